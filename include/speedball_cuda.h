@@ -570,12 +570,11 @@ typedef struct sb_tuning {
     uint32_t smemTlasNodes;   /* TLAS nodes staged in shared memory (0 = none)     */
     uint32_t bvhKind;         /* scene BVH over (triangle, instance) items, rebuilt
                                  on structural changes: 1 = 8-wide nodes with 8-bit
-                                 boxes for closest hits + binary for any hits
-                                 (default); 2 = binary only.
+                                 boxes (default; the binary tree beside it serves the
+                                 emitters' visibility); 2 = binary only.
                                  0 = the reference's TLAS + BLASes                */
-    uint32_t smemWideNodes;   /* bvhKind 1: the first (top-level) 8-wide nodes staged
-                                 in shared memory per CTA of the closest-hit stage,
-                                 80 bytes each (0 = none, at most 512)             */
+    uint32_t smemWideNodes;   /* at most 512; kept and returned, without effect: the
+                                 8-wide walk stages no nodes                       */
 } sb_tuning;
 sb_status sb_get_tuning(const sb_ctx* ctx, sb_tuning* out);
 /* The ray/triangle test this library was built with: 0 = the reference's
@@ -587,8 +586,7 @@ sb_status sb_get_tuning(const sb_ctx* ctx, sb_tuning* out);
 uint32_t sb_triangle_test(void);
 sb_status sb_set_tuning(sb_ctx* ctx, const sb_tuning* t);
 /* Time full solves of `cascade` under candidate tunings (bvhKind 1 / 2 / 0,
- * traceBlock 128 / 192 / 256, sortKey 0-3, for bvhKind 1 smemWideNodes
- * 0 / 73 / 512, and for bvhKind 0 TLAS staging
+ * traceBlock 128 / 192 / 256, sortKey 0-3, and for bvhKind 0 TLAS staging
  * off / 512 nodes), keep the fastest on the context and return it. The
  * cascade's histories and atlases are restored afterwards. Synchronizes. */
 sb_status sb_autotune(sb_ctx* ctx, uint32_t cascade, sb_tuning* chosen);

@@ -971,8 +971,8 @@ sb_status sb_solve(sb_ctx* ctx, uint32_t ci, uint32_t probeOffset, uint32_t upda
     const uint32_t chunk = (uint32_t)(ctx->jobCap / perProbe);
     const bool fullSolve = probeOffset == 0 && updatedCount == K.probeTotal && updatedCount <= chunk;
     if (ctx->tune.sortKey >= 2 && fullSolve) D.issueOrder = K.tileOrder;  // every probe in one chunk: tile by tile
-    // (the refill form on the 8-wide tree has no fixed batches to order)
-    const bool costOrder = ctx->tune.sortKey == 3 && fullSolve && !(SB_PRIMARY_REFILL && S.wideNodes);
+    // (the walk of the 8-wide tree has no fixed batches to order)
+    const bool costOrder = ctx->tune.sortKey == 3 && fullSolve && !S.wideNodes;
     if (costOrder) {  // this solve records its batch costs and orders the next one by them
         D.batchCost = K.batchCost;
         D.batchOrder = K.batchOrderReady ? K.batchOrder : nullptr;
@@ -1041,6 +1041,8 @@ static sb_status build_batch(const sb_solve_item* items, uint32_t count, BatchAr
         const uint32_t cnt = items[i].updatedCount > K.probeTotal ? K.probeTotal : items[i].updatedCount;
         BatchItem& I = B.it[i];
         I.W.S = dev_scene(c);
+        B.wideDepth = std::max(B.wideDepth, I.W.S.wideDepth);
+        if (I.W.S.wideNodes && I.W.S.dynCount) B.moved = 1u;
         I.W.C = dev_cascade(c, ci, items[i].probeOffset % K.probeTotal, cnt);
         std::memcpy(&I.W.P, &c->params, sizeof I.W.P);
         I.W.err = c->dErr;
@@ -1327,6 +1329,8 @@ static sb_status graph_launch(sb_ctx* lead) {
         cudaKernelNodeParams p = G.params[k];
         p.kernelParams = args;
         p.extra = nullptr;
+        // the walks' shared memory follows the trees' depth and the moved slots
+        if (k == 0 || k == 2) p.sharedMemBytes = trace_batch_smem(B, p.blockDim.x);
         CK(cudaGraphExecKernelNodeSetParams(G.exec, G.nodes[k], &p));
     }
     const std::vector<sb_ctx*> all = frame_contexts(G.lanes, G.items);
@@ -1462,9 +1466,8 @@ static sb_status time_min(sb_ctx* lead, const std::vector<sb_ctx*>& all, const s
 // Times full solves of cascade ci under each candidate tuning and keeps the
 // fastest. Candidates: the scene BVH kinds (8-wide / binary / the reference's
 // two-level walk), traversal block sizes 128 / 192 / 256, the four ray issue
-// orders (sortKey 0-3), for the 8-wide tree 0 / 73 / 512 top nodes staged in
-// shared memory, and for the two-level walk TLAS staging in shared memory off /
-// up to 512 nodes. The cascade's histories and atlases are restored afterwards, so
+// orders (sortKey 0-3), and for the two-level walk TLAS staging in shared memory
+// off / up to 512 nodes. The cascade's histories and atlases are restored afterwards, so
 // tuning leaves the probe state as it found it.
 sb_status sb_autotune(sb_ctx* ctx, uint32_t ci, sb_tuning* chosen) {
     if (!ctx) return SB_ERR_INVALID_ARG;
@@ -1480,14 +1483,12 @@ sb_status sb_autotune(sb_ctx* ctx, uint32_t ci, sb_tuning* chosen) {
     sb_tuning best = saved;
     float bestMs = 3.4e38f;
     const uint32_t kinds[3] = {1u, 2u, 0u}, blocks[3] = {128u, 192u, 256u};
-    const uint32_t wideDepth[3] = {0u, 73u, 512u};  // none, the top three levels, 512 nodes
-    // shared-memory staging: the TLAS for the two-level walk, the top 8-wide nodes for kind 1
+    // shared-memory staging: the TLAS for the two-level walk
     for (uint32_t kind : kinds)
         for (uint32_t block : blocks)
             for (uint32_t sort = 0; sort < 4 && s == SB_OK; ++sort)
-                for (uint32_t sm = 0; sm < (kind == 0 ? 2u : kind == 1 ? 3u : 1u) && s == SB_OK; ++sm) {
-                    sb_tuning t{block, sort, kind == 0 ? (sm ? 512u : 0u) : saved.smemTlasNodes, kind,
-                                kind == 1 ? wideDepth[sm] : 0u};
+                for (uint32_t sm = 0; sm < (kind == 0 ? 2u : 1u) && s == SB_OK; ++sm) {
+                    sb_tuning t{block, sort, kind == 0 ? (sm ? 512u : 0u) : saved.smemTlasNodes, kind, 0u};
                     if ((s = sb_set_tuning(ctx, &t)) != SB_OK) break;
                     float ms = 0.0f;
                     s = time_min(ctx, {ctx}, [&] { return sb_solve(ctx, ci, 0, probes); }, 3, ms);
@@ -1703,7 +1704,8 @@ sb_status sb_raycast(sb_ctx* ctx, const float* ro, const float* rd, uint32_t n, 
     CK(cudaMallocAsync(&dinst, (size_t)n * 4, ctx->stream));
     CK(cudaMemcpyAsync(dro, ro, (size_t)n * 12, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(drd, rd, (size_t)n * 12, cudaMemcpyHostToDevice, ctx->stream));
-    CK(launch_raycast(dev_scene(ctx), dro, drd, n, dt, dtri, dinst, ctx->dErr, ctx->stream));
+    CK(launch_raycast(dev_scene(ctx), dro, drd, n, dt, dtri, dinst, ctx->dWork + 8, ctx->numSms, ctx->dErr,
+                      ctx->stream));
     CK(cudaMemcpyAsync(tOut, dt, (size_t)n * 4, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaMemcpyAsync(triOut, dtri, (size_t)n * 4, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaMemcpyAsync(instOut, dinst, (size_t)n * 4, cudaMemcpyDeviceToHost, ctx->stream));
@@ -1730,7 +1732,8 @@ sb_status sb_raycast_device(sb_ctx* ctx, const float* ro, const float* rd, uint3
     if (n == 0) return ctx->sceneLoaded ? SB_OK : fail(ctx, SB_ERR_NOT_READY, "no scene uploaded");
     sb_status s = device_query_ready(ctx);
     if (s != SB_OK) return s;
-    CK(launch_raycast(dev_scene(ctx), ro, rd, n, tOut, triOut, instOut, ctx->dErr, ctx->stream));
+    CK(launch_raycast(dev_scene(ctx), ro, rd, n, tOut, triOut, instOut, ctx->dWork + 8, ctx->numSms, ctx->dErr,
+                      ctx->stream));
     return SB_OK;
 }
 
@@ -1740,7 +1743,8 @@ sb_status sb_occluded_device(sb_ctx* ctx, const float* ro, const float* rd, cons
     if (n == 0) return ctx->sceneLoaded ? SB_OK : fail(ctx, SB_ERR_NOT_READY, "no scene uploaded");
     sb_status s = device_query_ready(ctx);
     if (s != SB_OK) return s;
-    CK(launch_occluded(dev_scene(ctx), ro, rd, maxDist, n, blockedOut, ctx->dErr, ctx->stream));
+    CK(launch_occluded(dev_scene(ctx), ro, rd, maxDist, n, blockedOut, ctx->dWork + 8, ctx->numSms, ctx->dErr,
+                       ctx->stream));
     return SB_OK;
 }
 
@@ -1956,7 +1960,7 @@ sb_status sb_occluded(sb_ctx* ctx, const float* ro, const float* rd, const float
     CK(cudaMemcpyAsync(dro, ro, (size_t)n * 12, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(drd, rd, (size_t)n * 12, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(dm, maxDist, (size_t)n * 4, cudaMemcpyHostToDevice, ctx->stream));
-    CK(launch_occluded(dev_scene(ctx), dro, drd, dm, n, dout, ctx->dErr, ctx->stream));
+    CK(launch_occluded(dev_scene(ctx), dro, drd, dm, n, dout, ctx->dWork + 8, ctx->numSms, ctx->dErr, ctx->stream));
     CK(cudaMemcpyAsync(out, dout, (size_t)n, cudaMemcpyDeviceToHost, ctx->stream));
     cudaFreeAsync(dro, ctx->stream); cudaFreeAsync(drd, ctx->stream); cudaFreeAsync(dm, ctx->stream);
     cudaFreeAsync(dout, ctx->stream);

@@ -137,6 +137,22 @@ cudaError_t FlatScene::snapshot(const SceneBuffers& B, const uint32_t* order, ui
 
 namespace {
 
+// The nodes of sb_flat.h with the slots' meta bytes as one item mask and the scales
+// in bfloat16 (sb_walk8.cuh).
+void walk8_layout(std::vector<uint32_t>& nodes) {
+    for (size_t i = 0; i < nodes.size(); i += flat::WIDE_WORDS) {
+        uint32_t* w = nodes.data() + i;
+        const uint32_t imask = w[3] >> 24;
+        uint32_t items = 0;
+        for (uint32_t s = 0; s < 8; ++s)
+            if (!(imask >> s & 1u)) items |= (w[6 + s / 4] >> (8u * (s & 3u) + 5u) & 7u) << (3u * s);
+        // a scale 2^(e - 127) in bfloat16 is e << 7
+        w[7] = (w[3] >> 16 & 0xFFu) << 23;
+        w[3] = (w[3] & 0xFFu) << 7 | (w[3] >> 8 & 0xFFu) << 23;
+        w[6] = imask << 24 | items;
+    }
+}
+
 // One item per (triangle, active instance slot) with its world-space bounds
 // (the vertices under the inverse of the instance's inverse rows, in FP64,
 // widened), then the binned-SAH binary tree and the 8-wide tree beside it.
@@ -239,6 +255,7 @@ void compute(FlatScene::Job& j) {
         wideBuild = std::thread([&] { j.wideOk = flat::build_wide(boxes.data(), itTri.data(), itSlot.data(), n, j.wt); });
     j.treeOk = flat::build(boxes.data(), itTri.data(), itSlot.data(), n, j.tree);
     if (wideBuild.joinable()) wideBuild.join();
+    if (j.wideOk) walk8_layout(j.wt.nodes);
     if (!j.treeOk) j.why = "scene BVH: too many items";
 }
 

@@ -75,9 +75,9 @@ struct DevScene {
     // scene BVH (sb_flat.h): world-space tree over (triangle, slot) items;
     // slots marked in slotSkip moved or deformed since its build and are
     // walked through their own BLAS instead (dynList)
-    const uint4* flatNodes;    // binary child pairs (any hit; closest hit when wideNodes is null)
+    const uint4* flatNodes;    // binary child pairs (emitter visibility; every walk when wideNodes is null)
     const uint2* flatItems;
-    const uint4* wideNodes;    // the same items as 8-wide nodes with 8-bit boxes (closest hit), or null
+    const uint4* wideNodes;    // the same items as 8-wide nodes with 8-bit boxes (sb_walk8.cuh), or null
     const uint2* wideItems;
     const uint8_t* slotSkip;
     const uint32_t* dynList;
@@ -170,14 +170,13 @@ struct WaveCtx {
     DevParams P;
     uint32_t* err;
     unsigned long long* counters;  // [rays, shadowRays, tlasNodes, instances, blasNodes, triTests] or null
-    uint32_t* work;                // [0] primary cursor, [1] shadow cursor, [2] job count
+    uint32_t* work;                // [0] primary cursor, [1] shadow cursor, [2] job count, [3] batch-order
+                                   // claim, [4], [5] the moved slots' ray and job cursors
     float4* jobs;                  // 2 float4 per job: (origin, maxDist), (dir, ray << 6 | light)
     uint32_t jobCap;
     uint32_t slotBegin, slotCount; // probe slots of this chunk
     uint32_t smemTlas;             // TLAS nodes staged in shared memory (0 = read from global)
     uint32_t order;                // 0 probe-major, 1 direction-major
-    uint32_t smemWide;             // top 8-wide nodes staged in shared memory by the closest-hit stage
-    uint32_t sstk;                 // closest-hit walk stack entries per thread in shared memory (0: local)
 };
 
 // Several solves (scenes, cascades) through one launch of each stage: a
@@ -197,6 +196,8 @@ struct BatchArgs {
     uint32_t n;
     uint32_t totalRays;            // padded ray index space
     uint32_t blendBlocks;
+    uint32_t wideDepth;            // the deepest 8-wide tree among the items
+    uint32_t moved;                // some item has moved slots
     uint32_t* work;
     unsigned long long* counters;  // one set for the whole batch, or null
 };

@@ -8,20 +8,13 @@ namespace sb {
 void note_launch();
 uint64_t launches();
 
-// The closest-hit stage on the 8-wide tree hands each lane a new ray as soon
-// as its walk ends (per-lane refill) instead of running fixed 32-ray batches
-// per warp; 0 keeps the batches (and with them the costliest-first order).
-#ifndef SB_PRIMARY_REFILL
-#define SB_PRIMARY_REFILL 1
-#endif
-
 struct TraceTuning {
     uint32_t block;          // threads per block of the trace kernel
     uint32_t smemTlasNodes;  // stage the TLAS in shared memory when it has at most this many nodes
     uint32_t sortKey;        // ray issue order: 0 direction-major, 1 probe-major, 2 direction-major over probe
                              // tiles, 3 as 2 with closest-hit batches costliest first (last full solve's cycles)
     int numSms;
-    uint32_t smemWideNodes;  // top 8-wide scene-BVH nodes staged in shared memory per closest-hit CTA
+    uint32_t smemWideNodes;  // accepted and returned; the 8-wide walk stages no nodes
 };
 
 // Scene buffers in the reference layouts plus the derived layouts.
@@ -74,6 +67,8 @@ uint32_t blend_blocks(uint32_t updatedCount);  // CTAs of the blend for one solv
 // The batched kernels (stage 0 primary, 1 emit, 2 shadow, 3 shade; blend):
 // a captured graph refreshes their BatchArgs parameter on every replay.
 const void* trace_batch_kernel(int stage);
+// Dynamic shared memory of the batched walks (stages 0 and 2).
+uint32_t trace_batch_smem(const BatchArgs& B, uint32_t threads);
 const void* blend_batch_kernel();
 
 // Adjoint of shade + blend + upload (sb_adjoint.cu), over every probe of a
@@ -195,10 +190,12 @@ cudaError_t launch_emitter_vis(const DevScene& S, const DevCascade& C, const Dev
 // The FP32 probe rays of a solve as the trace forms them (sb_probe_rays).
 cudaError_t launch_probe_rays(const DevCascade& C, float jitter, float* ro, float* rd, cudaStream_t st);
 
-// Arbitrary-ray queries through the same traversal (raycastFirst-like).
+// Arbitrary-ray queries through the same traversal (raycastFirst-like); `cursor`: one word of
+// scratch for the stream's next query.
 cudaError_t launch_raycast(const DevScene& S, const float* ro, const float* rd, uint32_t n, float* tOut,
-                           int32_t* triOut, int32_t* instOut, uint32_t* err, cudaStream_t st);
+                           int32_t* triOut, int32_t* instOut, uint32_t* cursor, int numSms, uint32_t* err,
+                           cudaStream_t st);
 cudaError_t launch_occluded(const DevScene& S, const float* ro, const float* rd, const float* maxDist, uint32_t n,
-                            uint8_t* out, uint32_t* err, cudaStream_t st);
+                            uint8_t* out, uint32_t* cursor, int numSms, uint32_t* err, cudaStream_t st);
 
 }  // namespace sb

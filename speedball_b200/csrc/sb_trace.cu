@@ -13,9 +13,12 @@
 //                       the reference's summation order) + one-bounce atlas
 //                       read, or the SH-9 sky on a miss -> rayData.
 //
-// A and B are persistent and work-stealing (warps pull 32 items per atomic).
-// A issues rays direction-major: a warp holds ray k of 32 neighbouring probes,
-// i.e. 32 parallel rays, which keeps the BVH walks of a warp together.
+// A and B are persistent and work-stealing. On the 8-wide tree (*_walk8, *_batch) a
+// lane whose ray has ended takes the next one (sb_walk8.cuh, sb_walk2.cuh); on the
+// other layouts warps pull 32 items per atomic. A issues rays direction-major: a
+// warp holds ray k of 32 neighbouring probes, i.e. 32 parallel rays, which keeps
+// the BVH walks of a warp together.
+#include "sb_walk2.cuh"
 #include "sb_wave.cuh"
 
 namespace sb {
@@ -28,12 +31,14 @@ namespace sb {
 #ifndef SB_SHADOW_MIN_BLOCKS
 #define SB_SHADOW_MIN_BLOCKS 4
 #endif
-// Group-stack entries per thread held in shared memory by the closest-hit
-// stage's 8-wide walk (8 bytes each, one [entry][thread] array per CTA) when
-// the tree's depth fits; 0, or a deeper tree: the stack in local memory.
-#ifndef SB_SMEM_STACK
-#define SB_SMEM_STACK 16
+// The same for the walks of the 8-wide tree: 80 registers. Four blocks (64 registers,
+// less L1 beside the shared memory) measured 67 against 61 us on the room's primary
+// rays and 108 against 102 us on the atrium's, but 540 against 554 us for the plain
+// queries, whose rays come from arrays.
+#ifndef SB_WALK8_MIN_BLOCKS
+#define SB_WALK8_MIN_BLOCKS 3
 #endif
+constexpr int QUERY_MIN_BLOCKS = 4;
 
 // ---------------------------------------------------------------- bodies
 // Each stage's per-item work is a device function over `const WaveCtx&`; the
@@ -49,18 +54,15 @@ __device__ __forceinline__ void add_visits(unsigned long long* c, int at, uint32
     atomicAdd(&c[at + 3], (unsigned long long)v.tri);
 }
 
-// The raw record of a closest hit (FP32 t, no facing bit): k_emit finishes it.
-__device__ __forceinline__ void write_hit(const DevCascade& C, uint32_t slot, uint32_t k, int tri, int inst, float t,
-                                          float bu, float bv) {
-    const uint32_t uq = (uint32_t)__float2uint_rn(clampf(bu, 0.f, 1.f) * 65535.0f);
-    const uint32_t vq = (uint32_t)__float2uint_rn(clampf(bv, 0.f, 1.f) * 65535.0f);
-    C.hits[slot * C.rays + k] = tri >= 0 ? make_uint4((uint32_t)tri, (uint32_t)inst, __float_as_uint(t), uq | (vq << 16))
-                                         : make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, __float_as_uint(-1.0f), 0u);
+// The raw record of ray rayIdx's closest hit (FP32 t, no facing bit): k_emit finishes it.
+__device__ __forceinline__ void write_hit(const DevCascade& C, uint32_t rayIdx, int tri, int inst, float t,
+                                          uint32_t uv) {
+    C.hits[rayIdx] = tri >= 0 ? make_uint4((uint32_t)tri, (uint32_t)inst, __float_as_uint(t), uv)
+                              : make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, __float_as_uint(-1.0f), 0u);
 }
 
 // Stage A: the closest hit of one probe ray (item-local issue index g).
-__device__ __forceinline__ void primary_ray(const WaveCtx& W, const uint4* tl, bool pairs, uint32_t g, Visits& vis,
-                                            const uint4* sWide = nullptr, uint32_t nWide = 0) {
+__device__ __forceinline__ void primary_ray(const WaveCtx& W, const uint4* tl, bool pairs, uint32_t g, Visits& vis) {
     const DevCascade& C = W.C;
     uint32_t slot, k;
     ray_of(W, g, W.order != 0, slot, k);
@@ -69,62 +71,181 @@ __device__ __forceinline__ void primary_ray(const WaveCtx& W, const uint4* tl, b
     const float3 rd = ray_dir(k, C.rays, W.P.frameJitter);
     float bestT, bu, bv;
     int tri, inst;
-    trace_closest(W.S, tl, ro, rd, bestT, tri, inst, bu, bv, vis, W.err, pairs, sWide, nWide);
-    write_hit(C, slot, k, tri, inst, bestT, bu, bv);
+    trace_closest(W.S, tl, ro, rd, bestT, tri, inst, bu, bv, vis, W.err, pairs);
+    write_hit(C, slot * C.rays + k, tri, inst, bestT, pack_uv(bu, bv));
 }
 
-// Stage A on the 8-wide tree with per-lane refill, for a whole persistent warp
-// (all 32 lanes call it): each lane walks its own ray in rounds (wide_step),
-// and a lane whose walk has ended takes the next ray of the issue order before
-// the next round, so the lanes keep working instead of waiting for the slowest
-// ray of a fixed 32-ray batch. One atomicAdd per round fetches rays for all
-// the warp's idle lanes. Returns the rays traced.
+// The CTA's shared memory: the tables (filled here), then each warp's, used by the
+// moved slots' walk first and by the 8-wide one after it.
+struct WalkSmem {
+    Walk8Tables* tables;
+    Walk2Shared* w2;
+    Walk8Shared* w8;
+    uint2* stk;
+};
+__host__ __device__ __forceinline__ uint32_t walk_stride(uint32_t depth, bool moved) {
+    const uint32_t w8 = (uint32_t)(sizeof(Walk8Shared) + depth * 32u * sizeof(uint2));
+    return moved && sizeof(Walk2Shared) > w8 ? (uint32_t)sizeof(Walk2Shared) : w8;
+}
+static uint32_t walk_smem(uint32_t depth, bool moved, uint32_t threads) {
+    return (uint32_t)sizeof(Walk8Tables) + threads / 32u * walk_stride(depth, moved);
+}
+__device__ __forceinline__ WalkSmem walk_shared(void* smem, uint32_t depth, bool moved) {
+    WalkSmem m;
+    m.tables = reinterpret_cast<Walk8Tables*>(smem);
+    walk8_tables(*m.tables);
+    char* p = reinterpret_cast<char*>(smem) + sizeof(Walk8Tables) + (threadIdx.x / 32u) * walk_stride(depth, moved);
+    m.w2 = reinterpret_cast<Walk2Shared*>(p);
+    m.w8 = reinterpret_cast<Walk8Shared*>(p);
+    m.stk = reinterpret_cast<uint2*>(p + sizeof(Walk8Shared));
+    return m;
+}
+
+// A walk's next items for the lanes in `want`: positions of the shared cursor.
+__device__ __forceinline__ uint32_t take(uint32_t* cursor, uint32_t want) {
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t base = 0;
+    if (lane == 0) base = atomicAdd(cursor, (uint32_t)__popc(want));
+    return __shfl_sync(ALL_LANES, base, 0) + (uint32_t)__popc(want & ((1u << lane) - 1u));
+}
+
+// Stage A on the 8-wide tree. next(want, g) gives the lanes in `want` their
+// item-local issue positions (ok: this lane has one) and returns false when none
+// are left; dir(k) is ray direction k.
 //
-// sStack: this thread's column of the walk stack in shared memory (W.sstk
-// entries), or null for the stack in local memory.
-__device__ __forceinline__ uint32_t primary_refill(const WaveCtx& W, uint32_t total, Visits& vis, const uint4* sWide,
-                                                   uint32_t nWide, uint2* sStack = nullptr) {
+// The moved slots' hits go to the ray records (free until the shading), the tree's
+// to the hit records; emission takes the nearer one.
+template <class Next, class Dir>
+__device__ __forceinline__ void primary_moved(const WaveCtx& W, Walk2Shared& sm, Next next, Dir dir, Visits& vis) {
     const DevCascade& C = W.C;
     const uint32_t lane = threadIdx.x & 31u;
-    WideWalk w;
-    uint32_t slot = 0, k = 0, nRays = 0;
-    float bestT = T_MAX, bu = 0.0f, bv = 0.0f;
-    int tri = -1, inst = -1;
-    bool has = false, more = true;
-    for (;;) {
-        if (more) {
-            const uint32_t need = __ballot_sync(0xFFFFFFFFu, !has);
-            if (need) {
-                uint32_t base = 0;
-                if (lane == 0) base = atomicAdd(&W.work[0], (uint32_t)__popc(need));
-                base = __shfl_sync(0xFFFFFFFFu, base, 0);
-                if (base >= total) more = false;
-                const uint32_t g = base + (uint32_t)__popc(need & ((1u << lane) - 1u));
-                if (!has && g < total) {
-                    ray_of(W, g, W.order != 0, slot, k);
-                    const float3 ro = probe_world_pos(C, (C.probeOffset + slot) % C.probeTotal);
-                    const float3 rd = ray_dir(k, C.rays, W.P.frameJitter);
-                    bestT = T_MAX;
-                    tri = inst = -1;
-                    bu = bv = 0.0f;
-                    wide_begin<false>(W.S, w, ro, rd, bestT, tri, inst, bu, bv, vis, W.err);
-                    has = true;
-                }
-            }
-        }
-        if (!__any_sync(0xFFFFFFFFu, has)) {
-            if (!more) break;
-            continue;
-        }
-        if (has && wide_step<false>(W.S, w, bestT, tri, inst, bu, bv, vis, W.err, sWide, nWide, sStack,
-                                    (int)W.sstk)) {
-            wide_end<false>(W.S, w, bestT, tri, inst, bu, bv, vis, W.err);
-            write_hit(C, slot, k, tri, inst, bestT, bu, bv);
-            ++nRays;
-            has = false;
-        }
+    uint4* out = reinterpret_cast<uint4*>(C.rayData);
+    auto gen = [&](bool& more, uint32_t want, float3& o, float3& d, float& tmax, uint32_t& tag) {
+        uint32_t g;
+        bool ok;
+        more = next(want, g, ok);
+        if (!ok || !(want >> lane & 1u)) return false;
+        uint32_t slot, k;
+        ray_of(W, g, W.order != 0, slot, k);
+        o = probe_world_pos(C, (C.probeOffset + slot) % C.probeTotal);
+        d = dir(k);
+        tmax = T_MAX;
+        tag = slot * C.rays + k;
+        return true;
+    };
+    if (walk2_usable(W.S)) {
+        walk2<false>(W.S, sm, gen, [&](uint32_t tag, float t, uint4 hit, bool) {
+            out[tag] = make_uint4(hit.x, hit.y, __float_as_uint(t), hit.z);
+        }, vis, W.err);
+        return;
     }
+    for (bool more = true; more;) {  // a BLAS too deep for it: one ray per lane
+        float3 o, d;
+        float t, bu = 0.0f, bv = 0.0f;
+        uint32_t tag;
+        if (!gen(more, ALL_LANES, o, d, t, tag)) continue;
+        int tri = -1, inst = -1;
+        dyn_walk<false>(W.S, o, d, mk(1.0f / d.x, 1.0f / d.y, 1.0f / d.z), t, tri, inst, bu, bv, vis, W.err);
+        out[tag] = make_uint4((uint32_t)tri, (uint32_t)inst, __float_as_uint(t), pack_uv(bu, bv));
+    }
+}
+
+template <class Next, class Dir>
+__device__ __forceinline__ uint32_t primary_walk8(const WaveCtx& W, const WalkSmem& m, Next next, Dir dir,
+                                                  Visits& vis) {
+    const DevCascade& C = W.C;
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t nRays = 0;
+    auto gen = [&](bool& more, uint32_t want, float3& o, float3& d, float3& winv, float& tmax, uint32_t& tag,
+                   uint4& hit) {
+        uint32_t g;
+        bool ok;
+        more = next(want, g, ok);
+        if (!ok || !(want >> lane & 1u)) return false;
+        uint32_t slot, k;
+        ray_of(W, g, W.order != 0, slot, k);
+        o = probe_world_pos(C, (C.probeOffset + slot) % C.probeTotal);
+        d = dir(k);
+        winv = mk(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
+        tag = slot * C.rays + k;
+        tmax = T_MAX;
+        hit = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u);
+        ++nRays;
+        return true;
+    };
+    auto fin = [&](uint32_t tag, float t, uint4 hit, bool) { write_hit(C, tag, (int)hit.x, (int)hit.y, t, hit.z); };
+    walk8<false>(W.S, *m.tables, *m.w8, m.stk, W.S.wideDepth + 1u, gen, fin, vis, W.err);
     return nRays;
+}
+
+// A blocked light leaves its ray's mask (rayBase: the first ray index of the item).
+__device__ __forceinline__ void clear_light(const WaveCtx& W, uint32_t tag, uint32_t rayBase) {
+    const uint32_t li = tag & 63u;
+    uint4* v = W.C.vis + ((tag >> 6) - rayBase);
+    if (li < 32) atomicAnd(&v->z, ~(1u << li));
+    else atomicAnd(&v->w, ~(1u << (li - 32)));
+}
+
+// Stage B on the 8-wide tree, next(want, j) as for stage A, with jobs. A job that
+// the moved slots block loses its length: the tree's walk skips it when it comes to
+// it later (it may not see that yet, and then clears the same light again).
+template <class Next>
+__device__ __forceinline__ void shadow_moved(const WaveCtx& W, Walk2Shared& sm, uint32_t rayBase, Next next,
+                                             Visits& vis) {
+    const uint32_t lane = threadIdx.x & 31u;
+    auto gen = [&](bool& more, uint32_t want, float3& o, float3& d, float& tmax, uint32_t& tag) {
+        uint32_t j;
+        bool ok;
+        more = next(want, j, ok);
+        if (!ok || !(want >> lane & 1u)) return false;
+        const float4 a = W.jobs[2 * j], b = W.jobs[2 * j + 1];
+        o = xyz(a);
+        d = xyz(b);
+        tmax = a.w;
+        tag = j;
+        return true;
+    };
+    auto fin = [&](uint32_t j, float, uint4, bool blocked) {
+        if (!blocked) return;
+        clear_light(W, __float_as_uint(W.jobs[2 * j + 1].w), rayBase);
+        W.jobs[2 * j].w = 0.0f;
+    };
+    if (walk2_usable(W.S)) {
+        walk2<true>(W.S, sm, gen, fin, vis, W.err);
+        return;
+    }
+    for (bool more = true; more;) {
+        float3 o, d;
+        float t, u = 0.0f, v = 0.0f;
+        uint32_t tag;
+        if (!gen(more, ALL_LANES, o, d, t, tag)) continue;
+        int tri = -1, inst = -1;
+        if (dyn_walk<true>(W.S, o, d, mk(1.0f / d.x, 1.0f / d.y, 1.0f / d.z), t, tri, inst, u, v, vis, W.err))
+            fin(tag, t, make_uint4(0u, 0u, 0u, 0u), true);
+    }
+}
+
+template <class Next>
+__device__ __forceinline__ void shadow_walk8(const WaveCtx& W, const WalkSmem& m, uint32_t rayBase, Next next,
+                                             Visits& vis) {
+    const uint32_t lane = threadIdx.x & 31u;
+    auto gen = [&](bool& more, uint32_t want, float3& o, float3& d, float3& winv, float& tmax, uint32_t& tag, uint4&) {
+        uint32_t j;
+        bool ok;
+        more = next(want, j, ok);
+        if (!ok || !(want >> lane & 1u)) return false;
+        const float4 a = W.jobs[2 * j], b = W.jobs[2 * j + 1];
+        o = xyz(a);
+        d = xyz(b);
+        winv = mk(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
+        tmax = a.w;
+        tag = __float_as_uint(b.w);
+        return tmax > RAY_EPS;  // no hit lies nearer than that
+    };
+    auto fin = [&](uint32_t tag, float, uint4, bool blocked) {
+        if (blocked) clear_light(W, tag, rayBase);
+    };
+    walk8<true>(W.S, *m.tables, *m.w8, m.stk, W.S.wideDepth + 1u, gen, fin, vis, W.err);
 }
 
 // Stage A2, warp-collective (all 32 lanes call it; `active` lanes hold ray g):
@@ -151,6 +272,10 @@ __device__ __forceinline__ uint32_t emit_ray(const WaveCtx& W, bool active, uint
         ray_of(W, g, W.order != 0, slot, k);
         rayIdx = slot * N + k;
         h = C.hits[rayIdx];
+        if (W.S.wideNodes && W.S.dynCount) {  // the moved slots' hit, when it is no farther
+            const uint4 d = reinterpret_cast<const uint4*>(C.rayData)[rayIdx];
+            if (d.x != 0xFFFFFFFFu && (h.x == 0xFFFFFFFFu || __uint_as_float(d.z) <= __uint_as_float(h.z))) h = d;
+        }
         if (h.x != 0xFFFFFFFFu) {
             tri = (int)h.x;
             const uint32_t inst = h.y;
@@ -209,13 +334,8 @@ __device__ __forceinline__ uint32_t emit_ray(const WaveCtx& W, bool active, uint
 
 // Stage B: one shadow job; a blocked light is cleared from the ray's mask.
 __device__ __forceinline__ void shadow_job(const WaveCtx& W, const uint4* tl, bool pairs, float4 a, float4 b,
-                                           uint32_t rayIdx, Visits& vis) {
-    if (trace_any(W.S, tl, xyz(a), xyz(b), a.w, vis, W.err, pairs)) {
-        const uint32_t li = __float_as_uint(b.w) & 63u;
-        uint4* v = W.C.vis + rayIdx;
-        if (li < 32) atomicAnd(&v->z, ~(1u << li));
-        else atomicAnd(&v->w, ~(1u << (li - 32)));
-    }
+                                           uint32_t rayBase, Visits& vis) {
+    if (trace_any(W.S, tl, xyz(a), xyz(b), a.w, vis, W.err, pairs)) clear_light(W, __float_as_uint(b.w), rayBase);
 }
 
 // Stage C: emissive + unblocked NEE terms + bounce, or the sky, of one ray
@@ -273,29 +393,60 @@ __device__ __forceinline__ void shade_ray(const WaveCtx& W, uint32_t g) {
 
 // ---------------------------------------------------------------- per solve
 
+// The 8-wide tree (bvhKind 1). Each CTA forms the solve's N ray directions once.
+__global__ void __launch_bounds__(256, SB_WALK8_MIN_BLOCKS) k_trace_primary_walk8(WaveCtx W) {
+    extern __shared__ float4 smem[];
+    if (!*W.S.valid) return;
+    const uint32_t N = W.C.rays, total = W.slotCount * N;
+    for (uint32_t k = threadIdx.x; k < N; k += blockDim.x) {
+        const float3 d = ray_dir(k, N, W.P.frameJitter);
+        smem[k] = make_float4(d.x, d.y, d.z, 0.0f);
+    }
+    const WalkSmem m = walk_shared(smem + N, W.S.wideDepth + 1u, W.S.dynCount != 0u);  // (synchronizes)
+    Visits vis = {0, 0, 0, 0};
+    auto from = [&](uint32_t* cursor) {
+        return [cursor, total](uint32_t want, uint32_t& g, bool& ok) {
+            g = take(cursor, want);
+            ok = g < total;
+            return __any_sync(ALL_LANES, ok && (want >> (threadIdx.x & 31u) & 1u)) != 0;
+        };
+    };
+    auto dir = [&](uint32_t k) { return xyz(smem[k]); };
+    if (W.S.dynCount) primary_moved(W, *m.w2, from(&W.work[4]), dir, vis);
+    __syncwarp();
+    const uint32_t nRays = primary_walk8(W, m, from(&W.work[0]), dir, vis);
+    add_visits(W.counters, 2, nRays, vis);
+}
+
+__global__ void __launch_bounds__(256, SB_WALK8_MIN_BLOCKS) k_trace_shadow_walk8(WaveCtx W) {
+    extern __shared__ float4 smem[];
+    if (!*W.S.valid) return;
+    const uint32_t total = min(*(volatile uint32_t*)&W.work[2], W.jobCap);
+    const WalkSmem m = walk_shared(smem, W.S.wideDepth + 1u, W.S.dynCount != 0u);
+    Visits vis = {0, 0, 0, 0};
+    auto from = [&](uint32_t* cursor) {
+        return [cursor, total](uint32_t want, uint32_t& j, bool& ok) {
+            j = take(cursor, want);
+            ok = j < total;
+            return __any_sync(ALL_LANES, ok && (want >> (threadIdx.x & 31u) & 1u)) != 0;
+        };
+    };
+    if (W.S.dynCount) shadow_moved(W, *m.w2, 0u, from(&W.work[5]), vis);
+    __syncwarp();
+    shadow_walk8(W, m, 0u, from(&W.work[1]), vis);
+    add_visits(W.counters, 6, 0u, vis);
+}
+
+// The binary scene BVH and the two-level walk (bvhKind 2 and 0).
 __global__ void __launch_bounds__(256, SB_PRIMARY_MIN_BLOCKS) k_trace_primary(WaveCtx W) {
     extern __shared__ uint4 sTlas[];
     const bool pairs = closest_pairs(W.S);
     const uint4* tl = stage_tlas(W, sTlas, pairs);
-    // the scene BVH's top 8-wide nodes (the TLAS is not read on that walk:
-    // the buffer is free), staged once per CTA
-    const uint32_t nWide = W.S.wideNodes ? W.smemWide : 0u;
-    if (nWide) {
-        for (uint32_t i = threadIdx.x; i < 5u * nWide; i += blockDim.x) sTlas[i] = __ldg(W.S.wideNodes + i);
-        __syncthreads();
-    }
     if (!*W.S.valid) return;
     const uint32_t total = W.slotCount * W.C.rays;
     const uint32_t lane = threadIdx.x & 31u;
     Visits vis = {0, 0, 0, 0};
     uint32_t nRays = 0;
-    if (SB_PRIMARY_REFILL && W.S.wideNodes) {
-        // the walk stack after the staged nodes, one column per thread
-        uint2* sStack = W.sstk ? reinterpret_cast<uint2*>(sTlas + 5u * nWide) + threadIdx.x : nullptr;
-        nRays = primary_refill(W, total, vis, sTlas, nWide, sStack);
-        add_visits(W.counters, 2, nRays, vis);
-        return;
-    }
     for (;;) {
         uint32_t base = 0;
         if (lane == 0) base = atomicAdd(&W.work[0], 32u);
@@ -308,7 +459,7 @@ __global__ void __launch_bounds__(256, SB_PRIMARY_MIN_BLOCKS) k_trace_primary(Wa
         const uint32_t g = batch * 32u + lane;
         const long long t0 = W.C.batchCost ? clock64() : 0;
         if (g < total) {
-            primary_ray(W, tl, pairs, g, vis, sTlas, nWide);
+            primary_ray(W, tl, pairs, g, vis);
             ++nRays;
         }
         if (W.C.batchCost) {
@@ -383,7 +534,7 @@ __global__ void __launch_bounds__(256, SB_SHADOW_MIN_BLOCKS) k_trace_shadow(Wave
         uint32_t j = base + lane;
         if (j >= total) continue;
         const float4 a = W.jobs[2 * j], b = W.jobs[2 * j + 1];
-        shadow_job(W, tl, pairs, a, b, __float_as_uint(b.w) >> 6, vis);
+        shadow_job(W, tl, pairs, a, b, 0u, vis);
     }
     add_visits(W.counters, 6, 0u, vis);
     if (W.C.batchOrderOut) {
@@ -432,6 +583,11 @@ static int persistent_grid(const void* kernel, int block, size_t smem, const Tra
     return grid < 1 ? 1 : grid;
 }
 
+static int walk8_grid(const void* kernel, int block, size_t smem, const TraceTuning& tune, uint32_t items) {
+    if (smem > 48u * 1024u) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return persistent_grid(kernel, block, smem, tune, items);
+}
+
 cudaError_t launch_trace(const DevScene& S, const DevCascade& C, const DevParams& P, uint32_t* err,
                          unsigned long long* counters, uint32_t* work, const TraceTuning& tune, cudaStream_t st,
                          float4* jobs, uint32_t jobCap, uint32_t slotBegin, uint32_t slotCount,
@@ -452,34 +608,34 @@ cudaError_t launch_trace(const DevScene& S, const DevCascade& C, const DevParams
     // the scene-BVH walk reads no TLAS
     uint32_t smemNodes = !S.flatOn && S.tlasNodeCount <= tune.smemTlasNodes ? S.tlasNodeCount : 0u;
     W.smemTlas = smemNodes;
-    // the 8-wide walk's top nodes, staged by the closest-hit stage only
-    uint32_t wideNodes = S.wideNodes ? (tune.smemWideNodes < S.wideNodeCount ? tune.smemWideNodes : S.wideNodeCount) : 0u;
-    if (wideNodes > 512u) wideNodes = 512u;
-    W.smemWide = wideNodes;
-    size_t smem = (size_t)smemNodes * 64u;  // room for the child-pair TLAS (the 32-byte nodes need half)
-    size_t smemPrimary = smem > (size_t)wideNodes * 80u ? smem : (size_t)wideNodes * 80u;
-    // the walk stack in shared memory when the 8-wide tree's depth fits it (the
-    // stack holds at most one group per level below the root)
-    W.sstk = (SB_PRIMARY_REFILL && S.wideNodes && S.wideDepth + 1u <= (uint32_t)SB_SMEM_STACK) ? SB_SMEM_STACK : 0u;
-    smemPrimary += (size_t)W.sstk * (size_t)tune.block * 8u;
-    if (smemPrimary > 48u * 1024u)
-        cudaFuncSetAttribute(k_trace_primary, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smemPrimary);
-    if (smem > 48u * 1024u)
+    const size_t smem = (size_t)smemNodes * 64u;  // room for the child-pair TLAS (the 32-byte nodes need half)
+    if (smem > 48u * 1024u) {
+        cudaFuncSetAttribute(k_trace_primary, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         cudaFuncSetAttribute(k_trace_shadow, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    // ray, job-read and job-write cursors, and the batch-order claim
-    cudaError_t e = cudaMemsetAsync(work, 0, 4 * sizeof(uint32_t), st);
+    }
+    // ray, job-read and job-write cursors, the batch-order claim, the moved slots' cursors
+    cudaError_t e = cudaMemsetAsync(work, 0, 6 * sizeof(uint32_t), st);
     if (e != cudaSuccess) return e;
     const uint32_t rays = slotCount * C.rays;
-    int block = (int)tune.block;
-    k_trace_primary<<<persistent_grid((const void*)k_trace_primary, block, smemPrimary, tune, rays), block, smemPrimary,
-                      st>>>(W);
+    const int block = (int)tune.block;
+    const uint32_t smem8 = walk_smem(S.wideDepth + 1u, S.dynCount != 0u, tune.block);
+    const uint32_t smemP = smem8 + C.rays * (uint32_t)sizeof(float4);
+    if (S.wideNodes)
+        k_trace_primary_walk8<<<walk8_grid((const void*)k_trace_primary_walk8, block, smemP, tune, rays), block, smemP,
+                                st>>>(W);
+    else
+        k_trace_primary<<<persistent_grid((const void*)k_trace_primary, block, smem, tune, rays), block, smem, st>>>(W);
     note_launch();
     if (afterClosest) cudaEventRecord(afterClosest, st);
     k_emit<<<(rays + 127) / 128, 128, 0, st>>>(W);
     note_launch();
     if (afterPrimary) cudaEventRecord(afterPrimary, st);
     // shadow jobs: at most lightCount per ray (the queue is sized for it)
-    k_trace_shadow<<<persistent_grid((const void*)k_trace_shadow, block, smem, tune, rays * 4u), block, smem, st>>>(W);
+    if (S.wideNodes)
+        k_trace_shadow_walk8<<<walk8_grid((const void*)k_trace_shadow_walk8, block, smem8, tune, rays * 4u), block,
+                               smem8, st>>>(W);
+    else
+        k_trace_shadow<<<persistent_grid((const void*)k_trace_shadow, block, smem, tune, rays * 4u), block, smem, st>>>(W);
     note_launch();
     if (afterShadow) cudaEventRecord(afterShadow, st);
     k_shade<<<(rays + 127) / 128, 128, 0, st>>>(W);
@@ -491,102 +647,57 @@ cudaError_t launch_trace(const DevScene& S, const DevCascade& C, const DevParams
 // The same four stages over every item of a BatchArgs: one launch per stage
 // for all scenes and cascades, one shared ray index space and job queue.
 
-__global__ void __launch_bounds__(256, SB_PRIMARY_MIN_BLOCKS) k_trace_primary_batch(const __grid_constant__ BatchArgs B) {
+// Each warp takes 32-ray chunks and stays with one item while chunks of it follow
+// one another (the item index is warp-uniform, so the parameter-space reads of its
+// context stay uniform); items without an 8-wide tree run their chunks one ray per
+// lane (primary_ray). The moved slots of all items come first.
+__global__ void __launch_bounds__(256, SB_WALK8_MIN_BLOCKS) k_trace_primary_batch(const __grid_constant__ BatchArgs B) {
+    extern __shared__ float4 smem[];
     const uint32_t lane = threadIdx.x & 31u;
+    const WalkSmem m = walk_shared(smem, B.wideDepth + 1u, B.moved != 0u);
     Visits vis = {0, 0, 0, 0};
     uint32_t nRays = 0;
-    if (!SB_PRIMARY_REFILL) {
-        for (;;) {
+    for (int moved = B.moved ? 1 : 0; moved >= 0; --moved) {
+        uint32_t cur = 0, end = 0;  // the chunk in hand
+        auto chunk = [&]() {
+            if (cur < end) return true;
             uint32_t base = 0;
-            if (lane == 0) base = atomicAdd(&B.work[0], 32u);
-            base = __shfl_sync(0xFFFFFFFFu, base, 0);
-            if (base >= B.totalRays) break;
-            const BatchItem& I = B.it[batch_item(B, base)];
-            const uint32_t g = base + lane - I.rayBase;
-            if (g >= I.rays || !*I.W.S.valid) continue;
-            const bool pairs = closest_pairs(I.W.S);
-            primary_ray(I.W, pairs ? I.W.S.tlasPairs : I.W.S.tlas, pairs, g, vis);
-            ++nRays;
-        }
-        add_visits(B.counters, 2, nRays, vis);
-        return;
-    }
-    // Per-lane refill within one item at a time (the item index stays
-    // warp-uniform, so the parameter-space reads of its context stay uniform):
-    // the warp takes 32-ray chunks and hands their rays to idle lanes; a chunk
-    // of another item waits until every lane is idle. Items without an 8-wide
-    // tree run their chunks as 32-ray batches (primary_ray).
-    const uint32_t NONE = 0xFFFFFFFFu;
-    uint32_t item = NONE, cur = 0, curEnd = 0, pend = NONE;  // warp-uniform
-    bool more = true;
-    WideWalk w;
-    uint32_t slot = 0, k = 0;
-    float bestT = T_MAX, bu = 0.0f, bv = 0.0f;
-    int tri = -1, inst = -1;
-    bool has = false;
-    for (;;) {
-        const uint32_t need = __ballot_sync(0xFFFFFFFFu, !has);
-        if (cur == curEnd) {
-            if (pend == NONE && more) {
-                uint32_t base = 0;
-                if (lane == 0) base = atomicAdd(&B.work[0], 32u);
-                base = __shfl_sync(0xFFFFFFFFu, base, 0);
-                if (base >= B.totalRays) more = false;
-                else pend = base;
+            if (lane == 0) base = atomicAdd(&B.work[moved ? 4 : 0], 32u);
+            cur = __shfl_sync(ALL_LANES, base, 0);
+            end = min(cur + 32u, B.totalRays);
+            return cur < end;
+        };
+        while (chunk()) {
+            const BatchItem& I = B.it[batch_item(B, cur)];
+            const uint32_t stop = I.rayBase + I.rays;  // item ranges are 32-aligned
+            if (cur >= stop || !*I.W.S.valid || (moved && (!I.W.S.wideNodes || !I.W.S.dynCount))) {
+                cur = end;
+                continue;
             }
-            if (pend != NONE) {
-                const uint32_t pi = batch_item(B, pend);
-                if (pi == item || need == 0xFFFFFFFFu) {
-                    const BatchItem& P = B.it[pi];
-                    item = pi;
-                    cur = pend;
-                    curEnd = min(pend + 32u, P.rayBase + P.rays);  // item ranges are 32-aligned
-                    if (cur > curEnd || !*P.W.S.valid) cur = curEnd;
-                    pend = NONE;
-                }
-            }
-        }
-        if (cur < curEnd) {
-            const BatchItem& I = B.it[item];
             if (!I.W.S.wideNodes) {
-                if (need == 0xFFFFFFFFu) {  // a 32-ray batch, as without refill
-                    const uint32_t g = cur + lane - I.rayBase;
-                    if (cur + lane < curEnd) {
-                        const bool pairs = closest_pairs(I.W.S);
-                        primary_ray(I.W, pairs ? I.W.S.tlasPairs : I.W.S.tlas, pairs, g, vis);
-                        ++nRays;
-                    }
-                    cur = curEnd;
+                const uint32_t g = cur + lane;
+                if (g < min(end, stop)) {
+                    const bool pairs = closest_pairs(I.W.S);
+                    primary_ray(I.W, pairs ? I.W.S.tlasPairs : I.W.S.tlas, pairs, g - I.rayBase, vis);
+                    ++nRays;
                 }
-            } else if (need) {
-                const uint32_t rank = (uint32_t)__popc(need & ((1u << lane) - 1u));
-                const uint32_t n = min((uint32_t)__popc(need), curEnd - cur);
-                if (!has && rank < n) {
-                    ray_of(I.W, cur + rank - I.rayBase, I.W.order != 0, slot, k);
-                    const DevCascade& C = I.W.C;
-                    const float3 ro = probe_world_pos(C, (C.probeOffset + slot) % C.probeTotal);
-                    const float3 rd = ray_dir(k, C.rays, I.W.P.frameJitter);
-                    bestT = T_MAX;
-                    tri = inst = -1;
-                    bu = bv = 0.0f;
-                    wide_begin<false>(I.W.S, w, ro, rd, bestT, tri, inst, bu, bv, vis, I.W.err);
-                    has = true;
-                }
+                cur = end;
+                continue;
+            }
+            auto next = [&](uint32_t want, uint32_t& g, bool& ok) {
+                // the chunk's next rays; another item's chunk ends this walk
+                ok = false;
+                if (!chunk() || cur >= stop) return false;
+                const uint32_t n = min((uint32_t)__popc(want), end - cur), r = __popc(want & ((1u << lane) - 1u));
+                ok = r < n && cur + r < stop;
+                g = cur + r - I.rayBase;
                 cur += n;
-            }
-        }
-        if (!__any_sync(0xFFFFFFFFu, has)) {
-            if (!more && pend == NONE && cur == curEnd) break;
-            continue;
-        }
-        if (has) {
-            const BatchItem& I = B.it[item];
-            if (wide_step<false>(I.W.S, w, bestT, tri, inst, bu, bv, vis, I.W.err)) {
-                wide_end<false>(I.W.S, w, bestT, tri, inst, bu, bv, vis, I.W.err);
-                write_hit(I.W.C, slot, k, tri, inst, bestT, bu, bv);
-                ++nRays;
-                has = false;
-            }
+                return true;
+            };
+            auto dir = [&](uint32_t k) { return ray_dir(k, I.W.C.rays, I.W.P.frameJitter); };
+            if (moved) primary_moved(I.W, *m.w2, next, dir, vis);
+            else nRays += primary_walk8(I.W, m, next, dir, vis);
+            __syncwarp();
         }
     }
     add_visits(B.counters, 2, nRays, vis);
@@ -605,23 +716,58 @@ __global__ void __launch_bounds__(128) k_emit_batch(const __grid_constant__ Batc
     }
 }
 
-__global__ void __launch_bounds__(256, SB_SHADOW_MIN_BLOCKS) k_trace_shadow_batch(const __grid_constant__ BatchArgs B) {
+// As k_trace_primary_batch: a chunk of 32 jobs may hold several items' jobs, which
+// are walked one item after another.
+__global__ void __launch_bounds__(256, SB_WALK8_MIN_BLOCKS) k_trace_shadow_batch(const __grid_constant__ BatchArgs B) {
+    extern __shared__ float4 smem[];
     const BatchItem& I0 = B.it[0];
     const uint32_t total = min(*(volatile uint32_t*)&B.work[2], I0.W.jobCap);
     const uint32_t lane = threadIdx.x & 31u;
+    const WalkSmem m = walk_shared(smem, B.wideDepth + 1u, B.moved != 0u);
     Visits vis = {0, 0, 0, 0};
-    for (;;) {
-        uint32_t base = 0;
-        if (lane == 0) base = atomicAdd(&B.work[1], 32u);
-        base = __shfl_sync(0xFFFFFFFFu, base, 0);
-        if (base >= total) break;
-        uint32_t j = base + lane;
-        if (j >= total) continue;
-        const float4 a = I0.W.jobs[2 * j], b = I0.W.jobs[2 * j + 1];
-        const uint32_t ray = __float_as_uint(b.w) >> 6;
-        const BatchItem& I = B.it[batch_item(B, ray)];
-        const bool pairs = any_pairs(I.W.S);
-        shadow_job(I.W, pairs ? I.W.S.tlasPairs : I.W.S.tlas, pairs, a, b, ray - I.rayBase, vis);
+    for (int moved = B.moved ? 1 : 0; moved >= 0; --moved) {
+        uint32_t base = 0, left = 0;  // the chunk in hand and its jobs still to walk
+        uint32_t mine = 0;            // the item of this lane's job
+        auto chunk = [&]() {
+            if (left) return true;
+            if (lane == 0) base = atomicAdd(&B.work[moved ? 5 : 1], 32u);
+            base = __shfl_sync(ALL_LANES, base, 0);
+            const bool have = base < total && base + lane < total;
+            if (have) mine = batch_item(B, __float_as_uint(I0.W.jobs[2 * (base + lane) + 1].w) >> 6);
+            left = __ballot_sync(ALL_LANES, have);
+            return left != 0u;
+        };
+        while (chunk()) {
+            const uint32_t item = __shfl_sync(ALL_LANES, mine, __ffs(left) - 1);
+            const BatchItem& I = B.it[item];
+            if (!I.W.S.wideNodes || (moved && !I.W.S.dynCount)) {
+                const bool now = (left >> lane & 1u) && mine == item;
+                left &= ~__ballot_sync(ALL_LANES, now);
+                if (now && !moved) {
+                    const bool pairs = any_pairs(I.W.S);
+                    shadow_job(I.W, pairs ? I.W.S.tlasPairs : I.W.S.tlas, pairs, I0.W.jobs[2 * (base + lane)],
+                               I0.W.jobs[2 * (base + lane) + 1], I.rayBase, vis);
+                }
+                continue;
+            }
+            auto next = [&](uint32_t want, uint32_t& j, bool& ok) {
+                ok = false;
+                if (!chunk()) return false;
+                // this item's jobs of the chunk, as many as there are lanes for (the lowest
+                // run of neighbours among them)
+                const uint32_t own = __ballot_sync(ALL_LANES, (left >> lane & 1u) && mine == item);
+                if (!own) return false;  // another item's jobs end this walk
+                const uint32_t f = __ffs(own) - 1u, run = own >> f, len = ~run ? __ffs(~run) - 1u : 32u;
+                const uint32_t r = __popc(want & ((1u << lane) - 1u)), n = min((uint32_t)__popc(want), len);
+                ok = r < n;
+                j = base + f + r;
+                left &= ~((n < 32u ? (1u << n) - 1u : ALL_LANES) << f);
+                return true;
+            };
+            if (moved) shadow_moved(I.W, *m.w2, I.rayBase, next, vis);
+            else shadow_walk8(I.W, m, I.rayBase, next, vis);
+            __syncwarp();
+        }
     }
     add_visits(B.counters, 6, 0u, vis);
 }
@@ -645,21 +791,30 @@ const void* trace_batch_kernel(int stage) {
     }
 }
 
+uint32_t trace_batch_smem(const BatchArgs& B, uint32_t threads) {
+    const uint32_t smem = walk_smem(B.wideDepth + 1u, B.moved != 0u, threads);
+    if (smem > 48u * 1024u)
+        for (int stage = 0; stage <= 2; stage += 2)
+            cudaFuncSetAttribute(trace_batch_kernel(stage), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    return smem;
+}
+
 cudaError_t launch_trace_batch(const BatchArgs& B, const TraceTuning& tune, cudaStream_t st,
                                cudaEvent_t afterPrimary, cudaEvent_t afterShadow, cudaEvent_t afterClosest) {
     if (B.n == 0 || B.totalRays == 0) return cudaSuccess;
-    cudaError_t e = cudaMemsetAsync(B.work, 0, 3 * sizeof(uint32_t), st);
+    cudaError_t e = cudaMemsetAsync(B.work, 0, 6 * sizeof(uint32_t), st);
     if (e != cudaSuccess) return e;
     const int block = (int)tune.block;
     const uint32_t rays = B.totalRays;
-    k_trace_primary_batch<<<persistent_grid((const void*)k_trace_primary_batch, block, 0, tune, rays), block, 0,
+    const size_t smem = trace_batch_smem(B, tune.block);
+    k_trace_primary_batch<<<walk8_grid((const void*)k_trace_primary_batch, block, smem, tune, rays), block, smem,
                             st>>>(B);
     note_launch();
     if (afterClosest) cudaEventRecord(afterClosest, st);
     k_emit_batch<<<(rays + 127) / 128, 128, 0, st>>>(B);
     note_launch();
     if (afterPrimary) cudaEventRecord(afterPrimary, st);
-    k_trace_shadow_batch<<<persistent_grid((const void*)k_trace_shadow_batch, block, 0, tune, rays * 4u), block, 0,
+    k_trace_shadow_batch<<<walk8_grid((const void*)k_trace_shadow_batch, block, smem, tune, rays * 4u), block, smem,
                            st>>>(B);
     note_launch();
     if (afterShadow) cudaEventRecord(afterShadow, st);
@@ -679,7 +834,6 @@ __global__ void k_raycast(DevScene S, const float* ro, const float* rd, uint32_t
     float3 o = mk(ro[3 * i], ro[3 * i + 1], ro[3 * i + 2]), d = mk(rd[3 * i], rd[3 * i + 1], rd[3 * i + 2]);
     const bool pairs = closest_pairs(S);
     trace_closest(S, pairs ? S.tlasPairs : S.tlas, o, d, t, tri, inst, bu, bv, vis, err, pairs);
-    if (tri >= 0) t = refine_t(S, (uint32_t)tri, (uint32_t)inst, o, d);
     tOut[i] = t;
     triOut[i] = tri;
     instOut[i] = inst;
@@ -697,18 +851,92 @@ __global__ void k_occluded(DevScene S, const float* ro, const float* rd, const f
                  : 0;
 }
 
+// The same on the 8-wide tree.
+template <bool ANY>
+__global__ void __launch_bounds__(256, QUERY_MIN_BLOCKS) k_query_walk8(DevScene S, const float* ro, const float* rd,
+                                                                          const float* maxDist, uint32_t n,
+                                                                          float* tOut, int32_t* triOut,
+                                                                          int32_t* instOut, uint8_t* out,
+                                                                          uint32_t* cursor, uint32_t* err) {
+    extern __shared__ float4 smem[];
+    if (!*S.valid) return;
+    const uint32_t lane = threadIdx.x & 31u;
+    const WalkSmem m = walk_shared(smem, S.wideDepth + 1u, false);
+    Visits vis = {0, 0, 0, 0};
+    auto gen = [&](bool& more, uint32_t idle, float3& o, float3& d, float3& winv, float& tmax, uint32_t& tag,
+                   uint4& hit) {
+        const uint32_t i = take(cursor, idle);
+        const bool ok = i < n && (idle >> lane & 1u);
+        more = __any_sync(ALL_LANES, ok);
+        if (!ok) return false;
+        const size_t i3 = 3 * (size_t)i;
+        o = mk(ro[i3], ro[i3 + 1], ro[i3 + 2]);
+        d = mk(rd[i3], rd[i3 + 1], rd[i3 + 2]);
+        winv = mk(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
+        tmax = ANY ? maxDist[i] : T_MAX;
+        tag = i;
+        int tri = -1, inst = -1;
+        float bu = 0.0f, bv = 0.0f;
+        const bool blocked = dyn_walk<ANY>(S, o, d, winv, tmax, tri, inst, bu, bv, vis, err);
+        hit = make_uint4((uint32_t)tri, (uint32_t)inst, 0u, 0u);
+        if (ANY && blocked) out[i] = 1;
+        return !(ANY && blocked);
+    };
+    auto fin = [&](uint32_t i, float t, uint4 hit, bool blocked) {
+        if (ANY) {
+            out[i] = blocked ? 1 : 0;
+        } else {
+            tOut[i] = t;
+            triOut[i] = (int32_t)hit.x;
+            instOut[i] = (int32_t)hit.y;
+        }
+    };
+    walk8<ANY>(S, *m.tables, *m.w8, m.stk, S.wideDepth + 1u, gen, fin, vis, err);
+}
+
+// The hits' parameters in double-float (refine_t), one thread per ray.
+__global__ void k_refine_hits(DevScene S, const float* ro, const float* rd, uint32_t n, float* t, const int32_t* tri,
+                              const int32_t* inst) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n || !*S.valid || tri[i] < 0) return;
+    const size_t i3 = 3 * (size_t)i;
+    t[i] = refine_t(S, (uint32_t)tri[i], (uint32_t)inst[i], mk(ro[i3], ro[i3 + 1], ro[i3 + 2]),
+                    mk(rd[i3], rd[i3 + 1], rd[i3 + 2]));
+}
+
+static const TraceTuning query_tuning(int numSms) { return TraceTuning{256u, 0u, 0u, numSms, 0u}; }
+
 cudaError_t launch_raycast(const DevScene& S, const float* ro, const float* rd, uint32_t n, float* tOut,
-                           int32_t* triOut, int32_t* instOut, uint32_t* err, cudaStream_t st) {
+                           int32_t* triOut, int32_t* instOut, uint32_t* cursor, int numSms, uint32_t* err,
+                           cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    k_raycast<<<(n + 127) / 128, 128, 0, st>>>(S, ro, rd, n, tOut, triOut, instOut, err);
+    if (S.wideNodes) {
+        const size_t smem = walk_smem(S.wideDepth + 1u, false, 256u);
+        cudaError_t e = cudaMemsetAsync(cursor, 0, 4, st);
+        if (e != cudaSuccess) return e;
+        k_query_walk8<false><<<walk8_grid((const void*)k_query_walk8<false>, 256, smem, query_tuning(numSms), n), 256,
+                               smem, st>>>(S, ro, rd, nullptr, n, tOut, triOut, instOut, nullptr, cursor, err);
+    } else {
+        k_raycast<<<(n + 127) / 128, 128, 0, st>>>(S, ro, rd, n, tOut, triOut, instOut, err);
+    }
+    note_launch();
+    k_refine_hits<<<(n + 127) / 128, 128, 0, st>>>(S, ro, rd, n, tOut, triOut, instOut);
     note_launch();
     return cudaGetLastError();
 }
 
 cudaError_t launch_occluded(const DevScene& S, const float* ro, const float* rd, const float* maxDist, uint32_t n,
-                            uint8_t* out, uint32_t* err, cudaStream_t st) {
+                            uint8_t* out, uint32_t* cursor, int numSms, uint32_t* err, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    k_occluded<<<(n + 127) / 128, 128, 0, st>>>(S, ro, rd, maxDist, n, out, err);
+    if (S.wideNodes) {
+        const size_t smem = walk_smem(S.wideDepth + 1u, false, 256u);
+        cudaError_t e = cudaMemsetAsync(cursor, 0, 4, st);
+        if (e != cudaSuccess) return e;
+        k_query_walk8<true><<<walk8_grid((const void*)k_query_walk8<true>, 256, smem, query_tuning(numSms), n), 256,
+                              smem, st>>>(S, ro, rd, maxDist, n, nullptr, nullptr, nullptr, out, cursor, err);
+    } else {
+        k_occluded<<<(n + 127) / 128, 128, 0, st>>>(S, ro, rd, maxDist, n, out, err);
+    }
     note_launch();
     return cudaGetLastError();
 }

@@ -1,0 +1,217 @@
+// sb_walk2.cuh — the moved and deformed instance slots of a ray (DevScene's
+// dynList), walked by a persistent warp: per slot its world bounds (the reference's TLAS leaf test), then its BLAS as the child-pair
+// nodes the refits keep current, near child first.
+//
+// One thread that walks its ray's slots alone makes a chain of some hundred
+// dependent loads, and the few rays that graze a dense mesh set the kernel's end
+// while the chip is idle. So the triangles of the leaves a ray hits go to a queue
+// and are tested by 32 lanes at once, two leaves hit in one step are opened
+// together, and lanes whose rays meet no slot take new rays (as in sb_walk8.cuh).
+// The results meet the scene-BVH walk's only in the next stage, so a warp that has
+// no rays left here goes on with that walk while others finish theirs. The atrium's
+// three movers and one deformer cost 99 + 72 us in kernels of one thread per ray
+// (two rays in three meet none of them), 72 + 63 us in such kernels of this walk,
+// and 21 + 21 us ahead of the tree's walk in the same launch.
+#pragma once
+#include "sb_walk8.cuh"
+
+namespace sb {
+
+constexpr uint32_t WALK2_QUEUE = 256;  // at most 31 waiting, then 4 of every lane a pass
+constexpr uint32_t WALK2_DEPTH = 24;   // stacked far children; deeper BLASes: dyn_walk
+
+struct Walk2Shared {
+    float4 o[32];                 // local origin, determinant sign
+    float4 d[32];                 // local direction, slot
+    unsigned long long best[32];  // as in Walk8Shared
+    uint4 hit[32];
+    uint32_t item[WALK2_QUEUE];   // lane of its ray << 24 | triangle
+    uint32_t stk[WALK2_DEPTH][32];  // far children
+};
+
+// True when every slot's BLAS can be walked by walk2.
+__device__ __forceinline__ bool walk2_usable(const DevScene& S) {
+    if (!S.depth || !S.pairs) return false;
+    const uint32_t db = __ldg(S.depth);
+    return db != DEPTH_UNKNOWN && db <= WALK2_DEPTH;
+}
+
+// gen and fin as for walk8; the best hit starts as none within tmax.
+template <bool ANY, class Gen, class Fin>
+__device__ __forceinline__ void walk2(const DevScene& S, Walk2Shared& sm, Gen gen, Fin fin, Visits& vis,
+                                      uint32_t* err) {
+    const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
+    enum : uint32_t { FREE, WALK, ENDED };  // ENDED: this slot's nodes are done, items perhaps
+    uint32_t state = FREE;
+    float3 wo = mk(0.f, 0.f, 0.f), wd = wo, winv = wo, o = wo, inv = wo;
+    float tmax = 0.0f;
+    uint32_t tag = 0, k = 0, cur = PE_NONE, sp = 0, iter = 0, last = 0, head = 0, tail = 0;
+    bool more = true;
+    for (;;) {
+        const bool done = state == FREE || (state == ENDED && (int32_t)(last - head) <= 0);
+        const uint32_t idle = __ballot_sync(ALL_LANES, done);
+        if (__popc(idle) >= WALK8_IDLE || !__any_sync(ALL_LANES, state == WALK)) {
+            const bool blocked = ANY && state == ENDED && (uint32_t)sm.best[lane] == 0u;
+            bool have = done && state == ENDED && !blocked;  // a ray with slots left perhaps
+            if (done && state == ENDED && blocked) fin(tag, tmax, make_uint4(0u, 0u, 0u, 0u), true);
+            const uint32_t want = __ballot_sync(ALL_LANES, done && !have);
+            if (more && want) {
+                if (gen(more, want, wo, wd, tmax, tag)) {
+                    winv = mk(1.0f / wd.x, 1.0f / wd.y, 1.0f / wd.z);
+                    sm.best[lane] = (unsigned long long)__float_as_uint(tmax) << 32 | 0xFFFFFFFFull;
+                    if (!ANY) sm.hit[lane] = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u);
+                    k = iter = 0;
+                    have = true;
+                }
+            } else if (idle == ALL_LANES && !__any_sync(ALL_LANES, have)) {
+                break;
+            }
+            if (done) state = FREE;
+            if (have) {  // the ray's next slot
+                for (; k < S.dynCount && state == FREE; ++k) {
+                    const uint32_t slot = __ldg(S.dynList + k);
+                    if (S.slotBounds) {
+                        const float* b = S.slotBounds + 6u * slot;
+                        if (!slab(mk(__ldg(b), __ldg(b + 1), __ldg(b + 2)), mk(__ldg(b + 3), __ldg(b + 4), __ldg(b + 5)),
+                                  wo, winv, tmax))
+                            continue;
+                    }
+                    ++vis.inst;
+                    const float4 m = __ldg(S.inst + 4 * slot + 3);
+                    if (!(m.w > 0.5f)) continue;
+                    const float4 r0 = __ldg(S.inst + 4 * slot), r1 = __ldg(S.inst + 4 * slot + 1),
+                                 r2 = __ldg(S.inst + 4 * slot + 2);
+                    o = mk(dot3(xyz(r0), wo) + r0.w, dot3(xyz(r1), wo) + r1.w, dot3(xyz(r2), wo) + r2.w);
+                    const float3 d = mk(dot3(xyz(r0), wd), dot3(xyz(r1), wd), dot3(xyz(r2), wd));
+                    inv = mk(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
+                    const uint32_t root = __float_as_uint(m.x);
+                    if (root >= __float_as_uint(m.y) || root >= S.nodeCount) continue;
+                    const uint4 a = __ldg(S.nodes + 2 * root), b = __ldg(S.nodes + 2 * root + 1);
+                    ++vis.blas;
+                    if (!slab(mk(__uint_as_float(a.x), __uint_as_float(a.y), __uint_as_float(a.z)),
+                              mk(__uint_as_float(a.w), __uint_as_float(b.x), __uint_as_float(b.y)), o, inv, tmax))
+                        continue;
+                    cur = b.w == INTERIOR ? PE_BLAS | root : ((b.w >> 24) ? b.w : PE_NONE);
+                    if (cur == PE_NONE) continue;
+                    sm.o[lane] = make_float4(o.x, o.y, o.z, m.z);
+                    sm.d[lane] = make_float4(d.x, d.y, d.z, __uint_as_float(slot));
+                    sp = 0;
+                    last = head;
+                    state = WALK;
+                }
+                if (state == FREE)
+                    fin(tag, tmax, ANY ? make_uint4(0u, 0u, 0u, 0u) : sm.hit[lane], false);
+            }
+            __syncwarp();
+        }
+        // one node in every walking lane
+        uint32_t off0 = 0, n0 = 0, off1 = 0, n1 = 0;  // the hit leaves' triangles, nearer leaf first
+        if (state == WALK) {
+            if (cur >> 24) {  // a root that is a leaf
+                off0 = cur & 0x00FFFFFFu;
+                n0 = cur >> 24;
+                cur = PE_NONE;
+            } else {
+                const uint4* p = S.pairs + 4u * (cur & (PE_BLAS - 1u));
+                const uint4 q0 = __ldg(p), q1 = __ldg(p + 1), q2 = __ldg(p + 2), q3 = __ldg(p + 3);
+                vis.blas += 2;
+                float t0 = 0.f, t1 = 0.f;
+                const bool h0 = slab_near(__uint_as_float(q0.x), __uint_as_float(q0.z), __uint_as_float(q2.x),
+                                          __uint_as_float(q0.y), __uint_as_float(q0.w), __uint_as_float(q2.y), o, inv,
+                                          tmax, t0) && q3.x != PE_NONE;
+                const bool h1 = slab_near(__uint_as_float(q1.x), __uint_as_float(q1.z), __uint_as_float(q2.z),
+                                          __uint_as_float(q1.y), __uint_as_float(q1.w), __uint_as_float(q2.w), o, inv,
+                                          tmax, t1) && q3.y != PE_NONE;
+                const bool swap = h0 && h1 && t1 < t0;
+                uint32_t a = h0 ? q3.x : PE_NONE, b = h1 ? q3.y : PE_NONE;
+                if (swap) {
+                    const uint32_t x = a;
+                    a = b;
+                    b = x;
+                }
+                cur = PE_NONE;
+                if (a != PE_NONE) {
+                    if (a >> 24) { off0 = a & 0x00FFFFFFu; n0 = a >> 24; }
+                    else cur = a;
+                }
+                if (b != PE_NONE) {
+                    if (b >> 24) { off1 = b & 0x00FFFFFFu; n1 = b >> 24; }
+                    else if (cur == PE_NONE) cur = b;
+                    else if (sp < WALK2_DEPTH) sm.stk[sp++][lane] = b;
+                    else latch(err, ERR_CAPACITY);  // unreachable: walk2_usable bounds the depth
+                }
+                if (++iter > S.iterCapRef) {
+                    latch(err, ERR_WATCHDOG);
+                    cur = PE_NONE;
+                    sp = 0;
+                }
+            }
+            if (cur == PE_NONE && sp) cur = sm.stk[--sp][lane];
+            if (cur == PE_NONE) state = ENDED;
+        }
+        // the triangles to the queue, four of each lane a pass, and rounds of tests
+        for (;;) {
+            const uint32_t mine = min(n0 + n1, 4u);
+            const uint32_t c0 = __ballot_sync(ALL_LANES, mine & 1u), c1 = __ballot_sync(ALL_LANES, mine & 2u),
+                           c2 = __ballot_sync(ALL_LANES, mine & 4u);
+            uint32_t at = tail + __popc(c0 & below) + 2u * __popc(c1 & below) + 4u * __popc(c2 & below);
+            for (uint32_t i = 0; i < mine; ++i, ++at) {
+                if (!n0) {
+                    off0 = off1;
+                    n0 = n1;
+                    n1 = 0;
+                }
+                sm.item[at % WALK2_QUEUE] = lane << 24 | off0++;
+                --n0;
+            }
+            if (mine) last = at;
+            const bool any = (c0 | c1 | c2) != 0u;
+            tail += __popc(c0) + 2u * __popc(c1) + 4u * __popc(c2);
+            for (;;) {
+                if (tail - head < 32u) {
+                    if (tail == head) break;
+                    if (any) break;  // more may come
+                    const uint32_t wait = __ballot_sync(ALL_LANES, state == ENDED && (int32_t)(last - head) > 0);
+                    if (__popc(wait) < WALK8_WAIT && (!wait || __any_sync(ALL_LANES, state == WALK))) break;
+                }
+                __syncwarp();
+                const uint32_t n = min(32u, tail - head);
+                bool ok = false;
+                float t, u, v;
+                uint32_t tri = 0, of = 0, slot = 0;  // of: the lane whose ray it is
+                if (lane < n) {
+                    tri = sm.item[(head + lane) % WALK2_QUEUE];
+                    of = tri >> 24;
+                    tri &= 0x00FFFFFFu;
+                    const float4 ro = sm.o[of], rd = sm.d[of];
+                    const float limit = __uint_as_float((uint32_t)(sm.best[of] >> 32));
+                    slot = __float_as_uint(rd.w);
+                    float det;
+                    uint32_t hb;
+                    ok = tri_hit(S, tri, xyz(ro), xyz(rd), limit, t, det, u, v, hb) &&
+                         (hb & (ANY ? TB_SHADOW_OK : TB_CLOSEST_OK)) && side_ok(hb, det * ro.w);
+                    ++vis.tri;
+                }
+                if (__any_sync(ALL_LANES, ok)) {
+                    const unsigned long long key = ANY ? 0ull : (unsigned long long)__float_as_uint(t) << 32 | lane;
+                    if (ok) {
+                        if (ANY) sm.best[of] = 0ull;  // blocked
+                        else atomicMin(&sm.best[of], key);
+                    }
+                    __syncwarp();
+                    if (!ANY && ok && sm.best[of] == key) sm.hit[of] = make_uint4(tri, slot, pack_uv(u, v), 0u);
+                    __syncwarp();
+                    if (state != FREE) {
+                        const unsigned long long b = sm.best[lane];
+                        if (!ANY) tmax = __uint_as_float((uint32_t)(b >> 32));
+                        else if ((uint32_t)b == 0u) state = ENDED;
+                    }
+                }
+                head += n;
+            }
+            if (!any) break;
+        }
+    }
+}
+
+}  // namespace sb
