@@ -6,34 +6,59 @@
 // nodes (flattenBVHRoot, 658-721). This builder is a linear BVH (Karras,
 // "Maximizing Parallelism in the Construction of BVHs, Octrees, and k-d
 // Trees", HPG 2012) emitting that layout directly:
-//   1. per triangle its vertex bounds; the centroid bounds of the mesh;
-//   2. a 30-bit Morton code of each bounds centre within the centroid bounds;
-//   3. a stable LSD radix sort of (code, triangle), 4 passes of 8 bits, with
+//   1. per triangle the centre of its vertex bounds; the bounds of the centres;
+//   2. a 30-bit Morton code of each centre within those;
+//   3. a stable LSD radix sort of (code, triangle), 3 passes of 10 bits, with
 //      warp-level ranking (match.any) so equal digits keep their order;
 //   4. the binary radix tree over the sorted codes, equal codes ordered by
-//      position (Karras' tie rule), one thread per internal node;
-//   5. a bottom-up pass (one thread per triangle, arrival counters: the second
-//      child to arrive carries on) giving every node its bounds (exact min/max
-//      of its triangles' vertices, as the refit computes them) and its size in
-//      the output tree, where any node of at most `leafSize` triangles whose
-//      parent holds more becomes one leaf;
-//   6. every output node finds its pre-order index by walking to the root
-//      (adding 1 per ancestor and, when it lies right of an ancestor, the size
-//      of that ancestor's left subtree) and writes its record: bounds, miss =
-//      index + subtree size, payload (count << 24 | first position) or
-//      0xFFFFFFFF. The left child lands at index + 1.
+//      position (Karras' tie rule). It is the Cartesian tree of the common prefix
+//      lengths of neighbours: the node that splits between g and g + 1 reaches to
+//      the next shorter prefix on either side, which masks of 32 prefix bytes and
+//      the minima of 32, 1024, ... of them find in a few steps. A node of more than
+//      `leafSize` triangles is an interior node of the output; a child of one with
+//      at most that many is an output leaf;
+//   5. the output places without a climb: the tree below a node of K output leaves
+//      has 2 K - 1 nodes, and in pre-order a node comes after every output leaf and
+//      interior node that starts left of it and after its ancestors that start with
+//      it. So prefix sums over the positions, of leaves and of interior nodes by
+//      their first position, give every node its index and its miss link;
+//   6. the bounds: an output leaf's as the refit computes them (its triangles in
+//      order, strict < and >); an interior node's as the minimum and maximum of its
+//      range of output leaves, one warp per node, from the leaves' boxes and those
+//      of 32, 1024, ... positions. (The refit's unions order -0 below +0 and no
+//      leaf's bound is a NaN, so they are the minima and maxima of order-preserving
+//      integers, which the warp reduces in hardware.)
 // The output triangle order is the sorted order (triangle at each position).
-// No loop waits on another thread; every walk is bounded by the tree depth
-// (at most 64 levels: each level adds a bit of the 62-bit key + position).
+//
+// What bounds it is the chain of dependent phases, not their work: a mesh of a few
+// thousand triangles fills a few SMs. Up to BUILD_CLUSTER_TRIS triangles one launch
+// of a thread-block cluster of at most 8 CTAs runs all phases with hardware cluster
+// barriers between them; above that each phase is a launch over more SMs, placed
+// ahead of the end of the one before it (at 20,000 triangles 98 us by a cluster,
+// 69 us by launches; at 8,192 54 us by a cluster, at 10,000 67 us by launches). No loop waits on another thread; every
+// walk is bounded by the tree depth (at most 64 levels: each adds a bit of the
+// 62-bit key + position). A build of 1,024 / 8,192 / 65,537 / 600,000 triangles
+// takes 36 / 54 / 76 / 203 us; as 19 launches and copies with a bottom-up climb
+// over arrival counters (41 us on a mesh of 9k by itself) and a scan by one CTA it
+// took 142 / 168 / 195 / 627 us.
+#include <cooperative_groups.h>
+
+#include <algorithm>
+#include <cstddef>
+#include <type_traits>
+
 #include "sb_kernels.cuh"
 
 namespace sb {
 
 namespace {
 
-constexpr uint32_t kNone = 0xFFFFFFFFu;
-constexpr uint32_t kTile = 2048;   // keys per sort CTA (8 warps x 8 rounds x 32)
-constexpr uint32_t kSortThreads = 256;
+constexpr uint32_t kThreads = 1024;             // of every CTA
+constexpr uint32_t kWarps = kThreads / 32;
+constexpr uint32_t kBits = 10, kDigits = 1u << kBits;
+constexpr uint32_t kSortCtas = 148;             // of a sort pass: each reads the others' digit counts
+constexpr uint32_t kMaxCtas = 1024;             // of the other phases
+constexpr uint32_t BUILD_CLUSTER_TRIS = 8192;   // at most this many by one cluster
 
 __device__ __forceinline__ uint32_t f2o(float f) {
     const uint32_t u = __float_as_uint(f);
@@ -52,349 +77,599 @@ __device__ __forceinline__ uint32_t expand10(uint32_t v) {
     return v;
 }
 
-// 1. triangle bounds (source order) and the centroid bounds
-__global__ void k_tri_bounds(const float* pos, uint32_t V, const uint32_t* idx, uint32_t T, float4* lo, float4* hi,
-                             uint32_t* cbox, uint32_t* err) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    float c[3] = {0.f, 0.f, 0.f};
-    bool valid = false;
-    if (t < T) {
-        const uint32_t i0 = idx[3 * t], i1 = idx[3 * t + 1], i2 = idx[3 * t + 2];
-        if (i0 < V && i1 < V && i2 < V) {
+// One build's inputs, scratch and outputs.
+struct Build {
+    const float* pos;
+    const uint32_t* idx;
+    uint32_t V, T, leafSize, chunk;  // chunk: positions per CTA and phase, a multiple of kThreads
+    uint32_t levels;                 // prefix and box levels above the positions (32 per step)
+    float4* centre;                  // T
+    uint32_t* part;                  // kMaxCtas x 8: centre bounds; then leaf and node sums
+    uint32_t *keyA, *keyB, *valA;    // T each; the sorted triangles lie in `order`
+    uint32_t* hist;                  // kMaxCtas x kDigits
+    uint8_t* prefix;                 // per position and level: common prefix with the next, minima above
+    uint32_t *first, *last;          // T: range of the interior node of the output that splits after a position
+    uint32_t *starts, *leafCount;    // T: interior nodes that start here; triangles of the output leaf that does
+    uint2* before;                   // T + 1: output leaves, and all output nodes, that start left of a position
+    uint4 *boxLo, *boxHi;            // per position and level: box of 32^level positions' output leaves (f2o)
+    uint32_t levelAt[6];             // offset of each level in them and in prefix (a multiple of 32)
+    uint32_t *order, *nodes, *nodeCount;
+    uint32_t* err;
+};
+
+struct BuildShared {
+    uint2 sum2[kWarps];
+    uint32_t sum[kWarps];
+    uint32_t box[6];
+    uint32_t lo[kWarps][3], hi[kWarps][3];
+    union {
+        float tri[6][kThreads];            // bounds of the triangles of a tile
+        uint32_t far[kThreads + 1];        // splits of a tile whose range leaves their 32; their number
+    } u;
+    uint32_t cnt[kWarps][kDigits];         // a sort pass' digits per warp (launches of other phases end above)
+};
+
+__device__ __forceinline__ uint32_t warp_scan(uint32_t v) {  // inclusive
+    const uint32_t lane = threadIdx.x & 31u;
+#pragma unroll
+    for (int s = 1; s < 32; s <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, v, s);
+        if (lane >= (uint32_t)s) v += y;
+    }
+    return v;
+}
+// Exclusive scan over the CTA's threads; `total` of all. Synchronizes.
+__device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t* tmp, uint32_t& total) {
+    const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5, x = warp_scan(v);
+    if (lane == 31) tmp[w] = x;
+    __syncthreads();
+    const uint32_t sums = warp_scan(tmp[lane]);
+    total = __shfl_sync(0xFFFFFFFFu, sums, 31);
+    const uint32_t ahead = __shfl_sync(0xFFFFFFFFu, sums, (w + 31u) & 31u);
+    __syncthreads();
+    return (w ? ahead : 0u) + x - v;
+}
+
+// 1. centres (source order) and this CTA's part of their bounds
+__device__ __forceinline__ void build_centres(const Build& B, BuildShared& sm, uint32_t cta, uint32_t ctas) {
+    if (threadIdx.x < 6) sm.box[threadIdx.x] = threadIdx.x < 3 ? 0xFFFFFFFFu : 0u;
+    __syncthreads();
+    uint32_t omn[3] = {0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu}, omx[3] = {0u, 0u, 0u};
+    for (uint32_t t = cta * kThreads + threadIdx.x; t < B.T; t += ctas * kThreads) {
+        const uint32_t id[3] = {B.idx[3 * (size_t)t], B.idx[3 * (size_t)t + 1], B.idx[3 * (size_t)t + 2]};
+        float c[3] = {0.f, 0.f, 0.f};
+        if (id[0] < B.V && id[1] < B.V && id[2] < B.V) {
             float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
-            const uint32_t ids[3] = {i0, i1, i2};
             for (int k = 0; k < 3; ++k)
                 for (int a = 0; a < 3; ++a) {
-                    const float v = pos[3 * (size_t)ids[k] + a];
+                    const float v = B.pos[3 * (size_t)id[k] + a];
                     if (v < mn[a]) mn[a] = v;
                     if (v > mx[a]) mx[a] = v;
                 }
-            lo[t] = make_float4(mn[0], mn[1], mn[2], 0.0f);
-            hi[t] = make_float4(mx[0], mx[1], mx[2], 0.0f);
             for (int a = 0; a < 3; ++a) c[a] = mn[a] + (mx[a] - mn[a]) * 0.5f;
-            valid = isfinite(c[0]) && isfinite(c[1]) && isfinite(c[2]);
+            if (isfinite(c[0]) && isfinite(c[1]) && isfinite(c[2]))
+                for (int a = 0; a < 3; ++a) {
+                    omn[a] = min(omn[a], f2o(c[a]));
+                    omx[a] = max(omx[a], f2o(c[a]));
+                }
         } else {
-            latch(err, ERR_LAYOUT);
-            lo[t] = make_float4(0.f, 0.f, 0.f, 0.f);
-            hi[t] = lo[t];
+            latch(B.err, ERR_LAYOUT);
         }
+        B.centre[t] = make_float4(c[0], c[1], c[2], 0.0f);
     }
-    // warp-reduce the ordered-int centroid bounds, one atomic per warp and bound
-    uint32_t omn[3], omx[3];
     for (int a = 0; a < 3; ++a) {
-        omn[a] = valid ? f2o(c[a]) : 0xFFFFFFFFu;
-        omx[a] = valid ? f2o(c[a]) : 0u;
-        for (int s = 16; s; s >>= 1) {
-            omn[a] = min(omn[a], __shfl_xor_sync(0xFFFFFFFFu, omn[a], s));
-            omx[a] = max(omx[a], __shfl_xor_sync(0xFFFFFFFFu, omx[a], s));
+        const uint32_t mn = __reduce_min_sync(0xFFFFFFFFu, omn[a]), mx = __reduce_max_sync(0xFFFFFFFFu, omx[a]);
+        if ((threadIdx.x & 31u) == 0) {
+            atomicMin(&sm.box[a], mn);
+            atomicMax(&sm.box[3 + a], mx);
         }
     }
-    if ((threadIdx.x & 31) == 0)
+    __syncthreads();
+    if (threadIdx.x < 6) B.part[cta * 8u + threadIdx.x] = sm.box[threadIdx.x];
+}
+
+// 2. Morton codes; the tree's counters cleared
+__device__ __forceinline__ void build_codes(const Build& B, BuildShared& sm, uint32_t cta, uint32_t ctas) {
+    if (threadIdx.x < 32) {
+        for (uint32_t a = 0; a < 6; ++a) {
+            uint32_t v = a < 3 ? 0xFFFFFFFFu : 0u;
+            for (uint32_t c = threadIdx.x; c < ctas; c += 32) {
+                const uint32_t x = B.part[c * 8u + a];
+                v = a < 3 ? min(v, x) : max(v, x);
+            }
+            v = a < 3 ? __reduce_min_sync(0xFFFFFFFFu, v) : __reduce_max_sync(0xFFFFFFFFu, v);
+            if (threadIdx.x == 0) sm.box[a] = v;
+        }
+    }
+    __syncthreads();
+    const uint32_t end = min(B.T, (cta + 1u) * B.chunk);
+    for (uint32_t t = cta * B.chunk + threadIdx.x; t < end; t += kThreads) {
+        const float4 c4 = B.centre[t];
+        const float c[3] = {c4.x, c4.y, c4.z};
+        uint32_t q[3];
         for (int a = 0; a < 3; ++a) {
-            atomicMin(cbox + a, omn[a]);
-            atomicMax(cbox + 3 + a, omx[a]);
+            const float mn = o2f(sm.box[a]), mx = o2f(sm.box[3 + a]);
+            const float ext = mx - mn;
+            float x = ext > 0.0f ? (c[a] - mn) / ext : 0.0f;
+            x = isfinite(x) ? fminf(fmaxf(x, 0.0f), 1.0f) : 0.0f;
+            q[a] = min((uint32_t)(x * 1024.0f), 1023u);
         }
-}
-
-// 2. Morton codes of the bounds centres
-__global__ void k_morton(const float4* lo, const float4* hi, uint32_t T, const uint32_t* cbox, uint32_t* keys,
-                         uint32_t* vals) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= T) return;
-    const float4 l = lo[t], h = hi[t];
-    const float c[3] = {l.x + (h.x - l.x) * 0.5f, l.y + (h.y - l.y) * 0.5f, l.z + (h.z - l.z) * 0.5f};
-    uint32_t q[3];
-    for (int a = 0; a < 3; ++a) {
-        const float mn = o2f(cbox[a]), mx = o2f(cbox[3 + a]);
-        const float ext = mx - mn;
-        float x = ext > 0.0f ? (c[a] - mn) / ext : 0.0f;
-        x = isfinite(x) ? fminf(fmaxf(x, 0.0f), 1.0f) : 0.0f;
-        q[a] = min((uint32_t)(x * 1024.0f), 1023u);
+        B.keyA[t] = (expand10(q[0]) << 2) | (expand10(q[1]) << 1) | expand10(q[2]);
+        B.starts[t] = 0u;
+        B.leafCount[t] = 0u;
     }
-    keys[t] = (expand10(q[0]) << 2) | (expand10(q[1]) << 1) | expand10(q[2]);
-    vals[t] = t;
 }
 
-// 3. stable LSD radix sort, one 8-bit digit per pass
-__global__ void __launch_bounds__(kSortThreads) k_sort_hist(const uint32_t* keys, uint32_t T, uint32_t shift,
-                                                            uint32_t* hist, uint32_t tiles) {
-    __shared__ uint32_t cnt[256];
-    cnt[threadIdx.x] = 0u;
-    __syncthreads();
-    const uint32_t base = blockIdx.x * kTile;
-    for (uint32_t i = threadIdx.x; i < kTile; i += kSortThreads) {
-        const uint32_t p = base + i;
-        if (p < T) atomicAdd(&cnt[(keys[p] >> shift) & 0xFFu], 1u);
+// 3. stable LSD radix sort, one digit per pass: the digits of this CTA's chunk per
+// warp (each warp a contiguous part) and their sums, then, with all CTAs' sums
+// written, the keys and triangles to their places. Pass 0 reads triangle t at t.
+__device__ __forceinline__ uint32_t warp_part(const Build& B) { return B.chunk / kWarps; }  // a multiple of 32
+
+__device__ __forceinline__ void build_count(const Build& B, BuildShared& sm, uint32_t cta, const uint32_t* keys,
+                                            uint32_t shift) {
+    const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+    for (uint32_t d = lane; d < kDigits; d += 32) sm.cnt[w][d] = 0u;
+    __syncwarp();
+    const uint32_t from = cta * B.chunk + w * warp_part(B), to = min(B.T, from + warp_part(B));
+    for (uint32_t p = from; p < to; p += 32) {
+        const bool valid = p + lane < to;
+        const uint32_t digit = valid ? keys[p + lane] >> shift & (kDigits - 1u) : kDigits;
+        const uint32_t peers = __match_any_sync(0xFFFFFFFFu, digit);
+        if (valid && lane == (uint32_t)(__ffs(peers) - 1)) sm.cnt[w][digit] += __popc(peers);
+        __syncwarp();
     }
     __syncthreads();
-    hist[threadIdx.x * tiles + blockIdx.x] = cnt[threadIdx.x];
+    uint32_t n = 0;
+    for (uint32_t x = 0; x < kWarps; ++x) n += sm.cnt[x][threadIdx.x];
+    B.hist[cta * kDigits + threadIdx.x] = n;
 }
 
-// exclusive scan of n counts in place, one CTA of 1024 threads
-__global__ void __launch_bounds__(1024) k_scan(uint32_t* a, uint32_t n) {
-    __shared__ uint32_t warpSum[32];
-    __shared__ uint32_t carry;
-    if (threadIdx.x == 0) carry = 0u;
+__device__ __forceinline__ void build_place(const Build& B, BuildShared& sm, uint32_t cta, uint32_t ctas,
+                                            const uint32_t* keys, const uint32_t* vals, uint32_t shift,
+                                            uint32_t* keysOut, uint32_t* valsOut) {
+    const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5, d = threadIdx.x;  // one digit per thread
+    uint32_t ahead = 0, all = 0;
+#pragma unroll 8
+    for (uint32_t c = 0; c < ctas; ++c) {
+        const uint32_t x = B.hist[c * kDigits + d];
+        if (c < cta) ahead += x;
+        all += x;
+    }
+    uint32_t total;
+    uint32_t run = block_scan(all, sm.sum, total) + ahead;
+    for (uint32_t x = 0; x < kWarps; ++x) {
+        const uint32_t n = sm.cnt[x][d];
+        sm.cnt[x][d] = run;
+        run += n;
+    }
     __syncthreads();
-    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (uint32_t base = 0; base < n; base += 1024) {
-        const uint32_t i = base + threadIdx.x;
-        const uint32_t v = i < n ? a[i] : 0u;
-        uint32_t x = v;
-        for (int s = 1; s < 32; s <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, s);
-            if (lane >= (uint32_t)s) x += y;
+    const uint32_t from = cta * B.chunk + w * warp_part(B), to = min(B.T, from + warp_part(B));
+    for (uint32_t p = from; p < to; p += 32) {
+        const bool valid = p + lane < to;
+        const uint32_t key = valid ? keys[p + lane] : 0u;
+        const uint32_t digit = valid ? key >> shift & (kDigits - 1u) : kDigits;
+        const uint32_t peers = __match_any_sync(0xFFFFFFFFu, digit);
+        const uint32_t at = valid ? sm.cnt[w][digit] + __popc(peers & ((1u << lane) - 1u)) : 0u;
+        __syncwarp();
+        if (valid && lane == (uint32_t)(__ffs(peers) - 1)) sm.cnt[w][digit] += __popc(peers);
+        __syncwarp();
+        if (valid && at < B.T) {
+            keysOut[at] = key;
+            valsOut[at] = vals ? vals[p + lane] : p + lane;
         }
-        if (lane == 31) warpSum[w] = x;
+    }
+}
+
+// 4. common prefixes of neighbours in this CTA's chunk, and their minima over 32 and
+// 1024 positions. 0 (shorter than any) stands after the last position.
+__device__ __forceinline__ void build_prefixes(const Build& B, BuildShared& sm, const uint32_t* keys, uint32_t cta) {
+    const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+    const uint32_t end = min((B.T + 31u) & ~31u, (cta + 1u) * B.chunk);
+    for (uint32_t base = cta * B.chunk; base < end; base += kThreads) {
+        const uint32_t j = base + threadIdx.x;
+        uint32_t d = 0;
+        if (j + 1u < B.T) {
+            const uint32_t x = keys[j] ^ keys[j + 1u];
+            d = x ? __clz(x) : 32u + __clz(j ^ (j + 1u));  // keys have 30 bits: at least 2
+        }
+        if (j < end) B.prefix[j] = (uint8_t)d;
+        const uint32_t m = __reduce_min_sync(0xFFFFFFFFu, d);
+        if (lane == 0) {
+            if (j < end) B.prefix[B.levelAt[1] + (j >> 5)] = (uint8_t)m;
+            sm.sum[w] = m;
+        }
         __syncthreads();
         if (w == 0) {
-            uint32_t s = warpSum[lane];
-            for (int k = 1; k < 32; k <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, s, k);
-                if (lane >= (uint32_t)k) s += y;
+            const uint32_t n = __reduce_min_sync(0xFFFFFFFFu, sm.sum[lane]);
+            if (lane == 0) B.prefix[B.levelAt[2] + (base >> 10)] = (uint8_t)n;
+        }
+        __syncthreads();
+    }
+}
+
+// The entries shorter than v among the 32 of a level from `at` (a multiple of 32).
+__device__ __forceinline__ uint32_t shorter(const Build& B, uint32_t at, uint32_t v) {
+    const uint4* p = reinterpret_cast<const uint4*>(B.prefix + at);
+    const uint4 a = p[0], b = p[1];
+    const uint32_t vv = v * 0x01010101u, word[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    uint32_t m = 0;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) m |= ((__vcmpltu4(word[k], vv) & 0x01010101u) * 0x01020408u >> 24) << (4 * k);
+    return m;
+}
+// The nearest position right of g (left, or -1) with a prefix shorter than v, when
+// its own 32 hold none. n[k]: entries of level k.
+__device__ __forceinline__ int64_t shorter_far(const Build& B, uint32_t g, uint32_t v, bool right) {
+    uint32_t i = g >> 5;  // entry of level k
+    for (uint32_t k = 1;; ++k) {
+        const uint32_t top = k == B.levels, in = i & 31u;
+        for (uint32_t b = i >> 5;;) {
+            const uint32_t n = (k == 1 ? (B.T + 31u) >> 5 : k == 2 ? (B.T + 1023u) >> 10
+                                : k == 3 ? (B.T + 32767u) >> 15 : (B.T + 1048575u) >> 20);  // entries of this level
+            uint32_t m = shorter(B, B.levelAt[k] + 32u * b, v);
+            const uint32_t left = n - 32u * b;
+            if (left < 32u) m &= (1u << left) - 1u;
+            if (b == i >> 5) m &= right ? (in == 31u ? 0u : 0xFFFFFFFFu << (in + 1u)) : (1u << in) - 1u;
+            if (m) {  // down to the position
+                uint32_t e = 32u * b + (right ? __ffs(m) - 1u : 31u - __clz(m));
+                for (uint32_t l = k; l-- > 0;) {
+                    uint32_t q = shorter(B, (l ? B.levelAt[l] : 0u) + 32u * e, v);
+                    if (!q) return -2;  // unreachable: the minimum above said otherwise
+                    e = 32u * e + (right ? __ffs(q) - 1u : 31u - __clz(q));
+                }
+                return e;
             }
-            warpSum[lane] = s;  // inclusive over warps
+            if (!top) break;
+            if (right ? 32u * (b + 1u) >= n : b == 0u) return right ? (int64_t)B.T - 1 : -1;
+            b = right ? b + 1u : b - 1u;
         }
-        __syncthreads();
-        const uint32_t before = (w ? warpSum[w - 1] : 0u) + x - v;
-        if (i < n) a[i] = carry + before;
-        __syncthreads();
-        if (threadIdx.x == 1023) carry += warpSum[31];
-        __syncthreads();
+        i >>= 5;
     }
 }
 
-__global__ void __launch_bounds__(kSortThreads) k_sort_scatter(const uint32_t* keysIn, const uint32_t* valsIn,
-                                                               uint32_t T, uint32_t shift, const uint32_t* hist,
-                                                               uint32_t tiles, uint32_t* keysOut,
-                                                               uint32_t* valsOut) {
-    __shared__ uint32_t warpCnt[8][256];
-    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (uint32_t d = lane; d < 256; d += 32) warpCnt[w][d] = 0u;
-    __syncwarp();
-    const uint32_t seg = blockIdx.x * kTile + w * 256u;
-    const uint32_t ltMask = (1u << lane) - 1u;
-    uint32_t key[8], val[8], rank[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        const uint32_t p = seg + (uint32_t)k * 32u + lane;
-        const bool valid = p < T;
-        key[k] = valid ? keysIn[p] : 0u;
-        val[k] = valid ? valsIn[p] : 0u;
-        const uint32_t digit = (key[k] >> shift) & 0xFFu;
-        const uint32_t tag = valid ? digit : 0x100u;
-        const uint32_t peers = __match_any_sync(0xFFFFFFFFu, tag);
-        const uint32_t base = valid ? warpCnt[w][digit] : 0u;
-        __syncwarp();
-        if (valid && lane == (uint32_t)(__ffs(peers) - 1)) warpCnt[w][digit] = base + __popc(peers);
-        __syncwarp();
-        rank[k] = base + __popc(peers & ltMask);
-    }
-    __syncthreads();
-    // per digit: offsets of the warps in position order
-    {
-        const uint32_t d = threadIdx.x;
-        uint32_t run = 0u;
-        for (int ww = 0; ww < 8; ++ww) {
-            const uint32_t c = warpCnt[ww][d];
-            warpCnt[ww][d] = run;
-            run += c;
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        const uint32_t p = seg + (uint32_t)k * 32u + lane;
-        if (p >= T) continue;
-        const uint32_t digit = (key[k] >> shift) & 0xFFu;
-        const uint32_t dst = hist[digit * tiles + blockIdx.x] + warpCnt[w][digit] + rank[k];
-        keysOut[dst] = key[k];
-        valsOut[dst] = val[k];
-    }
-}
-
-// 4. binary radix tree (internal nodes 0..T-2, leaf j = T-1+j)
-__device__ __forceinline__ int delta(const uint32_t* keys, int64_t T, int64_t i, int64_t j) {
-    if (j < 0 || j >= T) return -1;
-    const uint32_t a = keys[i], b = keys[j];
-    if (a == b) return __clzll((unsigned long long)(i ^ j));  // >= 32 for positions below 2^32
-    return __clz(a ^ b);
-}
-
-__global__ void k_radix_tree(const uint32_t* keys, uint32_t T, uint32_t* parent, uint32_t* left, uint32_t* right,
-                             uint32_t* first, uint32_t* last, uint32_t* err) {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int64_t n = T;
-    if (i >= n - 1) return;
-    const int d = (delta(keys, n, i, i + 1) - delta(keys, n, i, i - 1)) >= 0 ? 1 : -1;
-    const int dmin = delta(keys, n, i, i - d);
-    int64_t lmax = 2;
-    while (delta(keys, n, i, i + lmax * d) > dmin) lmax *= 2;
-    int64_t l = 0;
-    for (int64_t t = lmax / 2; t >= 1; t /= 2)
-        if (delta(keys, n, i, i + (l + t) * d) > dmin) l += t;
-    const int64_t j = i + l * d;
-    const int dnode = delta(keys, n, i, j);
-    int64_t s = 0;
-    for (int64_t div = 2;; div *= 2) {
-        const int64_t t = (l + div - 1) / div;
-        if (delta(keys, n, i, i + (s + t) * d) > dnode) s += t;
-        if (t <= 1) break;
-    }
-    const int64_t g = i + s * d + (d < 0 ? -1 : 0);
-    const int64_t lo = i < j ? i : j, hiR = i < j ? j : i;
-    if (!(lo <= g && g < hiR && hiR < n)) {  // the split lies inside the node's range
-        latch(err, ERR_LAYOUT);
-        left[i] = right[i] = kNone;
-        first[i] = last[i] = (uint32_t)i;
+// The tree: the output's interior nodes and where its leaves start.
+__device__ __forceinline__ void build_tree(const Build& B, BuildShared& sm, uint32_t cta, uint32_t ctas) {
+    if (B.T <= B.leafSize) {  // the root is a leaf
+        if (cta == 0 && threadIdx.x == 0) B.leafCount[0] = B.T;
         return;
     }
-    const uint32_t L = (lo == g) ? (uint32_t)(n - 1 + g) : (uint32_t)g;
-    const uint32_t R = (hiR == g + 1) ? (uint32_t)(n - 1 + g + 1) : (uint32_t)(g + 1);
-    left[i] = L;
-    right[i] = R;
-    first[i] = (uint32_t)lo;
-    last[i] = (uint32_t)hiR;
-    parent[L] = (uint32_t)i;
-    parent[R] = (uint32_t)i;
-    if (i == 0) parent[0] = kNone;
+    auto emit = [&](uint32_t g, int64_t l, int64_t r) {  // the split between g and g + 1; l, r: the shorter prefixes
+        const int64_t lo = l + 1, hi = r;
+        uint32_t last = 0u;  // not an interior node of the output
+        if (!(l >= -1 && lo <= (int64_t)g && (int64_t)g < hi && hi < (int64_t)B.T)) {
+            latch(B.err, ERR_LAYOUT);
+        } else if (hi - lo + 1 > (int64_t)B.leafSize) {
+            last = (uint32_t)hi;
+            B.first[g] = (uint32_t)lo;
+            atomicAdd(B.starts + lo, 1u);
+            const uint32_t nl = g - (uint32_t)lo + 1u, nr = (uint32_t)hi - g;
+            if (nl <= B.leafSize) B.leafCount[lo] = nl;
+            if (nr <= B.leafSize) B.leafCount[g + 1u] = nr;
+        }
+        B.last[g] = last;
+    };
+    for (uint32_t g0 = cta * kThreads; g0 + 1u < B.T; g0 += ctas * kThreads) {
+        if (threadIdx.x == 0) sm.u.far[kThreads] = 0u;
+        __syncthreads();
+        const uint32_t g = g0 + threadIdx.x;
+        if (g + 1u < B.T) {
+            const uint32_t in = g & 31u, base = g & ~31u, m = shorter(B, base, B.prefix[g]);
+            const uint32_t mr = m & (in == 31u ? 0u : 0xFFFFFFFFu << (in + 1u)), ml = m & ((1u << in) - 1u);
+            if ((ml || base == 0u) && mr)
+                emit(g, ml ? (int64_t)base + 31 - __clz(ml) : -1, base + __ffs(mr) - 1u);
+            else
+                sm.u.far[atomicAdd(&sm.u.far[kThreads], 1u)] = g;
+        }
+        __syncthreads();
+        // the others, by full warps
+        for (uint32_t i = threadIdx.x; i < sm.u.far[kThreads]; i += kThreads) {
+            const uint32_t f = sm.u.far[i], in = f & 31u, base = f & ~31u, v = B.prefix[f], m = shorter(B, base, v);
+            const uint32_t mr = m & (in == 31u ? 0u : 0xFFFFFFFFu << (in + 1u)), ml = m & ((1u << in) - 1u);
+            emit(f, ml ? (int64_t)base + 31 - __clz(ml) : shorter_far(B, f, v, false),
+                 mr ? base + __ffs(mr) - 1u : shorter_far(B, f, v, true));
+        }
+        __syncthreads();
+    }
 }
 
-struct Tree {
-    uint32_t T, leafSize;
-    const uint32_t *parent, *left, *right, *first, *last, *vals;
-    const float4 *triLo, *triHi;
-    float4 *boxLo, *boxHi;
-    uint32_t* size;
-    uint32_t* arrive;
-    const float* pos;      // source vertices, 3 floats each
-    const uint32_t* idx;   // source triangles, 3 indices each
+// 5. output leaves and nodes that start in this CTA's chunk
+__device__ __forceinline__ void build_sums(const Build& B, BuildShared& sm, uint32_t cta) {
+    const uint32_t end = min(B.T, (cta + 1u) * B.chunk);
+    uint32_t leaves = 0, all = 0;
+    for (uint32_t j = cta * B.chunk + threadIdx.x; j < end; j += kThreads) {
+        const uint32_t leaf = B.leafCount[j] ? 1u : 0u;
+        leaves += leaf;
+        all += leaf + B.starts[j];
+    }
+    leaves = __reduce_add_sync(0xFFFFFFFFu, leaves);
+    all = __reduce_add_sync(0xFFFFFFFFu, all);
+    if ((threadIdx.x & 31u) == 0) sm.sum2[threadIdx.x >> 5] = make_uint2(leaves, all);
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        const uint2 x = sm.sum2[threadIdx.x];
+        const uint32_t a = __reduce_add_sync(0xFFFFFFFFu, x.x), b = __reduce_add_sync(0xFFFFFFFFu, x.y);
+        if (threadIdx.x == 0) {
+            B.part[cta * 8u + 6u] = a;
+            B.part[cta * 8u + 7u] = b;
+        }
+    }
+}
+
+struct BuildBox {
+    uint32_t lo[3], hi[3];  // f2o
 };
-
-// A leaf's bounds exactly as the refit computes them (gi_refit.js:108-113):
-// its triangles in BVH order, their vertices in index order, strict < / >
-// updates (so the sign of a zero bound matches the refit's).
-__device__ __forceinline__ void leaf_bounds(const Tree& R, uint32_t f, uint32_t l, float4& lo, float4& hi) {
-    float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
-    for (uint32_t q = f; q <= l; ++q) {
-        const uint32_t t = R.vals[q];
-        for (int k = 0; k < 3; ++k) {
-            const float* v = R.pos + 3 * (size_t)R.idx[3 * (size_t)t + k];
-            for (int a = 0; a < 3; ++a) {
-                if (v[a] < mn[a]) mn[a] = v[a];
-                if (v[a] > mx[a]) mx[a] = v[a];
-            }
-        }
-    }
-    lo = make_float4(mn[0], mn[1], mn[2], 0.0f);
-    hi = make_float4(mx[0], mx[1], mx[2], 0.0f);
+__device__ __forceinline__ BuildBox empty_box() {
+    return {{0xFFFFFFFFu, 0xFFFFFFFFu, 0xFFFFFFFFu}, {0u, 0u, 0u}};
 }
-
-__device__ __forceinline__ uint32_t count_of(const Tree& R, uint32_t node) {
-    return node < R.T - 1 ? R.last[node] - R.first[node] + 1u : 1u;
+__device__ __forceinline__ void unite(BuildBox& a, uint4 lo, uint4 hi) {
+    a.lo[0] = min(a.lo[0], lo.x); a.lo[1] = min(a.lo[1], lo.y); a.lo[2] = min(a.lo[2], lo.z);
+    a.hi[0] = max(a.hi[0], hi.x); a.hi[1] = max(a.hi[1], hi.y); a.hi[2] = max(a.hi[2], hi.z);
 }
-
-// 5. bottom-up: bounds and output sizes
-__global__ void k_climb(Tree R, uint32_t* err) {
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= R.T) return;
-    uint32_t node = R.T - 1 + j;
-    for (int level = 0;; ++level) {
-        const uint32_t p = R.parent[node];
-        if (p == kNone) break;
-        if (level >= 80) {  // deeper than any radix tree of 32-bit codes and positions
-            latch(err, ERR_LAYOUT);
-            break;
-        }
-        uint32_t prev;
-        asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(prev) : "l"(R.arrive + p) : "memory");
-        if (prev == 0u) break;
-        const uint32_t L = R.left[p], Rt = R.right[p];
-        if (p >= R.T - 1 || L >= 2 * R.T - 1 || Rt >= 2 * R.T - 1) {
-            latch(err, ERR_LAYOUT);
-            break;
-        }
-        float4 ll, lh, rl, rh;
-        uint32_t sl, sr;
-        if (L < R.T - 1) {
-            ll = __ldcg(R.boxLo + L); lh = __ldcg(R.boxHi + L); sl = __ldcg(R.size + L);
-        } else {
-            const uint32_t t = R.vals[L - (R.T - 1)];
-            ll = R.triLo[t]; lh = R.triHi[t]; sl = 1u;
-        }
-        if (Rt < R.T - 1) {
-            rl = __ldcg(R.boxLo + Rt); rh = __ldcg(R.boxHi + Rt); sr = __ldcg(R.size + Rt);
-        } else {
-            const uint32_t t = R.vals[Rt - (R.T - 1)];
-            rl = R.triLo[t]; rh = R.triHi[t]; sr = 1u;
-        }
-        if (count_of(R, p) <= R.leafSize) {  // one output leaf: bounds as the refit's leaf rule
-            float4 lo, hi;
-            leaf_bounds(R, R.first[p], R.last[p], lo, hi);
-            R.boxLo[p] = lo;
-            R.boxHi[p] = hi;
-            R.size[p] = 1u;
-        } else {                             // an interior node: the refit's union of its two children
-            R.boxLo[p] = make_float4(js_min(ll.x, rl.x), js_min(ll.y, rl.y), js_min(ll.z, rl.z), 0.0f);
-            R.boxHi[p] = make_float4(js_max(lh.x, rh.x), js_max(lh.y, rh.y), js_max(lh.z, rh.z), 0.0f);
-            R.size[p] = 1u + sl + sr;
-        }
-        node = p;
+__device__ __forceinline__ void unite_warp(BuildBox& a) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        a.lo[k] = __reduce_min_sync(0xFFFFFFFFu, a.lo[k]);
+        a.hi[k] = __reduce_max_sync(0xFFFFFFFFu, a.hi[k]);
     }
 }
-
-// 6. pre-order index and record of every output node
-__global__ void k_emit_nodes(Tree R, uint32_t* nodes, uint32_t* nodeCount, uint32_t* err) {
-    const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >= 2 * R.T - 1) return;
-    const uint32_t p0 = R.parent[x];
-    // emitted: the root, and every node whose parent is interior in the output
-    if (p0 != kNone && count_of(R, p0) <= R.leafSize) return;
-    uint32_t idx = 0u, c = x;
-    for (int level = 0;; ++level) {
-        const uint32_t a = R.parent[c];
-        if (a == kNone) break;
-        if (level >= 80) {
-            latch(err, ERR_LAYOUT);
-            return;
-        }
-        if (a >= R.T - 1) {
-            latch(err, ERR_LAYOUT);
-            return;
-        }
-        idx += 1u;
-        if (R.right[a] == c) {
-            const uint32_t L = R.left[a];
-            idx += L < R.T - 1 ? R.size[L] : 1u;
-        }
-        c = a;
-    }
-    const bool internal = x < R.T - 1;
-    float4 lo, hi;
-    uint32_t sz, payload;
-    if (internal) {
-        lo = R.boxLo[x];
-        hi = R.boxHi[x];
-        sz = R.size[x];
-        const uint32_t cnt = count_of(R, x);
-        payload = cnt <= R.leafSize ? ((cnt << 24) | R.first[x]) : 0xFFFFFFFFu;
-    } else {
-        const uint32_t j = x - (R.T - 1), t = R.vals[j];
-        lo = R.triLo[t];
-        hi = R.triHi[t];
-        sz = 1u;
-        payload = (1u << 24) | j;
-    }
-    if ((uint64_t)idx + sz > 2ull * R.T - 1ull) {  // sizes that do not add up: never write outside
-        latch(err, ERR_LAYOUT);
+__device__ __forceinline__ void store_box(const Build& B, uint32_t at, const BuildBox& b) {
+    B.boxLo[at] = make_uint4(b.lo[0], b.lo[1], b.lo[2], 0u);
+    B.boxHi[at] = make_uint4(b.hi[0], b.hi[1], b.hi[2], 0u);
+}
+__device__ __forceinline__ void store_node(const Build& B, uint32_t at, uint32_t size, const BuildBox& b,
+                                           uint32_t payload) {
+    if ((uint64_t)at + size > 2ull * B.T - 1ull) {  // sizes that do not add up: never write outside
+        latch(B.err, ERR_LAYOUT);
         return;
     }
-    uint32_t* n = nodes + 8ull * idx;
-    n[0] = __float_as_uint(lo.x); n[1] = __float_as_uint(lo.y); n[2] = __float_as_uint(lo.z);
-    n[3] = __float_as_uint(hi.x); n[4] = __float_as_uint(hi.y); n[5] = __float_as_uint(hi.z);
-    n[6] = idx + sz;
+    uint32_t* n = B.nodes + 8ull * at;
+    for (int a = 0; a < 3; ++a) {
+        n[a] = __float_as_uint(o2f(b.lo[a]));
+        n[3 + a] = __float_as_uint(o2f(b.hi[a]));
+    }
+    n[6] = at + size;
     n[7] = payload;
-    if (p0 == kNone) *nodeCount = sz;
+}
+
+// The vertices of the triangle at position q into bounds, as the refit does it:
+// in order, strict < and >.
+__device__ __forceinline__ void grow_by_triangle(const Build& B, uint32_t q, float mn[3], float mx[3]) {
+    const uint32_t t = B.order[q];
+    if (t >= B.T) return;
+    for (int k = 0; k < 3; ++k) {
+        const uint32_t v = B.idx[3 * (size_t)t + k];
+        if (v >= B.V) continue;
+        for (int x = 0; x < 3; ++x) {
+            const float y = B.pos[3 * (size_t)v + x];
+            if (y < mn[x]) mn[x] = y;
+            if (y > mx[x]) mx[x] = y;
+        }
+    }
+}
+
+// 5, 6. prefix sums of the chunk, its output leaves, and the box levels within it
+__device__ __forceinline__ void build_leaves(const Build& B, BuildShared& sm, uint32_t cta, uint32_t ctas) {
+    const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+    uint32_t leaves = 0, all = 0;  // ahead of the chunk
+    for (uint32_t c = lane; c < cta; c += 32) {
+        leaves += B.part[c * 8u + 6u];
+        all += B.part[c * 8u + 7u];
+    }
+    leaves = __reduce_add_sync(0xFFFFFFFFu, leaves);
+    all = __reduce_add_sync(0xFFFFFFFFu, all);
+    const uint32_t end = min(B.T, (cta + 1u) * B.chunk);
+    for (uint32_t base = cta * B.chunk; base < end; base += kThreads) {
+        const uint32_t j = base + threadIdx.x;
+        float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
+        if (j < end) grow_by_triangle(B, j, mn, mx);
+        for (int x = 0; x < 3; ++x) {
+            sm.u.tri[x][threadIdx.x] = mn[x];
+            sm.u.tri[3 + x][threadIdx.x] = mx[x];
+        }
+        const uint32_t cnt = j < end ? B.leafCount[j] : 0u, st = j < end ? B.starts[j] : 0u;
+        const uint32_t leaf = cnt ? 1u : 0u;
+        uint32_t nl, na;
+        const uint32_t l = leaves + block_scan(leaf, sm.sum, nl), a = all + block_scan(leaf + st, sm.sum, na);
+        leaves += nl;
+        all += na;
+        if (j < end) B.before[j] = make_uint2(l, a);
+        if (j + 1u == B.T) {
+            B.before[B.T] = make_uint2(l + leaf, a + leaf + st);
+            *B.nodeCount = a + leaf + st;
+        }
+        BuildBox b = empty_box();
+        if (leaf) {  // this position's triangle and the leaf's others; past the tile from their vertices
+            for (uint32_t i = 1; i < cnt; ++i) {
+                const uint32_t q = threadIdx.x + i;
+                if (q >= kThreads) {
+                    if (j + i < B.T) grow_by_triangle(B, j + i, mn, mx);
+                    continue;
+                }
+                for (int x = 0; x < 3; ++x) {
+                    const float lo = sm.u.tri[x][q], hi = sm.u.tri[3 + x][q];
+                    if (lo < mn[x]) mn[x] = lo;
+                    if (hi > mx[x]) mx[x] = hi;
+                }
+            }
+            for (int x = 0; x < 3; ++x) {
+                b.lo[x] = f2o(mn[x]);
+                b.hi[x] = f2o(mx[x]);
+            }
+            store_node(B, a + st, 1u, b, cnt << 24 | j);
+        }
+        if (j < end) store_box(B, j, b);
+        unite_warp(b);
+        if (lane == 0) {
+            if (j < end) store_box(B, B.levelAt[1] + (j >> 5), b);
+            for (int x = 0; x < 3; ++x) {
+                sm.lo[w][x] = b.lo[x];
+                sm.hi[w][x] = b.hi[x];
+            }
+        }
+        __syncthreads();
+        if (w == 0) {
+            for (int x = 0; x < 3; ++x) {
+                b.lo[x] = sm.lo[lane][x];
+                b.hi[x] = sm.hi[lane][x];
+            }
+            unite_warp(b);
+            if (lane == 0) store_box(B, B.levelAt[2] + (base >> 10), b);
+        }
+        __syncthreads();
+    }
+}
+
+// The prefix minima or the boxes of the levels above 1024 positions, one warp per
+// entry (one CTA).
+__device__ __forceinline__ void build_upper(const Build& B, bool boxes) {
+    const uint32_t lane = threadIdx.x & 31u, w = threadIdx.x >> 5;
+    uint32_t n = (B.T + 1023u) >> 10;
+    for (uint32_t k = 3; k <= B.levels; ++k) {
+        const uint32_t m = (n + 31u) >> 5;
+        for (uint32_t i = w; i < m; i += kWarps) {
+            const uint32_t c = 32u * i + lane, from = B.levelAt[k - 1] + c;
+            if (boxes) {
+                BuildBox b = empty_box();
+                if (c < n) unite(b, B.boxLo[from], B.boxHi[from]);
+                unite_warp(b);
+                if (lane == 0) store_box(B, B.levelAt[k] + i, b);
+            } else {
+                const uint32_t v = __reduce_min_sync(0xFFFFFFFFu, c < n ? (uint32_t)B.prefix[from] : 255u);
+                if (lane == 0) B.prefix[B.levelAt[k] + i] = (uint8_t)v;
+            }
+        }
+        __syncthreads();
+        n = m;
+    }
+}
+
+// 6. interior nodes: found one per thread, their boxes by the whole warp
+__device__ __forceinline__ void build_nodes(const Build& B, uint32_t cta, uint32_t ctas) {
+    const uint32_t lane = threadIdx.x & 31u;
+    if (B.T <= B.leafSize) return;  // the root is a leaf: no node was classified
+    for (uint32_t i0 = cta * kThreads + (threadIdx.x & ~31u); i0 + 1u < B.T; i0 += ctas * kThreads) {
+        const uint32_t i = i0 + lane;
+        const uint32_t l = i + 1u < B.T ? B.last[i] : 0u, f = l ? B.first[i] : 0u;
+        uint32_t at = 0, size = 0;
+        if (l) {
+            const uint2 from = B.before[f], to = B.before[l + 1u];
+            size = 2u * (to.x - from.x) - 1u;
+            at = from.y;
+            // the ancestors that start here too: a node is its parent's left child when
+            // the prefix after its range is longer than the one ahead of it
+            const uint32_t ahead = f ? B.prefix[f - 1u] : 0u;
+            for (uint32_t hi = l, level = 0; level < 80u && hi + 1u < B.T && B.prefix[hi] > ahead; ++level) {
+                ++at;
+                const uint32_t up = B.last[hi];
+                if (up <= hi || up >= B.T) break;
+                hi = up;
+            }
+        }
+        BuildBox b = empty_box();
+        uint32_t rest = __ballot_sync(0xFFFFFFFFu, l != 0u);
+        while (rest) {
+            const int src = __ffs(rest) - 1;
+            rest &= rest - 1u;
+            uint32_t p = __shfl_sync(0xFFFFFFFFu, f, src), q = __shfl_sync(0xFFFFFFFFu, l, src) + 1u;  // [p, q)
+            BuildBox x = empty_box();
+            for (uint32_t k = 0;; ++k) {  // the ends of the range that are not whole boxes of the next level
+                const uint32_t lv = k ? B.levelAt[k] : 0u, p2 = (p + 31u) >> 5, q2 = q >> 5;
+                if (k == B.levels || p2 >= q2) {
+                    for (uint32_t j = p + lane; j < q; j += 32) unite(x, B.boxLo[lv + j], B.boxHi[lv + j]);
+                    break;
+                }
+                if (p + lane < p2 << 5) unite(x, B.boxLo[lv + p + lane], B.boxHi[lv + p + lane]);
+                if ((q2 << 5) + lane < q) unite(x, B.boxLo[lv + (q2 << 5) + lane], B.boxHi[lv + (q2 << 5) + lane]);
+                p = p2;
+                q = q2;
+            }
+            unite_warp(x);
+            if ((int)lane == src) b = x;
+        }
+        if (l) store_node(B, at, size, b, 0xFFFFFFFFu);
+    }
+}
+
+__device__ __forceinline__ const uint32_t* pass_keys(const Build& B, uint32_t pass) { return pass & 1u ? B.keyB : B.keyA; }
+__device__ __forceinline__ uint32_t* pass_keys_out(const Build& B, uint32_t pass) { return pass & 1u ? B.keyA : B.keyB; }
+// the triangles go to `order`, to valA and to `order` again
+__device__ __forceinline__ const uint32_t* pass_vals(const Build& B, uint32_t pass) {
+    return pass == 0 ? nullptr : pass == 1 ? B.order : B.valA;
+}
+__device__ __forceinline__ uint32_t* pass_vals_out(const Build& B, uint32_t pass) { return pass == 1 ? B.valA : B.order; }
+
+// All phases by one cluster.
+__global__ void __launch_bounds__(kThreads) k_build_cluster(const __grid_constant__ Build B) {
+    extern __shared__ uint4 smem[];
+    BuildShared& sm = *reinterpret_cast<BuildShared*>(smem);
+    const cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    const uint32_t cta = cluster.block_rank(), ctas = cluster.num_blocks();
+    cudaTriggerProgrammaticLaunchCompletion();  // as in k_build_phase
+    cudaGridDependencySynchronize();
+    auto sync = [&] {
+        if (ctas > 1) cluster.sync();
+        else __syncthreads();
+    };
+    build_centres(B, sm, cta, ctas);
+    sync();
+    build_codes(B, sm, cta, ctas);
+    __syncthreads();
+    for (uint32_t pass = 0; pass < 3; ++pass) {
+        build_count(B, sm, cta, pass_keys(B, pass), pass * kBits);
+        sync();
+        build_place(B, sm, cta, ctas, pass_keys(B, pass), pass_vals(B, pass), pass * kBits, pass_keys_out(B, pass),
+                    pass_vals_out(B, pass));
+        sync();
+    }
+    build_prefixes(B, sm, pass_keys(B, 3), cta);
+    sync();
+    build_tree(B, sm, cta, ctas);
+    sync();
+    build_sums(B, sm, cta);
+    sync();
+    build_leaves(B, sm, cta, ctas);
+    sync();
+    build_nodes(B, cta, ctas);
+}
+
+// One phase per launch.
+enum : uint32_t { PHASE_CENTRES, PHASE_SORT, PHASE_PREFIXES = PHASE_SORT + 6, PHASE_UPPER, PHASE_TREE, PHASE_SUMS,
+                  PHASE_LEAVES, PHASE_UPPER_BOXES, PHASE_NODES, PHASES };
+__global__ void __launch_bounds__(kThreads) k_build_phase(const __grid_constant__ Build B, uint32_t phase) {
+    extern __shared__ uint4 smem[];
+    BuildShared& sm = *reinterpret_cast<BuildShared*>(smem);
+    const uint32_t cta = blockIdx.x, ctas = gridDim.x;
+    // the next phase's CTAs may be placed while this one's run; each waits here until
+    // the launches ahead of it are complete
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
+    if (phase == PHASE_CENTRES) {
+        build_centres(B, sm, cta, ctas);
+    } else if (phase < PHASE_PREFIXES) {  // count, then count and place, of the three passes
+        const uint32_t pass = (phase - PHASE_SORT) / 2u;
+        if (phase == PHASE_SORT) {
+            build_codes(B, sm, cta, ctas);
+            __syncthreads();
+        }
+        build_count(B, sm, cta, pass_keys(B, pass), pass * kBits);
+        if (phase - PHASE_SORT & 1u) {
+            __syncthreads();
+            build_place(B, sm, cta, ctas, pass_keys(B, pass), pass_vals(B, pass), pass * kBits,
+                        pass_keys_out(B, pass), pass_vals_out(B, pass));
+        }
+    } else if (phase == PHASE_PREFIXES) {
+        build_prefixes(B, sm, pass_keys(B, 3), cta);
+    } else if (phase == PHASE_TREE) {
+        build_tree(B, sm, cta, ctas);
+    } else if (phase == PHASE_SUMS) {
+        build_sums(B, sm, cta);
+    } else if (phase == PHASE_LEAVES) {
+        build_leaves(B, sm, cta, ctas);
+    } else if (phase == PHASE_UPPER || phase == PHASE_UPPER_BOXES) {
+        build_upper(B, phase == PHASE_UPPER_BOXES);
+    } else {
+        build_nodes(B, cta, ctas);
+    }
 }
 
 template <class Tp> cudaError_t grow(Tp*& p, size_t& cap, size_t n) {
@@ -410,40 +685,11 @@ template <class Tp> cudaError_t grow(Tp*& p, size_t& cap, size_t n) {
 }  // namespace
 
 struct BlasBuilder {
-    float4 *triLo = nullptr, *triHi = nullptr, *boxLo = nullptr, *boxHi = nullptr;
-    uint32_t *keyA = nullptr, *keyB = nullptr, *valA = nullptr, *valB = nullptr, *hist = nullptr;
-    uint32_t *cbox = nullptr, *parent = nullptr, *left = nullptr, *right = nullptr, *first = nullptr,
-             *last = nullptr, *arrive = nullptr, *size = nullptr;
-    size_t cT = 0, cT2 = 0, cK = 0, cH = 0, cN = 0, cBox = 0, cI = 0, cI2 = 0, cC = 0;
-    size_t cA = 0, cB = 0, cV = 0, cW = 0, cP = 0, cL = 0, cR = 0, cF = 0, cLa = 0, cAr = 0, cS = 0;
-
-    cudaError_t reserve(uint32_t T) {
-        const size_t tiles = (T + kTile - 1) / kTile;
-        cudaError_t e = cudaSuccess;
-        if (e == cudaSuccess) e = grow(triLo, cT, T);
-        if (e == cudaSuccess) e = grow(triHi, cT2, T);
-        if (e == cudaSuccess) e = grow(boxLo, cBox, T);
-        if (e == cudaSuccess) e = grow(boxHi, cN, T);
-        if (e == cudaSuccess) e = grow(keyA, cA, T);
-        if (e == cudaSuccess) e = grow(keyB, cB, T);
-        if (e == cudaSuccess) e = grow(valA, cV, T);
-        if (e == cudaSuccess) e = grow(valB, cW, T);
-        if (e == cudaSuccess) e = grow(hist, cH, 256 * tiles);
-        if (e == cudaSuccess) e = grow(cbox, cC, 6);
-        if (e == cudaSuccess) e = grow(parent, cP, 2 * (size_t)T);
-        if (e == cudaSuccess) e = grow(left, cL, T);
-        if (e == cudaSuccess) e = grow(right, cR, T);
-        if (e == cudaSuccess) e = grow(first, cF, T);
-        if (e == cudaSuccess) e = grow(last, cLa, T);
-        if (e == cudaSuccess) e = grow(arrive, cAr, T);
-        if (e == cudaSuccess) e = grow(size, cS, T);
-        return e;
-    }
+    uint8_t* scratch = nullptr;  // grows to the largest mesh built
+    size_t cap = 0;
+    bool ready = false;          // kernel attributes set
     ~BlasBuilder() {
-        for (void* p : {(void*)triLo, (void*)triHi, (void*)boxLo, (void*)boxHi, (void*)keyA, (void*)keyB,
-                        (void*)valA, (void*)valB, (void*)hist, (void*)cbox, (void*)parent, (void*)left,
-                        (void*)right, (void*)first, (void*)last, (void*)arrive, (void*)size})
-            if (p) cudaFree(p);
+        if (scratch) cudaFree(scratch);
     }
 };
 
@@ -454,40 +700,102 @@ cudaError_t blas_build(BlasBuilder* b, const float* pos, uint32_t V, const uint3
                        uint32_t leafSize, uint32_t* nodes, uint32_t* order, uint32_t* nodeCount, uint32_t* err,
                        cudaStream_t st) {
     if (T == 0) return cudaSuccess;
-    cudaError_t e = b->reserve(T);
+    Build B{};
+    B.pos = pos;
+    B.idx = idx;
+    B.V = V;
+    B.T = T;
+    B.leafSize = leafSize;
+    B.order = order;
+    B.nodes = nodes;
+    B.nodeCount = nodeCount;
+    B.err = err;
+    // box levels: 1 per position, 32, 1024, ... positions until at most 32 boxes are left
+    uint32_t boxes = (T + 31u) & ~31u, n = T;
+    for (uint32_t k = 1; k < 5; ++k) {
+        B.levelAt[k] = boxes;
+        n = (n + 31u) / 32u;
+        boxes += (n + 31u) & ~31u;
+        B.levels = k;
+        if (k >= 2 && n <= 32u) break;
+    }
+    // scratch, laid out 256-byte aligned; the first call sizes, the second places
+    uint8_t* base = nullptr;
+    size_t at = 0;
+    auto place = [&](auto*& p, size_t count) {
+        p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(base + at);
+        at += (count * sizeof(*p) + 255) & ~size_t(255);
+    };
+    auto layout = [&] {
+        at = 0;
+        place(B.centre, T);
+        place(B.part, kMaxCtas * 8);
+        place(B.keyA, T);
+        place(B.keyB, T);
+        place(B.valA, T);
+        place(B.hist, kSortCtas * kDigits);
+        place(B.prefix, boxes);
+        place(B.first, T);
+        place(B.last, T);
+        place(B.starts, T);
+        place(B.leafCount, T);
+        place(B.before, (size_t)T + 1);
+        place(B.boxLo, boxes);
+        place(B.boxHi, boxes);
+    };
+    layout();
+    cudaError_t e = grow(b->scratch, b->cap, at);
     if (e != cudaSuccess) return e;
-    const uint32_t tiles = (T + kTile - 1) / kTile;
-    const unsigned g = (T + 255) / 256;
-    // centroid bounds start empty: min words at the largest ordered value, max at 0
-    if ((e = cudaMemsetAsync(b->cbox, 0xFF, 3 * sizeof(uint32_t), st)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(b->cbox + 3, 0, 3 * sizeof(uint32_t), st)) != cudaSuccess) return e;
-    k_tri_bounds<<<g, 256, 0, st>>>(pos, V, idx, T, b->triLo, b->triHi, b->cbox, err); note_launch();
-    k_morton<<<g, 256, 0, st>>>(b->triLo, b->triHi, T, b->cbox, b->keyA, b->valA); note_launch();
-    uint32_t *kin = b->keyA, *vin = b->valA, *kout = b->keyB, *vout = b->valB;
-    for (uint32_t shift = 0; shift < 32; shift += 8) {
-        k_sort_hist<<<tiles, kSortThreads, 0, st>>>(kin, T, shift, b->hist, tiles); note_launch();
-        k_scan<<<1, 1024, 0, st>>>(b->hist, 256 * tiles); note_launch();
-        k_sort_scatter<<<tiles, kSortThreads, 0, st>>>(kin, vin, T, shift, b->hist, tiles, kout, vout); note_launch();
-        std::swap(kin, kout);
-        std::swap(vin, vout);
+    base = b->scratch;
+    layout();
+    const int smem = (int)sizeof(BuildShared);
+    if (!b->ready) {
+        for (const void* f : {(const void*)k_build_cluster, (const void*)k_build_phase})
+            if ((e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
+        b->ready = true;
     }
-    // after 4 passes the sorted keys and triangles are back in keyA / valA
-    if ((e = cudaMemcpyAsync(order, vin, (size_t)T * 4, cudaMemcpyDeviceToDevice, st)) != cudaSuccess) return e;
-    if (T == 1) {
-        // one triangle: the root is a leaf
-        Tree R{T, leafSize, b->parent, b->left, b->right, b->first, b->last, vin, b->triLo, b->triHi, b->boxLo,
-               b->boxHi, b->size, b->arrive, pos, idx};
-        if ((e = cudaMemsetAsync(b->parent, 0xFF, sizeof(uint32_t), st)) != cudaSuccess) return e;  // no parent
-        k_emit_nodes<<<1, 32, 0, st>>>(R, nodes, nodeCount, err); note_launch();
-        return cudaGetLastError();
+    if (T <= BUILD_CLUSTER_TRIS) {
+        B.levels = 2;  // up to 64 boxes of 1024 positions
+        uint32_t ctas = 1;
+        while (ctas < 8 && ctas * kThreads < T) ctas *= 2;
+        B.chunk = ((T + ctas - 1) / ctas + kThreads - 1) / kThreads * kThreads;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(ctas);
+        cfg.blockDim = dim3(kThreads);
+        cfg.dynamicSmemBytes = (size_t)smem;
+        cfg.stream = st;
+        cudaLaunchAttribute attr[2] = {};
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = ctas;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 2;
+        e = cudaLaunchKernelEx(&cfg, k_build_cluster, B);
+        note_launch();
+        return e != cudaSuccess ? e : cudaGetLastError();
     }
-    if ((e = cudaMemsetAsync(b->arrive, 0, (size_t)(T - 1) * 4, st)) != cudaSuccess) return e;
-    k_radix_tree<<<(T - 1 + 255) / 256, 256, 0, st>>>(kin, T, b->parent, b->left, b->right, b->first, b->last, err);
-    note_launch();
-    Tree R{T, leafSize, b->parent, b->left, b->right, b->first, b->last, vin, b->triLo, b->triHi, b->boxLo,
-           b->boxHi, b->size, b->arrive, pos, idx};
-    k_climb<<<g, 256, 0, st>>>(R, err); note_launch();
-    k_emit_nodes<<<(2 * T - 1 + 255) / 256, 256, 0, st>>>(R, nodes, nodeCount, err); note_launch();
+    cudaLaunchAttribute serial{};
+    serial.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    serial.val.programmaticStreamSerializationAllowed = 1;
+    for (uint32_t phase = 0; phase < PHASES; ++phase) {
+        const bool upper = phase == PHASE_UPPER || phase == PHASE_UPPER_BOXES;
+        const bool sort = phase >= PHASE_SORT && phase < PHASE_PREFIXES;
+        if (upper && B.levels < 3) continue;
+        const uint32_t most = phase < PHASE_PREFIXES ? kSortCtas : kMaxCtas;
+        const uint32_t ctas = std::min(most, (T + kThreads - 1u) / kThreads);
+        B.chunk = ((T + ctas - 1) / ctas + kThreads - 1) / kThreads * kThreads;
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(upper ? 1u : ctas);
+        cfg.blockDim = dim3(kThreads);
+        cfg.dynamicSmemBytes = sort ? (size_t)smem : offsetof(BuildShared, cnt);
+        cfg.stream = st;
+        cfg.attrs = &serial;
+        cfg.numAttrs = phase == 0 ? 0 : 1;
+        if ((e = cudaLaunchKernelEx(&cfg, k_build_phase, B, phase)) != cudaSuccess) return e;
+        note_launch();
+    }
     return cudaGetLastError();
 }
 
