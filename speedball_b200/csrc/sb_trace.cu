@@ -3,7 +3,7 @@
 //
 //   A  k_trace_primary  closest hit per probe ray (traverseClosest) -> raw
 //                       16-byte hit record.
-//      k_emit           per ray: hit t in double-float, hit frame, and the NEE
+//      k_emit           per ray: hit t in FP64, hit frame, and the NEE
 //                       pre-tests per candidate light (the reference's
 //                       ndl * peak > 0 and range gates); passing candidates
 //                       become shadow-ray jobs, one atomic per warp.
@@ -249,7 +249,7 @@ __device__ __forceinline__ void shadow_walk8(const WaveCtx& W, const WalkSmem& m
 }
 
 // Stage A2, warp-collective (all 32 lanes call it; `active` lanes hold ray g):
-// the hit parameter re-evaluated in double-float, the hit frame, and the NEE
+// the hit parameter re-evaluated in FP64, the hit frame, and the NEE
 // gates of every candidate light. Each lane runs the gates with no warp sync;
 // one warp scan and one atomicAdd then reserve the warp's shadow-ray jobs, and
 // each ray's passing candidates (gates evaluated again: the same pure
@@ -894,7 +894,7 @@ __global__ void __launch_bounds__(256, QUERY_MIN_BLOCKS) k_query_walk8(DevScene 
     walk8<ANY>(S, *m.tables, *m.w8, m.stk, S.wideDepth + 1u, gen, fin, vis, err);
 }
 
-// The hits' parameters in double-float (refine_t), one thread per ray.
+// The hits' parameters in FP64 (refine_t), one thread per ray.
 __global__ void k_refine_hits(DevScene S, const float* ro, const float* rd, uint32_t n, float* t, const int32_t* tri,
                               const int32_t* inst) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;

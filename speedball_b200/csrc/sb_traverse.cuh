@@ -1,5 +1,5 @@
 // sb_traverse.cuh — the closest-hit and any-hit queries (traverseClosest /
-// traverseAny, spectral_traverse.js:354-569), the double-float refinement of
+// traverseAny, spectral_traverse.js:354-569), the FP64 re-evaluation of
 // the final hit parameter, and the one-bounce atlas read (sampleAtlas,
 // gi_probes.js:1941-1974). The default walk is the 8-wide scene BVH's
 // (sb_walk8.cuh); the walks here answer the same query on the other layouts:
@@ -721,33 +721,35 @@ __device__ __forceinline__ bool trace_any(const DevScene& S, const uint4* tl, fl
 #endif
 }
 
-// The chosen hit's ray parameter re-evaluated in double-float: the same
-// Möller–Trumbore expression (spectral_traverse.js:396-408) on the local ray
-// (instLocalRay, 149-153), with the edges taken exactly from the pooled
-// vertices. FP32 alone loses ~1e-5 relative on near hits (the local origin is
-// rounded at scene scale); this keeps t within ~1e-7 of the exact value.
+// The chosen hit's ray parameter re-evaluated in FP64: the same Möller–Trumbore
+// expression (spectral_traverse.js:396-408) on the local ray (instLocalRay,
+// 149-153), with the edges taken from the pooled vertices. FP32 alone loses ~1e-5
+// relative on near hits (the local origin is rounded at scene scale); this keeps t
+// within ~1e-7 of the exact value.
 static __device__ float refine_t(const DevScene& S, uint32_t tri, uint32_t inst, float3 wro, float3 wrd) {
-    float4 r[3] = {__ldg(S.inst + 4 * inst), __ldg(S.inst + 4 * inst + 1), __ldg(S.inst + 4 * inst + 2)};
-    dfl lo[3], ld[3];
+    double o[3], d[3], v[3][3];
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
-        lo[k] = df_add(df_add(df_add(two_prod(r[k].x, wro.x), two_prod(r[k].y, wro.y)), two_prod(r[k].z, wro.z)),
-                       df(r[k].w));
-        ld[k] = df_add(df_add(two_prod(r[k].x, wrd.x), two_prod(r[k].y, wrd.y)), two_prod(r[k].z, wrd.z));
-    }
-    const float* p[3];
+        const float4 r = __ldg(S.inst + 4 * inst + k);
+        o[k] = (double)r.x * wro.x + (double)r.y * wro.y + (double)r.z * wro.z + (double)r.w;
+        d[k] = (double)r.x * wrd.x + (double)r.y * wrd.y + (double)r.z * wrd.z;
+        const float* p = S.vertexData + (size_t)__ldg(S.triIndex + 3 * tri + k) * 8u;
 #pragma unroll
-    for (int k = 0; k < 3; ++k) p[k] = S.vertexData + (size_t)__ldg(S.triIndex + 3 * tri + k) * 8u;
-    df3 p0 = {df(__ldg(p[0])), df(__ldg(p[0] + 1)), df(__ldg(p[0] + 2))};
-    df3 p1 = {df(__ldg(p[1])), df(__ldg(p[1] + 1)), df(__ldg(p[1] + 2))};
-    df3 p2 = {df(__ldg(p[2])), df(__ldg(p[2] + 1)), df(__ldg(p[2] + 2))};
-    df3 e1 = df3_sub(p1, p0), e2 = df3_sub(p2, p0);
-    df3 o = {lo[0], lo[1], lo[2]}, d = {ld[0], ld[1], ld[2]};
-    df3 pv = df3_cross(d, e2);
-    dfl det = df3_dot(e1, pv);
-    df3 tv = df3_sub(o, p0);
-    df3 qv = df3_cross(tv, e1);
-    return df_div(df3_dot(e2, qv), det);
+        for (int a = 0; a < 3; ++a) v[k][a] = __ldg(p + a);
+    }
+    double e1[3], e2[3], tv[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        e1[a] = v[1][a] - v[0][a];
+        e2[a] = v[2][a] - v[0][a];
+        tv[a] = o[a] - v[0][a];
+    }
+    // det = e1 . (d x e2), t = e2 . (tv x e1) / det
+    const double det = e1[0] * (d[1] * e2[2] - d[2] * e2[1]) + e1[1] * (d[2] * e2[0] - d[0] * e2[2]) +
+                       e1[2] * (d[0] * e2[1] - d[1] * e2[0]);
+    const double num = e2[0] * (tv[1] * e1[2] - tv[2] * e1[1]) + e2[1] * (tv[2] * e1[0] - tv[0] * e1[2]) +
+                       e2[2] * (tv[0] * e1[1] - tv[1] * e1[0]);
+    return (float)(num / det);
 }
 
 // sampleAtlas, gi_probes.js:1941-1974: 8-tap trilinear over the cage probes,
