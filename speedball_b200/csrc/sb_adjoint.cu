@@ -404,7 +404,7 @@ cudaError_t launch_blend_bwd(const DevCascade& C, const DevParams& P, const floa
 
 // The 32 texel taps of sample_atlas (8 cage probes x bilinear 2x2) with their
 // normalised weights: sample = sum_i w_i * atlas[texel_i].
-__device__ __forceinline__ void atlas_taps(const DevCascade& C, float3 P, float3 N, uint32_t* idx, float* wt) {
+__device__ __forceinline__ void atlas_taps(const DevCascade& C, float3 P, float3 N, uint32_t* idx, uint32_t* foot, float* wt) {
     float3 cell = mk(C.gridSize[0] / fmaxf(1.0f, float(C.res[0]) - 1.0f),
                      C.gridSize[1] / fmaxf(1.0f, float(C.res[1]) - 1.0f),
                      C.gridSize[2] / fmaxf(1.0f, float(C.res[2]) - 1.0f));
@@ -431,6 +431,8 @@ __device__ __forceinline__ void atlas_taps(const DevCascade& C, float3 P, float3
         float wz = dz ? frac[2] : 1.0f - frac[2];
         float w = wx * wy * wz + 1e-4f;
         const uint32_t t = ((uint32_t)pz * C.res[1] + (uint32_t)py) * 8u * Wu + (uint32_t)px * 8u + off;
+        foot[i] = (((uint32_t)pz * C.res[1] + (uint32_t)py) * C.res[0] + (uint32_t)px) * FOOT + (uint32_t)fy0 * 7u +
+                  (uint32_t)fx0;
         idx[4 * i] = t;
         idx[4 * i + 1] = t + 1u;
         idx[4 * i + 2] = t + Wu;
@@ -497,12 +499,13 @@ __global__ void __launch_bounds__(SHADE_BWD_THREADS) k_shade_bwd(WaveCtx W, cons
                 else atomicAdd(&gParam[6u * mc + li], (double)gl);
             }
             // bounce = sample (.) kd / pi, scaled by roll = C / max(C, luma(bounce))
-            uint32_t idx[32];
+            uint32_t idx[32], foot[8];
             float wt[32];
-            atlas_taps(C, fr.hitPos, fr.ng, idx, wt);
+            atlas_taps(C, fr.hitPos, fr.ng, idx, foot, wt);
             float3 smp = mk(0.f, 0.f, 0.f);
 #pragma unroll
-            for (int i = 0; i < 32; ++i) smp = smp + xyz(half4_to_float4(__ldg(C.atlasPrev + idx[i]))) * wt[i];
+            for (int i = 0; i < 8; ++i)
+                smp = smp + foot_rgb(C.footPrev, foot[i], make_float4(wt[4 * i], wt[4 * i + 1], wt[4 * i + 2], wt[4 * i + 3]));
             const float3 bounce = mul3(smp, kd) * (1.0f / PI_F);
             const float bl = luma3(bounce);
             const float Cc = P.radianceClamp;

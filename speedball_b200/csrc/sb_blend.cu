@@ -43,7 +43,20 @@ template <bool ROUGH> struct BlendSmem {
     float2 dep[BLEND_PROBES][BLEND_TEXELS];
     float4 rough[ROUGH ? BLEND_PROBES : 1][BLEND_TEXELS];  // blended rough history
     float wsum[BLEND_TEXELS], dwsum[BLEND_TEXELS], swsum[BLEND_TEXELS];  // the same for every probe
+    uint8_t src[TILE * TILE];  // the interior texel each texel of a tile shows
 };
+
+// Interior + canonical mirrored gutter (gi_probes.js:2816-2839): the interior texel
+// (row-major in OCT x OCT) that texel `texel` of a tile shows.
+__device__ __forceinline__ uint32_t tile_source(uint32_t texel) {
+    const int edge = TILE - 1, lo = BORDER, hi = BORDER + OCT - 1;
+    const int lx = (int)(texel % TILE), ly = (int)(texel / TILE);
+    const bool onLeft = lx == 0, onRight = lx == edge, onTop = ly == 0, onBottom = ly == edge;
+    const bool colB = onLeft || onRight, rowB = onTop || onBottom, corner = colB && rowB;
+    const int sx = corner ? (onLeft ? hi : lo) : (rowB ? edge - lx : (colB ? (onLeft ? lo : hi) : lx));
+    const int sy = corner ? (onTop ? hi : lo) : (rowB ? (onTop ? lo : hi) : (colB ? edge - ly : ly));
+    return (uint32_t)((sy - BORDER) * OCT + (sx - BORDER));
+}
 
 // Blend + upload of probe slots [block * BLEND_PROBES, + BLEND_PROBES) of one
 // solve; the body of the per-solve and the batched kernels.
@@ -62,6 +75,7 @@ __device__ __forceinline__ void blend_upload_block(const DevCascade& C, const De
     const bool cosUnit = cosPow == 1.0f;  // pow(x, 1) == x exactly
     const uint32_t sharpN = (uint32_t)P.depthSharpness;
     const bool sharpInt = P.depthSharpness >= 1.0f && P.depthSharpness <= 16.0f && float(sharpN) == P.depthSharpness;
+    if (tid < TILE * TILE) S.src[tid] = (uint8_t)tile_source((uint32_t)tid);
     if (tid < BLEND_TEXELS) {
         float u = (float(tid % OCT) + 0.5f) / 6.0f, v = (float(tid / OCT) + 0.5f) / 6.0f;
         float3 d = oct_decode(u, v);
@@ -296,17 +310,11 @@ __device__ __forceinline__ void blend_upload_block(const DevCascade& C, const De
     }
     __syncthreads();
 
-    // 64 texels per probe: interior + canonical mirrored gutter (gi_probes.js:2816-2839)
+    // 64 texels per probe
     for (uint32_t e = tid; e < nProbes * 64u; e += BLEND_THREADS) {
         const uint32_t q = e / 64u, texel = e % 64u;
         const uint32_t probeIndex = (C.probeOffset + base + q) % C.probeTotal;
-        const int edge = TILE - 1, lo = BORDER, hi = BORDER + OCT - 1;
-        int lx = (int)(texel % TILE), ly = (int)(texel / TILE);
-        bool onLeft = lx == 0, onRight = lx == edge, onTop = ly == 0, onBottom = ly == edge;
-        bool colB = onLeft || onRight, rowB = onTop || onBottom, corner = colB && rowB;
-        int sx = corner ? (onLeft ? hi : lo) : (rowB ? edge - lx : (colB ? (onLeft ? lo : hi) : lx));
-        int sy = corner ? (onTop ? hi : lo) : (rowB ? (onTop ? lo : hi) : (colB ? edge - ly : ly));
-        int src = (sy - BORDER) * OCT + (sx - BORDER);
+        const uint32_t lx = texel % TILE, ly = texel / TILE, src = S.src[texel];
         uint32_t col = probeIndex % C.res[0];
         uint32_t row = (probeIndex / (C.res[0] * C.res[1])) * C.res[1] + (probeIndex / C.res[0]) % C.res[1];
         size_t t = (size_t)(row * TILE + ly) * C.atlasW + col * TILE + lx;
@@ -314,6 +322,22 @@ __device__ __forceinline__ void blend_upload_block(const DevCascade& C, const De
         float2 d = S.dep[q][src];
         C.depthAtlas[t] = float4_to_half4(make_float4(d.x, d.y, 0.0f, 1.0f));
         if (ROUGH) C.roughAtlas[t] = float4_to_half4(S.rough[q][src]);  // unfiltered (gi_probes.js:2789-2795, 2841-2843)
+    }
+    // and the 49 footprints of the same texels, for the one-bounce read and the receivers
+    for (uint32_t e = tid; e < nProbes * FOOT; e += BLEND_THREADS) {
+        const uint32_t q = e / FOOT, f = e % FOOT;
+        const uint32_t at = ((C.probeOffset + base + q) % C.probeTotal) * FOOT + f;
+        const uint32_t c = (f / 7u) * TILE + f % 7u;  // its first texel
+        const uint32_t s0 = S.src[c], s1 = S.src[c + 1u], s2 = S.src[c + TILE], s3 = S.src[c + TILE + 1u];
+        store_foot(C.foot, at, float4_to_half4(S.u.out[q][s0]), float4_to_half4(S.u.out[q][s1]),
+                   float4_to_half4(S.u.out[q][s2]), float4_to_half4(S.u.out[q][s3]));
+        const float2 d0 = S.dep[q][s0], d1 = S.dep[q][s1], d2 = S.dep[q][s2], d3 = S.dep[q][s3];
+        const uint2 lo = float4_to_half4(make_float4(d0.x, d0.y, d1.x, d1.y)),
+                    hi = float4_to_half4(make_float4(d2.x, d2.y, d3.x, d3.y));
+        C.footDepth[at] = make_uint4(lo.x, lo.y, hi.x, hi.y);
+        if (ROUGH)
+            store_foot(C.footRough, at, float4_to_half4(S.rough[q][s0]), float4_to_half4(S.rough[q][s1]),
+                       float4_to_half4(S.rough[q][s2]), float4_to_half4(S.rough[q][s3]));
     }
 }
 
@@ -577,9 +601,26 @@ __global__ void k_clear_cascade(DevCascade C) {
     }
 }
 
+// The footprints of the atlases as they are (a host upload, a clear).
+__global__ void k_footprints(DevCascade C) {
+    const uint32_t at = blockIdx.x * blockDim.x + threadIdx.x;
+    if (at >= C.probeTotal * FOOT) return;
+    const uint32_t probe = at / FOOT, f = at % FOOT;
+    const uint32_t col = probe % C.res[0], row = (probe / (C.res[0] * C.res[1])) * C.res[1] + (probe / C.res[0]) % C.res[1];
+    const size_t t = (size_t)(row * TILE + f / 7u) * C.atlasW + col * TILE + f % 7u, W = C.atlasW;
+    store_foot(C.foot, at, C.atlas[t], C.atlas[t + 1], C.atlas[t + W], C.atlas[t + W + 1]);
+    C.footDepth[at] = make_uint4(C.depthAtlas[t].x, C.depthAtlas[t + 1].x, C.depthAtlas[t + W].x, C.depthAtlas[t + W + 1].x);
+}
+
+cudaError_t launch_footprints(const DevCascade& C, cudaStream_t st) {
+    const uint32_t n = C.probeTotal * FOOT;
+    k_footprints<<<(n + 255) / 256, 256, 0, st>>>(C); note_launch();
+    return cudaGetLastError();
+}
+
 cudaError_t launch_clear_cascade(const DevCascade& C, cudaStream_t st) {
     k_clear_cascade<<<148 * 4, 256, 0, st>>>(C); note_launch();
-    return cudaGetLastError();
+    return launch_footprints(C, st);
 }
 
 }  // namespace sb

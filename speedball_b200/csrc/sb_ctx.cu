@@ -14,6 +14,7 @@
 
 #include "sb_flat_scene.cuh"
 #include "sb_kernels.cuh"
+#include "sb_math.cuh"
 
 using namespace sb;
 
@@ -33,6 +34,7 @@ struct Cascade {
     float2* depth = nullptr;
     uint2* atlas = nullptr;
     uint2* depthAtlas = nullptr;
+    uint4 *foot = nullptr, *footDepth = nullptr, *footRough = nullptr;  // the atlases' footprints (sb_math.cuh)
     float4* rayData = nullptr;
     uint4* hits = nullptr;
     uint4* vis = nullptr;
@@ -161,7 +163,7 @@ struct sb_ctx {
         uint4* hits = nullptr; size_t hitsCap = 0;       // solves x probes x rays
         uint4* vis = nullptr; size_t visCap = 0;
         float4* hist = nullptr; size_t histCap = 0;      // (solves + 1) x probes x 64: history before each solve
-        uint2* atlas = nullptr; size_t atlasCap = 0;     // solves x texels: the atlas each solve's bounce reads
+        uint4* foot = nullptr; size_t footCap = 0;       // per solve: the footprints its bounce reads
         float4* E = nullptr; size_t ECap = 0;            // probes x 36: last solve's upload output
         float4* gE = nullptr; size_t gECap = 0;
         float* target = nullptr; size_t targetCap = 0;   // probes x 36 x 3
@@ -282,8 +284,10 @@ DevCascade dev_cascade(const sb_ctx* c, uint32_t ci, uint32_t probeOffset, uint3
     D.vis = K.vis;
     D.irr = K.irr;
     D.depth = K.depth;
-    D.atlasPrev = K.atlas;
+    D.footPrev = K.foot;
     D.atlas = K.atlas;
+    D.foot = K.foot;
+    D.footDepth = K.footDepth;
     D.depthAtlas = K.depthAtlas;
     D.eOut = c->recordE;
     D.lights = c->B.lights;
@@ -293,6 +297,7 @@ DevCascade dev_cascade(const sb_ctx* c, uint32_t ci, uint32_t probeOffset, uint3
     D.reflect = K.reflTier;
     D.roughSpec = K.roughSpec;
     D.roughAtlas = K.roughAtlas;
+    D.footRough = K.footRough;
     D.glossyNum = K.glossyNum;
     D.glossyDen = K.glossyDen;
     D.glossyAtlas = K.glossyAtlas;
@@ -311,7 +316,7 @@ DevCascade dev_cascade(const sb_ctx* c, uint32_t ci, uint32_t probeOffset, uint3
 // and glossy atlases to vec4(0) (clearAtlasKernel / clearGlossyAtlasKernel,
 // 2703-2724). The glossy phase restarts at 0.
 sb_status alloc_reflection(sb_ctx* ctx, Cascade& K) {
-    release(K.roughSpec); release(K.roughAtlas); release(K.glossyNum); release(K.glossyDen);
+    release(K.roughSpec); release(K.roughAtlas); release(K.footRough); release(K.glossyNum); release(K.glossyDen);
     release(K.glossyAtlas);
     const uint32_t tier = ctx->reflectTier, P = K.probeTotal;
     K.reflTier = tier;
@@ -326,6 +331,9 @@ sb_status alloc_reflection(sb_ctx* ctx, Cascade& K) {
     const size_t texels = (size_t)P * 64u;
     CK(grow(K.roughSpec, c, texels)); c = 0;
     CK(grow(K.roughAtlas, c, texels)); c = 0;
+    const size_t foot = (size_t)P * FOOT * FOOT_U4;
+    CK(grow(K.footRough, c, foot)); c = 0;
+    CK(cudaMemsetAsync(K.footRough, 0, foot * sizeof(uint4), ctx->stream));
     CK(cudaMemsetAsync(K.roughSpec, 0, texels * sizeof(float4), ctx->stream));
     CK(cudaMemsetAsync(K.roughAtlas, 0, texels * sizeof(uint2), ctx->stream));
     if (tier >= SB_REFLECT_HIGH) {
@@ -511,6 +519,7 @@ void sb_destroy(sb_ctx* ctx) {
         release(K.tileOrder); release(K.batchCost); release(K.batchOrder);
         release(K.vis);
         release(K.roughSpec); release(K.roughAtlas); release(K.glossyNum); release(K.glossyDen);
+        release(K.foot); release(K.footDepth); release(K.footRough);
         release(K.glossyAtlas);
     }
     release(ctx->jobs);
@@ -521,7 +530,7 @@ void sb_destroy(sb_ctx* ctx) {
     for (cudaEvent_t e : G.joins) cudaEventDestroy(e);
     if (G.fork) cudaEventDestroy(G.fork);
     auto& T = ctx->tape;
-    release(T.hits); release(T.vis); release(T.hist); release(T.atlas); release(T.E); release(T.gE);
+    release(T.hits); release(T.vis); release(T.hist); release(T.foot); release(T.E); release(T.gE);
     release(T.target); release(T.shaded); release(T.gR); release(T.gH); release(T.gA); release(T.gParam);
     release(T.loss);
     for (cudaEvent_t e : {T.evF0, T.evF1, T.evB0, T.evB1})
@@ -698,6 +707,8 @@ sb_status sb_upload_range(sb_ctx* ctx, uint32_t which, uint32_t start, uint32_t 
     if (!dst) return fail(ctx, SB_ERR_NOT_READY, "buffer %u not allocated", buf);
     if ((size_t)start + count > len) return fail(ctx, SB_ERR_INVALID_ARG, "range [%u,+%u) outside %zu", start, count, len);
     CK(cudaMemcpyAsync((char*)dst + (size_t)start * esz, src, (size_t)count * esz, cudaMemcpyHostToDevice, ctx->stream));
+    if (buf == SB_BUF_IRRADIANCE_ATLAS || buf == SB_BUF_DEPTH_ATLAS)
+        CK(launch_footprints(dev_cascade(ctx, ci, 0, 0), ctx->stream));
     ++ctx->epoch;
     if (buf <= SB_BUF_MATERIALS && !(buf == SB_BUF_MATERIALS && shading_only(B, start, count))) {
         ++ctx->structGen;
@@ -861,6 +872,7 @@ sb_status sb_configure_cascade(sb_ctx* ctx, uint32_t ci, const sb_grid* g) {
     size_t rays = (size_t)probeTotal * g->raysPerProbe;
     if (!sameDims) {
         release(K.irr); release(K.depth); release(K.atlas); release(K.depthAtlas); release(K.tileOrder);
+        release(K.foot); release(K.footDepth);
         release(K.emitterVis);
         size_t c = 0;
         CK(grow(K.emitterVis, c, (size_t)probeTotal * EMITTER_CAP)); c = 0;
@@ -869,6 +881,8 @@ sb_status sb_configure_cascade(sb_ctx* ctx, uint32_t ci, const sb_grid* g) {
         CK(grow(K.depth, c, (size_t)probeTotal * 64)); c = 0;
         CK(grow(K.atlas, c, (size_t)probeTotal * 64)); c = 0;
         CK(grow(K.depthAtlas, c, (size_t)probeTotal * 64)); c = 0;
+        CK(grow(K.foot, c, (size_t)probeTotal * FOOT * FOOT_U4)); c = 0;
+        CK(grow(K.footDepth, c, (size_t)probeTotal * FOOT)); c = 0;
         // the probes in 4 x 4 x 2 tiles (row-major over tiles, x fastest inside;
         // edge tiles clipped): 32 consecutive entries form one compact block
         std::vector<uint32_t> order;
@@ -1423,7 +1437,9 @@ struct CascadeSnapshot {
         const size_t hist = (size_t)K.probeTotal * 64, texels = (size_t)K.atlasW * K.atlasH;
         const size_t gt = (size_t)K.probeTotal * K.glossyTile * K.glossyTile;
         const size_t ga = (size_t)K.glossyTilesX * K.glossyTile * K.glossyTilesY * K.glossyTile;
-        const Region want[] = {{K.irr, nullptr, hist * 16}, {K.depth, nullptr, hist * 8},
+        const size_t foot = (size_t)K.probeTotal * FOOT * 16;
+        const Region want[] = {{K.foot, nullptr, foot * FOOT_U4}, {K.footDepth, nullptr, foot},
+                               {K.footRough, nullptr, foot * FOOT_U4}, {K.irr, nullptr, hist * 16}, {K.depth, nullptr, hist * 8},
                                {K.atlas, nullptr, texels * 8}, {K.depthAtlas, nullptr, texels * 8},
                                {K.emitterVis, nullptr, (size_t)K.probeTotal * EMITTER_CAP * 4},
                                {K.roughSpec, nullptr, hist * 16}, {K.roughAtlas, nullptr, texels * 8},
@@ -1580,7 +1596,8 @@ sb_status sb_forward_record(sb_ctx* ctx, uint32_t ci, uint32_t solves, const flo
     CK(grow(T.hits, T.hitsCap, solves * nRay));
     CK(grow(T.vis, T.visCap, solves * nRay));
     CK(grow(T.hist, T.histCap, (solves + 1) * (size_t)probes * 64));
-    CK(grow(T.atlas, T.atlasCap, solves * texels));
+    const size_t foot = (size_t)probes * FOOT * FOOT_U4;
+    CK(grow(T.foot, T.footCap, solves * foot));
     CK(grow(T.E, T.ECap, (size_t)probes * 36));
     CK(grow(T.loss, T.lossCap, 1));
     if (!T.evF0) {
@@ -1588,10 +1605,10 @@ sb_status sb_forward_record(sb_ctx* ctx, uint32_t ci, uint32_t solves, const flo
     }
     CK(cudaEventRecord(T.evF0, ctx->stream));
     CK(launch_clear_cascade(dev_cascade(ctx, ci, 0, 0), ctx->stream));
-    const size_t histBytes = (size_t)probes * 64 * sizeof(float4), atlasBytes = texels * sizeof(uint2);
+    const size_t histBytes = (size_t)probes * 64 * sizeof(float4);
     for (uint32_t s = 0; s < solves; ++s) {
         CK(cudaMemcpyAsync(T.hist + s * (size_t)probes * 64, K.irr, histBytes, cudaMemcpyDeviceToDevice, ctx->stream));
-        CK(cudaMemcpyAsync(T.atlas + s * texels, K.atlas, atlasBytes, cudaMemcpyDeviceToDevice, ctx->stream));
+        CK(cudaMemcpyAsync(T.foot + s * foot, K.foot, foot * sizeof(uint4), cudaMemcpyDeviceToDevice, ctx->stream));
         ctx->recordE = s + 1 == solves ? T.E : nullptr;
         sb_status st = sb_solve(ctx, ci, 0, probes);
         ctx->recordE = nullptr;
@@ -1652,7 +1669,7 @@ sb_status sb_backward(sb_ctx* ctx, sb_grads* grads) {
         DevCascade D = dev_cascade(ctx, T.cascade, 0, probes);
         D.hits = T.hits + s * nRay;
         D.vis = T.vis + s * nRay;
-        D.atlasPrev = T.atlas + (size_t)s * T.texels;
+        D.footPrev = T.foot + (size_t)s * probes * FOOT * FOOT_U4;
         D.rayData = T.shaded;
         D.eOut = nullptr;
         const float4* Hs = T.hist + (size_t)s * hist;
@@ -1874,19 +1891,22 @@ static sb_status gather_args(sb_ctx* ctx, const sb_gather_params* prm, const flo
         for (int a = 0; a < 3; ++a) {
             A.c[c].gridMin[a] = K.grid.gridMin[a];
             A.c[c].gridSize[a] = K.grid.gridSize[a];
-            A.c[c].res[a] = float(K.grid.res[a]);
+            const float res = float(K.grid.res[a]);
+            A.c[c].cell[a] = K.grid.gridSize[a] / std::max(res - 1.0f, 1.0f);
+            A.c[c].perCell[a] = 1.0f / std::max(A.c[c].cell[a], 1e-6f);
+            A.c[c].lastBase[a] = std::max(res - 2.0f, 0.0f);
         }
-        A.c[c].atlasW = K.atlasW;
-        A.c[c].atlasH = K.atlasH;
-        A.c[c].atlas = K.atlas;
-        A.c[c].depth = K.depthAtlas;
-        A.c[c].rough = K.roughAtlas;
+        A.c[c].resX = K.grid.res[0];
+        A.c[c].resY = K.grid.res[1];
+        A.c[c].foot = K.foot;
+        A.c[c].footDepth = K.footDepth;
+        A.c[c].footRough = K.footRough;
         A.c[c].glossy = K.reflTier >= SB_REFLECT_HIGH ? K.glossyAtlas : nullptr;
-        A.c[c].glossyOct = K.glossyOct;
+        A.c[c].glossyOct = float(K.glossyOct);
+        A.c[c].perGlossyRow = 1.0f / float(K.glossyTilesX);
         A.c[c].glossyTile = K.glossyTile;
         A.c[c].glossyTilesX = K.glossyTilesX;
         A.c[c].glossyW = K.glossyTilesX * K.glossyTile;
-        A.c[c].glossyH = K.glossyTilesY * K.glossyTile;
     }
     A.cascades = prm->cascades;
     A.dualDetail = prm->dualDetail ? 1u : 0u;

@@ -112,8 +112,9 @@ struct DevCascade {
     uint4* vis;                // NEE masks: tested lights (lo, hi), unblocked lights (lo, hi)
     float4* irr;               // history, probeTotal*64
     float2* depth;             // history
-    const uint2* atlasPrev;    // RGBA16F texels as 4 halves (the previous upload)
-    uint2* atlas;              // RGBA16F output
+    const uint4* footPrev;     // the previous upload's colour footprints (sb_math.cuh)
+    uint2* atlas;              // RGBA16F output, texels as 4 halves
+    uint4 *foot, *footDepth;   // the outputs' footprints
     uint2* depthAtlas;
     float4* eOut;              // optional: FP32 upload output of the 36 interior texels per probe (adjoint tape)
     const uint32_t* issueOrder;  // optional (full updates from slot 0): direction-major issue visits the
@@ -136,6 +137,7 @@ struct DevCascade {
     uint32_t reflect;
     float4* roughSpec;
     uint2* roughAtlas;
+    uint4* footRough;
     float4* glossyNum;
     float* glossyDen;
     uint2* glossyAtlas;

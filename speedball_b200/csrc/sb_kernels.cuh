@@ -89,6 +89,8 @@ cudaError_t launch_light_grid(float* lights, uint32_t lightCount, const DevCasca
 // (direction, type), (colour, emitter class).
 cudaError_t launch_light_gates(const float* lights, float4* gates, cudaStream_t st);
 cudaError_t launch_clear_cascade(const DevCascade& C, cudaStream_t st);
+// The footprints of the irradiance and depth atlases as they are.
+cudaError_t launch_footprints(const DevCascade& C, cudaStream_t st);
 
 // Validation + derived-layout packing (sb_pack.cu).
 cudaError_t launch_pack_scene(const SceneBuffers& B, uint32_t* err, cudaStream_t st);
@@ -144,15 +146,18 @@ cudaError_t launch_tlas_pairs(const SceneBuffers& B, cudaStream_t st);
 // Receiver gather (sb_gather.cu): one cascade's atlases and grid as the gather
 // reads them, and one launch's G-buffer.
 struct GatherCascade {
-    float gridMin[3], gridSize[3], res[3];
-    uint32_t atlasW, atlasH;
-    const uint2* atlas;   // RGBA16F irradiance atlas
-    const uint2* depth;   // RGBA16F depth-moment atlas
-    // reflection lobes (combined receiver): rough atlas in the irradiance
-    // layout; glossy atlas (null below tier high) of glossyTile-texel tiles
-    const uint2* rough;
+    float gridMin[3], gridSize[3];
+    float cell[3], perCell[3];  // cell edges; 1 / max(edge, 1e-6)
+    float lastBase[3];          // the last cage's first probe: max(res - 2, 0)
+    uint32_t resX, resY;
+    const uint4* foot;       // footprints of the irradiance atlas (sb_math.cuh)
+    const uint4* footDepth;  // of the depth-moment atlas
+    // reflection lobes (combined receiver): footprints of the rough atlas; glossy
+    // atlas (null below tier high) of glossyTile-texel tiles
+    const uint4* footRough;
     const uint2* glossy;
-    uint32_t glossyOct, glossyTile, glossyTilesX, glossyW, glossyH;
+    float glossyOct, perGlossyRow;  // texels of a glossy tile's edge; 1 / tiles per row
+    uint32_t glossyTile, glossyTilesX, glossyW;
 };
 struct GatherArgs {
     GatherCascade c[2];

@@ -105,4 +105,64 @@ __device__ __forceinline__ uint2 float4_to_half4(float4 v) {
     return r;
 }
 
+// Footprints: what a bilinear read inside a probe's 8 x 8 tile needs, side by side.
+// The tile-local coordinate 0.5 + uv * 6 lies in [0.5, 6.5], so a read starts at one
+// of 7 x 7 texels; footprint (x, y) of probe p, at p * 49 + y * 7 + x, holds texels
+// (x, y), (x + 1, y), (x, y + 1), (x + 1, y + 1) as binary16: the colours' (r, g)
+// pairs, then b and the alphas of the rows (32 bytes); the depth moments' pairs (16
+// bytes). The atlases hold the same texels for the host; the readers here take one
+// load per tap instead of four, in one to two cache lines per probe instead of one
+// per texel row.
+constexpr uint32_t FOOT = 7u * 7u;
+constexpr uint32_t FOOT_U4 = 2u;  // uint4 per colour footprint
+
+struct FootTap {
+    uint32_t at;  // y * 7 + x
+    float fx, fy;
+};
+__device__ __forceinline__ FootTap foot_tap(float2 o) {
+    const float xl = fmaf(o.x, 6.0f, 0.5f), yl = fmaf(o.y, 6.0f, 0.5f);
+    const float x0 = floorf(xl), y0 = floorf(yl);
+    return {(uint32_t)y0 * 7u + (uint32_t)x0, xl - x0, yl - y0};
+}
+// The bilinear weights of texels 00, 10, 01, 11.
+__device__ __forceinline__ float4 foot_weights(const FootTap& t) {
+    return make_float4((1.0f - t.fx) * (1.0f - t.fy), t.fx * (1.0f - t.fy), (1.0f - t.fx) * t.fy, t.fx * t.fy);
+}
+__device__ __forceinline__ float2 half2_at(uint32_t w) { return __half22float2(*reinterpret_cast<const __half2*>(&w)); }
+__device__ __forceinline__ void load_foot(const uint4* p, uint32_t w[8]) {
+    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
+        : "l"(p));
+}
+__device__ __forceinline__ float bilerp(float a, float b, float c, float d, float4 w) {
+    return a * w.x + b * w.y + c * w.z + d * w.w;
+}
+__device__ __forceinline__ float3 foot_rgb(const uint4* foot, uint32_t at, float4 w) {
+    uint32_t u[8];
+    load_foot(foot + FOOT_U4 * at, u);
+    const float2 a = half2_at(u[0]), b = half2_at(u[1]), c = half2_at(u[2]), d = half2_at(u[3]);
+    const float2 b0 = half2_at(u[4]), b1 = half2_at(u[5]);
+    return mk(bilerp(a.x, b.x, c.x, d.x, w), bilerp(a.y, b.y, c.y, d.y, w), bilerp(b0.x, b0.y, b1.x, b1.y, w));
+}
+__device__ __forceinline__ float4 foot_rgba(const uint4* foot, uint32_t at, float4 w) {
+    uint32_t u[8];
+    load_foot(foot + FOOT_U4 * at, u);
+    const float2 a = half2_at(u[0]), b = half2_at(u[1]), c = half2_at(u[2]), d = half2_at(u[3]);
+    const float2 b0 = half2_at(u[4]), b1 = half2_at(u[5]), a0 = half2_at(u[6]), a1 = half2_at(u[7]);
+    return make_float4(bilerp(a.x, b.x, c.x, d.x, w), bilerp(a.y, b.y, c.y, d.y, w), bilerp(b0.x, b0.y, b1.x, b1.y, w),
+                       bilerp(a0.x, a0.y, a1.x, a1.y, w));
+}
+__device__ __forceinline__ float2 foot_depth(const uint4* foot, uint32_t at, float4 w) {
+    const uint4 u = __ldg(foot + at);
+    const float2 a = half2_at(u.x), b = half2_at(u.y), c = half2_at(u.z), d = half2_at(u.w);
+    return make_float2(bilerp(a.x, b.x, c.x, d.x, w), bilerp(a.y, b.y, c.y, d.y, w));
+}
+// A footprint from its four texels (RGBA16F: rg | ba).
+__device__ __forceinline__ void store_foot(uint4* foot, uint32_t at, uint2 t00, uint2 t10, uint2 t01, uint2 t11) {
+    foot[FOOT_U4 * at] = make_uint4(t00.x, t10.x, t01.x, t11.x);
+    foot[FOOT_U4 * at + 1u] = make_uint4(__byte_perm(t00.y, t10.y, 0x5410u), __byte_perm(t01.y, t11.y, 0x5410u),
+                                         __byte_perm(t00.y, t10.y, 0x7632u), __byte_perm(t01.y, t11.y, 0x7632u));
+}
+
 }  // namespace sb

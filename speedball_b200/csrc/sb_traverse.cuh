@@ -767,13 +767,9 @@ static __device__ float3 sample_atlas(const DevCascade& C, float3 P, float3 N) {
         base[a] = clampf(floorf(gf[a]), 0.0f, fmaxf(float(C.res[a]) - 2.0f, 0.0f));
         frac[a] = clampf(gf[a] - base[a], 0.0f, 1.0f);
     }
-    // the bilinear footprint inside each cage probe's tile: tile-local coordinate
-    // 0.5 + uv * 6 in [0.5, 6.5], the same offset and weights for all 8 taps
-    const float2 ouv = oct_encode(normalize3(N));
-    const float xl = fmaf(ouv.x, 6.0f, 0.5f), yl = fmaf(ouv.y, 6.0f, 0.5f);
-    const float fx0 = floorf(xl), fy0 = floorf(yl), fx = xl - fx0, fy = yl - fy0;
-    const uint32_t Wu = C.atlasW, off = (uint32_t)fy0 * Wu + (uint32_t)fx0;
-    const float w00 = (1.0f - fx) * (1.0f - fy), w10 = fx * (1.0f - fy), w01 = (1.0f - fx) * fy, w11 = fx * fy;
+    // the bilinear read inside each cage probe's tile: the same footprint and weights for all 8 taps
+    const FootTap tap = foot_tap(oct_encode(normalize3(N)));
+    const float4 bw = foot_weights(tap);
     float3 acc = mk(0.f, 0.f, 0.f);
     float wsum = 0.0f;
 #pragma unroll
@@ -784,14 +780,8 @@ static __device__ float3 sample_atlas(const DevCascade& C, float3 P, float3 N) {
         float wy = dy ? frac[1] : 1.0f - frac[1];
         float wz = dz ? frac[2] : 1.0f - frac[2];
         float w = wx * wy * wz + 1e-4f;
-        const uint32_t tile = ((uint32_t)pz * C.res[1] + (uint32_t)py) * 8u * Wu + (uint32_t)px * 8u;
-        const uint2* p = C.atlasPrev + tile + off;
-        float4 t00 = half4_to_float4(__ldg(p)), t10 = half4_to_float4(__ldg(p + 1));
-        float4 t01 = half4_to_float4(__ldg(p + Wu)), t11 = half4_to_float4(__ldg(p + Wu + 1));
-        float3 s = mk(t00.x * w00 + t10.x * w10 + t01.x * w01 + t11.x * w11,
-                      t00.y * w00 + t10.y * w10 + t01.y * w01 + t11.y * w11,
-                      t00.z * w00 + t10.z * w10 + t01.z * w01 + t11.z * w11);
-        acc = acc + s * w;
+        const uint32_t probe = ((uint32_t)pz * C.res[1] + (uint32_t)py) * C.res[0] + (uint32_t)px;
+        acc = acc + foot_rgb(C.footPrev, probe * FOOT + tap.at, bw) * w;
         wsum += w;
     }
     return acc * (1.0f / fmaxf(wsum, 1e-4f));
