@@ -212,6 +212,7 @@ template <class T> void release(T*& p) {
     p = nullptr;
 }
 
+constexpr uint32_t QUERY_CURSOR = SB_BATCH_MAX * WORK_WORDS;  // in dWork, behind the solves' words
 constexpr uint64_t kJobCapMax = 64ull << 20;  // 64 Mi shadow jobs (2 GiB) per trace chunk
 
 uint32_t tlas_nodes_for(uint32_t n) {
@@ -469,7 +470,7 @@ sb_status sb_create(const sb_device_opts* opts, sb_ctx** out) {
         if (cudaStreamCreateWithFlags(&ctx->ownStream, cudaStreamNonBlocking) != cudaSuccess) { st = SB_ERR_CUDA; break; }
         ctx->stream = ctx->ownStream;
         if (cudaMalloc(&ctx->dErr, 4) != cudaSuccess || cudaMalloc(&ctx->dGate, 32 * 4) != cudaSuccess ||
-            cudaMalloc(&ctx->dWork, 64) != cudaSuccess || cudaMalloc(&ctx->dCounters, 16 * 8) != cudaSuccess ||
+            cudaMalloc(&ctx->dWork, (QUERY_CURSOR + 8) * 4) != cudaSuccess || cudaMalloc(&ctx->dCounters, 16 * 8) != cudaSuccess ||
             cudaMalloc(&ctx->B.valid, 4) != cudaSuccess || cudaMalloc(&ctx->B.depth, 8) != cudaSuccess) {
             st = SB_ERR_OOM;
             break;
@@ -1056,12 +1057,13 @@ static sb_status build_batch(const sb_solve_item* items, uint32_t count, BatchAr
         BatchItem& I = B.it[i];
         I.W.S = dev_scene(c);
         B.wideDepth = std::max(B.wideDepth, I.W.S.wideDepth);
+        B.maxRays = std::max(B.maxRays, c->casc[ci].grid.raysPerProbe);
         if (I.W.S.wideNodes && I.W.S.dynCount) B.moved = 1u;
         I.W.C = dev_cascade(c, ci, items[i].probeOffset % K.probeTotal, cnt);
         std::memcpy(&I.W.P, &c->params, sizeof I.W.P);
         I.W.err = c->dErr;
         I.W.counters = nullptr;
-        I.W.work = lead->dWork;
+        I.W.work = lead->dWork + i * WORK_WORDS;
         I.W.slotBegin = 0;
         I.W.slotCount = cnt;
         I.W.smemTlas = 0;
@@ -1074,6 +1076,7 @@ static sb_status build_batch(const sb_solve_item* items, uint32_t count, BatchAr
         I.blendBase = blend;
         I.blendBlocks = blend_blocks(cnt);
         blend += I.blendBlocks;
+        I.W.jobCap = (uint32_t)std::min<uint64_t>(rays * (c->lightCount ? c->lightCount : 1u), kJobCapMax);
         jobs += rays * (c->lightCount ? c->lightCount : 1u);
     }
     if (rayBase >= (1ull << 26))
@@ -1089,9 +1092,10 @@ static sb_status build_batch(const sb_solve_item* items, uint32_t count, BatchAr
         CK(grow(lead->jobs, c, (size_t)jobs * 2));
         lead->jobCap = (uint32_t)jobs;
     }
+    float4* at = lead->jobs;  // (jobs fit: each item's part holds a job per ray and light)
     for (uint32_t i = 0; i < count; ++i) {
-        B.it[i].W.jobs = lead->jobs;
-        B.it[i].W.jobCap = lead->jobCap;
+        B.it[i].W.jobs = at;
+        at += 2 * (size_t)B.it[i].W.jobCap;
     }
     B.n = count;
     B.totalRays = (uint32_t)rayBase;
@@ -1721,8 +1725,8 @@ sb_status sb_raycast(sb_ctx* ctx, const float* ro, const float* rd, uint32_t n, 
     CK(cudaMallocAsync(&dinst, (size_t)n * 4, ctx->stream));
     CK(cudaMemcpyAsync(dro, ro, (size_t)n * 12, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(drd, rd, (size_t)n * 12, cudaMemcpyHostToDevice, ctx->stream));
-    CK(launch_raycast(dev_scene(ctx), dro, drd, n, dt, dtri, dinst, ctx->dWork + 8, ctx->numSms, ctx->dErr,
-                      ctx->stream));
+    CK(launch_raycast(dev_scene(ctx), dro, drd, n, dt, dtri, dinst, ctx->dWork + QUERY_CURSOR, ctx->numSms,
+                      ctx->dErr, ctx->stream));
     CK(cudaMemcpyAsync(tOut, dt, (size_t)n * 4, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaMemcpyAsync(triOut, dtri, (size_t)n * 4, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaMemcpyAsync(instOut, dinst, (size_t)n * 4, cudaMemcpyDeviceToHost, ctx->stream));
@@ -1749,8 +1753,8 @@ sb_status sb_raycast_device(sb_ctx* ctx, const float* ro, const float* rd, uint3
     if (n == 0) return ctx->sceneLoaded ? SB_OK : fail(ctx, SB_ERR_NOT_READY, "no scene uploaded");
     sb_status s = device_query_ready(ctx);
     if (s != SB_OK) return s;
-    CK(launch_raycast(dev_scene(ctx), ro, rd, n, tOut, triOut, instOut, ctx->dWork + 8, ctx->numSms, ctx->dErr,
-                      ctx->stream));
+    CK(launch_raycast(dev_scene(ctx), ro, rd, n, tOut, triOut, instOut, ctx->dWork + QUERY_CURSOR, ctx->numSms,
+                      ctx->dErr, ctx->stream));
     return SB_OK;
 }
 
@@ -1760,8 +1764,8 @@ sb_status sb_occluded_device(sb_ctx* ctx, const float* ro, const float* rd, cons
     if (n == 0) return ctx->sceneLoaded ? SB_OK : fail(ctx, SB_ERR_NOT_READY, "no scene uploaded");
     sb_status s = device_query_ready(ctx);
     if (s != SB_OK) return s;
-    CK(launch_occluded(dev_scene(ctx), ro, rd, maxDist, n, blockedOut, ctx->dWork + 8, ctx->numSms, ctx->dErr,
-                       ctx->stream));
+    CK(launch_occluded(dev_scene(ctx), ro, rd, maxDist, n, blockedOut, ctx->dWork + QUERY_CURSOR, ctx->numSms,
+                       ctx->dErr, ctx->stream));
     return SB_OK;
 }
 
@@ -1980,7 +1984,7 @@ sb_status sb_occluded(sb_ctx* ctx, const float* ro, const float* rd, const float
     CK(cudaMemcpyAsync(dro, ro, (size_t)n * 12, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(drd, rd, (size_t)n * 12, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(dm, maxDist, (size_t)n * 4, cudaMemcpyHostToDevice, ctx->stream));
-    CK(launch_occluded(dev_scene(ctx), dro, drd, dm, n, dout, ctx->dWork + 8, ctx->numSms, ctx->dErr, ctx->stream));
+    CK(launch_occluded(dev_scene(ctx), dro, drd, dm, n, dout, ctx->dWork + QUERY_CURSOR, ctx->numSms, ctx->dErr, ctx->stream));
     CK(cudaMemcpyAsync(out, dout, (size_t)n, cudaMemcpyDeviceToHost, ctx->stream));
     cudaFreeAsync(dro, ctx->stream); cudaFreeAsync(drd, ctx->stream); cudaFreeAsync(dm, ctx->stream);
     cudaFreeAsync(dout, ctx->stream);

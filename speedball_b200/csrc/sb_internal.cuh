@@ -181,15 +181,17 @@ struct WaveCtx {
     uint32_t order;                // 0 probe-major, 1 direction-major
 };
 
+constexpr uint32_t WORK_WORDS = 8;  // WaveCtx::work of one solve
+
 // Several solves (scenes, cascades) through one launch of each stage: a
 // shared ray index space in which item i owns [rayBase, rayBase + rays), with
-// rayBase a multiple of 32 so a warp's 32 rays never straddle two items, and a
-// shared shadow-job queue whose jobs carry the global ray index. The blend
+// rayBase a multiple of 32 so a warp's 32 rays never straddle two items, and
+// cursors and a part of the lead's shadow-job queue for each item. The blend
 // grid is split the same way (blendBase / blendBlocks CTAs per item). Passed
 // by value as a __grid_constant__ kernel parameter and indexed in place.
 constexpr uint32_t SB_BATCH_MAX = 16;
 struct BatchItem {
-    WaveCtx W;                     // W.work / W.jobs / W.jobCap are the batch's shared ones
+    WaveCtx W;
     uint32_t rayBase, rays;
     uint32_t blendBase, blendBlocks;
 };
@@ -200,7 +202,8 @@ struct BatchArgs {
     uint32_t blendBlocks;
     uint32_t wideDepth;            // the deepest 8-wide tree among the items
     uint32_t moved;                // some item has moved slots
-    uint32_t* work;
+    uint32_t maxRays;              // the most rays per probe among the items
+    uint32_t* work;                // the items' cursors (WORK_WORDS each)
     unsigned long long* counters;  // one set for the whole batch, or null
 };
 static_assert(sizeof(BatchArgs) <= 32000, "BatchArgs must fit the kernel parameter space");
