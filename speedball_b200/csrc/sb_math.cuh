@@ -130,6 +130,12 @@ __device__ __forceinline__ float4 foot_weights(const FootTap& t) {
     return make_float4((1.0f - t.fx) * (1.0f - t.fy), t.fx * (1.0f - t.fy), (1.0f - t.fx) * t.fy, t.fx * t.fy);
 }
 __device__ __forceinline__ float2 half2_at(uint32_t w) { return __half22float2(*reinterpret_cast<const __half2*>(&w)); }
+// Two float4 as one 32-byte operation (p 32-byte aligned).
+__device__ __forceinline__ void store32(float4* p, float4 a, float4 b) {
+    asm volatile("st.global.v8.f32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "f"(a.x), "f"(a.y), "f"(a.z),
+                 "f"(a.w), "f"(b.x), "f"(b.y), "f"(b.z), "f"(b.w)
+                 : "memory");
+}
 __device__ __forceinline__ void load_foot(const uint4* p, uint32_t w[8]) {
     asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
         : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])

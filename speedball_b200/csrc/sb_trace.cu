@@ -250,11 +250,12 @@ __device__ __forceinline__ void shadow_walk8(const WaveCtx& W, const WalkSmem& m
 // the hit parameter re-evaluated in FP64, the hit frame, and the NEE
 // gates of every candidate light. Each lane runs the gates with no warp sync;
 // one warp scan and one atomicAdd then reserve the warp's shadow-ray jobs, and
-// each ray's passing candidates (gates evaluated again: the same pure
-// function) are written together in list order, so a shadow warp mostly holds
-// rays that share an origin. Jobs carry the ray's record index.
-__device__ __forceinline__ uint32_t emit_ray(const WaveCtx& W, bool active, uint32_t g) {
+// each ray's passing candidates are written together in list order, so a shadow
+// warp mostly holds rays that share an origin. Jobs carry the ray's record index.
+// `gates`: GATE_LIGHTS entries of shared memory, the warp's own.
+__device__ __forceinline__ uint32_t emit_ray(const WaveCtx& W, bool active, uint32_t g, float4* gates) {
     const DevCascade& C = W.C;
+    const GateTable T = gate_table(W, gates);
     const uint32_t N = C.rays;
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t rayIdx = 0;
@@ -289,7 +290,7 @@ __device__ __forceinline__ uint32_t emit_ray(const WaveCtx& W, bool active, uint
     if (tri >= 0) L = light_list(W, fr.hitPos);
     unsigned long long pass = 0ull;
     for (uint32_t i = 0; i < L.count; ++i)
-        if (light_gate(W, light_at(L, i), fr.hitPos, fr.ng)) pass |= 1ull << i;
+        if (table_gate(W, T, light_at(L, i), fr.hitPos, fr.ng)) pass |= 1ull << i;
     const uint32_t mine = (uint32_t)__popcll(pass);
     uint32_t incl = mine;
 #pragma unroll
@@ -312,9 +313,9 @@ __device__ __forceinline__ uint32_t emit_ray(const WaveCtx& W, bool active, uint
         if (j < W.jobCap) {
             float3 wi;
             float dist;
-            light_ray(W, li, fr.hitPos, wi, dist);
-            W.jobs[2 * j] = make_float4(fr.hitPos.x, fr.hitPos.y, fr.hitPos.z, dist - fr.traceBias);
-            W.jobs[2 * j + 1] = make_float4(wi.x, wi.y, wi.z, __uint_as_float(tag | li));
+            light_ray(T, li, fr.hitPos, wi, dist);
+            store32(W.jobs + 2 * j, make_float4(fr.hitPos.x, fr.hitPos.y, fr.hitPos.z, dist - fr.traceBias),
+                    make_float4(wi.x, wi.y, wi.z, __uint_as_float(tag | li)));
             if (li < 32) tested0 |= 1u << li;
             else tested1 |= 1u << (li - 32);
             ++nJobs;
@@ -519,11 +520,15 @@ __device__ void order_batches(const uint32_t* cost, uint32_t* order, uint32_t n,
     for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) order[atomicAdd(&at[cost_bin(__ldcg(cost + i))], 1u)] = i;
 }
 
-__global__ void __launch_bounds__(128) k_emit(WaveCtx W) {
+// 64 registers: left to itself the compiler takes 84, and the atrium's emission 48 us
+// instead of 41 (40 registers: 46).
+constexpr int EMIT_MIN_BLOCKS = 8;
+__global__ void __launch_bounds__(128, EMIT_MIN_BLOCKS) k_emit(WaveCtx W) {
+    __shared__ float4 gates[4][GATE_LIGHTS];
     if (!*W.S.valid) return;
     const uint32_t total = W.slotCount * W.C.rays;
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t nJobs = emit_ray(W, g < total, g);
+    const uint32_t nJobs = emit_ray(W, g < total, g, gates[threadIdx.x / 32u]);
     if (W.counters) {
         const uint32_t warpDone = __reduce_add_sync(0xFFFFFFFFu, nJobs);
         if ((threadIdx.x & 31u) == 0 && warpDone) atomicAdd(&W.counters[1], (unsigned long long)warpDone);
@@ -700,13 +705,14 @@ __global__ void __launch_bounds__(256, SB_WALK8_MIN_BLOCKS) k_trace_primary_batc
     add_visits(B.counters, 2, nRays, vis);
 }
 
-__global__ void __launch_bounds__(128) k_emit_batch(const __grid_constant__ BatchArgs B) {
+__global__ void __launch_bounds__(128, EMIT_MIN_BLOCKS) k_emit_batch(const __grid_constant__ BatchArgs B) {
+    __shared__ float4 gates[4][GATE_LIGHTS];
     const uint32_t gg = blockIdx.x * blockDim.x + threadIdx.x;
     if (gg - (threadIdx.x & 31u) >= B.totalRays) return;  // whole warps only
     const BatchItem& I = B.it[batch_item(B, gg & ~31u)];
     if (!*I.W.S.valid) return;
     const uint32_t g = gg - I.rayBase;
-    const uint32_t nJobs = emit_ray(I.W, g < I.rays, g);
+    const uint32_t nJobs = emit_ray(I.W, g < I.rays, g, gates[threadIdx.x / 32u]);
     if (B.counters) {
         const uint32_t warpDone = __reduce_add_sync(0xFFFFFFFFu, nJobs);
         if ((threadIdx.x & 31u) == 0 && warpDone) atomicAdd(&B.counters[1], (unsigned long long)warpDone);
