@@ -471,8 +471,7 @@ __global__ void __launch_bounds__(SHADE_BWD_THREADS) k_shade_bwd(WaveCtx W, cons
         const float3 gr = xyz(gR[g]);
         if (hrec.x != 0xFFFFFFFFu && (gr.x != 0.f || gr.y != 0.f || gr.z != 0.f)) {
             const uint32_t tri = hrec.x, inst = hrec.y & 0x7FFFFFFFu;
-            const float3 ro = probe_world_pos(C, slot);
-            const float3 rd = ray_dir(k, N, P.frameJitter);
+            const float3 ro = slot_origin(C, slot), rd = wave_dir(W, k);
             const HitFrame fr = hit_frame(W, tri, inst, ro, rd, __uint_as_float(hrec.z), (int)(hrec.y >> 31));
             const uint32_t m = __ldg(W.S.triMaterial + tri);
             const float* M = W.S.materials + (size_t)m * 28u;
@@ -545,8 +544,8 @@ __global__ void __launch_bounds__(SHADE_BWD_THREADS) k_shade_bwd(WaveCtx W, cons
     }
 }
 
-cudaError_t launch_shade_bwd(const DevScene& S, const DevCascade& C, const DevParams& P, const float4* gR,
-                             double* gParam, float4* gA, cudaStream_t st) {
+cudaError_t launch_shade_bwd(const DevScene& S, const DevCascade& C, const DevParams& P, const float4* dirs,
+                             const float4* gR, double* gParam, float4* gA, cudaStream_t st) {
     const uint32_t rays = C.probeTotal * C.rays;
     if (rays == 0) return cudaSuccess;
     WaveCtx W{};
@@ -554,6 +553,7 @@ cudaError_t launch_shade_bwd(const DevScene& S, const DevCascade& C, const DevPa
     W.C = C;
     W.P = P;
     W.slotCount = C.probeTotal;
+    W.dirs = const_cast<float4*>(dirs);
     const uint32_t nParam = 6u * S.materialCount + S.lightCount;
     const size_t smem = (size_t)nParam * sizeof(float);
     const int useSmem = smem <= 32u * 1024u ? 1 : 0;

@@ -39,6 +39,7 @@ struct Cascade {
     uint4* hits = nullptr;
     uint4* vis = nullptr;
     size_t rayCap = 0;
+    float4* probePos = nullptr;     // every probe's position
     uint32_t* tileOrder = nullptr;  // probe index per issue position in 4 x 4 x 2 tiles (sortKey 2)
     // sortKey 3: cycles per 32-ray closest-hit batch of the last full solve, and the batch
     // order (costliest first) built from them; ready once a full solve has recorded costs
@@ -100,6 +101,7 @@ struct sb_ctx {
     RefitRange refitRanges[16];
     uint32_t packEpoch = 1, refitNext = 0;
     uint32_t* dWork = nullptr;
+    float4* dDirs = nullptr;  // ray directions: a batch's items (a solve: the first), then the adjoint's
     unsigned long long* dCounters = nullptr;
     bool countersOn = false;
 
@@ -213,6 +215,7 @@ template <class T> void release(T*& p) {
 }
 
 constexpr uint32_t QUERY_CURSOR = SB_BATCH_MAX * WORK_WORDS;  // in dWork, behind the solves' words
+constexpr uint32_t ADJOINT_DIRS = SB_BATCH_MAX * MAX_RAYS;    // in dDirs
 constexpr uint64_t kJobCapMax = 64ull << 20;  // 64 Mi shadow jobs (2 GiB) per trace chunk
 
 uint32_t tlas_nodes_for(uint32_t n) {
@@ -280,6 +283,7 @@ DevCascade dev_cascade(const sb_ctx* c, uint32_t ci, uint32_t probeOffset, uint3
     }
     D.probeOffset = probeOffset;
     D.updatedCount = updated;
+    D.probePos = K.probePos;
     D.rayData = K.rayData;
     D.hits = K.hits;
     D.vis = K.vis;
@@ -470,7 +474,9 @@ sb_status sb_create(const sb_device_opts* opts, sb_ctx** out) {
         if (cudaStreamCreateWithFlags(&ctx->ownStream, cudaStreamNonBlocking) != cudaSuccess) { st = SB_ERR_CUDA; break; }
         ctx->stream = ctx->ownStream;
         if (cudaMalloc(&ctx->dErr, 4) != cudaSuccess || cudaMalloc(&ctx->dGate, 32 * 4) != cudaSuccess ||
-            cudaMalloc(&ctx->dWork, (QUERY_CURSOR + 8) * 4) != cudaSuccess || cudaMalloc(&ctx->dCounters, 16 * 8) != cudaSuccess ||
+            cudaMalloc(&ctx->dWork, (QUERY_CURSOR + 8) * 4) != cudaSuccess ||
+            cudaMalloc(&ctx->dDirs, (ADJOINT_DIRS + MAX_RAYS) * sizeof(float4)) != cudaSuccess ||
+            cudaMalloc(&ctx->dCounters, 16 * 8) != cudaSuccess ||
             cudaMalloc(&ctx->B.valid, 4) != cudaSuccess || cudaMalloc(&ctx->B.depth, 8) != cudaSuccess) {
             st = SB_ERR_OOM;
             break;
@@ -517,7 +523,7 @@ void sb_destroy(sb_ctx* ctx) {
     for (auto& K : ctx->casc) {
         release(K.irr); release(K.depth); release(K.atlas); release(K.depthAtlas); release(K.rayData); release(K.hits);
         release(K.emitterVis);
-        release(K.tileOrder); release(K.batchCost); release(K.batchOrder);
+        release(K.probePos); release(K.tileOrder); release(K.batchCost); release(K.batchOrder);
         release(K.vis);
         release(K.roughSpec); release(K.roughAtlas); release(K.glossyNum); release(K.glossyDen);
         release(K.foot); release(K.footDepth); release(K.footRough);
@@ -536,7 +542,7 @@ void sb_destroy(sb_ctx* ctx) {
     release(T.loss);
     for (cudaEvent_t e : {T.evF0, T.evF1, T.evB0, T.evB1})
         if (e) cudaEventDestroy(e);
-    release(ctx->dErr); release(ctx->dGate); release(ctx->dWork); release(ctx->dCounters);
+    release(ctx->dErr); release(ctx->dGate); release(ctx->dWork); release(ctx->dDirs); release(ctx->dCounters);
     if (ctx->syncEv) cudaEventDestroy(ctx->syncEv);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
     if (ctx->evMid) cudaEventDestroy(ctx->evMid);
@@ -874,8 +880,9 @@ sb_status sb_configure_cascade(sb_ctx* ctx, uint32_t ci, const sb_grid* g) {
     if (!sameDims) {
         release(K.irr); release(K.depth); release(K.atlas); release(K.depthAtlas); release(K.tileOrder);
         release(K.foot); release(K.footDepth);
-        release(K.emitterVis);
+        release(K.emitterVis); release(K.probePos);
         size_t c = 0;
+        CK(grow(K.probePos, c, (size_t)probeTotal)); c = 0;
         CK(grow(K.emitterVis, c, (size_t)probeTotal * EMITTER_CAP)); c = 0;
         CK(cudaMemsetAsync(K.emitterVis, 0, (size_t)probeTotal * EMITTER_CAP * sizeof(float), ctx->stream));
         CK(grow(K.irr, c, (size_t)probeTotal * 64)); c = 0;
@@ -928,6 +935,7 @@ sb_status sb_configure_cascade(sb_ctx* ctx, uint32_t ci, const sb_grid* g) {
         s = alloc_reflection(ctx, K);
         if (s != SB_OK) return s;
     }
+    CK(launch_probe_positions(dev_cascade(ctx, ci, 0, 0), K.probePos, ctx->stream));
     K.glossyPhase = 0;  // every rebuild restarts the glossy interleave (gi_probes.js:3162, 3193, 3224)
     ++ctx->epoch;
     ++ctx->structGen;
@@ -999,7 +1007,7 @@ sb_status sb_solve(sb_ctx* ctx, uint32_t ci, uint32_t probeOffset, uint32_t upda
     ctx->singleChunk = updatedCount <= chunk;
     for (uint32_t s0 = 0; s0 < updatedCount; s0 += chunk) {
         uint32_t n = updatedCount - s0 < chunk ? updatedCount - s0 : chunk;
-        CK(launch_trace(S, D, P, ctx->dErr, ctx->countersOn ? ctx->dCounters : nullptr, ctx->dWork, ctx->tune,
+        CK(launch_trace(S, D, P, ctx->dErr, ctx->countersOn ? ctx->dCounters : nullptr, ctx->dWork, ctx->dDirs, ctx->tune,
                         ctx->stream, ctx->jobs, ctx->jobCap, s0, n, timing ? ctx->evA : nullptr,
                         timing ? ctx->evB : nullptr, timing ? ctx->evC : nullptr));
     }
@@ -1064,6 +1072,9 @@ static sb_status build_batch(const sb_solve_item* items, uint32_t count, BatchAr
         I.W.err = c->dErr;
         I.W.counters = nullptr;
         I.W.work = lead->dWork + i * WORK_WORDS;
+        I.W.dirs = lead->dDirs + i * MAX_RAYS;
+        I.W.slotMagic = div_magic(cnt);
+        I.W.rayMagic = div_magic(K.grid.raysPerProbe);
         I.W.slotBegin = 0;
         I.W.slotCount = cnt;
         I.W.smemTlas = 0;
@@ -1667,6 +1678,8 @@ sb_status sb_backward(sb_ctx* ctx, sb_grads* grads) {
     const DevScene S = dev_scene(ctx);
     DevParams P;
     std::memcpy(&P, &ctx->params, sizeof P);
+    float4* dirs = ctx->dDirs + ADJOINT_DIRS;
+    CK(launch_ray_dirs(T.rays, P.frameJitter, dirs, ctx->stream));
     float4* gHnext = T.gH;              // dL/dH after solve s (from solve s + 1's blend)
     const float4* gAnext = nullptr;     // dL/dAtlas written by solve s (read by solve s + 1)
     for (int s = (int)T.solves - 1; s >= 0; --s) {
@@ -1683,9 +1696,9 @@ sb_status sb_backward(sb_ctx* ctx, sb_grads* grads) {
         float4* gAcur = T.gA + (size_t)(s & 1) * T.texels;
         float4* gHprev = gHnext == T.gH ? T.gH + hist : T.gH;
         CK(cudaMemsetAsync(gAcur, 0, (size_t)T.texels * sizeof(float4), ctx->stream));
-        CK(launch_shade(S, D, P, probes, ctx->stream));
+        CK(launch_shade(S, D, P, dirs, probes, ctx->stream));
         CK(launch_blend_bwd(D, P, T.shaded, Hs, gHnext, gHprev, T.gR, ctx->stream));
-        CK(launch_shade_bwd(S, D, P, T.gR, T.gParam, gAcur, ctx->stream));
+        CK(launch_shade_bwd(S, D, P, dirs, T.gR, T.gParam, gAcur, ctx->stream));
         gHnext = gHprev;
         gAnext = gAcur;
     }

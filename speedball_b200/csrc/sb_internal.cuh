@@ -107,6 +107,7 @@ struct DevCascade {
     // cascade 0's grid, for the clustered cell lookup
     float g0Min[3], g0Size[3];
     uint32_t g0Res[3];
+    const float4* probePos;    // every probe's position (probe_world_pos)
     float4* rayData;           // updatedCount*rays
     uint4* hits;               // 16-byte hit records: tri, inst | facing << 31, t, packed uv
     uint4* vis;                // NEE masks: tested lights (lo, hi), unblocked lights (lo, hi)
@@ -176,11 +177,27 @@ struct WaveCtx {
                                    // claim, [4], [5] the moved slots' ray and job cursors
     float4* jobs;                  // 2 float4 per job: (origin, maxDist), (dir, ray << 6 | light)
     uint32_t jobCap;
+    float4* dirs;                  // the solve's ray directions (written by stage A, read by the later ones)
     uint32_t slotBegin, slotCount; // probe slots of this chunk
+    uint32_t slotMagic, rayMagic;  // div_magic of slotCount and the rays per probe
     uint32_t smemTlas;             // TLAS nodes staged in shared memory (0 = read from global)
     uint32_t order;                // 0 probe-major, 1 direction-major
 };
 
+// Quotient and remainder by a divisor known ahead, magic = floor((2^32 - 1) / d): the
+// high product is the quotient or one less (it is short by g / 2^32 at most).
+inline uint32_t div_magic(uint32_t d) { return d ? 0xFFFFFFFFu / d : 0u; }
+__device__ __forceinline__ uint32_t divide(uint32_t g, uint32_t d, uint32_t magic, uint32_t& rest) {
+    uint32_t q = __umulhi(g, magic);
+    rest = g - q * d;
+    if (rest >= d) {
+        ++q;
+        rest -= d;
+    }
+    return q;
+}
+
+constexpr uint32_t MAX_RAYS = 256;  // per probe
 constexpr uint32_t WORK_WORDS = 8;  // WaveCtx::work of one solve
 
 // Several solves (scenes, cascades) through one launch of each stage: a

@@ -44,8 +44,8 @@ struct SceneBuffers {
 // The three trace stages over probe slots [slotBegin, slotBegin + slotCount);
 // `jobs` holds up to jobCap shadow-ray jobs (32 bytes each).
 cudaError_t launch_trace(const DevScene& S, const DevCascade& C, const DevParams& P, uint32_t* err,
-                         unsigned long long* counters, uint32_t* work, const TraceTuning& tune, cudaStream_t st,
-                         float4* jobs, uint32_t jobCap, uint32_t slotBegin, uint32_t slotCount,
+                         unsigned long long* counters, uint32_t* work, float4* dirs, const TraceTuning& tune,
+                         cudaStream_t st, float4* jobs, uint32_t jobCap, uint32_t slotBegin, uint32_t slotCount,
                          cudaEvent_t afterPrimary = nullptr, cudaEvent_t afterShadow = nullptr,
                          cudaEvent_t afterClosest = nullptr);
 cudaError_t launch_blend_upload(const DevCascade& C, const DevParams& P, cudaStream_t st);
@@ -54,11 +54,10 @@ cudaError_t launch_blend_upload(const DevCascade& C, const DevParams& P, cudaStr
 cudaError_t launch_scatter_vertices(float* vertexData8, const float* positions, const float* normals, uint32_t n,
                                     cudaStream_t st);
 cudaError_t launch_glossy(const DevCascade& C, const DevParams& P, cudaStream_t st);
-cudaError_t launch_shade(const DevScene& S, const DevCascade& C, const DevParams& P, uint32_t slotCount,
-                         cudaStream_t st);
+cudaError_t launch_shade(const DevScene& S, const DevCascade& C, const DevParams& P, const float4* dirs,
+                         uint32_t slotCount, cudaStream_t st);
 
-// Batched stages (every item of B in one launch per stage). B.work must hold
-// 3 words; every item's W.jobs / W.jobCap / W.work are the batch's shared ones.
+// Batched stages (every item of B in one launch per stage).
 cudaError_t launch_trace_batch(const BatchArgs& B, const TraceTuning& tune, cudaStream_t st,
                                cudaEvent_t afterPrimary = nullptr, cudaEvent_t afterShadow = nullptr,
                          cudaEvent_t afterClosest = nullptr);
@@ -82,8 +81,8 @@ cudaError_t launch_upload_bwd(const DevCascade& C, const DevParams& P, const flo
                               const float4* gA, float4* gH, cudaStream_t st);
 cudaError_t launch_blend_bwd(const DevCascade& C, const DevParams& P, const float4* rays, const float4* Hprev,
                              const float4* gH, float4* gHprev, float4* gR, cudaStream_t st);
-cudaError_t launch_shade_bwd(const DevScene& S, const DevCascade& C, const DevParams& P, const float4* gR,
-                             double* gParam, float4* gA, cudaStream_t st);
+cudaError_t launch_shade_bwd(const DevScene& S, const DevCascade& C, const DevParams& P, const float4* dirs,
+                             const float4* gR, double* gParam, float4* gA, cudaStream_t st);
 cudaError_t launch_light_grid(float* lights, uint32_t lightCount, const DevCascade& g0, cudaStream_t st);
 // The 64 light records' gate fields as three aligned float4 each: (position, range),
 // (direction, type), (colour, emitter class).
@@ -193,6 +192,9 @@ bool fine_box_from_hist(const uint32_t* hist, const double mn[3], const double s
 cudaError_t launch_emitter_vis(const DevScene& S, const DevCascade& C, const DevParams& P, uint32_t* err,
                                cudaStream_t st);
 // The FP32 probe rays of a solve as the trace forms them (sb_probe_rays).
+// The tables a solve's stages read: probe positions, ray directions.
+cudaError_t launch_probe_positions(const DevCascade& C, float4* pos, cudaStream_t st);
+cudaError_t launch_ray_dirs(uint32_t rays, float jitter, float4* dirs, cudaStream_t st);
 cudaError_t launch_probe_rays(const DevCascade& C, float jitter, float* ro, float* rd, cudaStream_t st);
 
 // Arbitrary-ray queries through the same traversal (raycastFirst-like); `cursor`: one word of

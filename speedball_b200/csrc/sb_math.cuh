@@ -33,6 +33,12 @@ __device__ __forceinline__ void kahan_fma(float& s, float& c, float w, float x) 
     s = t;
 }
 
+// The probe of an update slot (both less than probeTotal).
+__device__ __forceinline__ uint32_t probe_of(const DevCascade& C, uint32_t slot) {
+    const uint32_t p = C.probeOffset + slot;
+    return p < C.probeTotal ? p : p - C.probeTotal;
+}
+
 // Probe position, gi_probes.js:1714-1726 (relocation x classifyStrength = 0).
 __device__ __forceinline__ float3 probe_world_pos(const DevCascade& C, uint32_t p) {
     uint32_t ix = p % C.res[0], iy = (p / C.res[0]) % C.res[1], iz = p / (C.res[0] * C.res[1]);

@@ -66,8 +66,7 @@ __device__ __forceinline__ void primary_ray(const WaveCtx& W, const uint4* tl, b
     const DevCascade& C = W.C;
     uint32_t slot, k;
     ray_of(W, g, W.order != 0, slot, k);
-    const uint32_t probeIndex = (C.probeOffset + slot) % C.probeTotal;
-    const float3 ro = probe_world_pos(C, probeIndex);
+    const float3 ro = slot_origin(C, slot);
     const float3 rd = ray_dir(k, C.rays, W.P.frameJitter);
     float bestT, bu, bv;
     int tri, inst;
@@ -111,7 +110,7 @@ __device__ __forceinline__ uint32_t take(uint32_t* cursor, uint32_t want) {
 
 // Stage A on the 8-wide tree. next(want, g) gives the lanes in `want` their
 // item-local issue positions (ok: this lane has one) and returns false when none
-// are left; dir(k) is ray direction k.
+// are left; dir(k, inv) is ray direction k with its inverse.
 //
 // The moved slots' hits go to the ray records (free until the shading), the tree's
 // to the hit records; emission takes the nearer one.
@@ -120,15 +119,15 @@ __device__ __forceinline__ void primary_moved(const WaveCtx& W, Walk2Shared& sm,
     const DevCascade& C = W.C;
     const uint32_t lane = threadIdx.x & 31u;
     uint4* out = reinterpret_cast<uint4*>(C.rayData);
-    auto gen = [&](bool& more, uint32_t want, float3& o, float3& d, float& tmax, uint32_t& tag) {
+    auto gen = [&](bool& more, uint32_t want, float3& o, float3& d, float3& winv, float& tmax, uint32_t& tag) {
         uint32_t g;
         bool ok;
         more = next(want, g, ok);
         if (!ok || !(want >> lane & 1u)) return false;
         uint32_t slot, k;
         ray_of(W, g, W.order != 0, slot, k);
-        o = probe_world_pos(C, (C.probeOffset + slot) % C.probeTotal);
-        d = dir(k);
+        o = slot_origin(C, slot);
+        d = dir(k, winv);
         tmax = T_MAX;
         tag = slot * C.rays + k;
         return true;
@@ -140,12 +139,12 @@ __device__ __forceinline__ void primary_moved(const WaveCtx& W, Walk2Shared& sm,
         return;
     }
     for (bool more = true; more;) {  // a BLAS too deep for it: one ray per lane
-        float3 o, d;
+        float3 o, d, winv;
         float t, bu = 0.0f, bv = 0.0f;
         uint32_t tag;
-        if (!gen(more, ALL_LANES, o, d, t, tag)) continue;
+        if (!gen(more, ALL_LANES, o, d, winv, t, tag)) continue;
         int tri = -1, inst = -1;
-        dyn_walk<false>(W.S, o, d, mk(1.0f / d.x, 1.0f / d.y, 1.0f / d.z), t, tri, inst, bu, bv, vis, W.err);
+        dyn_walk<false>(W.S, o, d, winv, t, tri, inst, bu, bv, vis, W.err);
         out[tag] = make_uint4((uint32_t)tri, (uint32_t)inst, __float_as_uint(t), pack_uv(bu, bv));
     }
 }
@@ -164,9 +163,8 @@ __device__ __forceinline__ uint32_t primary_walk8(const WaveCtx& W, const WalkSm
         if (!ok || !(want >> lane & 1u)) return false;
         uint32_t slot, k;
         ray_of(W, g, W.order != 0, slot, k);
-        o = probe_world_pos(C, (C.probeOffset + slot) % C.probeTotal);
-        d = dir(k);
-        winv = mk(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
+        o = slot_origin(C, slot);
+        d = dir(k, winv);
         tag = slot * C.rays + k;
         tmax = T_MAX;
         hit = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u);
@@ -192,7 +190,7 @@ __device__ __forceinline__ void clear_light(const WaveCtx& W, uint32_t tag) {
 template <class Next>
 __device__ __forceinline__ void shadow_moved(const WaveCtx& W, Walk2Shared& sm, Next next, Visits& vis) {
     const uint32_t lane = threadIdx.x & 31u;
-    auto gen = [&](bool& more, uint32_t want, float3& o, float3& d, float& tmax, uint32_t& tag) {
+    auto gen = [&](bool& more, uint32_t want, float3& o, float3& d, float3& winv, float& tmax, uint32_t& tag) {
         uint32_t j;
         bool ok;
         more = next(want, j, ok);
@@ -200,6 +198,7 @@ __device__ __forceinline__ void shadow_moved(const WaveCtx& W, Walk2Shared& sm, 
         const float4 a = W.jobs[2 * j], b = W.jobs[2 * j + 1];
         o = xyz(a);
         d = xyz(b);
+        winv = mk(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
         tmax = a.w;
         tag = j;
         return true;
@@ -214,12 +213,12 @@ __device__ __forceinline__ void shadow_moved(const WaveCtx& W, Walk2Shared& sm, 
         return;
     }
     for (bool more = true; more;) {
-        float3 o, d;
+        float3 o, d, winv;
         float t, u = 0.0f, v = 0.0f;
         uint32_t tag;
-        if (!gen(more, ALL_LANES, o, d, t, tag)) continue;
+        if (!gen(more, ALL_LANES, o, d, winv, t, tag)) continue;
         int tri = -1, inst = -1;
-        if (dyn_walk<true>(W.S, o, d, mk(1.0f / d.x, 1.0f / d.y, 1.0f / d.z), t, tri, inst, u, v, vis, W.err))
+        if (dyn_walk<true>(W.S, o, d, winv, t, tri, inst, u, v, vis, W.err))
             fin(tag, t, make_uint4(0u, 0u, 0u, 0u), true);
     }
 }
@@ -278,8 +277,7 @@ __device__ __forceinline__ uint32_t emit_ray(const WaveCtx& W, bool active, uint
         if (h.x != 0xFFFFFFFFu) {
             tri = (int)h.x;
             const uint32_t inst = h.y;
-            const float3 ro = probe_world_pos(C, (C.probeOffset + slot) % C.probeTotal);
-            const float3 rd = ray_dir(k, N, W.P.frameJitter);
+            const float3 ro = slot_origin(C, slot), rd = wave_dir(W, k);
             const float t = refine_t(W.S, (uint32_t)tri, inst, ro, rd);
             fr = hit_frame(W, (uint32_t)tri, inst, ro, rd, t, -1);
             h.y = inst | (fr.faceFwd ? 0x80000000u : 0u);
@@ -345,9 +343,7 @@ __device__ __forceinline__ void shade_ray(const WaveCtx& W, uint32_t g) {
     uint32_t slot, k;
     ray_of(W, g, false, slot, k);
     const uint32_t rayIdx = slot * N + k;
-    uint32_t probeIndex = (C.probeOffset + slot) % C.probeTotal;
-    float3 ro = probe_world_pos(C, probeIndex);
-    float3 rd = ray_dir(k, N, W.P.frameJitter);
+    const float3 ro = slot_origin(C, slot), rd = wave_dir(W, k);
     uint4 h = C.hits[rayIdx];
     float3 outRgb;
     float hitT = -1.0f;
@@ -422,22 +418,36 @@ __device__ __forceinline__ uint32_t job_count(const WaveCtx& W) {
     return min(*(volatile uint32_t*)&W.work[2], W.jobCap);
 }
 
-// The N ray directions of a solve, by a CTA (for stage A; walk_shared synchronizes).
-__device__ __forceinline__ void ray_dirs(const WaveCtx& W, float4* dirs) {
+// The ray directions of a solve, by a CTA: for the later stages, and with their
+// inverses for this CTA's walks (walk_shared synchronizes).
+__device__ __forceinline__ void write_dirs(const WaveCtx& W) {
     for (uint32_t k = threadIdx.x; k < W.C.rays; k += blockDim.x) {
         const float3 d = ray_dir(k, W.C.rays, W.P.frameJitter);
-        dirs[k] = make_float4(d.x, d.y, d.z, 0.0f);
+        W.dirs[k] = make_float4(d.x, d.y, d.z, 0.0f);
     }
+}
+__device__ __forceinline__ void stage_dirs(const WaveCtx& W, float4* sm) {
+    for (uint32_t k = threadIdx.x; k < W.C.rays; k += blockDim.x) {
+        const float3 d = ray_dir(k, W.C.rays, W.P.frameJitter);
+        sm[2 * k] = make_float4(d.x, d.y, d.z, 0.0f);
+        sm[2 * k + 1] = make_float4(1.0f / d.x, 1.0f / d.y, 1.0f / d.z, 0.0f);
+    }
+}
+__device__ __forceinline__ float3 staged_dir(const float4* sm, uint32_t k, float3& winv) {
+    winv = xyz(sm[2 * k + 1]);
+    return xyz(sm[2 * k]);
 }
 
 // The 8-wide tree (bvhKind 1).
 __global__ void __launch_bounds__(256, SB_WALK8_MIN_BLOCKS) k_trace_primary_walk8(WaveCtx W) {
     extern __shared__ float4 smem[];
     if (!*W.S.valid) return;
-    ray_dirs(W, smem);
-    const WalkSmem m = walk_shared(smem + W.C.rays, W.S.wideDepth + 1u, W.S.dynCount != 0u);
+    if (blockIdx.x == 0) write_dirs(W);
+    stage_dirs(W, smem);
+    const WalkSmem m = walk_shared(smem + 2 * W.C.rays, W.S.wideDepth + 1u, W.S.dynCount != 0u);
     Visits vis = {0, 0, 0, 0};
-    const uint32_t nRays = primary_stage(W, m, [&](uint32_t k) { return xyz(smem[k]); }, vis);
+    const uint32_t nRays = primary_stage(
+        W, m, [&](uint32_t k, float3& winv) { return staged_dir(smem, k, winv); }, vis);
     add_visits(W.counters, 2, nRays, vis);
 }
 
@@ -456,6 +466,7 @@ __global__ void __launch_bounds__(256, SB_PRIMARY_MIN_BLOCKS) k_trace_primary(Wa
     const bool pairs = closest_pairs(W.S);
     const uint4* tl = stage_tlas(W, sTlas, pairs);
     if (!*W.S.valid) return;
+    if (blockIdx.x == 0) write_dirs(W);
     const uint32_t total = W.slotCount * W.C.rays;
     const uint32_t lane = threadIdx.x & 31u;
     Visits vis = {0, 0, 0, 0};
@@ -575,8 +586,8 @@ __global__ void __launch_bounds__(128) k_shade(WaveCtx W) {
 
 // Stage C alone over probe slots [0, slotCount) from the records already in
 // C.hits / C.vis (the adjoint re-evaluates shading this way).
-cudaError_t launch_shade(const DevScene& S, const DevCascade& C, const DevParams& P, uint32_t slotCount,
-                         cudaStream_t st) {
+cudaError_t launch_shade(const DevScene& S, const DevCascade& C, const DevParams& P, const float4* dirs,
+                         uint32_t slotCount, cudaStream_t st) {
     if (slotCount == 0) return cudaSuccess;
     WaveCtx W{};
     W.S = S;
@@ -584,6 +595,8 @@ cudaError_t launch_shade(const DevScene& S, const DevCascade& C, const DevParams
     W.P = P;
     W.slotBegin = 0;
     W.slotCount = slotCount;
+    W.rayMagic = div_magic(C.rays);
+    W.dirs = const_cast<float4*>(dirs);
     const uint32_t rays = slotCount * C.rays;
     k_shade<<<(rays + 127) / 128, 128, 0, st>>>(W);
     note_launch();
@@ -606,8 +619,8 @@ static int walk8_grid(const void* kernel, int block, size_t smem, const TraceTun
 }
 
 cudaError_t launch_trace(const DevScene& S, const DevCascade& C, const DevParams& P, uint32_t* err,
-                         unsigned long long* counters, uint32_t* work, const TraceTuning& tune, cudaStream_t st,
-                         float4* jobs, uint32_t jobCap, uint32_t slotBegin, uint32_t slotCount,
+                         unsigned long long* counters, uint32_t* work, float4* dirs, const TraceTuning& tune,
+                         cudaStream_t st, float4* jobs, uint32_t jobCap, uint32_t slotBegin, uint32_t slotCount,
                          cudaEvent_t afterPrimary, cudaEvent_t afterShadow, cudaEvent_t afterClosest) {
     if (slotCount == 0) return cudaSuccess;
     WaveCtx W;
@@ -619,8 +632,11 @@ cudaError_t launch_trace(const DevScene& S, const DevCascade& C, const DevParams
     W.work = work;
     W.jobs = jobs;
     W.jobCap = jobCap;
+    W.dirs = dirs;
     W.slotBegin = slotBegin;
     W.slotCount = slotCount;
+    W.slotMagic = div_magic(slotCount);
+    W.rayMagic = div_magic(C.rays);
     W.order = tune.sortKey == 1 ? 0u : 1u;  // direction-major (sortKey 0, and 2 over probe tiles); 1 = probe-major
     // the scene-BVH walk reads no TLAS
     uint32_t smemNodes = !S.flatOn && S.tlasNodeCount <= tune.smemTlasNodes ? S.tlasNodeCount : 0u;
@@ -636,7 +652,7 @@ cudaError_t launch_trace(const DevScene& S, const DevCascade& C, const DevParams
     const uint32_t rays = slotCount * C.rays;
     const int block = (int)tune.block;
     const uint32_t smem8 = walk_smem(S.wideDepth + 1u, S.dynCount != 0u, tune.block);
-    const uint32_t smemP = smem8 + C.rays * (uint32_t)sizeof(float4);
+    const uint32_t smemP = smem8 + 2u * C.rays * (uint32_t)sizeof(float4);
     if (S.wideNodes)
         k_trace_primary_walk8<<<walk8_grid((const void*)k_trace_primary_walk8, block, smemP, tune, rays), block, smemP,
                                 st>>>(W);
@@ -675,8 +691,9 @@ __global__ void __launch_bounds__(256, SB_WALK8_MIN_BLOCKS) k_trace_primary_batc
     extern __shared__ float4 smem[];
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t first = batch_item(B, (uint32_t)((uint64_t)blockIdx.x * B.totalRays / gridDim.x));
-    ray_dirs(B.it[first].W, smem);
-    const WalkSmem m = walk_shared(smem + B.maxRays, B.wideDepth + 1u, B.moved != 0u);
+    for (uint32_t j = blockIdx.x; j < B.n; j += gridDim.x) write_dirs(B.it[j].W);
+    stage_dirs(B.it[first].W, smem);
+    const WalkSmem m = walk_shared(smem + 2 * B.maxRays, B.wideDepth + 1u, B.moved != 0u);
     Visits vis = {0, 0, 0, 0};
     uint32_t nRays = 0;
     uint32_t i = first;
@@ -684,8 +701,11 @@ __global__ void __launch_bounds__(256, SB_WALK8_MIN_BLOCKS) k_trace_primary_batc
         const WaveCtx& W = B.it[i].W;
         if (!*W.S.valid) continue;
         if (W.S.wideNodes) {
-            nRays += primary_stage(W, m, [&](uint32_t k) {
-                return i == first ? xyz(smem[k]) : ray_dir(k, W.C.rays, W.P.frameJitter);
+            nRays += primary_stage(W, m, [&](uint32_t k, float3& winv) {
+                if (i == first) return staged_dir(smem, k, winv);
+                const float3 d = ray_dir(k, W.C.rays, W.P.frameJitter);
+                winv = mk(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
+                return d;
             }, vis);
             continue;
         }
@@ -782,7 +802,7 @@ const void* trace_batch_kernel(int stage) {
 
 uint32_t trace_batch_smem(const BatchArgs& B, uint32_t threads) {
     const uint32_t smem =
-        walk_smem(B.wideDepth + 1u, B.moved != 0u, threads) + B.maxRays * (uint32_t)sizeof(float4);
+        walk_smem(B.wideDepth + 1u, B.moved != 0u, threads) + 2u * B.maxRays * (uint32_t)sizeof(float4);
     if (smem > 48u * 1024u)
         for (int stage = 0; stage <= 2; stage += 2)
             cudaFuncSetAttribute(trace_batch_kernel(stage), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -841,8 +861,9 @@ __global__ void k_occluded(DevScene S, const float* ro, const float* rd, const f
                  : 0;
 }
 
-// The same on the 8-wide tree.
-template <bool ANY>
+// The same on the 8-wide tree. MOVED: the scene has moved slots, walked as a ray is
+// taken; without that walk's code the kernel keeps its registers (QUERY_MOVED_FIGURES).
+template <bool ANY, bool MOVED>
 __global__ void __launch_bounds__(256, QUERY_MIN_BLOCKS) k_query_walk8(DevScene S, const float* ro, const float* rd,
                                                                           const float* maxDist, uint32_t n,
                                                                           float* tOut, int32_t* triOut,
@@ -867,7 +888,7 @@ __global__ void __launch_bounds__(256, QUERY_MIN_BLOCKS) k_query_walk8(DevScene 
         tag = i;
         int tri = -1, inst = -1;
         float bu = 0.0f, bv = 0.0f;
-        const bool blocked = dyn_walk<ANY>(S, o, d, winv, tmax, tri, inst, bu, bv, vis, err);
+        const bool blocked = MOVED && dyn_walk<ANY>(S, o, d, winv, tmax, tri, inst, bu, bv, vis, err);
         hit = make_uint4((uint32_t)tri, (uint32_t)inst, 0u, 0u);
         if (ANY && blocked) out[i] = 1;
         return !(ANY && blocked);
@@ -904,8 +925,9 @@ cudaError_t launch_raycast(const DevScene& S, const float* ro, const float* rd, 
         const size_t smem = walk_smem(S.wideDepth + 1u, false, 256u);
         cudaError_t e = cudaMemsetAsync(cursor, 0, 4, st);
         if (e != cudaSuccess) return e;
-        k_query_walk8<false><<<walk8_grid((const void*)k_query_walk8<false>, 256, smem, query_tuning(numSms), n), 256,
-                               smem, st>>>(S, ro, rd, nullptr, n, tOut, triOut, instOut, nullptr, cursor, err);
+        const auto kernel = S.dynCount ? k_query_walk8<false, true> : k_query_walk8<false, false>;
+        kernel<<<walk8_grid((const void*)kernel, 256, smem, query_tuning(numSms), n), 256, smem, st>>>(
+            S, ro, rd, nullptr, n, tOut, triOut, instOut, nullptr, cursor, err);
     } else {
         k_raycast<<<(n + 127) / 128, 128, 0, st>>>(S, ro, rd, n, tOut, triOut, instOut, err);
     }
@@ -922,8 +944,9 @@ cudaError_t launch_occluded(const DevScene& S, const float* ro, const float* rd,
         const size_t smem = walk_smem(S.wideDepth + 1u, false, 256u);
         cudaError_t e = cudaMemsetAsync(cursor, 0, 4, st);
         if (e != cudaSuccess) return e;
-        k_query_walk8<true><<<walk8_grid((const void*)k_query_walk8<true>, 256, smem, query_tuning(numSms), n), 256,
-                              smem, st>>>(S, ro, rd, maxDist, n, nullptr, nullptr, nullptr, out, cursor, err);
+        const auto kernel = S.dynCount ? k_query_walk8<true, true> : k_query_walk8<true, false>;
+        kernel<<<walk8_grid((const void*)kernel, 256, smem, query_tuning(numSms), n), 256, smem, st>>>(
+            S, ro, rd, maxDist, n, nullptr, nullptr, nullptr, out, cursor, err);
     } else {
         k_occluded<<<(n + 127) / 128, 128, 0, st>>>(S, ro, rd, maxDist, n, out, err);
     }
@@ -940,7 +963,7 @@ __global__ void k_probe_rays(const DevCascade C, float jitter, float* ro, float*
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= C.updatedCount * C.rays) return;
     const uint32_t slot = i / C.rays, k = i % C.rays;
-    const float3 o = probe_world_pos(C, (C.probeOffset + slot) % C.probeTotal);
+    const float3 o = slot_origin(C, slot);
     const float3 d = ray_dir(k, C.rays, jitter);
     ro[3 * i] = o.x; ro[3 * i + 1] = o.y; ro[3 * i + 2] = o.z;
     rd[3 * i] = d.x; rd[3 * i + 1] = d.y; rd[3 * i + 2] = d.z;
@@ -953,8 +976,8 @@ __global__ void k_emitter_vis(DevScene S, DevCascade C, DevParams P, uint32_t* e
     const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
     const uint32_t slot = gid / EMITTER_CAP, e = gid % EMITTER_CAP;
     if (slot >= C.updatedCount || e >= C.emitterCount || !*S.valid) return;
-    const uint32_t probeIndex = (C.probeOffset + slot) % C.probeTotal;
-    const float3 ro = probe_world_pos(C, probeIndex);
+    const uint32_t probeIndex = probe_of(C, slot);
+    const float3 ro = slot_origin(C, slot);
     const float* L = C.lights + (size_t)(C.emitterBase + e) * 17u;
     const float3 center = mk(L[1], L[2], L[3]);
     const float sourceRadius = fmaxf(L[14], 0.0f);
@@ -991,6 +1014,31 @@ cudaError_t launch_emitter_vis(const DevScene& S, const DevCascade& C, const Dev
     const uint32_t n = C.updatedCount * EMITTER_CAP;
     if (n == 0 || C.emitterCount == 0) return cudaSuccess;
     k_emitter_vis<<<(n + 127) / 128, 128, 0, st>>>(S, C, P, err);
+    note_launch();
+    return cudaGetLastError();
+}
+
+// The tables of slot_origin (with a cascade's grid) and wave_dir.
+__global__ void k_probe_positions(DevCascade C, float4* pos) {
+    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= C.probeTotal) return;
+    const float3 v = probe_world_pos(C, p);
+    pos[p] = make_float4(v.x, v.y, v.z, 0.0f);
+}
+cudaError_t launch_probe_positions(const DevCascade& C, float4* pos, cudaStream_t st) {
+    if (C.probeTotal == 0) return cudaSuccess;
+    k_probe_positions<<<(C.probeTotal + 255) / 256, 256, 0, st>>>(C, pos);
+    note_launch();
+    return cudaGetLastError();
+}
+__global__ void k_ray_dirs(uint32_t rays, float jitter, float4* dirs) {
+    const uint32_t k = threadIdx.x;
+    if (k >= rays) return;
+    const float3 d = ray_dir(k, rays, jitter);
+    dirs[k] = make_float4(d.x, d.y, d.z, 0.0f);
+}
+cudaError_t launch_ray_dirs(uint32_t rays, float jitter, float4* dirs, cudaStream_t st) {
+    k_ray_dirs<<<1, MAX_RAYS, 0, st>>>(rays, jitter, dirs);
     note_launch();
     return cudaGetLastError();
 }

@@ -56,8 +56,7 @@ __device__ __forceinline__ void walk2(const DevScene& S, Walk2Shared& sm, Gen ge
             if (done && state == ENDED && blocked) fin(tag, tmax, make_uint4(0u, 0u, 0u, 0u), true);
             const uint32_t want = __ballot_sync(ALL_LANES, done && !have);
             if (more && want) {
-                if (gen(more, want, wo, wd, tmax, tag)) {
-                    winv = mk(1.0f / wd.x, 1.0f / wd.y, 1.0f / wd.z);
+                if (gen(more, want, wo, wd, winv, tmax, tag)) {
                     sm.best[lane] = (unsigned long long)__float_as_uint(tmax) << 32 | 0xFFFFFFFFull;
                     if (!ANY) sm.hit[lane] = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u);
                     k = iter = 0;

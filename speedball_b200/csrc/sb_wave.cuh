@@ -214,18 +214,24 @@ __device__ __forceinline__ void ray_of(const WaveCtx& W, uint32_t g, bool dirMaj
     const uint32_t N = W.C.rays;
     uint32_t s;
     if (dirMajor) {
-        k = g / W.slotCount;
-        s = g - k * W.slotCount;
+        k = divide(g, W.slotCount, W.slotMagic, s);
         if (W.C.issueOrder) {  // a permutation of every probe (the solve covers them all from slot 0)
             slot = __ldg(W.C.issueOrder + s);
             return;
         }
     } else {
-        s = g / N;
-        k = g - s * N;
+        s = divide(g, N, W.rayMagic, k);
     }
     slot = W.slotBegin + s;
 }
+
+// Origin and direction k of a slot's rays (probe_world_pos and ray_dir) from the
+// tables: evaluated per ray they were a fifth of the emission's instructions and, at
+// the few lanes that take new rays, of the walks'.
+__device__ __forceinline__ float3 slot_origin(const DevCascade& C, uint32_t slot) {
+    return xyz(__ldg(C.probePos + probe_of(C, slot)));
+}
+__device__ __forceinline__ float3 wave_dir(const WaveCtx& W, uint32_t k) { return xyz(__ldg(W.dirs + k)); }
 
 // SH-9 sky radiance of a miss (gi_probes.js:2190-2206).
 __device__ __forceinline__ float3 sky_sh(const DevParams& P, float3 rd) {
