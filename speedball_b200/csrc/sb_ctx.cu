@@ -94,11 +94,11 @@ struct sb_ctx {
     size_t stageCap = 0;
 
     uint32_t* dErr = nullptr;
-    uint32_t* dGate = nullptr;     // 16 layout verdicts, one per cached refit range, then their 16 subtree counts
+    uint32_t* dGate = nullptr;     // the cached refit ranges' verdicts, subtree and top-node counts, progress
     // Refit ranges whose parent links and layout checks are current: valid while
     // packEpoch is unchanged (no upload touched nodes, indices or materials since).
     struct RefitRange { uint32_t root = 0, end = 0, epoch = 0; bool used = false; };
-    RefitRange refitRanges[16];
+    RefitRange refitRanges[REFIT_RANGES];
     uint32_t packEpoch = 1, refitNext = 0;
     uint32_t* dWork = nullptr;
     float4* dDirs = nullptr;  // ray directions: a batch's items (a solve: the first), then the adjoint's
@@ -473,7 +473,7 @@ sb_status sb_create(const sb_device_opts* opts, sb_ctx** out) {
         ctx->tune.numSms = ctx->numSms;
         if (cudaStreamCreateWithFlags(&ctx->ownStream, cudaStreamNonBlocking) != cudaSuccess) { st = SB_ERR_CUDA; break; }
         ctx->stream = ctx->ownStream;
-        if (cudaMalloc(&ctx->dErr, 4) != cudaSuccess || cudaMalloc(&ctx->dGate, 32 * 4) != cudaSuccess ||
+        if (cudaMalloc(&ctx->dErr, 4) != cudaSuccess || cudaMalloc(&ctx->dGate, 4 * REFIT_RANGES * 4) != cudaSuccess ||
             cudaMalloc(&ctx->dWork, (QUERY_CURSOR + 8) * 4) != cudaSuccess ||
             cudaMalloc(&ctx->dDirs, (ADJOINT_DIRS + MAX_RAYS) * sizeof(float4)) != cudaSuccess ||
             cudaMalloc(&ctx->dCounters, 16 * 8) != cudaSuccess ||
@@ -2016,7 +2016,7 @@ sb_status sb_refit_blas(sb_ctx* ctx, uint32_t root, uint32_t end) {
     if (s != SB_OK) return s;
     // a range checked on the current layout refits with the bottom-up pass alone
     int slot = -1;
-    for (int k = 0; k < 16; ++k) {
+    for (int k = 0; k < (int)REFIT_RANGES; ++k) {
         const auto& r = ctx->refitRanges[k];
         if (r.used && r.root == root && r.end == end && r.epoch == ctx->packEpoch) slot = k;
     }
@@ -2025,7 +2025,7 @@ sb_status sb_refit_blas(sb_ctx* ctx, uint32_t root, uint32_t end) {
         // relinking rewrites the parents of [root, end): overlapping cached ranges are stale
         for (auto& r : ctx->refitRanges)
             if (r.used && r.root < end && root < r.end) r.used = false;
-        slot = (int)(ctx->refitNext++ % 16u);
+        slot = (int)(ctx->refitNext++ % REFIT_RANGES);
         ctx->refitRanges[slot] = {root, end, ctx->packEpoch, true};
     }
     CK(launch_refit_blas(ctx->B, root, end, ctx->dErr, ctx->dGate + slot, ctx->stream, validated));

@@ -25,8 +25,16 @@ __device__ __forceinline__ void bad(uint32_t* gate, uint32_t* err) {
 }
 
 // ------------------------------------------------------------- BLAS refit
-__global__ void k_refit_reset(uint32_t* parent, uint32_t* arrive, uint32_t root, uint32_t end) {
+// The words of a cached range: its verdict, its number of subtrees, the number of top
+// nodes in its plan (NONE: no plan), the subtrees finished in a running refit.
+constexpr uint32_t GATE = 0, GATE_SUBS = REFIT_RANGES, GATE_TOPS = 2 * REFIT_RANGES, GATE_DONE = 3 * REFIT_RANGES;
+
+__global__ void k_refit_reset(uint32_t* parent, uint32_t* arrive, uint32_t root, uint32_t end, uint32_t* gate) {
     uint32_t i = root + blockIdx.x * blockDim.x + threadIdx.x;
+    if (i == root) {
+        gate[GATE] = 1u;  // valid until a check fails
+        gate[GATE_SUBS] = gate[GATE_TOPS] = gate[GATE_DONE] = 0u;
+    }
     if (i >= end) return;
     parent[i] = NONE;
     arrive[i] = 0u;
@@ -81,247 +89,285 @@ __global__ void k_refit_orphans(const uint32_t* parent, uint32_t root, uint32_t 
     if (parent[i] == NONE) bad(gate, err);
 }
 
-__device__ __forceinline__ float vload(const uint32_t* p) { return __uint_as_float(*(const volatile uint32_t*)p); }
+__device__ __forceinline__ uint32_t arrive_at(uint32_t* counter) {
+    uint32_t prev;
+    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(prev) : "l"(counter) : "memory");
+    return prev;
+}
 
-#ifndef SB_REFIT_ACQREL
-#define SB_REFIT_ACQREL 1
-#endif
-// One node of the node-by-node refit: a leaf's box (and its re-gathered
-// triangles), then the climb: the second child to finish computes its parent.
-__device__ __forceinline__ void refit_node_climb(uint32_t* nodes, const uint32_t* triIndex, const float* vertexData,
-                                                 const uint32_t* triMaterial, const uint32_t* matBits, float4* tris,
-                                                 const uint32_t* parent, uint32_t* arrive, uint32_t i, uint4* pairs) {
-    uint32_t info = nodes[8 * i + 7];
-    if (info == INTERIOR) return;
-    uint32_t off = info & 0x00FFFFFFu, cnt = info >> 24;
-    if (cnt != 0u) {
-        float mnx = INFINITY, mny = INFINITY, mnz = INFINITY, mxx = -INFINITY, mxy = -INFINITY, mxz = -INFINITY;
-        for (uint32_t t = off; t < off + cnt; ++t) {
-            float3 p[3];
-            for (int k = 0; k < 3; ++k) {
-                const float* v = vertexData + (size_t)triIndex[3 * t + k] * 8u;
-                float x = v[0], y = v[1], z = v[2];
-                p[k] = make_float3(x, y, z);
-                if (x < mnx) mnx = x;
-                if (x > mxx) mxx = x;
-                if (y < mny) mny = y;
-                if (y > mxy) mxy = y;
-                if (z < mnz) mnz = z;
-                if (z > mxz) mxz = z;
-            }
-            // re-gather the pre-gathered triangle from the deformed vertices
-            tris[3 * t] = make_float4(p[0].x, p[0].y, p[0].z, __uint_as_float(matBits[triMaterial[t]]));
-            tris[3 * t + 1] = make_float4(p[1].x, p[1].y, p[1].z, 0.0f);
-            tris[3 * t + 2] = make_float4(p[2].x, p[2].y, p[2].z, 0.0f);
-        }
-        uint32_t* n = nodes + 8 * i;
-        n[0] = __float_as_uint(mnx); n[1] = __float_as_uint(mny); n[2] = __float_as_uint(mnz);
-        n[3] = __float_as_uint(mxx); n[4] = __float_as_uint(mxy); n[5] = __float_as_uint(mxz);
+// What a refit reads of the scene, and writes.
+struct RefitArrays {
+    uint32_t* nodes;
+    const uint32_t* triIndex;
+    const float4* vertices;  // two float4 per vertex, the position first
+    const uint32_t *triMaterial, *matBits;
+    float4* tris;
+    const uint32_t* parent;
+    uint32_t* arrive;
+    uint4* pairs;
+};
+
+// A leaf's box over its triangles in order (cnt > 0), and its pre-gathered triangles
+// from the deformed vertices. Four triangles' loads are in flight together.
+__device__ __forceinline__ void refit_leaf(const RefitArrays& R, uint32_t off, uint32_t cnt, float box[6]) {
+    for (int k = 0; k < 3; ++k) {
+        box[k] = INFINITY;
+        box[3 + k] = -INFINITY;
     }
-    uint32_t node = i;
+    for (uint32_t at = 0; at < cnt; at += 4u) {
+        float4 v[4][3];
+        uint32_t bits[4];
+#pragma unroll
+        for (uint32_t j = 0; j < 4u; ++j) {
+            const uint32_t t = off + min(at + j, cnt - 1u);
+            bits[j] = __ldg(R.matBits + __ldg(R.triMaterial + t));
+#pragma unroll
+            for (int k = 0; k < 3; ++k) v[j][k] = __ldg(R.vertices + 2 * (size_t)__ldg(R.triIndex + 3 * t + k));
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < 4u; ++j) {
+            if (at + j >= cnt) break;
+            const uint32_t t = off + at + j;
+#pragma unroll
+            for (int k = 0; k < 3; ++k) {
+                const float p[3] = {v[j][k].x, v[j][k].y, v[j][k].z};
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    if (p[a] < box[a]) box[a] = p[a];
+                    if (p[a] > box[3 + a]) box[3 + a] = p[a];
+                }
+                R.tris[3 * t + k] = make_float4(p[0], p[1], p[2], k == 0 ? __uint_as_float(bits[j]) : 0.0f);
+            }
+        }
+    }
+}
+
+// A node's box from its children's.
+__device__ __forceinline__ void join_boxes(const uint32_t lb[6], const uint32_t rb[6], uint32_t box[6]) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        box[k] = __float_as_uint(js_min(__uint_as_float(lb[k]), __uint_as_float(rb[k])));
+        box[3 + k] = __float_as_uint(js_max(__uint_as_float(lb[3 + k]), __uint_as_float(rb[3 + k])));
+    }
+}
+__device__ __forceinline__ void store_box(uint32_t* nodes, uint32_t i, const uint32_t b[6]) {
+    *reinterpret_cast<uint4*>(nodes + 8 * (size_t)i) = make_uint4(b[0], b[1], b[2], b[3]);
+    *reinterpret_cast<uint2*>(nodes + 8 * (size_t)i + 4) = make_uint2(b[4], b[5]);
+}
+
+// The climb through global memory: the second child to finish computes its parent.
+__device__ __forceinline__ void refit_climb(const RefitArrays& R, uint32_t node) {
     for (;;) {
-        uint32_t p = parent[node];
+        const uint32_t p = R.parent[node];
         if (p == NONE) break;
         // arrival: release publishes this thread's box stores, acquire orders the
         // sibling's box reads below after the sibling's release (one acq_rel atomic)
-#if SB_REFIT_ACQREL
-        uint32_t prev;
-        asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(prev) : "l"(arrive + p) : "memory");
-        if (prev == 0u) break;
-#else
-        __threadfence();
-        if (atomicAdd(&arrive[p], 1u) == 0u) break;
-        __threadfence();
-#endif
-        arrive[p] = 0u;  // both children arrived: ready for the next refit of this range
-        uint32_t l = p + 1;
-        uint32_t r = *(const volatile uint32_t*)(nodes + 8 * l + 6);
-        const uint32_t* L = nodes + 8 * l;
-        const uint32_t* R = nodes + 8 * r;
-        uint32_t lb[6], rb[6];
+        if (arrive_at(R.arrive + p) == 0u) break;
+        R.arrive[p] = 0u;  // both children arrived: ready for the next refit of this range
+        const uint32_t l = p + 1;
+        const uint32_t r = *(const volatile uint32_t*)(R.nodes + 8 * l + 6);
+        uint32_t lb[6], rb[6], box[6];
 #pragma unroll
         for (int k = 0; k < 6; ++k) {
-            lb[k] = *(const volatile uint32_t*)(L + k);
-            rb[k] = *(const volatile uint32_t*)(R + k);
+            lb[k] = *(const volatile uint32_t*)(R.nodes + 8 * l + k);
+            rb[k] = *(const volatile uint32_t*)(R.nodes + 8 * r + k);
         }
-        uint32_t* n = nodes + 8 * p;
-#pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            n[k] = __float_as_uint(js_min(__uint_as_float(lb[k]), __uint_as_float(rb[k])));
-            n[3 + k] = __float_as_uint(js_max(__uint_as_float(lb[3 + k]), __uint_as_float(rb[3 + k])));
-        }
-        if (pairs) store_pair_boxes(pairs + 4u * p, lb, rb);  // the traversal's copy of both child boxes
+        join_boxes(lb, rb, box);
+        store_box(R.nodes, p, box);
+        if (R.pairs) store_pair_boxes(R.pairs + 4u * p, lb, rb);  // the traversal's copy of both child boxes
         node = p;
     }
 }
 
-__global__ void k_refit_run(uint32_t* nodes, const uint32_t* triIndex, const float* vertexData,
-                            const uint32_t* triMaterial, const uint32_t* matBits, float4* tris,
-                            const uint32_t* parent, uint32_t* arrive, uint32_t root, uint32_t end,
-                            const uint32_t* gate, uint4* pairs, uint32_t* err) {
-    uint32_t i = root + blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= end) return;
-    if (*gate == 0u) {
-        if (i == root) latch(err, ERR_LAYOUT);  // the range's layout verdict stands until a new upload
-        return;
-    }
-    refit_node_climb(nodes, triIndex, vertexData, triMaterial, matBits, tris, parent, arrive, i, pairs);
-}
-
-// Subtrees of at most REFIT_SUB nodes refit inside one CTA: the threaded
-// layout stores a node's subtree as [i, miss(i)) (to the range end on the right
-// spine), so a CTA takes one such range, computes its leaves, and climbs with
-// shared-memory arrival counters; the thread that completes the subtree root
-// carries on through the global climb above it. The partition (every node
-// whose subtree fits while its parent's does not) is made once per validated
-// range, next to the layout checks.
-#ifndef SB_REFIT_CTA
-#define SB_REFIT_CTA 1
-#endif
-#ifndef SB_REFIT_SUB
-#define SB_REFIT_SUB 256
-#endif
-constexpr uint32_t REFIT_SUB = SB_REFIT_SUB;  // nodes per CTA subtree (= threads per CTA)
+// Subtrees of at most REFIT_SUB nodes refit inside one CTA: the threaded layout stores
+// a node's subtree as [i, miss(i)) (to the range end on the right spine), one node per
+// thread. The partition (every node whose subtree fits while its parent's does not)
+// is made once per validated range, next to the layout checks, and with it, when there
+// are at most REFIT_SUB subtrees, a plan of the nodes above them, which the CTA that
+// finishes last computes in the same way.
+//
+// What bounds it is the chain of dependent loads, not work: a deforming mesh of some
+// thousand triangles is 0.4 MB. So a thread's node, triangle indices and vertices are
+// loaded once, four triangles' at a time; the boxes climb in shared memory, one
+// level per barrier (a counter per node and its fences cost more than the levels that
+// nothing happens in); and what is above the subtrees costs one more load of their
+// boxes. The atrium's deforming mesh refits in 15 us instead of 31 node by node.
+constexpr uint32_t REFIT_SUB = 256;  // nodes per CTA subtree (= threads per CTA)
 
 __device__ __forceinline__ uint32_t sub_size(const uint32_t* nodes, uint32_t i, uint32_t end) {
     const uint32_t miss = nodes[8 * i + 6];
     return (miss > i && miss <= end) ? miss - i : end - i;
 }
 
+// The subtrees' roots from the front of the range's words in subRoots, the nodes above
+// them from the back (roots and top nodes are different nodes of the range).
 __global__ void k_refit_partition(const uint32_t* nodes, const uint32_t* parent, uint32_t root, uint32_t end,
-                                  const uint32_t* gate, uint32_t* subRoots, uint32_t* count) {
+                                  uint32_t* gate, uint32_t* subRoots) {
     const uint32_t i = root + blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= end || *gate != 1u) return;
-    if (sub_size(nodes, i, end) > REFIT_SUB) return;
+    if (i >= end || gate[GATE] != 1u) return;
+    if (sub_size(nodes, i, end) > REFIT_SUB) {
+        subRoots[end - 1u - atomicAdd(gate + GATE_TOPS, 1u)] = i;
+        return;
+    }
     const uint32_t p = parent[i];
     if (p != NONE && sub_size(nodes, p, end) <= REFIT_SUB) return;
-    subRoots[root + atomicAdd(count, 1u)] = i;  // at most end - root entries
+    subRoots[root + atomicAdd(gate + GATE_SUBS, 1u)] = i;
 }
 
-__global__ void __launch_bounds__(REFIT_SUB) k_refit_cta(uint32_t* nodes, const uint32_t* triIndex,
-                                                         const float* vertexData, const uint32_t* triMaterial,
-                                                         const uint32_t* matBits, float4* tris,
-                                                         const uint32_t* parent, uint32_t* arrive, uint32_t root,
-                                                         uint32_t end, const uint32_t* gate, uint4* pairs,
-                                                         const uint32_t* subRoots, const uint32_t* count,
-                                                         uint32_t* err) {
-    __shared__ float sBox[6 * REFIT_SUB];
-    __shared__ uint32_t sArr[REFIT_SUB];
-    const uint32_t g = *gate;
+// The plan: behind the n roots, per top node (its index, left unit, right unit, 0),
+// where units 0 .. n - 1 are the subtrees and n + t is top node t. One CTA.
+__global__ void __launch_bounds__(REFIT_SUB) k_refit_plan(const uint32_t* nodes, uint32_t root, uint32_t end,
+                                                          uint32_t* gate, uint32_t* subRoots) {
+    __shared__ uint32_t unit[2 * REFIT_SUB];
+    __shared__ uint32_t bad;
+    const uint32_t n = gate[GATE_SUBS], tops = gate[GATE_TOPS], tid = threadIdx.x;
+    const bool planned = gate[GATE] == 1u && n != 0u && n <= REFIT_SUB && tops + 1u == n &&
+                         n + 4u * tops <= end - root;
+    if (tid == 0) bad = 0u;
+    if (planned) {
+        if (tid < n) unit[tid] = subRoots[root + tid];
+        if (tid < tops) unit[n + tid] = subRoots[end - 1u - tid];
+    }
+    __syncthreads();
+    if (planned && tid < tops) {
+        const uint32_t l = unit[n + tid] + 1u, r = nodes[8 * l + 6];
+        uint32_t ul = NONE, ur = NONE;
+        for (uint32_t u = 0; u < n + tops; ++u) {
+            if (unit[u] == l) ul = u;
+            if (unit[u] == r) ur = u;
+        }
+        if (ul == NONE || ur == NONE) bad = 1u;
+        uint32_t* e = subRoots + root + n + 4u * tid;
+        e[0] = unit[n + tid];
+        e[1] = ul;
+        e[2] = ur;
+        e[3] = 0u;
+    }
+    __syncthreads();
+    if (tid == 0 && (!planned || bad)) gate[GATE_TOPS] = NONE;
+}
+
+__global__ void __launch_bounds__(REFIT_SUB) k_refit_cta(const RefitArrays R, uint32_t root, uint32_t end,
+                                                         uint32_t* gate, const uint32_t* subRoots, uint32_t* err) {
+    __shared__ uint32_t sBox[6][2 * REFIT_SUB];
+    __shared__ uint32_t sMiss[REFIT_SUB];
+    __shared__ volatile uint32_t sDone[2 * REFIT_SUB];  // the round that computed a box
+    __shared__ uint32_t sLast;
+    const uint32_t tid = threadIdx.x;
+    const uint32_t g = gate[GATE], nSub = gate[GATE_SUBS], tops = gate[GATE_TOPS];
     if (g == 0u) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) latch(err, ERR_LAYOUT);  // the range's verdict stands
+        if (blockIdx.x == 0 && tid == 0) latch(err, ERR_LAYOUT);  // the range's verdict stands
         return;
     }
     if (g != 1u) {  // no subtree partition for this layout: node by node, grid-stride
-        for (uint32_t i = root + blockIdx.x * blockDim.x + threadIdx.x; i < end; i += gridDim.x * blockDim.x)
-            refit_node_climb(nodes, triIndex, vertexData, triMaterial, matBits, tris, parent, arrive, i, pairs);
+        for (uint32_t i = root + blockIdx.x * blockDim.x + tid; i < end; i += gridDim.x * blockDim.x) {
+            const uint32_t info = R.nodes[8 * i + 7];
+            if (info == INTERIOR) continue;
+            if (info >> 24) {
+                float b[6];
+                refit_leaf(R, info & 0x00FFFFFFu, info >> 24, b);
+                uint32_t w[6];
+                for (int k = 0; k < 6; ++k) w[k] = __float_as_uint(b[k]);
+                store_box(R.nodes, i, w);
+            }
+            refit_climb(R, i);
+        }
         return;
     }
-    const uint32_t nSub = *count;
-    const uint32_t tid = threadIdx.x;
+    // one level of boxes per round: unit u (children l, r) once both are done
+    auto round = [&](uint32_t u, uint32_t l, uint32_t r, uint32_t now) {
+        if (sDone[u] != NONE || sDone[l] >= now || sDone[r] >= now) return;
+        uint32_t lb[6], rb[6], box[6];
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            lb[k] = sBox[k][l];
+            rb[k] = sBox[k][r];
+        }
+        join_boxes(lb, rb, box);
+#pragma unroll
+        for (int k = 0; k < 6; ++k) sBox[k][u] = box[k];
+        sDone[u] = now;
+    };
+    auto store = [&](uint32_t node, uint32_t u, uint32_t l, uint32_t r, bool interior) {
+        uint32_t b[6], lb[6], rb[6];
+#pragma unroll
+        for (int k = 0; k < 6; ++k) {
+            b[k] = sBox[k][u];
+            lb[k] = sBox[k][l];
+            rb[k] = sBox[k][r];
+        }
+        store_box(R.nodes, node, b);
+        if (interior && R.pairs) store_pair_boxes(R.pairs + 4u * node, lb, rb);
+    };
     for (uint32_t t = blockIdx.x; t < nSub; t += gridDim.x) {
         const uint32_t r0 = subRoots[root + t];
-        const uint32_t sz = min(sub_size(nodes, r0, end), REFIT_SUB);
-        sArr[tid] = 0u;
+        uint4 lo = make_uint4(0u, 0u, 0u, 0u), hi = lo;
+        if (tid < end - r0) {
+            lo = *reinterpret_cast<const uint4*>(R.nodes + 8 * (size_t)(r0 + tid));
+            hi = *reinterpret_cast<const uint4*>(R.nodes + 8 * (size_t)(r0 + tid) + 4);
+        }
+        sMiss[tid] = hi.z;
         __syncthreads();
-        uint32_t node = NONE;  // the node this thread carries up
-        if (tid < sz) {
-            const uint32_t i = r0 + tid;
-            const uint32_t info = nodes[8 * i + 7];
-            if (info != INTERIOR) {
-                const uint32_t off = info & 0x00FFFFFFu, cnt = info >> 24;
-                uint32_t* n = nodes + 8 * i;
-                if (cnt != 0u) {
-                    float mnx = INFINITY, mny = INFINITY, mnz = INFINITY, mxx = -INFINITY, mxy = -INFINITY,
-                          mxz = -INFINITY;
-                    for (uint32_t tr = off; tr < off + cnt; ++tr) {
-                        float3 p[3];
-                        for (int k = 0; k < 3; ++k) {
-                            const float* v = vertexData + (size_t)triIndex[3 * tr + k] * 8u;
-                            const float x = v[0], y = v[1], z = v[2];
-                            p[k] = make_float3(x, y, z);
-                            if (x < mnx) mnx = x;
-                            if (x > mxx) mxx = x;
-                            if (y < mny) mny = y;
-                            if (y > mxy) mxy = y;
-                            if (z < mnz) mnz = z;
-                            if (z > mxz) mxz = z;
-                        }
-                        tris[3 * tr] = make_float4(p[0].x, p[0].y, p[0].z, __uint_as_float(matBits[triMaterial[tr]]));
-                        tris[3 * tr + 1] = make_float4(p[1].x, p[1].y, p[1].z, 0.0f);
-                        tris[3 * tr + 2] = make_float4(p[2].x, p[2].y, p[2].z, 0.0f);
-                    }
-                    n[0] = __float_as_uint(mnx); n[1] = __float_as_uint(mny); n[2] = __float_as_uint(mnz);
-                    n[3] = __float_as_uint(mxx); n[4] = __float_as_uint(mxy); n[5] = __float_as_uint(mxz);
-                }
-                for (int k = 0; k < 6; ++k) sBox[6 * tid + k] = __uint_as_float(n[k]);
-                node = i;
+        const uint32_t m0 = sMiss[0], sz = min(m0 > r0 && m0 <= end ? m0 - r0 : end - r0, REFIT_SUB);
+        const bool mine = tid < sz, interior = mine && hi.w == INTERIOR;
+        uint32_t l = tid, r = tid;
+        if (interior) {
+            l = tid + 1u;
+            r = l < sz ? sMiss[l] - r0 : NONE;
+            if (r >= sz || r <= l) {  // a partition that does not match the layout
+                latch(err, ERR_LAYOUT);
+                l = r = tid;          // (never done: nothing above it is written)
             }
         }
-        // inside the subtree: the second child to finish computes its parent
-        volatile float* vb = sBox;
-        while (node != NONE && node != r0) {
-            const uint32_t p = parent[node];
-            const uint32_t pl = p - r0;  // p lies in [r0, node): the subtree is [r0, r0 + sz)
-            if (p == NONE || pl >= sz) {  // a partition that does not match the layout
-                latch(err, ERR_LAYOUT);
-                node = NONE;
-                break;
+        if (mine && !interior) {
+            uint32_t box[6] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y};
+            if (hi.w >> 24) {
+                float b[6];
+                refit_leaf(R, hi.w & 0x00FFFFFFu, hi.w >> 24, b);
+#pragma unroll
+                for (int k = 0; k < 6; ++k) box[k] = __float_as_uint(b[k]);
             }
-            __threadfence_block();
-            if (atomicAdd(&sArr[pl], 1u) == 0u) {
-                node = NONE;
-                break;
-            }
-            __threadfence_block();
-            const uint32_t l = p + 1, r = nodes[8 * l + 6];
-            const uint32_t ll = l - r0, rl = r - r0;
-            if (ll >= sz || rl >= sz) {
-                latch(err, ERR_LAYOUT);
-                node = NONE;
-                break;
-            }
-            uint32_t lb[6], rb[6];
-            for (int k = 0; k < 6; ++k) {
-                lb[k] = __float_as_uint(vb[6 * ll + k]);
-                rb[k] = __float_as_uint(vb[6 * rl + k]);
-            }
-            uint32_t* n = nodes + 8 * p;
-            for (int k = 0; k < 3; ++k) {
-                const float mn = js_min(__uint_as_float(lb[k]), __uint_as_float(rb[k]));
-                const float mx = js_max(__uint_as_float(lb[3 + k]), __uint_as_float(rb[3 + k]));
-                n[k] = __float_as_uint(mn);
-                n[3 + k] = __float_as_uint(mx);
-                vb[6 * pl + k] = mn;
-                vb[6 * pl + 3 + k] = mx;
-            }
-            if (pairs) store_pair_boxes(pairs + 4u * p, lb, rb);
-            node = p;
+#pragma unroll
+            for (int k = 0; k < 6; ++k) sBox[k][tid] = box[k];
         }
-        // the subtree root is done: the levels above through global memory
-        while (node != NONE) {
-            const uint32_t p = parent[node];
-            if (p == NONE) break;
-            uint32_t prev;
-            asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(prev) : "l"(arrive + p) : "memory");
-            if (prev == 0u) break;
-            arrive[p] = 0u;
-            const uint32_t l = p + 1;
-            const uint32_t r = *(const volatile uint32_t*)(nodes + 8 * l + 6);
-            const uint32_t* L = nodes + 8 * l;
-            const uint32_t* Rn = nodes + 8 * r;
-            uint32_t lb[6], rb[6];
-            for (int k = 0; k < 6; ++k) {
-                lb[k] = *(const volatile uint32_t*)(L + k);
-                rb[k] = *(const volatile uint32_t*)(Rn + k);
+        sDone[tid] = mine && !interior ? 0u : NONE;
+        bool open = interior;
+        for (uint32_t now = 1; now <= sz && __syncthreads_or(open); ++now) {
+            if (interior) round(tid, l, r, now);
+            open = interior && sDone[tid] == NONE;
+        }
+        __syncthreads();
+        if (mine && sDone[tid] != NONE && (interior || hi.w >> 24)) store(r0 + tid, tid, l, r, interior);
+        // above the subtree: through global memory, or by the CTA that finishes last
+        if (tid == 0) {
+            sLast = 0u;
+            if (tops == NONE) refit_climb(R, r0);
+            else if (tops) sLast = arrive_at(gate + GATE_DONE) + 1u == nSub ? 1u : 0u;
+        }
+        __syncthreads();
+        if (sLast) {
+            uint32_t node = 0, ul = 0, ur = 0;
+            if (tid < tops) {
+                const uint32_t* e = subRoots + root + nSub + 4u * tid;
+                node = e[0];
+                ul = e[1];
+                ur = e[2];
+                sDone[nSub + tid] = NONE;
             }
-            uint32_t* n = nodes + 8 * p;
-            for (int k = 0; k < 3; ++k) {
-                n[k] = __float_as_uint(js_min(__uint_as_float(lb[k]), __uint_as_float(rb[k])));
-                n[3 + k] = __float_as_uint(js_max(__uint_as_float(lb[3 + k]), __uint_as_float(rb[3 + k])));
+            if (tid < nSub) {
+                const uint32_t* n = R.nodes + 8 * (size_t)subRoots[root + tid];
+#pragma unroll
+                for (int k = 0; k < 6; ++k) sBox[k][tid] = *(const volatile uint32_t*)(n + k);
+                sDone[tid] = 0u;
             }
-            if (pairs) store_pair_boxes(pairs + 4u * p, lb, rb);
-            node = p;
+            open = true;
+            for (uint32_t now = 1; now <= tops && __syncthreads_or(open); ++now) {
+                if (tid < tops) round(nSub + tid, ul, ur, now);
+                open = tid < tops && sDone[nSub + tid] == NONE;
+            }
+            __syncthreads();
+            if (tid < tops && sDone[nSub + tid] != NONE) store(node, nSub + tid, ul, ur, true);
+            if (tid == 0) gate[GATE_DONE] = 0u;
         }
         __syncthreads();  // the shared arrays serve the next subtree
     }
@@ -355,30 +401,20 @@ cudaError_t launch_refit_blas(const SceneBuffers& B, uint32_t root, uint32_t end
     uint32_t n = end - root;
     unsigned g = (n + 255) / 256;
     if (!validated) {
-        cudaError_t e = cudaMemsetAsync(gate, 1, sizeof(uint32_t), st);  // nonzero: valid until a check fails
-        if (e != cudaSuccess) return e;
-        k_refit_reset<<<g, 256, 0, st>>>(B.parent, B.arrive, root, end); note_launch();
+        k_refit_reset<<<g, 256, 0, st>>>(B.parent, B.arrive, root, end, gate); note_launch();
         k_refit_link<<<g, 256, 0, st>>>(B.nodes, B.triIndex, B.triMaterial, B.triCount, B.vertexCount,
                                         B.materialCount, B.parent, root, end, gate, err); note_launch();
         k_refit_orphans<<<g, 256, 0, st>>>(B.parent, root, end, gate, err); note_launch();
-        if (SB_REFIT_CTA) {
-            cudaError_t e2 = cudaMemsetAsync(gate + 16, 0, sizeof(uint32_t), st);  // the range's subtree count
-            if (e2 != cudaSuccess) return e2;
-            k_refit_partition<<<g, 256, 0, st>>>(B.nodes, B.parent, root, end, gate, B.subRoots, gate + 16);
-            note_launch();
-        }
+        k_refit_partition<<<g, 256, 0, st>>>(B.nodes, B.parent, root, end, gate, B.subRoots); note_launch();
+        k_refit_plan<<<1, REFIT_SUB, 0, st>>>(B.nodes, root, end, gate, B.subRoots); note_launch();
     }
-    if (SB_REFIT_CTA) {
-        // one CTA per subtree (the count is on the device; idle CTAs return at once)
-        const unsigned ctas = n < 1184u ? n : 1184u;
-        k_refit_cta<<<ctas, REFIT_SUB, 0, st>>>(B.nodes, B.triIndex, B.vertexData, B.triMaterial, B.matBits, B.tris,
-                                                B.parent, B.arrive, root, end, gate, B.pairs, B.subRoots, gate + 16,
-                                                err);
-        note_launch();
-        return cudaGetLastError();
-    }
-    k_refit_run<<<g, 256, 0, st>>>(B.nodes, B.triIndex, B.vertexData, B.triMaterial, B.matBits, B.tris, B.parent,
-                                   B.arrive, root, end, gate, B.pairs, err); note_launch();
+    // one CTA per subtree: how many there are is on the device (a subtree of a balanced
+    // tree has 128 nodes or more; CTAs take further ones in turn)
+    const RefitArrays R{B.nodes, B.triIndex, reinterpret_cast<const float4*>(B.vertexData), B.triMaterial, B.matBits,
+                        B.tris, B.parent, B.arrive, B.pairs};
+    const unsigned ctas = (n + 63u) / 64u;
+    k_refit_cta<<<ctas < 1184u ? ctas : 1184u, REFIT_SUB, 0, st>>>(R, root, end, gate, B.subRoots, err);
+    note_launch();
     return cudaGetLastError();
 }
 
