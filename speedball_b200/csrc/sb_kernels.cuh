@@ -126,11 +126,7 @@ constexpr uint32_t TLAS_BUILD_MAX = 4096;  // instances per single-CTA TLAS buil
 cudaError_t launch_tlas_build(const SceneBuffers& B, const InstanceTable& I, uint32_t* err, cudaStream_t st);
 // srcList/world16 are device arrays (count entries); srcList == null updates every
 // source instance from its stored matrix (rewriteRows = 0 after a BLAS refit).
-cudaError_t launch_update_instances(const SceneBuffers& B, const InstanceTable& I, const uint32_t* srcList,
-                                    const double* world16, uint32_t count, int rewriteRows, uint32_t* err,
-                                    cudaStream_t st);
-cudaError_t launch_tlas_refit(const SceneBuffers& B, const InstanceTable& I, uint32_t* err, cudaStream_t st);
-// launch_update_instances followed by launch_tlas_refit, as one single-CTA launch.
+// The transform lane (instances, then the TLAS over them) as one single-CTA launch.
 cudaError_t launch_update_refit_tlas(const SceneBuffers& B, const InstanceTable& I, const uint32_t* srcList,
                                      const double* world16, uint32_t count, int rewriteRows, uint32_t* err,
                                      cudaStream_t st);

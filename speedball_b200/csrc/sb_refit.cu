@@ -441,6 +441,16 @@ __device__ double det4(const double* m) {
     return DS(DA(DS(DM(mat(m, 0, 0), c0), DM(mat(m, 0, 1), c1)), DM(mat(m, 0, 2), c2)), DM(mat(m, 0, 3), c3));
 }
 
+// Entry (r, c) of the adjugate.
+__device__ __forceinline__ double cofactor(const double* m, int r, int c) {
+    const int r0 = c == 0, r1 = 1 + (c <= 1), r2 = 2 + (c <= 2), c0 = r == 0, c1 = 1 + (r <= 1), c2 = 2 + (r <= 2);
+    const double t0 = DM(mat(m, r0, c0), DS(DM(mat(m, r1, c1), mat(m, r2, c2)), DM(mat(m, r1, c2), mat(m, r2, c1))));
+    const double t1 = DM(mat(m, r0, c1), DS(DM(mat(m, r1, c0), mat(m, r2, c2)), DM(mat(m, r1, c2), mat(m, r2, c0))));
+    const double t2 = DM(mat(m, r0, c2), DS(DM(mat(m, r1, c0), mat(m, r2, c1)), DM(mat(m, r1, c1), mat(m, r2, c0))));
+    const double m3 = DA(DS(t0, t1), t2);
+    return ((r + c) & 1) ? -m3 : m3;
+}
+
 // First three rows of the inverse (adjugate / determinant), zeros if singular.
 __device__ void inverse_rows(const double* m, double out[12]) {
     double det = det4(m);
@@ -450,36 +460,22 @@ __device__ void inverse_rows(const double* m, double out[12]) {
     }
     double inv = __ddiv_rn(1.0, det);
     for (int r = 0; r < 3; ++r)
-        for (int c = 0; c < 4; ++c) {
-            int rows[3], cols[3];
-            for (int i = 0, k = 0; i < 4; ++i) if (i != c) rows[k++] = i;
-            for (int j = 0, k = 0; j < 4; ++j) if (j != r) cols[k++] = j;
-            double t0 = DM(mat(m, rows[0], cols[0]),
-                           DS(DM(mat(m, rows[1], cols[1]), mat(m, rows[2], cols[2])),
-                              DM(mat(m, rows[1], cols[2]), mat(m, rows[2], cols[1]))));
-            double t1 = DM(mat(m, rows[0], cols[1]),
-                           DS(DM(mat(m, rows[1], cols[0]), mat(m, rows[2], cols[2])),
-                              DM(mat(m, rows[1], cols[2]), mat(m, rows[2], cols[0]))));
-            double t2 = DM(mat(m, rows[0], cols[2]),
-                           DS(DM(mat(m, rows[1], cols[0]), mat(m, rows[2], cols[1])),
-                              DM(mat(m, rows[1], cols[1]), mat(m, rows[2], cols[0]))));
-            double m3 = DA(DS(t0, t1), t2);
-            double cof = ((r + c) & 1) ? -m3 : m3;
-            out[r * 4 + c] = DM(cof, inv);
-        }
+        for (int c = 0; c < 4; ++c) out[r * 4 + c] = DM(cofactor(m, r, c), inv);
+}
+
+__device__ __forceinline__ void transform_corner(const double* m, double x, double y, double z, double p[3]) {
+    const double w = __ddiv_rn(1.0, DA(DA(DA(DM(m[3], x), DM(m[7], y)), DM(m[11], z)), m[15]));
+    p[0] = DM(DA(DA(DA(DM(m[0], x), DM(m[4], y)), DM(m[8], z)), m[12]), w);
+    p[1] = DM(DA(DA(DA(DM(m[1], x), DM(m[5], y)), DM(m[9], z)), m[13]), w);
+    p[2] = DM(DA(DA(DA(DM(m[2], x), DM(m[6], y)), DM(m[10], z)), m[14]), w);
 }
 
 __device__ void transform_box(const double* m, const double lmin[3], const double lmax[3], double wmin[3],
                               double wmax[3]) {
     for (int a = 0; a < 3; ++a) { wmin[a] = INFINITY; wmax[a] = -INFINITY; }
     for (int i = 0; i < 8; ++i) {
-        double x = (i & 1) ? lmax[0] : lmin[0];
-        double y = (i & 2) ? lmax[1] : lmin[1];
-        double z = (i & 4) ? lmax[2] : lmin[2];
-        double w = __ddiv_rn(1.0, DA(DA(DA(DM(m[3], x), DM(m[7], y)), DM(m[11], z)), m[15]));
-        double p[3] = {DM(DA(DA(DA(DM(m[0], x), DM(m[4], y)), DM(m[8], z)), m[12]), w),
-                       DM(DA(DA(DA(DM(m[1], x), DM(m[5], y)), DM(m[9], z)), m[13]), w),
-                       DM(DA(DA(DA(DM(m[2], x), DM(m[6], y)), DM(m[10], z)), m[14]), w)};
+        double p[3];
+        transform_corner(m, (i & 1) ? lmax[0] : lmin[0], (i & 2) ? lmax[1] : lmin[1], (i & 4) ? lmax[2] : lmin[2], p);
         for (int a = 0; a < 3; ++a) {
             if (p[a] < wmin[a]) wmin[a] = p[a];
             if (p[a] > wmax[a]) wmax[a] = p[a];
@@ -785,27 +781,86 @@ cudaError_t launch_tlas_build(const SceneBuffers& B, const InstanceTable& I, uin
 
 // ------------------------------------------------------ transform lane
 // updateTransforms (spectral_scene.js:1402-1514): recompute the listed source
-// instances (all when srcList is null) and write their slots.
-__global__ void k_update_instances(SceneBuffers B, InstanceTable I, const uint32_t* srcList, const double* world16,
-                                   uint32_t count, int rewriteRows, uint32_t* err) {
-    uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t total = srcList ? count : I.count;
-    if (i >= total) return;
-    uint32_t src = srcList ? srcList[i] : i;
-    if (src >= I.count) { latch(err, ERR_LAYOUT); return; }
-    if (srcList && world16)
-        for (int k = 0; k < 16; ++k) I.world[(size_t)src * 16u + k] = world16[(size_t)i * 16u + k];
-    compute_instance(B, I, src, err);
-    write_slot(B, I, I.slotOf[src], src, rewriteRows != 0);
-}
+// instances (all when srcList is null) and write their slots, then refit the TLAS.
 
-cudaError_t launch_update_instances(const SceneBuffers& B, const InstanceTable& I, const uint32_t* srcList,
-                                    const double* world16, uint32_t count, int rewriteRows, uint32_t* err,
-                                    cudaStream_t st) {
-    uint32_t total = srcList ? count : I.count;
-    if (total == 0) return cudaSuccess;
-    k_update_instances<<<(total + 127) / 128, 128, 0, st>>>(B, I, srcList, world16, count, rewriteRows, err); note_launch();
-    return cudaGetLastError();
+// compute_instance and write_slot by a warp: every operation the same, an inverse
+// entry per lane, then a box corner per lane. m: 16 doubles of shared memory, corner: 24.
+// Returns the slot; bounds (of lane a < 3): its liveBounds entries a and 3 + a.
+__device__ uint32_t update_instance_warp(const SceneBuffers& B, const InstanceTable& I, uint32_t src,
+                                         const double* world, bool rows, double* m, double* corner, float& lo,
+                                         float& hi, uint32_t* err) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t root = I.blasRoot[src], end = I.blasEnd[src], slot = I.slotOf[src];
+    const bool active = I.active[src];
+    if (lane < 16u) {
+        const double v = world ? world[lane] : I.world[(size_t)src * 16u + lane];
+        if (world) I.world[(size_t)src * 16u + lane] = v;
+        m[lane] = v;
+    }
+    __syncwarp();
+    // without new matrices or rows the inverses stand as they are
+    const bool inside = root < end && end <= B.nodeCount, inverse = rows || world;
+    const float* nb = reinterpret_cast<const float*>(B.nodes + (size_t)(inside ? root : 0u) * 8u);
+    float b[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) b[k] = nb[k];
+    float row = 0.0f, sign = 1.0f;
+    if (inverse) {
+        const double det = det4(m);
+        const double inv = __ddiv_rn(1.0, det);
+        if (lane < 12u) {
+            row = __double2float_rn(det == 0.0 ? 0.0 : DM(cofactor(m, (int)(lane / 4u), (int)(lane % 4u)), inv));
+            I.invRows[(size_t)src * 12u + lane] = row;
+        }
+        sign = det < 0.0 ? -1.0f : 1.0f;
+    }
+    if (lane < 8u) {
+        double p[3];
+        transform_corner(m, (lane & 1u) ? b[3] : b[0], (lane & 2u) ? b[4] : b[1], (lane & 4u) ? b[5] : b[2], p);
+        for (int a = 0; a < 3; ++a) corner[3 * lane + a] = p[a];
+    }
+    __syncwarp();
+    if (lane == 0) {
+        if (inverse) I.detSign[src] = sign;
+        if (active && !inside) latch(err, ERR_LAYOUT);
+    }
+    lo = hi = 0.0f;
+    if (lane < 3u) {
+        double mn = INFINITY, mx = -INFINITY;
+        if (!active) mn = mx = m[12 + lane];
+        else if (!inside) mn = mx = 0.0;
+        else
+            for (int i = 0; i < 8; ++i) {
+                const double v = corner[3 * i + lane];
+                if (v < mn) mn = v;
+                if (v > mx) mx = v;
+            }
+        double* o = I.aabb + (size_t)src * 9u + lane;
+        const double mid = DM(DA(mn, mx), 0.5);
+        o[0] = mn;
+        o[3] = mx;
+        o[6] = mid;
+        if (mid != mid) latch(err, ERR_NAN_KEY);
+        lo = __double2float_rn(mn);
+        hi = __double2float_rn(mx);
+        I.liveBounds[(size_t)slot * 6u + lane] = lo;
+        I.liveBounds[(size_t)slot * 6u + 3u + lane] = hi;
+    }
+    if (rows) {
+        const float act = active ? 1.0f : 0.0f;
+        float v = row;
+        if (lane == 12u) v = float(root);
+        if (lane == 13u) v = float(end);
+        if (lane == 14u) v = sign;
+        if (lane == 15u) v = act;
+        if (lane >= 16u) v = 0.0f;
+        if (lane < 28u) B.materials[B.instBase + (size_t)slot * 28u + lane] = v;
+        if (lane == 12u) v = __uint_as_float(root);
+        if (lane == 13u) v = __uint_as_float(end);
+        if (lane < 16u) reinterpret_cast<float*>(B.inst)[16u * (size_t)slot + lane] = v;
+    }
+    __syncwarp();
+    return slot;
 }
 
 // refitFlatTlasRange over the frozen partition, deepest level first (the
@@ -861,87 +916,138 @@ __device__ __forceinline__ void tlas_refit_pairs(const SceneBuffers& B, uint32_t
     }
 }
 
-// TLASes of up to this many nodes run the level pass on a shared-memory copy
-// of the boxes, structure words and depths (the same min / max on the same
-// values; every node is still written to the records as it is refit), so a
-// level reads its children from shared memory instead of global memory.
-#ifndef SB_TLAS_STAGE_NODES
-#define SB_TLAS_STAGE_NODES 512
-#endif
-constexpr uint32_t TLAS_STAGE_NODES = SB_TLAS_STAGE_NODES > 0 ? SB_TLAS_STAGE_NODES : 1;
+// TLASes of up to this many nodes and slots refit in shared memory.
+constexpr uint32_t TLAS_STAGE = 512;
+// Up to this many listed instances are updated by a warp each, more by a thread each.
+constexpr uint32_t TLAS_WARPS = 16, TLAS_WARP_UPDATES = 3 * TLAS_WARPS;
 
-__device__ __forceinline__ void tlas_refit_body(const SceneBuffers& B, const InstanceTable& I) {
-    const uint32_t nn = B.tlasNodeCount;
+// The transform lane in one CTA: the listed (or every) source instance's rows and
+// bounds, then the TLAS refit over them, deepest level first.
+//
+// One CTA's latency bounds it: loads, the FP64 chain of an inverse and the levels. So
+// the TLAS's structure and slot bounds are staged while the instances are computed (a
+// warp each: a determinant, then one cofactor and one corner per lane), the levels
+// run on shared memory alone, and everything is written at the end. With
+// three movers in the atrium's 34 instances 6.8 us instead of 13.5.
+__global__ void __launch_bounds__(32 * TLAS_WARPS) k_update_refit_tlas(SceneBuffers B, InstanceTable I,
+                                                                       const uint32_t* srcList, const double* world16,
+                                                                       uint32_t count, int rewriteRows,
+                                                                       uint32_t* err) {
+    __shared__ uint32_t sBox[6][TLAS_STAGE];
+    __shared__ float sBounds[6][TLAS_STAGE];
+    __shared__ uint16_t sMiss[TLAS_STAGE], sOff[TLAS_STAGE], sCnt[TLAS_STAGE], sDepth[TLAS_STAGE];
+    __shared__ double sM[TLAS_WARPS][16], sCorner[TLAS_WARPS][24];
+    __shared__ float sNew[6][TLAS_WARP_UPDATES];
+    __shared__ uint32_t sSlot[TLAS_WARP_UPDATES];
+    const uint32_t total = srcList ? count : I.count, nn = B.tlasNodeCount, slots = B.instCount;
     const int maxDepth = (int)*(volatile uint32_t*)I.scratch;
-    if (SB_TLAS_STAGE_NODES > 0 && nn <= TLAS_STAGE_NODES) {
-        __shared__ float sBox[6 * TLAS_STAGE_NODES];
-        __shared__ uint32_t sMiss[TLAS_STAGE_NODES], sOff[TLAS_STAGE_NODES], sCnt[TLAS_STAGE_NODES],
-            sDepth[TLAS_STAGE_NODES];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    const bool staged = nn <= TLAS_STAGE && slots <= TLAS_STAGE, byWarp = total <= TLAS_WARP_UPDATES;
+    // with few instances their warps start on them at once and the others stage
+    const uint32_t firstStage = byWarp && total <= TLAS_WARPS / 2 ? 32u * total : 0u;
+    if (staged && threadIdx.x >= firstStage) {
         const float* T = B.materials + B.tlasBase;
-        for (uint32_t i = threadIdx.x; i < nn; i += blockDim.x) {
+        const uint32_t step = blockDim.x - firstStage;
+        for (uint32_t i = threadIdx.x - firstStage; i < nn; i += step) {
             const float* N = T + (size_t)i * 12u;
-            for (int k = 0; k < 6; ++k) sBox[6 * i + k] = N[k];
-            sMiss[i] = (uint32_t)N[6];
-            sOff[i] = (uint32_t)N[7];
-            sCnt[i] = N[8] > 0.0f ? (uint32_t)N[8] : 0u;
-            sDepth[i] = I.nodeDepth[i];
+            sMiss[i] = (uint16_t)N[6];
+            sOff[i] = (uint16_t)N[7];
+            sCnt[i] = N[8] > 0.0f ? (uint16_t)N[8] : 0u;
+            sDepth[i] = (uint16_t)I.nodeDepth[i];
         }
-        __syncthreads();
-        for (int d = maxDepth; d >= 0; --d) {
-            for (uint32_t i = threadIdx.x; i < nn; i += blockDim.x) {
-                if (sDepth[i] != (uint32_t)d) continue;
-                float bx[6];
-                const uint32_t cnt = sCnt[i];
-                if (cnt > 0u) {
-                    const uint32_t off = sOff[i];
-                    float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
-                    for (uint32_t s = off; s < off + cnt; ++s) {
-                        const float* b = I.liveBounds + (size_t)s * 6u;
-                        for (int k = 0; k < 3; ++k) {
-                            if (b[k] < mn[k]) mn[k] = b[k];
-                            if (b[3 + k] > mx[k]) mx[k] = b[3 + k];
-                        }
-                    }
-                    for (int k = 0; k < 3; ++k) { bx[k] = mn[k]; bx[3 + k] = mx[k]; }
-                } else {
-                    const uint32_t l = i + 1, r = sMiss[l];
-                    for (int k = 0; k < 3; ++k) {
-                        bx[k] = js_min(sBox[6 * l + k], sBox[6 * r + k]);
-                        bx[3 + k] = js_max(sBox[6 * l + 3 + k], sBox[6 * r + 3 + k]);
-                    }
+        for (uint32_t i = threadIdx.x - firstStage; i < 6u * slots; i += step) sBounds[i % 6u][i / 6u] = I.liveBounds[i];
+    }
+    if (byWarp) {
+        for (uint32_t i = warp; i < total; i += TLAS_WARPS) {
+            const uint32_t src = srcList ? srcList[i] : i;
+            if (src >= I.count) {
+                if (lane == 0) {
+                    latch(err, ERR_LAYOUT);
+                    sSlot[i] = NONE;
                 }
-                for (int k = 0; k < 6; ++k) sBox[6 * i + k] = bx[k];
-                write_tlas_node(B, i, bx, sMiss[i], sOff[i], cnt);
+                continue;
             }
-            __syncthreads();
+            float lo, hi;
+            const uint32_t slot =
+                update_instance_warp(B, I, src, srcList && world16 ? world16 + (size_t)i * 16u : nullptr,
+                                     rewriteRows != 0, sM[warp], sCorner[warp], lo, hi, err);
+            if (lane == 0) sSlot[i] = slot;
+            if (lane < 3u) {
+                sNew[lane][i] = lo;
+                sNew[3u + lane][i] = hi;
+            }
         }
     } else {
-        tlas_refit_levels(B, I, nn, maxDepth);
-    }
-    tlas_refit_pairs(B, nn);
-}
-
-__global__ void __launch_bounds__(1024) k_tlas_refit(SceneBuffers B, InstanceTable I) { tlas_refit_body(B, I); }
-
-// The transform lane in one CTA: the listed (or every) source instance's rows
-// and bounds, then the TLAS refit over them, with one launch.
-__global__ void __launch_bounds__(512) k_update_refit_tlas(SceneBuffers B, InstanceTable I, const uint32_t* srcList,
-                                                            const double* world16, uint32_t count, int rewriteRows,
-                                                            uint32_t* err) {
-    const uint32_t total = srcList ? count : I.count;
-    for (uint32_t i = threadIdx.x; i < total; i += blockDim.x) {
-        const uint32_t src = srcList ? srcList[i] : i;
-        if (src >= I.count) {
-            latch(err, ERR_LAYOUT);
-            continue;
+        for (uint32_t i = threadIdx.x; i < total; i += blockDim.x) {
+            const uint32_t src = srcList ? srcList[i] : i;
+            if (src >= I.count) {
+                latch(err, ERR_LAYOUT);
+                continue;
+            }
+            if (srcList && world16)
+                for (int k = 0; k < 16; ++k) I.world[(size_t)src * 16u + k] = world16[(size_t)i * 16u + k];
+            compute_instance(B, I, src, err);
+            write_slot(B, I, I.slotOf[src], src, rewriteRows != 0);
         }
-        if (srcList && world16)
-            for (int k = 0; k < 16; ++k) I.world[(size_t)src * 16u + k] = world16[(size_t)i * 16u + k];
-        compute_instance(B, I, src, err);
-        write_slot(B, I, I.slotOf[src], src, rewriteRows != 0);
     }
     __syncthreads();
-    tlas_refit_body(B, I);
+    if (!staged) {
+        tlas_refit_levels(B, I, nn, maxDepth);
+        tlas_refit_pairs(B, nn);
+        return;
+    }
+    if (byWarp) {
+        if (threadIdx.x < 6u)
+            for (uint32_t i = 0; i < total; ++i)
+                if (sSlot[i] < slots) sBounds[threadIdx.x][sSlot[i]] = sNew[threadIdx.x][i];
+    } else {
+        for (uint32_t i = threadIdx.x; i < 6u * slots; i += blockDim.x) sBounds[i % 6u][i / 6u] = I.liveBounds[i];
+    }
+    __syncthreads();
+    for (int d = maxDepth; d >= 0; --d) {
+        for (uint32_t i = threadIdx.x; i < nn; i += blockDim.x) {
+            if (sDepth[i] != (uint32_t)d) continue;
+            uint32_t box[6];
+            const uint32_t cnt = sCnt[i];
+            if (cnt > 0u) {
+                float mn[3] = {INFINITY, INFINITY, INFINITY}, mx[3] = {-INFINITY, -INFINITY, -INFINITY};
+                for (uint32_t s = sOff[i]; s < sOff[i] + cnt; ++s)
+                    for (int k = 0; k < 3; ++k) {
+                        if (sBounds[k][s] < mn[k]) mn[k] = sBounds[k][s];
+                        if (sBounds[3 + k][s] > mx[k]) mx[k] = sBounds[3 + k][s];
+                    }
+                for (int k = 0; k < 3; ++k) {
+                    box[k] = __float_as_uint(mn[k]);
+                    box[3 + k] = __float_as_uint(mx[k]);
+                }
+            } else {
+                const uint32_t l = i + 1, r = sMiss[l];
+                uint32_t lb[6], rb[6];
+                for (int k = 0; k < 6; ++k) {
+                    lb[k] = sBox[k][l];
+                    rb[k] = sBox[k][r];
+                }
+                join_boxes(lb, rb, box);
+            }
+            for (int k = 0; k < 6; ++k) sBox[k][i] = box[k];
+        }
+        __syncthreads();
+    }
+    for (uint32_t i = threadIdx.x; i < nn; i += blockDim.x) {
+        if ((int)sDepth[i] > maxDepth) continue;
+        float b[6];
+        for (int k = 0; k < 6; ++k) b[k] = __uint_as_float(sBox[k][i]);
+        write_tlas_node(B, i, b, sMiss[i], sOff[i], sCnt[i]);
+        // the traversal's child-pair copy of the bounds (entries are structural)
+        const uint32_t l = i + 1u;
+        if (!B.tlasPairs || sCnt[i] || l >= nn || !(sMiss[l] > l && sMiss[l] < nn)) continue;
+        uint32_t lb[6], rb[6];
+        for (int k = 0; k < 6; ++k) {
+            lb[k] = sBox[k][l];
+            rb[k] = sBox[k][sMiss[l]];
+        }
+        store_pair_boxes(B.tlasPairs + 4u * i, lb, rb);
+    }
 }
 
 // Depth of every TLAS node and the refit-index checks of
@@ -989,13 +1095,7 @@ __global__ void k_tlas_index(SceneBuffers B, InstanceTable I, uint32_t* owner, u
 cudaError_t launch_update_refit_tlas(const SceneBuffers& B, const InstanceTable& I, const uint32_t* srcList,
                                      const double* world16, uint32_t count, int rewriteRows, uint32_t* err,
                                      cudaStream_t st) {
-    k_update_refit_tlas<<<1, 512, 0, st>>>(B, I, srcList, world16, count, rewriteRows, err); note_launch();
-    return cudaGetLastError();
-}
-
-cudaError_t launch_tlas_refit(const SceneBuffers& B, const InstanceTable& I, uint32_t* err, cudaStream_t st) {
-    if (B.tlasNodeCount == 0) return cudaSuccess;
-    k_tlas_refit<<<1, 1024, 0, st>>>(B, I); note_launch();
+    k_update_refit_tlas<<<1, 32 * TLAS_WARPS, 0, st>>>(B, I, srcList, world16, count, rewriteRows, err); note_launch();
     return cudaGetLastError();
 }
 
