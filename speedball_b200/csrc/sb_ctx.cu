@@ -1011,7 +1011,7 @@ sb_status sb_solve(sb_ctx* ctx, uint32_t ci, uint32_t probeOffset, uint32_t upda
                         ctx->stream, ctx->jobs, ctx->jobCap, s0, n, timing ? ctx->evA : nullptr,
                         timing ? ctx->evB : nullptr, timing ? ctx->evC : nullptr));
     }
-    if (ctx->emitterCount) CK(launch_emitter_vis(S, D, P, ctx->dErr, ctx->stream));
+    if (ctx->emitterCount) CK(launch_emitter_vis(S, D, ctx->stream));
     if (timing) CK(cudaEventRecord(ctx->evMid, ctx->stream));
     CK(launch_blend_upload(D, P, ctx->stream));
     if (K.reflTier >= SB_REFLECT_HIGH) {

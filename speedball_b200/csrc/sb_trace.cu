@@ -369,7 +369,7 @@ __device__ __forceinline__ void shade_ray(const WaveCtx& W, uint32_t g) {
             if (!(diffuseEnergy > 0.02f || emissivePeak > 1e-6f)) hitT = -(t + ROUGH_UNSHADED_T_BIAS);
         }
         uint4 v = C.vis[rayIdx];
-        unsigned long long ok = (unsigned long long)v.z | ((unsigned long long)v.w << 32);
+        unsigned long long ok = (unsigned long long)(v.z & v.x) | (unsigned long long)(v.w & v.y) << 32;
         while (ok) {
             uint32_t li = (uint32_t)(__ffsll((long long)ok) - 1);
             ok &= ok - 1ull;
@@ -584,6 +584,90 @@ __global__ void __launch_bounds__(128) k_shade(WaveCtx W) {
     shade_ray(W, g);
 }
 
+// emitterVisKernel (gi_probes.js:2216-2260): per (updated probe, emitter) a
+// shadow ray from the probe to a point of the emitter's disk, chosen by a sin
+// hash of (probe, emitter, epoch seed) evaluated in separately rounded FP32,
+// folded into the emitter's visibility history with retention 0.8.
+//
+// The rays join stage B's jobs. By themselves they are too few to fill the chip (2,197
+// probes and 3 emitters: 206 warps) and take as long as their longest walk, 72 us,
+// while stage B walks ninety times as many in 155: there they cost 9 us, the jobs' and
+// the fold's launches included. A ray's outcome is its emitter's record bit in the
+// unblocked mask of its probe's ray 0: the NEE tests no such record, so the bit is free
+// until the fold takes it out again.
+__global__ void __launch_bounds__(128) k_emitter_jobs(WaveCtx W) {
+    if (!*W.S.valid) return;
+    const DevCascade& C = W.C;
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
+    const bool active = i < W.slotCount;
+    const uint32_t slot = W.slotBegin + (active ? i : 0u), probeIndex = probe_of(C, slot);
+    const uint32_t ray = slot * C.rays;
+    const float3 ro = slot_origin(C, slot);
+    unsigned long long open = 0ull;
+    for (uint32_t e = 0; e < C.emitterCount; ++e) {
+        const uint32_t li = C.emitterBase + e;
+        const float* L = C.lights + (size_t)li * 17u;
+        const float3 center = mk(L[1], L[2], L[3]);
+        const float sourceRadius = fmaxf(L[14], 0.0f);
+        const float3 axis = center - ro;
+        const float dist = sqrtf(dot3(axis, axis));
+        const bool far = active && dist > fmaxf(sourceRadius, 1e-3f);
+        const uint32_t jobs = __ballot_sync(ALL_LANES, far);
+        if (!jobs) continue;
+        uint32_t j = 0;
+        if (lane == 0) j = atomicAdd(&W.work[2], (uint32_t)__popc(jobs));
+        j = __shfl_sync(ALL_LANES, j, 0) + (uint32_t)__popc(jobs & ((1u << lane) - 1u));
+        if (!far) continue;
+        if (j >= W.jobCap) {
+            latch(W.err, ERR_CAPACITY);  // (unreachable: no ray tests an emitter's record)
+            continue;
+        }
+        const float3 d = axis * (1.0f / dist);
+        const float3 up = fabsf(d.y) < 0.999f ? mk(0.0f, 1.0f, 0.0f) : mk(1.0f, 0.0f, 0.0f);
+        const float3 tangent = normalize3(cross3(up, d));
+        const float3 bitangent = cross3(d, tangent);
+        const float seed = __fadd_rn(__fadd_rn(__fmul_rn(float(probeIndex), 12.9898f), __fmul_rn(float(e), 78.233f)),
+                                     __fmul_rn(W.P.emitterVisSeed, 37.719f));
+        const float h0 = __fmul_rn(sinf(seed), 43758.5453f);
+        const float h1 = __fmul_rn(sinf(__fadd_rn(seed, 19.19f)), 24634.6345f);
+        const float u = h0 - floorf(h0), v = h1 - floorf(h1);
+        const float diskRadius = sqrtf(u) * sourceRadius;
+        const float diskAngle = v * 6.283185307179586f;
+        const float3 target = center + (tangent * (cosf(diskAngle) * diskRadius) + bitangent * (sinf(diskAngle) * diskRadius));
+        const float3 sdir = normalize3(target - ro);
+        const float traceBias = fmaxf(C.cellMin * 0.005f * W.P.debugTraceBiasScale, RAY_EPS * W.P.debugRayEpsScale);
+        store32(W.jobs + 2 * j, make_float4(ro.x, ro.y, ro.z, fmaxf(dist - sourceRadius - traceBias, 1e-4f)),
+                make_float4(sdir.x, sdir.y, sdir.z, __uint_as_float(ray << 6 | li)));
+        open |= 1ull << li;
+    }
+    if (open) {
+        C.vis[ray].z |= (uint32_t)open;
+        C.vis[ray].w |= (uint32_t)(open >> 32);
+    }
+}
+
+__global__ void __launch_bounds__(128) k_emitter_vis(DevScene S, DevCascade C) {
+    const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
+    if (slot >= C.updatedCount || !*S.valid) return;
+    uint4* ray = C.vis + (size_t)slot * C.rays;
+    const uint4 v = *ray;
+    const unsigned long long open = (unsigned long long)v.z | (unsigned long long)v.w << 32;
+    float* vp = C.emitterVis + (size_t)probe_of(C, slot) * EMITTER_CAP;
+    for (uint32_t e = 0; e < C.emitterCount; ++e) {
+        const float sample = open >> (C.emitterBase + e) & 1ull ? 1.0f : 0.0f;
+        vp[e] = sample * (1.0f - EMITTER_VIS_RETENTION) + vp[e] * EMITTER_VIS_RETENTION;
+    }
+    ray->z = v.z & v.x;
+    ray->w = v.w & v.y;
+}
+
+cudaError_t launch_emitter_vis(const DevScene& S, const DevCascade& C, cudaStream_t st) {
+    if (C.updatedCount == 0 || C.emitterCount == 0) return cudaSuccess;
+    k_emitter_vis<<<(C.updatedCount + 127) / 128, 128, 0, st>>>(S, C);
+    note_launch();
+    return cudaGetLastError();
+}
+
 // Stage C alone over probe slots [0, slotCount) from the records already in
 // C.hits / C.vis (the adjoint re-evaluates shading this way).
 cudaError_t launch_shade(const DevScene& S, const DevCascade& C, const DevParams& P, const float4* dirs,
@@ -662,6 +746,10 @@ cudaError_t launch_trace(const DevScene& S, const DevCascade& C, const DevParams
     if (afterClosest) cudaEventRecord(afterClosest, st);
     k_emit<<<(rays + 127) / 128, 128, 0, st>>>(W);
     note_launch();
+    if (C.emitterCount) {
+        k_emitter_jobs<<<(slotCount + 127) / 128, 128, 0, st>>>(W);
+        note_launch();
+    }
     if (afterPrimary) cudaEventRecord(afterPrimary, st);
     // shadow jobs: at most lightCount per ray (the queue is sized for it)
     if (S.wideNodes)
@@ -969,56 +1057,6 @@ __global__ void k_probe_rays(const DevCascade C, float jitter, float* ro, float*
     ro[3 * i] = o.x; ro[3 * i + 1] = o.y; ro[3 * i + 2] = o.z;
     rd[3 * i] = d.x; rd[3 * i + 1] = d.y; rd[3 * i + 2] = d.z;
 }
-// emitterVisKernel (gi_probes.js:2216-2260): per (updated probe, emitter) a
-// shadow ray from the probe to a point of the emitter's disk, chosen by a sin
-// hash of (probe, emitter, epoch seed) evaluated in separately rounded FP32,
-// folded into the emitter's visibility history with retention 0.8.
-__global__ void k_emitter_vis(DevScene S, DevCascade C, DevParams P, uint32_t* err) {
-    const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
-    const uint32_t slot = gid / EMITTER_CAP, e = gid % EMITTER_CAP;
-    if (slot >= C.updatedCount || e >= C.emitterCount || !*S.valid) return;
-    const uint32_t probeIndex = probe_of(C, slot);
-    const float3 ro = slot_origin(C, slot);
-    const float* L = C.lights + (size_t)(C.emitterBase + e) * 17u;
-    const float3 center = mk(L[1], L[2], L[3]);
-    const float sourceRadius = fmaxf(L[14], 0.0f);
-    const float3 axis = center - ro;
-    const float dist = sqrtf(dot3(axis, axis));
-    float sample = 0.0f;
-    if (dist > fmaxf(sourceRadius, 1e-3f)) {
-        const float3 d = axis * (1.0f / dist);
-        const float3 up = fabsf(d.y) < 0.999f ? mk(0.0f, 1.0f, 0.0f) : mk(1.0f, 0.0f, 0.0f);
-        const float3 tangent = normalize3(cross3(up, d));
-        const float3 bitangent = cross3(d, tangent);
-        const float seed = __fadd_rn(__fadd_rn(__fmul_rn(float(probeIndex), 12.9898f), __fmul_rn(float(e), 78.233f)),
-                                     __fmul_rn(P.emitterVisSeed, 37.719f));
-        const float h0 = __fmul_rn(sinf(seed), 43758.5453f);
-        const float h1 = __fmul_rn(sinf(__fadd_rn(seed, 19.19f)), 24634.6345f);
-        const float u = h0 - floorf(h0), v = h1 - floorf(h1);
-        const float diskRadius = sqrtf(u) * sourceRadius;
-        const float diskAngle = v * 6.283185307179586f;
-        const float3 target = center + (tangent * (cosf(diskAngle) * diskRadius) + bitangent * (sinf(diskAngle) * diskRadius));
-        const float3 sdir = normalize3(target - ro);
-        const float traceBias = fmaxf(C.cellMin * 0.005f * P.debugTraceBiasScale, RAY_EPS * P.debugRayEpsScale);
-        Visits vis = {0, 0, 0, 0};
-        const bool pairs = any_pairs(S);
-        const bool blocked = trace_any(S, pairs ? S.tlasPairs : S.tlas, ro, sdir,
-                                       fmaxf(dist - sourceRadius - traceBias, 1e-4f), vis, err, pairs);
-        sample = blocked ? 0.0f : 1.0f;
-    }
-    float* vp = C.emitterVis + (size_t)probeIndex * EMITTER_CAP + e;
-    *vp = sample * (1.0f - EMITTER_VIS_RETENTION) + *vp * EMITTER_VIS_RETENTION;
-}
-
-cudaError_t launch_emitter_vis(const DevScene& S, const DevCascade& C, const DevParams& P, uint32_t* err,
-                               cudaStream_t st) {
-    const uint32_t n = C.updatedCount * EMITTER_CAP;
-    if (n == 0 || C.emitterCount == 0) return cudaSuccess;
-    k_emitter_vis<<<(n + 127) / 128, 128, 0, st>>>(S, C, P, err);
-    note_launch();
-    return cudaGetLastError();
-}
-
 // The tables of slot_origin (with a cascade's grid) and wave_dir.
 __global__ void k_probe_positions(DevCascade C, float4* pos) {
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
