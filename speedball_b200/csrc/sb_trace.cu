@@ -32,13 +32,12 @@ namespace sb {
 #define SB_SHADOW_MIN_BLOCKS 4
 #endif
 // The same for the walks of the 8-wide tree: 80 registers. Four blocks (64 registers,
-// less L1 beside the shared memory) measured 67 against 61 us on the room's primary
-// rays and 108 against 102 us on the atrium's, but 540 against 554 us for the plain
-// queries, whose rays come from arrays.
+// spills, less L1 beside the shared memory) measured 59 against 48 us on the room's
+// primary rays, 122 against 98 us on the atrium's and 966 against 932 us for 2.07M
+// bounce rays with a shadow ray each.
 #ifndef SB_WALK8_MIN_BLOCKS
 #define SB_WALK8_MIN_BLOCKS 3
 #endif
-constexpr int QUERY_MIN_BLOCKS = 4;
 
 // ---------------------------------------------------------------- bodies
 // Each stage's per-item work is a device function over `const WaveCtx&`; the
@@ -100,12 +99,15 @@ __device__ __forceinline__ WalkSmem walk_shared(void* smem, uint32_t depth, bool
     return m;
 }
 
-// A walk's next items for the lanes in `want`: positions of the shared cursor.
-__device__ __forceinline__ uint32_t take(uint32_t* cursor, uint32_t want) {
+// A walk's next items for the lanes in `want`: positions of the shared cursor; whether
+// it has more (before it is asked in vain, so that the walk knows its last rays).
+__device__ __forceinline__ uint32_t take(uint32_t* cursor, uint32_t total, uint32_t want, bool& more) {
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t base = 0;
     if (lane == 0) base = atomicAdd(cursor, (uint32_t)__popc(want));
-    return __shfl_sync(ALL_LANES, base, 0) + (uint32_t)__popc(want & ((1u << lane) - 1u));
+    base = __shfl_sync(ALL_LANES, base, 0);
+    more = base < total && total - base > (uint32_t)__popc(want);
+    return base + (uint32_t)__popc(want & ((1u << lane) - 1u));
 }
 
 // Stage A on the 8-wide tree. next(want, g) gives the lanes in `want` their
@@ -388,12 +390,20 @@ __device__ __forceinline__ void shade_ray(const WaveCtx& W, uint32_t g) {
 
 // ---------------------------------------------------------------- per solve
 
-// Positions from a cursor up to `total`.
-__device__ __forceinline__ auto from_cursor(uint32_t* cursor, uint32_t total) {
-    return [cursor, total](uint32_t want, uint32_t& g, bool& ok) {
-        g = take(cursor, want);
-        ok = g < total;
-        return __any_sync(ALL_LANES, ok && (want >> (threadIdx.x & 31u) & 1u)) != 0;
+// Positions from a cursor up to `total`. Neighbouring rays are alike, and a warp whose 32
+// are all long ones ends late where warps take only a few; `mix` then gives it eight
+// from each quarter of the positions: 48 -> 42 us for the room's 32,768 closest hits,
+// 79 -> 76 for 210,912 (59 a warp). Larger launches and the shadow jobs, whose
+// neighbours share their first nodes, measured the same to 4% slower mixed.
+__device__ __forceinline__ auto from_cursor(uint32_t* cursor, uint32_t total, bool mix = false) {
+    mix = mix && total <= 64u * gridDim.x * (blockDim.x / 32u);
+    const uint32_t row = mix ? ((total + 7u) / 8u + 3u) / 4u : 0u, end = mix ? row * 32u : total;
+    return [cursor, total, row, end](uint32_t want, uint32_t& g, bool& ok) {
+        bool more;
+        const uint32_t p = take(cursor, end, want, more), b = p / 8u;
+        g = row ? ((b % 4u) * row + b / 4u) * 8u + p % 8u : p;
+        ok = p < end && g < total;
+        return more;
     };
 }
 
@@ -404,7 +414,7 @@ __device__ __forceinline__ uint32_t primary_stage(const WaveCtx& W, const WalkSm
     const uint32_t total = W.slotCount * W.C.rays;
     if (W.S.dynCount) primary_moved(W, *m.w2, from_cursor(&W.work[4], total), dir, vis);
     __syncwarp();
-    const uint32_t n = primary_walk8(W, m, from_cursor(&W.work[0], total), dir, vis);
+    const uint32_t n = primary_walk8(W, m, from_cursor(&W.work[0], total, true), dir, vis);
     __syncwarp();
     return n;
 }
@@ -950,10 +960,10 @@ __global__ void k_occluded(DevScene S, const float* ro, const float* rd, const f
 }
 
 // The same on the 8-wide tree. MOVED: the scene has moved slots, walked as a ray is
-// taken; without that walk's code the kernel spills less: 554 -> 528 us
+// taken; without that walk's code the kernel spilled less at 64 registers: 554 -> 528 us
 // (closest) and 362 -> 341 us (any) for 2.07M bounce rays.
 template <bool ANY, bool MOVED>
-__global__ void __launch_bounds__(256, QUERY_MIN_BLOCKS) k_query_walk8(DevScene S, const float* ro, const float* rd,
+__global__ void __launch_bounds__(256, SB_WALK8_MIN_BLOCKS) k_query_walk8(DevScene S, const float* ro, const float* rd,
                                                                           const float* maxDist, uint32_t n,
                                                                           float* tOut, int32_t* triOut,
                                                                           int32_t* instOut, uint8_t* out,
@@ -965,9 +975,8 @@ __global__ void __launch_bounds__(256, QUERY_MIN_BLOCKS) k_query_walk8(DevScene 
     Visits vis = {0, 0, 0, 0};
     auto gen = [&](bool& more, uint32_t idle, float3& o, float3& d, float3& winv, float& tmax, uint32_t& tag,
                    uint4& hit) {
-        const uint32_t i = take(cursor, idle);
+        const uint32_t i = take(cursor, n, idle, more);
         const bool ok = i < n && (idle >> lane & 1u);
-        more = __any_sync(ALL_LANES, ok);
         if (!ok) return false;
         const size_t i3 = 3 * (size_t)i;
         o = mk(ro[i3], ro[i3 + 1], ro[i3 + 2]);
