@@ -8,10 +8,13 @@
 // and are tested by 32 lanes at once, two leaves hit in one step are opened
 // together, and lanes whose rays meet no slot take new rays (as in sb_walk8.cuh).
 // The results meet the scene-BVH walk's only in the next stage, so a warp that has
-// no rays left here goes on with that walk while others finish theirs. The atrium's
-// three movers and one deformer cost 99 + 72 us in kernels of one thread per ray
-// (two rays in three meet none of them), 72 + 63 us in such kernels of this walk,
-// and 21 + 21 us ahead of the tree's walk in the same launch.
+// no rays left here goes on with that walk while others finish theirs. Its last rays
+// its lanes share, as in walk8: one that grazes a dense mesh in each of its slots had
+// kept its warp here to the end of the launch. The atrium's three movers and one
+// deformer cost 99 + 72 us in kernels of one thread per ray (two rays in three meet
+// none of them), 72 + 63 us in such kernels of this walk, and 21 + 21 us ahead of the
+// tree's walk in the same launch; shared, the launches took 96 -> 92 and 101 -> 95 us,
+// of 1,536 probes' rays 66 -> 56 and 57 -> 40.
 #pragma once
 #include "sb_walk8.cuh"
 
@@ -27,6 +30,7 @@ struct Walk2Shared {
     uint4 hit[32];
     uint32_t item[WALK2_QUEUE];   // lane of its ray << 24 | triangle
     uint32_t stk[WALK2_DEPTH][32];  // far children
+    uint2 give[32];               // far children on their way to idle lanes; donor, lane of its ray
 };
 
 // True when every slot's BLAS can be walked by walk2.
@@ -47,61 +51,134 @@ __device__ __forceinline__ void walk2(const DevScene& S, Walk2Shared& sm, Gen ge
     float tmax = 0.0f;
     uint32_t tag = 0, k = 0, cur = PE_NONE, sp = 0, iter = 0, last = 0, head = 0, tail = 0;
     bool more = true;
+    uint32_t home = lane, base = 0;  // as in walk8
+    bool own = false, alone = S.iterCapRef < SB_WALK_STEPS_REF_DEFAULT, again = false;
+    uint32_t ties = 0;
+    // the lane's ray into its next slot; false: none left
+    auto next_slot = [&]() {
+        for (; k < S.dynCount; ) {
+            const uint32_t slot = __ldg(S.dynList + k++);
+            if (S.slotBounds) {
+                const float* b = S.slotBounds + 6u * slot;
+                if (!slab(mk(__ldg(b), __ldg(b + 1), __ldg(b + 2)), mk(__ldg(b + 3), __ldg(b + 4), __ldg(b + 5)), wo,
+                          winv, tmax))
+                    continue;
+            }
+            ++vis.inst;
+            const float4 m = __ldg(S.inst + 4 * slot + 3);
+            if (!(m.w > 0.5f)) continue;
+            const float4 r0 = __ldg(S.inst + 4 * slot), r1 = __ldg(S.inst + 4 * slot + 1),
+                         r2 = __ldg(S.inst + 4 * slot + 2);
+            o = mk(dot3(xyz(r0), wo) + r0.w, dot3(xyz(r1), wo) + r1.w, dot3(xyz(r2), wo) + r2.w);
+            const float3 d = mk(dot3(xyz(r0), wd), dot3(xyz(r1), wd), dot3(xyz(r2), wd));
+            inv = mk(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
+            const uint32_t root = __float_as_uint(m.x);
+            if (root >= __float_as_uint(m.y) || root >= S.nodeCount) continue;
+            const uint4 a = __ldg(S.nodes + 2 * root), b = __ldg(S.nodes + 2 * root + 1);
+            ++vis.blas;
+            if (!slab(mk(__uint_as_float(a.x), __uint_as_float(a.y), __uint_as_float(a.z)),
+                      mk(__uint_as_float(a.w), __uint_as_float(b.x), __uint_as_float(b.y)), o, inv, tmax))
+                continue;
+            cur = b.w == INTERIOR ? PE_BLAS | root : ((b.w >> 24) ? b.w : PE_NONE);
+            if (cur == PE_NONE) continue;
+            sm.o[lane] = make_float4(o.x, o.y, o.z, m.z);
+            sm.d[lane] = make_float4(d.x, d.y, d.z, __uint_as_float(slot));
+            sp = base = 0;
+            home = lane;
+            last = head;
+            state = WALK;
+            return true;
+        }
+        return false;
+    };
     for (;;) {
-        const bool done = state == FREE || (state == ENDED && (int32_t)(last - head) <= 0);
-        const uint32_t idle = __ballot_sync(ALL_LANES, done);
-        if (__popc(idle) >= WALK8_IDLE || !__any_sync(ALL_LANES, state == WALK)) {
-            const bool blocked = ANY && state == ENDED && (uint32_t)sm.best[lane] == 0u;
-            bool have = done && state == ENDED && !blocked;  // a ray with slots left perhaps
-            if (done && state == ENDED && blocked) fin(tag, tmax, make_uint4(0u, 0u, 0u, 0u), true);
-            const uint32_t want = __ballot_sync(ALL_LANES, done && !have);
-            if (more && want) {
-                if (gen(more, want, wo, wd, winv, tmax, tag)) {
+        bool flush = false;
+        if (more) {
+            const bool done = state == FREE || (state == ENDED && (int32_t)(last - head) <= 0);
+            const uint32_t idle = __ballot_sync(ALL_LANES, done);
+            if (__popc(idle) >= WALK8_IDLE || !__any_sync(ALL_LANES, state == WALK)) {
+                const bool blocked = ANY && done && own && (uint32_t)sm.best[lane] == 0u;
+                if (blocked) {
+                    fin(tag, tmax, make_uint4(0u, 0u, 0u, 0u), true);
+                    own = false;
+                }
+                const uint32_t want = __ballot_sync(ALL_LANES, done && !own);
+                if (want && gen(more, want, wo, wd, winv, tmax, tag)) {
                     sm.best[lane] = (unsigned long long)__float_as_uint(tmax) << 32 | 0xFFFFFFFFull;
                     if (!ANY) sm.hit[lane] = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u);
                     k = iter = 0;
-                    have = true;
+                    own = true;
                 }
-            } else if (idle == ALL_LANES && !__any_sync(ALL_LANES, have)) {
-                break;
-            }
-            if (done) state = FREE;
-            if (have) {  // the ray's next slot
-                for (; k < S.dynCount && state == FREE; ++k) {
-                    const uint32_t slot = __ldg(S.dynList + k);
-                    if (S.slotBounds) {
-                        const float* b = S.slotBounds + 6u * slot;
-                        if (!slab(mk(__ldg(b), __ldg(b + 1), __ldg(b + 2)), mk(__ldg(b + 3), __ldg(b + 4), __ldg(b + 5)),
-                                  wo, winv, tmax))
-                            continue;
+                if (done) {
+                    state = FREE;
+                    if (own && !next_slot()) {
+                        fin(tag, tmax, ANY ? make_uint4(0u, 0u, 0u, 0u) : sm.hit[lane], false);
+                        own = false;
                     }
-                    ++vis.inst;
-                    const float4 m = __ldg(S.inst + 4 * slot + 3);
-                    if (!(m.w > 0.5f)) continue;
-                    const float4 r0 = __ldg(S.inst + 4 * slot), r1 = __ldg(S.inst + 4 * slot + 1),
-                                 r2 = __ldg(S.inst + 4 * slot + 2);
-                    o = mk(dot3(xyz(r0), wo) + r0.w, dot3(xyz(r1), wo) + r1.w, dot3(xyz(r2), wo) + r2.w);
-                    const float3 d = mk(dot3(xyz(r0), wd), dot3(xyz(r1), wd), dot3(xyz(r2), wd));
-                    inv = mk(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
-                    const uint32_t root = __float_as_uint(m.x);
-                    if (root >= __float_as_uint(m.y) || root >= S.nodeCount) continue;
-                    const uint4 a = __ldg(S.nodes + 2 * root), b = __ldg(S.nodes + 2 * root + 1);
-                    ++vis.blas;
-                    if (!slab(mk(__uint_as_float(a.x), __uint_as_float(a.y), __uint_as_float(a.z)),
-                              mk(__uint_as_float(a.w), __uint_as_float(b.x), __uint_as_float(b.y)), o, inv, tmax))
-                        continue;
-                    cur = b.w == INTERIOR ? PE_BLAS | root : ((b.w >> 24) ? b.w : PE_NONE);
-                    if (cur == PE_NONE) continue;
-                    sm.o[lane] = make_float4(o.x, o.y, o.z, m.z);
-                    sm.d[lane] = make_float4(d.x, d.y, d.z, __uint_as_float(slot));
-                    sp = 0;
-                    last = head;
+                }
+                __syncwarp();
+            }
+        } else {
+            // no rays are left to take: the lanes share those in hand, as in walk8. A ray goes
+            // on to its next slot when no lane is in this one and the queue is empty (its
+            // local ray is the lanes' and the items'); a tie sends it through its slots again.
+            const uint32_t busy = __reduce_or_sync(ALL_LANES, state == WALK ? 1u << home : 0u);
+            const bool ready = own && state != WALK && !(busy >> lane & 1u);
+            flush = __any_sync(ALL_LANES, ready);
+            if (!flush && !busy && tail == head) break;
+            if (flush && tail == head) {
+                bool settled = false;
+                if (ready) {
+                    const unsigned long long b = sm.best[lane];
+                    const bool blocked = ANY && (uint32_t)b == 0u;
+                    tmax = __uint_as_float((uint32_t)(b >> 32));
+                    state = FREE;
+                    bool ended = blocked || !next_slot();
+                    settled = ended;
+                    if (ended && ties >> lane & 1u) {
+                        tmax = __uint_as_float((uint32_t)(b >> 32) + 1u);
+                        sm.best[lane] = (unsigned long long)__float_as_uint(tmax) << 32 | 0xFFFFFFFFull;
+                        k = 0;
+                        alone = again = true;
+                        ended = !next_slot();
+                    }
+                    if (ended) {
+                        const unsigned long long e = sm.best[lane];
+                        const uint32_t t = (uint32_t)(e >> 32) - (again && (uint32_t)e == 0xFFFFFFFFu ? 1u : 0u);
+                        fin(tag, __uint_as_float(t), ANY ? make_uint4(0u, 0u, 0u, 0u) : sm.hit[lane], blocked);
+                        own = false;
+                    }
+                }
+                ties &= ~__ballot_sync(ALL_LANES, settled);
+                __syncwarp();
+            }
+            // (a lane whose own ray waits for the queue takes nothing)
+            const uint32_t walking =
+                __ballot_sync(ALL_LANES, state == WALK || (ready && tail != head));
+            const bool spare = state == WALK && sp > base && !(home == lane && alone);
+            const uint32_t donors = __popc(~walking) >= WALK8_GIVE ? __ballot_sync(ALL_LANES, spare) : 0u;
+            if (donors) {
+                const uint32_t n = min(__popc(donors), __popc(~walking)), r = __popc(donors & below);
+                if (spare && r < n) sm.give[r] = make_uint2(sm.stk[base++][lane], lane << 8 | home);
+                __syncwarp();
+                const uint32_t q = __popc(~walking & below);
+                const bool take = !(walking >> lane & 1u) && q < n;
+                const uint2 e = take ? sm.give[q] : make_uint2(0u, lane << 8);
+                const uint32_t from = e.y >> 8;
+                o.x = __shfl_sync(ALL_LANES, o.x, from);
+                o.y = __shfl_sync(ALL_LANES, o.y, from);
+                o.z = __shfl_sync(ALL_LANES, o.z, from);
+                inv.x = __shfl_sync(ALL_LANES, inv.x, from);
+                inv.y = __shfl_sync(ALL_LANES, inv.y, from);
+                inv.z = __shfl_sync(ALL_LANES, inv.z, from);
+                tmax = __shfl_sync(ALL_LANES, tmax, from);
+                if (take) {
+                    cur = e.x;
+                    home = e.y & 31u;
+                    sp = base = 0;
                     state = WALK;
                 }
-                if (state == FREE)
-                    fin(tag, tmax, ANY ? make_uint4(0u, 0u, 0u, 0u) : sm.hit[lane], false);
             }
-            __syncwarp();
         }
         // one node in every walking lane
         uint32_t off0 = 0, n0 = 0, off1 = 0, n1 = 0;  // the hit leaves' triangles, nearer leaf first
@@ -142,10 +219,10 @@ __device__ __forceinline__ void walk2(const DevScene& S, Walk2Shared& sm, Gen ge
                 if (++iter > S.iterCapRef) {
                     latch(err, ERR_WATCHDOG);
                     cur = PE_NONE;
-                    sp = 0;
+                    sp = base;
                 }
             }
-            if (cur == PE_NONE && sp) cur = sm.stk[--sp][lane];
+            if (cur == PE_NONE && sp > base) cur = sm.stk[--sp][lane];
             if (cur == PE_NONE) state = ENDED;
         }
         // the triangles to the queue, four of each lane a pass, and rounds of tests
@@ -160,7 +237,7 @@ __device__ __forceinline__ void walk2(const DevScene& S, Walk2Shared& sm, Gen ge
                     n0 = n1;
                     n1 = 0;
                 }
-                sm.item[at % WALK2_QUEUE] = lane << 24 | off0++;
+                sm.item[at % WALK2_QUEUE] = home << 24 | off0++;
                 --n0;
             }
             if (mine) last = at;
@@ -170,13 +247,16 @@ __device__ __forceinline__ void walk2(const DevScene& S, Walk2Shared& sm, Gen ge
                 if (tail - head < 32u) {
                     if (tail == head) break;
                     if (any) break;  // more may come
-                    const uint32_t wait = __ballot_sync(ALL_LANES, state == ENDED && (int32_t)(last - head) > 0);
-                    if (__popc(wait) < WALK8_WAIT && (!wait || __any_sync(ALL_LANES, state == WALK))) break;
+                    const uint32_t wait =
+                        __ballot_sync(ALL_LANES, more ? state == ENDED && (int32_t)(last - head) > 0 : state != WALK);
+                    if (!flush && __popc(wait) < (more ? WALK8_WAIT : WALK8_TAIL) &&
+                        (!wait || __any_sync(ALL_LANES, state == WALK)))
+                        break;
                 }
                 __syncwarp();
                 const uint32_t n = min(32u, tail - head);
-                bool ok = false;
-                float t, u, v;
+                bool ok = false, tie = false;
+                float t = 0.0f, u, v;
                 uint32_t tri = 0, of = 0, slot = 0;  // of: the lane whose ray it is
                 if (lane < n) {
                     tri = sm.item[(head + lane) % WALK2_QUEUE];
@@ -187,11 +267,14 @@ __device__ __forceinline__ void walk2(const DevScene& S, Walk2Shared& sm, Gen ge
                     slot = __float_as_uint(rd.w);
                     float det;
                     uint32_t hb;
-                    ok = tri_hit(S, tri, xyz(ro), xyz(rd), limit, t, det, u, v, hb) &&
+                    const float upTo = ANY || more ? limit : __uint_as_float(__float_as_uint(limit) + 1u);
+                    ok = tri_hit(S, tri, xyz(ro), xyz(rd), upTo, t, det, u, v, hb) &&
                          (hb & (ANY ? TB_SHADOW_OK : TB_CLOSEST_OK)) && side_ok(hb, det * ro.w);
+                    tie = ok;
+                    ok = ok && t < limit;
                     ++vis.tri;
                 }
-                if (__any_sync(ALL_LANES, ok)) {
+                if (__any_sync(ALL_LANES, ok || tie)) {
                     const unsigned long long key = ANY ? 0ull : (unsigned long long)__float_as_uint(t) << 32 | lane;
                     if (ok) {
                         if (ANY) sm.best[of] = 0ull;  // blocked
@@ -199,9 +282,14 @@ __device__ __forceinline__ void walk2(const DevScene& S, Walk2Shared& sm, Gen ge
                     }
                     __syncwarp();
                     if (!ANY && ok && sm.best[of] == key) sm.hit[of] = make_uint4(tri, slot, pack_uv(u, v), 0u);
+                    if (!ANY && !more) {
+                        const unsigned long long b = sm.best[of];
+                        tie = tie && (uint32_t)(b >> 32) == __float_as_uint(t) && b != key && (uint32_t)b != 0xFFFFFFFFu;
+                        ties |= __reduce_or_sync(ALL_LANES, tie ? 1u << of : 0u) & ~__ballot_sync(ALL_LANES, alone);
+                    }
                     __syncwarp();
                     if (state != FREE) {
-                        const unsigned long long b = sm.best[lane];
+                        const unsigned long long b = sm.best[home];
                         if (!ANY) tmax = __uint_as_float((uint32_t)(b >> 32));
                         else if ((uint32_t)b == 0u) state = ENDED;
                     }
