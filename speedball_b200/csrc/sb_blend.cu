@@ -344,12 +344,14 @@ __device__ __forceinline__ void blend_upload_block(const DevCascade& C, const De
 template <bool ROUGH>
 __global__ void __launch_bounds__(BLEND_THREADS) k_blend_upload(DevCascade C, DevParams P) {
     __shared__ BlendSmem<ROUGH> S;
+    stage_begin(C.stamps, 4);
     blend_upload_block<ROUGH>(C, P, blockIdx.x, S);
 }
 
 // Every item of a batch: CTAs [blendBase, blendBase + blendBlocks) belong to item i.
 __global__ void __launch_bounds__(BLEND_THREADS) k_blend_upload_batch(const __grid_constant__ BatchArgs B) {
     __shared__ BlendSmem<false> S;  // batches carry no reflection lobes
+    stage_begin(B.it[0].W.C.stamps, 4);
     uint32_t i = 0;
     while (i + 1 < B.n && blockIdx.x >= B.it[i + 1].blendBase) ++i;
     const BatchItem& I = B.it[i];
@@ -360,12 +362,8 @@ __global__ void __launch_bounds__(BLEND_THREADS) k_blend_upload_batch(const __gr
 cudaError_t launch_blend_upload(const DevCascade& C, const DevParams& P, cudaStream_t st) {
     if (C.updatedCount == 0) return cudaSuccess;
     const uint32_t blocks = (C.updatedCount + BLEND_PROBES - 1) / BLEND_PROBES;
-    if (C.reflect && C.roughSpec)
-        k_blend_upload<true><<<blocks, BLEND_THREADS, 0, st>>>(C, P);
-    else
-        k_blend_upload<false><<<blocks, BLEND_THREADS, 0, st>>>(C, P);
-    note_launch();
-    return cudaGetLastError();
+    return launch_stage(C.reflect && C.roughSpec ? k_blend_upload<true> : k_blend_upload<false>, blocks,
+                        (uint32_t)BLEND_THREADS, 0, st, C, P);
 }
 
 const void* blend_batch_kernel() { return (const void*)k_blend_upload_batch; }
@@ -404,6 +402,7 @@ __device__ __forceinline__ float pow64(float c) {
 
 __global__ void __launch_bounds__(352) k_glossy(DevCascade C, DevParams P, uint32_t groupThreads) {
     extern __shared__ float4 gsm[];
+    stage_wait();
     const uint32_t N = C.rays;
     const uint32_t groups = blockDim.x / groupThreads;
     float4* dir = gsm;  // N ray directions, then groups x GLOSSY_PROBES x N rays: rgb, coverage
@@ -526,8 +525,7 @@ cudaError_t launch_glossy(const DevCascade& C, const DevParams& P, cudaStream_t 
     const size_t smem = (size_t)C.rays * (1u + groups * GLOSSY_PROBES) * sizeof(float4);
     const uint32_t perCta = groups * GLOSSY_PROBES;
     const uint32_t blocks = (C.updatedCount + perCta - 1u) / perCta;
-    k_glossy<<<blocks, groups * groupThreads, smem, st>>>(C, P, groupThreads); note_launch();
-    return cudaGetLastError();
+    return launch_stage(k_glossy, blocks, groups * groupThreads, smem, st, C, P, groupThreads);
 }
 
 // lightGridKernel, gi_probes.js:1893-1937. Every operation is separately

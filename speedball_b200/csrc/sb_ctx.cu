@@ -122,7 +122,10 @@ struct sb_ctx {
     FlatScene flat;
     float4* jobs = nullptr;        // shadow-ray job queue (2 float4 per job)
     uint32_t jobCap = 0;
-    cudaEvent_t ev0 = nullptr, evMid = nullptr, ev1 = nullptr, evA = nullptr, evB = nullptr, evC = nullptr;
+    cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    unsigned long long* dStamps = nullptr;  // when the last solve's stages started
+    bool stamped = false;          // the last solve had probes to update
+    bool workClear = false;        // dWork's cursors are zero (each solve's shading leaves them so)
     cudaEvent_t syncEv = nullptr;  // cross-context ordering of batched solves
     bool timed = false;
     bool lastWasGraph = false;     // ev0..ev1 bracket a graph launch (whole frame, no stage events)
@@ -284,6 +287,7 @@ DevCascade dev_cascade(const sb_ctx* c, uint32_t ci, uint32_t probeOffset, uint3
     D.probeOffset = probeOffset;
     D.updatedCount = updated;
     D.probePos = K.probePos;
+    D.stamps = c->dStamps;
     D.rayData = K.rayData;
     D.hits = K.hits;
     D.vis = K.vis;
@@ -475,6 +479,7 @@ sb_status sb_create(const sb_device_opts* opts, sb_ctx** out) {
         ctx->stream = ctx->ownStream;
         if (cudaMalloc(&ctx->dErr, 4) != cudaSuccess || cudaMalloc(&ctx->dGate, 4 * REFIT_RANGES * 4) != cudaSuccess ||
             cudaMalloc(&ctx->dWork, (QUERY_CURSOR + 8) * 4) != cudaSuccess ||
+            cudaMalloc(&ctx->dStamps, STAGE_STAMPS * 8) != cudaSuccess ||
             cudaMalloc(&ctx->dDirs, (ADJOINT_DIRS + MAX_RAYS) * sizeof(float4)) != cudaSuccess ||
             cudaMalloc(&ctx->dCounters, 16 * 8) != cudaSuccess ||
             cudaMalloc(&ctx->B.valid, 4) != cudaSuccess || cudaMalloc(&ctx->B.depth, 8) != cudaSuccess) {
@@ -486,11 +491,7 @@ sb_status sb_create(const sb_device_opts* opts, sb_ctx** out) {
         cudaMemset(ctx->B.depth, 0xFF, 8);
         cudaMemset(ctx->dCounters, 0, 128);
         cudaEventCreate(&ctx->ev0);
-        cudaEventCreate(&ctx->evMid);
         cudaEventCreate(&ctx->ev1);
-        cudaEventCreate(&ctx->evA);
-        cudaEventCreate(&ctx->evB);
-        cudaEventCreate(&ctx->evC);
         sb_params_defaults(&ctx->params);
         if (cudaDeviceSynchronize() != cudaSuccess) { st = SB_ERR_CUDA; break; }
     } while (0);
@@ -542,13 +543,9 @@ void sb_destroy(sb_ctx* ctx) {
     release(T.loss);
     for (cudaEvent_t e : {T.evF0, T.evF1, T.evB0, T.evB1})
         if (e) cudaEventDestroy(e);
-    release(ctx->dErr); release(ctx->dGate); release(ctx->dWork); release(ctx->dDirs); release(ctx->dCounters);
+    release(ctx->dErr); release(ctx->dGate); release(ctx->dWork); release(ctx->dDirs); release(ctx->dStamps); release(ctx->dCounters);
     if (ctx->syncEv) cudaEventDestroy(ctx->syncEv);
     if (ctx->ev0) cudaEventDestroy(ctx->ev0);
-    if (ctx->evMid) cudaEventDestroy(ctx->evMid);
-    if (ctx->evA) cudaEventDestroy(ctx->evA);
-    if (ctx->evB) cudaEventDestroy(ctx->evB);
-    if (ctx->evC) cudaEventDestroy(ctx->evC);
     if (ctx->evDeform) cudaEventDestroy(ctx->evDeform);
     if (ctx->hDeform) cudaFreeHost(ctx->hDeform);
     if (ctx->dDeform) cudaFree(ctx->dDeform);
@@ -958,6 +955,15 @@ sb_status sb_configure_cascade(sb_ctx* ctx, uint32_t ci, const sb_grid* g) {
     return SB_OK;
 }
 
+// The stages' cursors are zero when a solve starts: the shading of the last one has
+// cleared them, unless it was not enqueued to its end.
+static cudaError_t clear_work(sb_ctx* ctx) {
+    cudaError_t e = cudaSuccess;
+    if (!ctx->workClear) e = cudaMemsetAsync(ctx->dWork, 0, QUERY_CURSOR * sizeof(uint32_t), ctx->stream);
+    ctx->workClear = false;
+    return e;
+}
+
 sb_status sb_solve(sb_ctx* ctx, uint32_t ci, uint32_t probeOffset, uint32_t updatedCount) {
     if (!ctx) return SB_ERR_INVALID_ARG;
     if (ci >= SB_MAX_CASCADES || !ctx->casc[ci].configured)
@@ -1005,14 +1011,15 @@ sb_status sb_solve(sb_ctx* ctx, uint32_t ci, uint32_t probeOffset, uint32_t upda
     const bool timing = !ctx->capturing;  // events inside a capture would not be re-recorded by replays
     if (timing) CK(cudaEventRecord(ctx->ev0, ctx->stream));
     ctx->singleChunk = updatedCount <= chunk;
+    ctx->stamped = updatedCount != 0;
+    CK(clear_work(ctx));
     for (uint32_t s0 = 0; s0 < updatedCount; s0 += chunk) {
         uint32_t n = updatedCount - s0 < chunk ? updatedCount - s0 : chunk;
         CK(launch_trace(S, D, P, ctx->dErr, ctx->countersOn ? ctx->dCounters : nullptr, ctx->dWork, ctx->dDirs, ctx->tune,
-                        ctx->stream, ctx->jobs, ctx->jobCap, s0, n, timing ? ctx->evA : nullptr,
-                        timing ? ctx->evB : nullptr, timing ? ctx->evC : nullptr));
+                        ctx->stream, ctx->jobs, ctx->jobCap, s0, n));
     }
     if (ctx->emitterCount) CK(launch_emitter_vis(S, D, ctx->stream));
-    if (timing) CK(cudaEventRecord(ctx->evMid, ctx->stream));
+    ctx->workClear = true;
     CK(launch_blend_upload(D, P, ctx->stream));
     if (K.reflTier >= SB_REFLECT_HIGH) {
         // glossyKernel after the blend (gi_probes.js:3829-3835): this solve resolves
@@ -1154,14 +1161,15 @@ static sb_status enqueue_batch(const sb_solve_item* items, uint32_t count) {
     const bool timing = !lead->capturing;
     if (B.counters) CK(cudaMemsetAsync(lead->dCounters, 0, 128, lead->stream));
     if (timing) CK(cudaEventRecord(lead->ev0, lead->stream));
-    CK(launch_trace_batch(B, lead->tune, lead->stream, timing ? lead->evA : nullptr, timing ? lead->evB : nullptr,
-                          timing ? lead->evC : nullptr));
-    if (timing) CK(cudaEventRecord(lead->evMid, lead->stream));
+    CK(clear_work(lead));
+    CK(launch_trace_batch(B, lead->tune, lead->stream));
+    lead->workClear = true;
     CK(launch_blend_upload_batch(B, lead->stream));
     if (timing) {
         CK(cudaEventRecord(lead->ev1, lead->stream));
         lead->timed = true;
         lead->singleChunk = true;
+        lead->stamped = B.totalRays != 0;
         lead->lastWasGraph = false;
     }
     if (!lead->capturing) return join_streams(items, count, false);
@@ -1689,6 +1697,7 @@ sb_status sb_backward(sb_ctx* ctx, sb_grads* grads) {
         D.footPrev = T.foot + (size_t)s * probes * FOOT * FOOT_U4;
         D.rayData = T.shaded;
         D.eOut = nullptr;
+        D.stamps = nullptr;
         const float4* Hs = T.hist + (size_t)s * hist;
         const float4* Hs1 = T.hist + (size_t)(s + 1) * hist;
         const bool last = s + 1 == (int)T.solves;
@@ -2203,13 +2212,19 @@ sb_status sb_get_stats(sb_ctx* ctx, sb_stats* out) {
     } else if (ctx->timed) {
         float ms = 0.0f;
         if (cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1) == cudaSuccess) out->lastSolveMs = ms;
-        if (cudaEventElapsedTime(&ms, ctx->ev0, ctx->evMid) == cudaSuccess) out->lastTraceMs = ms;
-        if (cudaEventElapsedTime(&ms, ctx->evMid, ctx->ev1) == cudaSuccess) out->lastBlendMs = ms;
-        if (ctx->singleChunk) {
-            if (cudaEventElapsedTime(&ms, ctx->ev0, ctx->evC) == cudaSuccess) out->lastPrimaryMs = ms;
-            if (cudaEventElapsedTime(&ms, ctx->evC, ctx->evA) == cudaSuccess) out->lastEmitMs = ms;
-            if (cudaEventElapsedTime(&ms, ctx->evA, ctx->evB) == cudaSuccess) out->lastShadowMs = ms;
-            if (cudaEventElapsedTime(&ms, ctx->evB, ctx->evMid) == cudaSuccess) out->lastShadeMs = ms;
+        // a stage from its start to the next one's; the blend what the trace leaves of the solve
+        unsigned long long t[STAGE_STAMPS];
+        CK(cudaMemcpy(t, ctx->dStamps, sizeof t, cudaMemcpyDeviceToHost));
+        auto between = [&](int a, int b) { return t[b] > t[a] ? (float)((double)(t[b] - t[a]) * 1e-6) : 0.0f; };
+        if (ctx->stamped) {
+            out->lastTraceMs = std::min(between(0, 4), out->lastSolveMs);
+            out->lastBlendMs = out->lastSolveMs - out->lastTraceMs;
+        }
+        if (ctx->stamped && ctx->singleChunk) {
+            out->lastPrimaryMs = between(0, 1);
+            out->lastEmitMs = between(1, 2);
+            out->lastShadowMs = between(2, 3);
+            out->lastShadeMs = between(3, 4);
         }
     }
     float fms = 0.0f;

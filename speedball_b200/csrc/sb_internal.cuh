@@ -108,6 +108,7 @@ struct DevCascade {
     float g0Min[3], g0Size[3];
     uint32_t g0Res[3];
     const float4* probePos;    // every probe's position (probe_world_pos)
+    unsigned long long* stamps;  // when each stage started (stage_begin), or null
     float4* rayData;           // updatedCount*rays
     uint4* hits;               // 16-byte hit records: tri, inst | facing << 31, t, packed uv
     uint4* vis;                // NEE masks: tested lights (lo, hi), unblocked lights (lo, hi)
@@ -230,6 +231,25 @@ __device__ __forceinline__ uint32_t batch_item(const BatchArgs& B, uint32_t g) {
 #pragma unroll 1
     while (i + 1 < B.n && g >= B.it[i + 1].rayBase) ++i;
     return i;
+}
+
+// The stages of a solve follow one another as programmatic dependent launches: each
+// starts by waiting for the end of the one ahead, whose launch it then need not wait for
+// in the stream. (Letting the next stage's CTAs come up earlier, with a trigger at a
+// stage's start, costs more than it hides: they hold shared memory and change its split
+// with the L1. Room update 172 us so, 159 without dependent launches, 149 as it is.)
+// Stage `i` (0 closest hits .. 4 blend) also notes when it started, for the per-stage
+// times: an event record between two kernels costs some 2 us of the device (room 169
+// with events and a memset of the cursors).
+constexpr int STAGE_STAMPS = 5;
+__device__ __forceinline__ void stage_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void stage_begin(unsigned long long* stamps, int i) {
+    stage_wait();
+    if (stamps && blockIdx.x == 0 && threadIdx.x == 0) {
+        unsigned long long t;
+        asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+        stamps[i] = t;
+    }
 }
 
 __device__ __forceinline__ void latch(uint32_t* err, uint32_t bit) {

@@ -6,6 +6,25 @@ namespace sb {
 
 // Process-wide count of kernels this library launched (reported in sb_stats).
 void note_launch();
+
+// A programmatic dependent launch: the kernel (and any that it follows so) starts with
+// stage_wait.
+template <class... P, class... A>
+inline cudaError_t launch_stage(void (*kernel)(P...), uint32_t grid, uint32_t block, size_t smem, cudaStream_t st,
+                                const A&... args) {
+    cudaLaunchAttribute serial{};
+    serial.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    serial.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &serial;
+    cfg.numAttrs = 1;
+    note_launch();
+    return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
 uint64_t launches();
 
 struct TraceTuning {
@@ -46,9 +65,7 @@ struct SceneBuffers {
 // `jobs` holds up to jobCap shadow-ray jobs (32 bytes each).
 cudaError_t launch_trace(const DevScene& S, const DevCascade& C, const DevParams& P, uint32_t* err,
                          unsigned long long* counters, uint32_t* work, float4* dirs, const TraceTuning& tune,
-                         cudaStream_t st, float4* jobs, uint32_t jobCap, uint32_t slotBegin, uint32_t slotCount,
-                         cudaEvent_t afterPrimary = nullptr, cudaEvent_t afterShadow = nullptr,
-                         cudaEvent_t afterClosest = nullptr);
+                         cudaStream_t st, float4* jobs, uint32_t jobCap, uint32_t slotBegin, uint32_t slotCount);
 cudaError_t launch_blend_upload(const DevCascade& C, const DevParams& P, cudaStream_t st);
 // Positions (and normals when given), 3 floats per vertex, into the first six
 // floats of n pooled 8-float vertices.
@@ -59,9 +76,7 @@ cudaError_t launch_shade(const DevScene& S, const DevCascade& C, const DevParams
                          uint32_t slotCount, cudaStream_t st);
 
 // Batched stages (every item of B in one launch per stage).
-cudaError_t launch_trace_batch(const BatchArgs& B, const TraceTuning& tune, cudaStream_t st,
-                               cudaEvent_t afterPrimary = nullptr, cudaEvent_t afterShadow = nullptr,
-                         cudaEvent_t afterClosest = nullptr);
+cudaError_t launch_trace_batch(const BatchArgs& B, const TraceTuning& tune, cudaStream_t st);
 cudaError_t launch_blend_upload_batch(const BatchArgs& B, cudaStream_t st);
 uint32_t blend_blocks(uint32_t updatedCount);  // CTAs of the blend for one solve
 // The batched kernels (stage 0 primary, 1 emit, 2 shadow, 3 shade; blend):

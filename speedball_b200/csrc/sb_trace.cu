@@ -451,6 +451,7 @@ __device__ __forceinline__ float3 staged_dir(const float4* sm, uint32_t k, float
 // The 8-wide tree (bvhKind 1).
 __global__ void __launch_bounds__(256, SB_WALK8_MIN_BLOCKS) k_trace_primary_walk8(WaveCtx W) {
     extern __shared__ float4 smem[];
+    stage_begin(W.slotBegin ? nullptr : W.C.stamps, 0);  // (a later chunk of the same solve)
     if (!*W.S.valid) return;
     if (blockIdx.x == 0) write_dirs(W);
     stage_dirs(W, smem);
@@ -463,6 +464,7 @@ __global__ void __launch_bounds__(256, SB_WALK8_MIN_BLOCKS) k_trace_primary_walk
 
 __global__ void __launch_bounds__(256, SB_WALK8_MIN_BLOCKS) k_trace_shadow_walk8(WaveCtx W) {
     extern __shared__ float4 smem[];
+    stage_begin(W.C.stamps, 2);
     if (!*W.S.valid) return;
     const WalkSmem m = walk_shared(smem, W.S.wideDepth + 1u, W.S.dynCount != 0u);
     Visits vis = {0, 0, 0, 0};
@@ -473,6 +475,7 @@ __global__ void __launch_bounds__(256, SB_WALK8_MIN_BLOCKS) k_trace_shadow_walk8
 // The binary scene BVH and the two-level walk (bvhKind 2 and 0).
 __global__ void __launch_bounds__(256, SB_PRIMARY_MIN_BLOCKS) k_trace_primary(WaveCtx W) {
     extern __shared__ uint4 sTlas[];
+    stage_begin(W.slotBegin ? nullptr : W.C.stamps, 0);  // (a later chunk of the same solve)
     const bool pairs = closest_pairs(W.S);
     const uint4* tl = stage_tlas(W, sTlas, pairs);
     if (!*W.S.valid) return;
@@ -546,6 +549,7 @@ __device__ void order_batches(const uint32_t* cost, uint32_t* order, uint32_t n,
 constexpr int EMIT_MIN_BLOCKS = 8;
 __global__ void __launch_bounds__(128, EMIT_MIN_BLOCKS) k_emit(WaveCtx W) {
     __shared__ float4 gates[4][GATE_LIGHTS];
+    stage_begin(W.C.stamps, 1);
     if (!*W.S.valid) return;
     const uint32_t total = W.slotCount * W.C.rays;
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
@@ -558,6 +562,7 @@ __global__ void __launch_bounds__(128, EMIT_MIN_BLOCKS) k_emit(WaveCtx W) {
 
 __global__ void __launch_bounds__(256, SB_SHADOW_MIN_BLOCKS) k_trace_shadow(WaveCtx W) {
     extern __shared__ uint4 sTlas[];
+    stage_begin(W.C.stamps, 2);
     const bool pairs = any_pairs(W.S);
     const uint4* tl = stage_tlas(W, sTlas, pairs);
     if (!*W.S.valid) return;
@@ -587,7 +592,15 @@ __global__ void __launch_bounds__(256, SB_SHADOW_MIN_BLOCKS) k_trace_shadow(Wave
     }
 }
 
+// The cursors of the stages ahead, for the next solve (128 threads).
+static_assert(SB_BATCH_MAX * WORK_WORDS <= 128, "one word per thread of a CTA");
+__device__ __forceinline__ void clear_work(uint32_t* work, uint32_t words) {
+    if (work && blockIdx.x == 0 && threadIdx.x < words) work[threadIdx.x] = 0u;
+}
+
 __global__ void __launch_bounds__(128) k_shade(WaveCtx W) {
+    stage_begin(W.C.stamps, 3);
+    clear_work(W.work, WORK_WORDS);
     if (!*W.S.valid) return;
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= W.slotCount * W.C.rays) return;
@@ -606,6 +619,7 @@ __global__ void __launch_bounds__(128) k_shade(WaveCtx W) {
 // unblocked mask of its probe's ray 0: the NEE tests no such record, so the bit is free
 // until the fold takes it out again.
 __global__ void __launch_bounds__(128) k_emitter_jobs(WaveCtx W) {
+    stage_wait();
     if (!*W.S.valid) return;
     const DevCascade& C = W.C;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
@@ -657,6 +671,7 @@ __global__ void __launch_bounds__(128) k_emitter_jobs(WaveCtx W) {
 }
 
 __global__ void __launch_bounds__(128) k_emitter_vis(DevScene S, DevCascade C) {
+    stage_wait();
     const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
     if (slot >= C.updatedCount || !*S.valid) return;
     uint4* ray = C.vis + (size_t)slot * C.rays;
@@ -673,9 +688,7 @@ __global__ void __launch_bounds__(128) k_emitter_vis(DevScene S, DevCascade C) {
 
 cudaError_t launch_emitter_vis(const DevScene& S, const DevCascade& C, cudaStream_t st) {
     if (C.updatedCount == 0 || C.emitterCount == 0) return cudaSuccess;
-    k_emitter_vis<<<(C.updatedCount + 127) / 128, 128, 0, st>>>(S, C);
-    note_launch();
-    return cudaGetLastError();
+    return launch_stage(k_emitter_vis, (C.updatedCount + 127) / 128, 128, 0, st, S, C);
 }
 
 // Stage C alone over probe slots [0, slotCount) from the records already in
@@ -714,8 +727,7 @@ static int walk8_grid(const void* kernel, int block, size_t smem, const TraceTun
 
 cudaError_t launch_trace(const DevScene& S, const DevCascade& C, const DevParams& P, uint32_t* err,
                          unsigned long long* counters, uint32_t* work, float4* dirs, const TraceTuning& tune,
-                         cudaStream_t st, float4* jobs, uint32_t jobCap, uint32_t slotBegin, uint32_t slotCount,
-                         cudaEvent_t afterPrimary, cudaEvent_t afterShadow, cudaEvent_t afterClosest) {
+                         cudaStream_t st, float4* jobs, uint32_t jobCap, uint32_t slotBegin, uint32_t slotCount) {
     if (slotCount == 0) return cudaSuccess;
     WaveCtx W;
     W.S = S;
@@ -740,38 +752,31 @@ cudaError_t launch_trace(const DevScene& S, const DevCascade& C, const DevParams
         cudaFuncSetAttribute(k_trace_primary, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         cudaFuncSetAttribute(k_trace_shadow, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     }
-    // ray, job-read and job-write cursors, the batch-order claim, the moved slots' cursors
-    cudaError_t e = cudaMemsetAsync(work, 0, 6 * sizeof(uint32_t), st);
-    if (e != cudaSuccess) return e;
-    const uint32_t rays = slotCount * C.rays;
+    const uint32_t rays = slotCount * C.rays, perRay = (rays + 127) / 128;
     const int block = (int)tune.block;
-    const uint32_t smem8 = walk_smem(S.wideDepth + 1u, S.dynCount != 0u, tune.block);
-    const uint32_t smemP = smem8 + 2u * C.rays * (uint32_t)sizeof(float4);
+    const size_t smem8 = walk_smem(S.wideDepth + 1u, S.dynCount != 0u, tune.block);
+    const size_t smemP = smem8 + 2u * C.rays * sizeof(float4);
+    cudaError_t e;
     if (S.wideNodes)
         k_trace_primary_walk8<<<walk8_grid((const void*)k_trace_primary_walk8, block, smemP, tune, rays), block, smemP,
                                 st>>>(W);
     else
         k_trace_primary<<<persistent_grid((const void*)k_trace_primary, block, smem, tune, rays), block, smem, st>>>(W);
     note_launch();
-    if (afterClosest) cudaEventRecord(afterClosest, st);
-    k_emit<<<(rays + 127) / 128, 128, 0, st>>>(W);
-    note_launch();
-    if (C.emitterCount) {
-        k_emitter_jobs<<<(slotCount + 127) / 128, 128, 0, st>>>(W);
-        note_launch();
-    }
-    if (afterPrimary) cudaEventRecord(afterPrimary, st);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if ((e = launch_stage(k_emit, perRay, 128, 0, st, W)) != cudaSuccess) return e;
+    if (C.emitterCount && (e = launch_stage(k_emitter_jobs, (slotCount + 127) / 128, 128, 0, st, W)) != cudaSuccess)
+        return e;
     // shadow jobs: at most lightCount per ray (the queue is sized for it)
     if (S.wideNodes)
-        k_trace_shadow_walk8<<<walk8_grid((const void*)k_trace_shadow_walk8, block, smem8, tune, rays * 4u), block,
-                               smem8, st>>>(W);
+        e = launch_stage(k_trace_shadow_walk8,
+                         (uint32_t)walk8_grid((const void*)k_trace_shadow_walk8, block, smem8, tune, rays * 4u),
+                         (uint32_t)block, smem8, st, W);
     else
-        k_trace_shadow<<<persistent_grid((const void*)k_trace_shadow, block, smem, tune, rays * 4u), block, smem, st>>>(W);
-    note_launch();
-    if (afterShadow) cudaEventRecord(afterShadow, st);
-    k_shade<<<(rays + 127) / 128, 128, 0, st>>>(W);
-    note_launch();
-    return cudaGetLastError();
+        e = launch_stage(k_trace_shadow,
+                         (uint32_t)persistent_grid((const void*)k_trace_shadow, block, smem, tune, rays * 4u),
+                         (uint32_t)block, smem, st, W);
+    return e != cudaSuccess ? e : launch_stage(k_shade, perRay, 128, 0, st, W);
 }
 
 // ---------------------------------------------------------------- batched
@@ -787,6 +792,7 @@ __device__ __forceinline__ uint32_t next_item(const BatchArgs& B, uint32_t i) { 
 
 __global__ void __launch_bounds__(256, SB_WALK8_MIN_BLOCKS) k_trace_primary_batch(const __grid_constant__ BatchArgs B) {
     extern __shared__ float4 smem[];
+    stage_begin(B.it[0].W.C.stamps, 0);
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t first = batch_item(B, (uint32_t)((uint64_t)blockIdx.x * B.totalRays / gridDim.x));
     for (uint32_t j = blockIdx.x; j < B.n; j += gridDim.x) write_dirs(B.it[j].W);
@@ -825,6 +831,7 @@ __global__ void __launch_bounds__(256, SB_WALK8_MIN_BLOCKS) k_trace_primary_batc
 
 __global__ void __launch_bounds__(128, EMIT_MIN_BLOCKS) k_emit_batch(const __grid_constant__ BatchArgs B) {
     __shared__ float4 gates[4][GATE_LIGHTS];
+    stage_begin(B.it[0].W.C.stamps, 1);
     const uint32_t gg = blockIdx.x * blockDim.x + threadIdx.x;
     if (gg - (threadIdx.x & 31u) >= B.totalRays) return;  // whole warps only
     const BatchItem& I = B.it[batch_item(B, gg & ~31u)];
@@ -839,6 +846,7 @@ __global__ void __launch_bounds__(128, EMIT_MIN_BLOCKS) k_emit_batch(const __gri
 
 __global__ void __launch_bounds__(256, SB_WALK8_MIN_BLOCKS) k_trace_shadow_batch(const __grid_constant__ BatchArgs B) {
     extern __shared__ float4 smem[];
+    stage_begin(B.it[0].W.C.stamps, 2);
     const uint32_t lane = threadIdx.x & 31u;
     const WalkSmem m = walk_shared(smem, B.wideDepth + 1u, B.moved != 0u);
     Visits vis = {0, 0, 0, 0};
@@ -880,6 +888,8 @@ __global__ void __launch_bounds__(256, SB_WALK8_MIN_BLOCKS) k_trace_shadow_batch
 }
 
 __global__ void __launch_bounds__(128) k_shade_batch(const __grid_constant__ BatchArgs B) {
+    stage_begin(B.it[0].W.C.stamps, 3);
+    clear_work(B.work, SB_BATCH_MAX * WORK_WORDS);
     const uint32_t gg = blockIdx.x * blockDim.x + threadIdx.x;
     if (gg >= B.totalRays) return;
     const BatchItem& I = B.it[batch_item(B, gg & ~31u)];
@@ -907,25 +917,19 @@ uint32_t trace_batch_smem(const BatchArgs& B, uint32_t threads) {
     return smem;
 }
 
-cudaError_t launch_trace_batch(const BatchArgs& B, const TraceTuning& tune, cudaStream_t st,
-                               cudaEvent_t afterPrimary, cudaEvent_t afterShadow, cudaEvent_t afterClosest) {
+cudaError_t launch_trace_batch(const BatchArgs& B, const TraceTuning& tune, cudaStream_t st) {
     if (B.n == 0 || B.totalRays == 0) return cudaSuccess;
-    cudaError_t e = cudaMemsetAsync(B.work, 0, SB_BATCH_MAX * WORK_WORDS * sizeof(uint32_t), st);
-    if (e != cudaSuccess) return e;
     const int block = (int)tune.block;
     const uint32_t rays = B.totalRays;
     const size_t smem = trace_batch_smem(B, tune.block);
     k_trace_primary_batch<<<walk8_grid((const void*)k_trace_primary_batch, block, smem, tune, rays), block, smem,
                             st>>>(B);
     note_launch();
-    if (afterClosest) cudaEventRecord(afterClosest, st);
     k_emit_batch<<<(rays + 127) / 128, 128, 0, st>>>(B);
     note_launch();
-    if (afterPrimary) cudaEventRecord(afterPrimary, st);
     k_trace_shadow_batch<<<walk8_grid((const void*)k_trace_shadow_batch, block, smem, tune, rays * 4u), block, smem,
                            st>>>(B);
     note_launch();
-    if (afterShadow) cudaEventRecord(afterShadow, st);
     k_shade_batch<<<(rays + 127) / 128, 128, 0, st>>>(B);
     note_launch();
     return cudaGetLastError();
