@@ -723,9 +723,10 @@ __device__ __forceinline__ bool trace_any(const DevScene& S, const uint4* tl, fl
 
 // The chosen hit's ray parameter re-evaluated in FP64: the same Möller–Trumbore
 // expression (spectral_traverse.js:396-408) on the local ray (instLocalRay,
-// 149-153), with the edges taken from the pooled vertices. FP32 alone loses ~1e-5
+// 149-153), on the triangle's vertices as the walks test them. FP32 alone loses ~1e-5
 // relative on near hits (the local origin is rounded at scene scale); this keeps t
-// within ~1e-7 of the exact value.
+// within ~1e-7 of the exact value. The pre-gathered vertices instead of three indices
+// and nine values: 47 -> 29 us for 2.07M hits, the atrium's emission 39.5 -> 36.2 us.
 static __device__ float refine_t(const DevScene& S, uint32_t tri, uint32_t inst, float3 wro, float3 wrd) {
     double o[3], d[3], v[3][3];
 #pragma unroll
@@ -733,9 +734,10 @@ static __device__ float refine_t(const DevScene& S, uint32_t tri, uint32_t inst,
         const float4 r = __ldg(S.inst + 4 * inst + k);
         o[k] = (double)r.x * wro.x + (double)r.y * wro.y + (double)r.z * wro.z + (double)r.w;
         d[k] = (double)r.x * wrd.x + (double)r.y * wrd.y + (double)r.z * wrd.z;
-        const float* p = S.vertexData + (size_t)__ldg(S.triIndex + 3 * tri + k) * 8u;
-#pragma unroll
-        for (int a = 0; a < 3; ++a) v[k][a] = __ldg(p + a);
+        const float4 p = __ldg(S.tris + 3 * tri + k);
+        v[k][0] = p.x;
+        v[k][1] = p.y;
+        v[k][2] = p.z;
     }
     double e1[3], e2[3], tv[3];
 #pragma unroll
