@@ -9,6 +9,32 @@
 
 namespace sb {
 
+// Two Kahan sums (kahan_fma) side by side in packed operations: the same roundings, with
+// the compensation kept negated (t - s and y - d as fma by -1, which is exact). The sums
+// are half of the blend's instructions, and issue bounds it: 32 -> 29.5 us for the
+// atrium's 4,096 probes x 64 rays, 51 -> 47 for 128 rays. Packed, they take 68 registers;
+// held to 56 (four CTAs per SM) 29.5 us, at three CTAs 32.7.
+__device__ __forceinline__ unsigned long long f32x2(float lo, float hi) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ void kahan_fma2(unsigned long long& s, unsigned long long& nc, unsigned long long w,
+                                           unsigned long long x) {
+    const unsigned long long neg = 0xBF800000BF800000ull;  // (-1, -1)
+    unsigned long long y, t, d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(y) : "l"(w), "l"(x), "l"(nc));
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(t) : "l"(s), "l"(y));
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(s), "l"(neg), "l"(t));
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(nc) : "l"(d), "l"(neg), "l"(y));
+    s = t;
+}
+
 // One CTA blends BLEND_PROBES probes, one thread per (probe, interior texel).
 // The cosine weight pow(max(dot(texelDir, rayDir), 0), cosPow) and the depth
 // weight pow(cw, depthSharpness) depend on (texel, ray) only, not on the probe,
@@ -29,8 +55,7 @@ template <bool ROUGH> struct BlendSmem {
     static constexpr int CH = ROUGH ? 32 : 64;  // rays staged per pass
     float4 texDir[BLEND_TEXELS];
     float4 rayDir[CH];
-    float wc[CH][BLEND_TEXELS];               // cosine weight  [ray][texel]
-    float wd[CH][BLEND_TEXELS];               // depth weight   [ray][texel]
+    float2 w[CH][BLEND_TEXELS];               // cosine and depth weight [ray][texel]
     float wr[ROUGH ? CH : 1][BLEND_TEXELS];   // rough lobe weight cd^8
     union {
         struct {
@@ -82,11 +107,11 @@ __device__ __forceinline__ void blend_upload_block(const DevCascade& C, const De
         S.texDir[tid] = make_float4(d.x, d.y, d.z, 0.0f);
     }
 
-    float sr = 0.f, sg = 0.f, sb = 0.f, sl = 0.f, sl2 = 0.f, ws = 0.f, sd = 0.f, sd2 = 0.f, dws = 0.f;
-    float cr = 0.f, cg = 0.f, cb = 0.f, cl = 0.f, cl2 = 0.f, cws = 0.f, cd = 0.f, cd2 = 0.f, cdw = 0.f;
+    // pairs of sums and their negated compensations: r g, b luma, luma^2 distance; rough lobe r g, b coverage
+    unsigned long long srg = 0, sbl = 0, sld = 0, crg = 0, cbl = 0, cld = 0, xrg = 0, xbh = 0, kxrg = 0, kxbh = 0;
+    float ws = 0.f, sd2 = 0.f, dws = 0.f, cws = 0.f, cd2 = 0.f, cdw = 0.f;
     // rough lobe sums (sAcc, sHit, sWsum of gi_probes.js:2358-2360) and their compensations
-    float xr = 0.f, xg = 0.f, xb = 0.f, xh = 0.f, xws = 0.f;
-    float kxr = 0.f, kxg = 0.f, kxb = 0.f, kxh = 0.f, kxws = 0.f;
+    float xws = 0.f, kxws = 0.f;
     // a true miss feeds the lobe only with an explicit sky fallback (gi_probes.js:2364-2367)
     const float skyValid = ROUGH ? P.reflectionSkyFallback * P.skyConfigured * (P.skyIntensity > 0.0f ? 1.0f : 0.0f)
                                  : 0.0f;
@@ -126,8 +151,7 @@ __device__ __forceinline__ void blend_upload_block(const DevCascade& C, const De
             } else {
                 dw = powf(cw, P.depthSharpness);
             }
-            S.wc[k][j] = cw;
-            S.wd[k][j] = dw;
+            S.w[k][j] = make_float2(cw, dw);
             if (ROUGH) {  // fixed power-8 lobe as ((cd^2)^2)^2 (gi_probes.js:2389-2393)
                 const float c2 = cd * cd, c4 = c2 * c2;
                 S.wr[k][j] = c4 * c4;
@@ -137,32 +161,34 @@ __device__ __forceinline__ void blend_upload_block(const DevCascade& C, const De
         if (live) {
 #pragma unroll 4
             for (uint32_t k = 0; k < n; ++k) {
-                float w = S.wc[k][lane], v = S.wd[k][lane];
-                float4 a = S.u.f.fa[p][k], b = S.u.f.fb[p][k];
-                kahan_fma(sr, cr, w, a.x);
-                kahan_fma(sg, cg, w, a.y);
-                kahan_fma(sb, cb, w, a.z);
-                kahan_fma(sl, cl, w, a.w);
-                kahan_fma(sl2, cl2, w, b.x);
-                kahan_fma(sd, cd, v, b.y);
-                kahan_fma(sd2, cd2, v, b.z);
+                const float2 wv = S.w[k][lane];
+                const float4 a = S.u.f.fa[p][k], b = S.u.f.fb[p][k];
+                const unsigned long long ww = f32x2(wv.x, wv.x);
+                kahan_fma2(srg, crg, ww, f32x2(a.x, a.y));
+                kahan_fma2(sbl, cbl, ww, f32x2(a.z, a.w));
+                kahan_fma2(sld, cld, f32x2(wv.x, wv.y), f32x2(b.x, b.y));  // luma^2, distance
+                kahan_fma(sd2, cd2, wv.y, b.z);
                 if (ROUGH) {
                     const float r = S.wr[k][lane];
                     const float rv = r * b.w;  // coverage is 0 or 1: exact
-                    kahan_fma(xr, kxr, rv, a.x);
-                    kahan_fma(xg, kxg, rv, a.y);
-                    kahan_fma(xb, kxb, rv, a.z);
-                    kahan_fma(xh, kxh, rv, 1.0f);
+                    const unsigned long long rr = f32x2(rv, rv);
+                    kahan_fma2(xrg, kxrg, rr, f32x2(a.x, a.y));
+                    kahan_fma2(xbh, kxbh, rr, f32x2(a.z, 1.0f));
                 }
             }
             if (p == 0)  // the weight sums depend on (texel, ray) only: the first probe's lanes form them
                 for (uint32_t k = 0; k < n; ++k) {
-                    kahan_fma(ws, cws, S.wc[k][lane], 1.0f);
-                    kahan_fma(dws, cdw, S.wd[k][lane], 1.0f);
+                    kahan_fma(ws, cws, S.w[k][lane].x, 1.0f);
+                    kahan_fma(dws, cdw, S.w[k][lane].y, 1.0f);
                     if (ROUGH) kahan_fma(xws, kxws, S.wr[k][lane], 1.0f);
                 }
         }
     }
+    float sr = unpack2(srg).x, sg = unpack2(srg).y, sb = unpack2(sbl).x, sl = unpack2(sbl).y, sl2 = unpack2(sld).x;
+    float sd = unpack2(sld).y;
+    float cr = -unpack2(crg).x, cg = -unpack2(crg).y, cb = -unpack2(cbl).x, cl = -unpack2(cbl).y, cl2 = -unpack2(cld).x;
+    float xr = unpack2(xrg).x, xg = unpack2(xrg).y, xb = unpack2(xbh).x, xh = unpack2(xbh).y;
+    float kxr = -unpack2(kxrg).x, kxg = -unpack2(kxrg).y, kxb = -unpack2(kxbh).x, kxh = -unpack2(kxbh).y;
     if (p == 0) {
         S.wsum[lane] = ws;
         S.dwsum[lane] = dws;
@@ -341,15 +367,16 @@ __device__ __forceinline__ void blend_upload_block(const DevCascade& C, const De
     }
 }
 
+constexpr int BLEND_MIN_BLOCKS = 4;
 template <bool ROUGH>
-__global__ void __launch_bounds__(BLEND_THREADS) k_blend_upload(DevCascade C, DevParams P) {
+__global__ void __launch_bounds__(BLEND_THREADS, BLEND_MIN_BLOCKS) k_blend_upload(DevCascade C, DevParams P) {
     __shared__ BlendSmem<ROUGH> S;
     stage_begin(C.stamps, 4);
     blend_upload_block<ROUGH>(C, P, blockIdx.x, S);
 }
 
 // Every item of a batch: CTAs [blendBase, blendBase + blendBlocks) belong to item i.
-__global__ void __launch_bounds__(BLEND_THREADS) k_blend_upload_batch(const __grid_constant__ BatchArgs B) {
+__global__ void __launch_bounds__(BLEND_THREADS, BLEND_MIN_BLOCKS) k_blend_upload_batch(const __grid_constant__ BatchArgs B) {
     __shared__ BlendSmem<false> S;  // batches carry no reflection lobes
     stage_begin(B.it[0].W.C.stamps, 4);
     uint32_t i = 0;
