@@ -956,12 +956,19 @@ sb_status sb_configure_cascade(sb_ctx* ctx, uint32_t ci, const sb_grid* g) {
 }
 
 // The stages' cursors are zero when a solve starts: the shading of the last one has
-// cleared them, unless it was not enqueued to its end.
+// cleared them, unless it was not enqueued to its end. A captured solve, which may be
+// replayed after any other, always clears them itself.
+static bool in_capture(const sb_ctx* ctx) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    return ctx->capturing || (cudaStreamIsCapturing(ctx->stream, &st) == cudaSuccess && st != cudaStreamCaptureStatusNone);
+}
 static cudaError_t clear_work(sb_ctx* ctx) {
-    cudaError_t e = cudaSuccess;
-    if (!ctx->workClear) e = cudaMemsetAsync(ctx->dWork, 0, QUERY_CURSOR * sizeof(uint32_t), ctx->stream);
-    ctx->workClear = false;
-    return e;
+    const bool captured = in_capture(ctx);
+    if (!captured && ctx->workClear) {
+        ctx->workClear = false;
+        return cudaSuccess;
+    }
+    return cudaMemsetAsync(ctx->dWork, 0, QUERY_CURSOR * sizeof(uint32_t), ctx->stream);
 }
 
 sb_status sb_solve(sb_ctx* ctx, uint32_t ci, uint32_t probeOffset, uint32_t updatedCount) {
@@ -1019,7 +1026,7 @@ sb_status sb_solve(sb_ctx* ctx, uint32_t ci, uint32_t probeOffset, uint32_t upda
                         ctx->stream, ctx->jobs, ctx->jobCap, s0, n));
     }
     if (ctx->emitterCount) CK(launch_emitter_vis(S, D, ctx->stream));
-    ctx->workClear = true;
+    ctx->workClear = ctx->workClear || !in_capture(ctx);
     CK(launch_blend_upload(D, P, ctx->stream));
     if (K.reflTier >= SB_REFLECT_HIGH) {
         // glossyKernel after the blend (gi_probes.js:3829-3835): this solve resolves
@@ -1163,7 +1170,7 @@ static sb_status enqueue_batch(const sb_solve_item* items, uint32_t count) {
     if (timing) CK(cudaEventRecord(lead->ev0, lead->stream));
     CK(clear_work(lead));
     CK(launch_trace_batch(B, lead->tune, lead->stream));
-    lead->workClear = true;
+    lead->workClear = lead->workClear || !in_capture(lead);
     CK(launch_blend_upload_batch(B, lead->stream));
     if (timing) {
         CK(cudaEventRecord(lead->ev1, lead->stream));
