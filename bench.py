@@ -223,24 +223,24 @@ def run_ours(args, dist: Dist):
                    shadow_blas=st.shadowBlasNodeVisits, shadow_tri=st.shadowTriangleTests)
     # algorithmic bytes per launch of each stage. Per-unit figures: 32 B TLAS node, 64 B instance
     # record, 48 B pre-gathered triangle; per box test 32 B (a BLAS node, or half a 64 B child-pair
-    # node) or 10 B on the 8-wide closest-hit tree (80 B node / 8 boxes); 16 B raw hit record per ray
+    # node) or 10 B on the 8-wide tree (80 B node / 8 boxes; the moved slots' pair nodes, a few
+    # percent of the tests, are counted the same); 16 B raw hit record per ray
     # (written by the closest-hit stage, read by the emission stage); emission per ray 16 B visibility
     # mask, per hit 16 B final hit record + 48 B instance rows + 48 B pre-gathered triangle + 48 B
     # reference triangle (3 indices, 3 vertices) for the refined t, 32 B per shadow job (written by the
     # emission stage, read by the shadow stage); per hit 80 B of triangle/instance rows, 40 B material,
-    # 256 B of bounce taps (8 taps x 4 texels x 8 B); 16 B ray record write; 3,776 B per probe for
+    # 256 B of bounce taps (8 footprints of 32 B); 16 B ray record write; 3,776 B per probe for
     # blend + upload.
     tun = _abi.sb_tuning()
     _abi.check(lib.sb_get_tuning(ctx, C.byref(tun)), ctx)
-    closest_box = 10 if tun.bvhKind == 1 else 32
+    box = 10 if tun.bvhKind == 1 else 32
 
-    def trav(t, i, b, tr, box=32):
+    def trav(t, i, b, tr):
         return 32 * t + 64 * i + box * b + 48 * tr
     jobs = counted["shadow"]
     stage_bytes = {
         "k_trace_primary": trav(counted["tlas"] - counted["shadow_tlas"], counted["inst"] - counted["shadow_inst"],
-                                counted["blas"] - counted["shadow_blas"], counted["tri"] - counted["shadow_tri"],
-                                closest_box)
+                                counted["blas"] - counted["shadow_blas"], counted["tri"] - counted["shadow_tri"])
         + 16 * rays,
         "k_emit": 32 * rays + 160 * hits + 32 * jobs,
         "k_trace_shadow": trav(counted["shadow_tlas"], counted["shadow_inst"], counted["shadow_blas"],
@@ -1068,7 +1068,7 @@ def run_large(args, dist: Dist):
     its vertices uploaded from page-locked memory, its BLAS refit, instance
     bounds + TLAS refit, then full solves of both cascades (16.8M primary
     rays). Timed once per scene-BVH layout: bvhKind 2 (binary, FP32 boxes),
-    1 (8-wide, 8-bit boxes for closest hits) and 0 (the reference's TLAS +
+    1 (8-wide, 8-bit boxes) and 0 (the reference's TLAS +
     BLAS walk); hit records of the layouts are compared on a fixed pose."""
     from speedball_b200 import _abi, synth
     device = dist.local

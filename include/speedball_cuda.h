@@ -570,8 +570,8 @@ typedef struct sb_tuning {
     uint32_t smemTlasNodes;   /* TLAS nodes staged in shared memory (0 = none)     */
     uint32_t bvhKind;         /* scene BVH over (triangle, instance) items, rebuilt
                                  on structural changes: 1 = 8-wide nodes with 8-bit
-                                 boxes (default; the binary tree beside it serves the
-                                 emitters' visibility); 2 = binary only.
+                                 boxes (default; the binary tree beside it serves when
+                                 those are too deep for the walk's stack); 2 = binary only.
                                  0 = the reference's TLAS + BLASes                */
     uint32_t smemWideNodes;   /* at most 512; kept and returned, without effect: the
                                  8-wide walk stages no nodes                       */
@@ -600,11 +600,13 @@ typedef struct sb_stats {
     uint64_t primaryRays, shadowRays;
     uint64_t tlasNodeVisits, instanceVisits, blasNodeVisits, triangleTests;
     float lastSolveMs;        /* trace + blend/upload of the last sb_solve (device time) */
-    float lastTraceMs;        /* the three trace stages (primary, shadow, shade)          */
-    float lastBlendMs;        /* blend + upload kernel alone                              */
+    float lastTraceMs;        /* the trace stages, to the start of the blend              */
+    float lastBlendMs;        /* blend + upload (and the glossy lobe): the solve's time
+                                 after the trace                                         */
     uint64_t kernelLaunches;  /* kernels this library launched, process-wide              */
-    float lastPrimaryMs;      /* per stage, for solves that fit one shadow-job chunk: the
-                                 closest-hit stage (k_trace_primary)                     */
+    float lastPrimaryMs;      /* per stage, for solves that fit one shadow-job chunk, from a
+                                 stage's start to the next one's: the closest-hit stage
+                                 (k_trace_primary)                                       */
     float lastShadowMs;
     float lastShadeMs;
     /* the shadow-ray share of the visit counters above */

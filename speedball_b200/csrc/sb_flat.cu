@@ -290,7 +290,6 @@ cudaError_t FlatScene::install(Job& j, cudaStream_t st, std::string& why) {
         if (e == cudaSuccess) e = cudaMemcpy(witems, j.wt.items.data(), j.wt.items.size() * 4, cudaMemcpyHostToDevice);
         if (e != cudaSuccess) return e;
         wideReady = true;
-        wideCount = (uint32_t)(j.wt.nodes.size() / flat::WIDE_WORDS);
         wideDepth = j.wt.depth;
     }
     root = j.tree.root;
@@ -407,7 +406,6 @@ void FlatScene::fill(DevScene& S) const {
     S.flatItems = on ? items : nullptr;
     S.wideNodes = on && wide && wideReady ? wnodes : nullptr;
     S.wideItems = on && wide && wideReady ? witems : nullptr;
-    S.wideNodeCount = on && wide && wideReady ? wideCount : 0u;
     S.wideDepth = on && wide && wideReady ? wideDepth : 0u;
     S.flatRoot = on ? root : flat::ENTRY_NONE;
     S.slotSkip = on ? dSkip : nullptr;

@@ -75,7 +75,7 @@ struct DevScene {
     // scene BVH (sb_flat.h): world-space tree over (triangle, slot) items;
     // slots marked in slotSkip moved or deformed since its build and are
     // walked through their own BLAS instead (dynList)
-    const uint4* flatNodes;    // binary child pairs (emitter visibility; every walk when wideNodes is null)
+    const uint4* flatNodes;    // binary child pairs (every walk when wideNodes is null)
     const uint2* flatItems;
     const uint4* wideNodes;    // the same items as 8-wide nodes with 8-bit boxes (sb_walk8.cuh), or null
     const uint2* wideItems;
@@ -83,7 +83,6 @@ struct DevScene {
     const uint32_t* dynList;
     const float* slotBounds;   // world AABB per slot (the TLAS leaf bounds), or null
     uint32_t flatRoot, dynCount;
-    uint32_t wideNodeCount;    // nodes of the 8-wide tree (0 when it is not built)
     uint32_t wideDepth;        // its depth (levels below the root)
     int32_t flatOn;
     uint32_t nodeCount, triCount, instCount, tlasNodeCount, materialCount;

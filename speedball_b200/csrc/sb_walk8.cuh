@@ -28,11 +28,11 @@
 // pipe, which takes one every second cycle. So what is not a plane distance is kept
 // short: the box tests end in subtractions whose signs one three-input logic
 // operation and one funnel shift per child collect, and the masks of hit children
-// go through small tables in shared memory. Measured against one walk per lane:
-// closest hits 1431 -> 542 us there, 194 -> 118 us for the atrium's probe rays with
-// its moved slots, 119 -> 61 us for the room's 32,768; any hits (which had a binary
-// tree) 438 -> 362, 163 -> 110 and 102 -> 66 us. Four lanes per ray, two children
-// each, measured 1359 us on the bounce: item tests found too few lanes.
+// go through small tables in shared memory. Measured against one walk per lane (for
+// any hits on a binary tree), the last rays shared: closest hits 1431 -> 507 us there,
+// 194 -> 92 us for the atrium's probe rays with its moved slots, 119 -> 42 us for the
+// room's 32,768; any hits 438 -> 360, 163 -> 95 and 102 -> 49 us. Four lanes per ray, two
+// children each, measured 1359 us on the bounce: item tests found too few lanes.
 #pragma once
 #include "sb_traverse.cuh"
 
