@@ -24,14 +24,18 @@ __device__ __forceinline__ float2 unpack2(unsigned long long v) {
     asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
     return r;
 }
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
 __device__ __forceinline__ void kahan_fma2(unsigned long long& s, unsigned long long& nc, unsigned long long w,
                                            unsigned long long x) {
     const unsigned long long neg = 0xBF800000BF800000ull;  // (-1, -1)
-    unsigned long long y, t, d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(y) : "l"(w), "l"(x), "l"(nc));
+    const unsigned long long y = fma2(w, x, nc);
+    unsigned long long t;
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(t) : "l"(s), "l"(y));
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(s), "l"(neg), "l"(t));
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(nc) : "l"(d), "l"(neg), "l"(y));
+    nc = fma2(fma2(s, neg, t), neg, y);
     s = t;
 }
 
@@ -418,7 +422,8 @@ uint32_t blend_blocks(uint32_t updatedCount) { return (updatedCount + BLEND_PROB
 // own GLOSSY_PROBES probes) when a group is small (tier high: 50 resolved
 // texels), as far as the staged rays fit 48 KB. Measured on the atrium (4,096
 // probes x 64 rays): tier ultra 0.127 ms with one probe per CTA, 0.084 ms with
-// 8 probes per thread, 0.069 ms (ncu) with 4 and the higher occupancy.
+// 8 probes per thread, 0.069 ms (ncu) with 4 and the higher occupancy. The sums in
+// packed pairs: 52 -> 49 us for 2,197 probes x 96 rays (ultra).
 constexpr uint32_t GLOSSY_PROBES = 4;
 constexpr uint32_t GLOSSY_MAX_RAYS = 256;  // raysPerProbe <= 256 (gi_probes.js:988-992)
 
@@ -470,9 +475,9 @@ __global__ void __launch_bounds__(352) k_glossy(DevCascade C, DevParams P, uint3
     const float3 td = active ? oct_decode((float(sx - BORDER) + 0.5f) / float(oct),
                                           (float(sy - BORDER) + 0.5f) / float(oct))
                              : mk(0.0f, 0.0f, 0.0f);
-    float ar[GLOSSY_PROBES], ag[GLOSSY_PROBES], ab[GLOSSY_PROBES], ah[GLOSSY_PROBES];
+    unsigned long long arg[GLOSSY_PROBES], abh[GLOSSY_PROBES];  // r g, b coverage
 #pragma unroll
-    for (uint32_t q = 0; q < GLOSSY_PROBES; ++q) ar[q] = ag[q] = ab[q] = ah[q] = 0.0f;
+    for (uint32_t q = 0; q < GLOSSY_PROBES; ++q) arg[q] = abh[q] = 0ull;
     float aw = 0.0f;
     // every group slot is accumulated (a short last group's extra slots hold zero
     // rays whose sums are never stored): no branch in the loop
@@ -480,14 +485,13 @@ __global__ void __launch_bounds__(352) k_glossy(DevCascade C, DevParams P, uint3
     for (uint32_t k = 0; k < N; ++k) {
         const float4 d = dir[k];
         const float gw = pow64(fmaxf(td.x * d.x + td.y * d.y + td.z * d.z, 0.0f));
+        const unsigned long long ww = f32x2(gw, gw);
         aw += gw;
 #pragma unroll
         for (uint32_t q = 0; q < GLOSSY_PROBES; ++q) {
             const float4 r = rad[q * N + k];
-            ar[q] = fmaf(gw, r.x, ar[q]);
-            ag[q] = fmaf(gw, r.y, ag[q]);
-            ab[q] = fmaf(gw, r.z, ab[q]);
-            ah[q] = fmaf(gw, r.w, ah[q]);
+            arg[q] = fma2(ww, f32x2(r.x, r.y), arg[q]);
+            abh[q] = fma2(ww, f32x2(r.z, r.w), abh[q]);
         }
     }
     if (!active) return;
@@ -499,7 +503,7 @@ __global__ void __launch_bounds__(352) k_glossy(DevCascade C, DevParams P, uint3
     for (uint32_t q = 0; q < GLOSSY_PROBES; ++q) {
         if (q >= nProbes) break;
         const uint32_t probeIndex = (C.probeOffset + base + q) % C.probeTotal;
-        float r = ar[q], g = ag[q], b = ab[q], h = ah[q], w = aw;
+        float r = unpack2(arg[q]).x, g = unpack2(arg[q]).y, b = unpack2(abh[q]).x, h = unpack2(abh[q]).y, w = aw;
         // the emitters' virtual rays with the power-64 weight (gi_probes.js:2624-2638)
         if (C.emitterCount) {
             const float3 ro = probe_world_pos(C, probeIndex);
