@@ -744,7 +744,17 @@ cudaError_t blas_build(BlasBuilder* b, const float* pos, uint32_t V, const uint3
         place(B.boxHi, boxes);
     };
     layout();
-    cudaError_t e = grow(b->scratch, b->cap, at);
+    // grown in powers of two, so that a pass over meshes of rising size frees and
+    // allocates a few times, not for each; exactly where that much is not to be had
+    cudaError_t e = cudaSuccess;
+    if (at > b->cap) {
+        size_t want = 1u << 20;
+        while (want < at) want *= 2;
+        if ((e = grow(b->scratch, b->cap, want)) != cudaSuccess) {
+            cudaGetLastError();
+            e = grow(b->scratch, b->cap, at);
+        }
+    }
     if (e != cudaSuccess) return e;
     base = b->scratch;
     layout();
