@@ -226,9 +226,8 @@ def run_ours(args, dist: Dist):
     # node) or 10 B on the 8-wide tree (80 B node / 8 boxes; the moved slots' pair nodes, a few
     # percent of the tests, are counted the same); 16 B raw hit record per ray
     # (written by the closest-hit stage, read by the emission stage); emission per ray 16 B visibility
-    # mask, per hit 16 B final hit record + 48 B instance rows + 48 B pre-gathered triangle + 48 B
-    # reference triangle (3 indices, 3 vertices) for the refined t, 32 B per shadow job (written by the
-    # emission stage, read by the shadow stage); per hit 80 B of triangle/instance rows, 40 B material,
+    # mask, per hit 16 B final hit record + 48 B instance rows + 48 B pre-gathered triangle, 32 B per
+    # shadow job (written by the emission stage, read by the shadow stage); per hit 80 B of triangle/instance rows, 40 B material,
     # 256 B of bounce taps (8 footprints of 32 B); 16 B ray record write; 3,776 B per probe for
     # blend + upload.
     tun = _abi.sb_tuning()
@@ -242,7 +241,7 @@ def run_ours(args, dist: Dist):
         "k_trace_primary": trav(counted["tlas"] - counted["shadow_tlas"], counted["inst"] - counted["shadow_inst"],
                                 counted["blas"] - counted["shadow_blas"], counted["tri"] - counted["shadow_tri"])
         + 16 * rays,
-        "k_emit": 32 * rays + 160 * hits + 32 * jobs,
+        "k_emit": 32 * rays + 112 * hits + 32 * jobs,
         "k_trace_shadow": trav(counted["shadow_tlas"], counted["shadow_inst"], counted["shadow_blas"],
                                counted["shadow_tri"]) + 32 * jobs,
         "k_shade": 48 * rays + 376 * hits,
