@@ -284,7 +284,7 @@ __device__ __forceinline__ void walk2(const DevScene& S, Walk2Shared& sm, Gen ge
                     if (!ANY && ok && sm.best[of] == key) sm.hit[of] = make_uint4(tri, slot, pack_uv(u, v), 0u);
                     if (!ANY && !more) {
                         const unsigned long long b = sm.best[of];
-                        tie = tie && (uint32_t)(b >> 32) == __float_as_uint(t) && b != key && (uint32_t)b != 0xFFFFFFFFu;
+                        tie = tie && (uint32_t)(b >> 32) == __float_as_uint(t) && !(ok && b == key) && (uint32_t)b != 0xFFFFFFFFu;
                         ties |= __reduce_or_sync(ALL_LANES, tie ? 1u << of : 0u) & ~__ballot_sync(ALL_LANES, alone);
                     }
                     __syncwarp();

@@ -407,7 +407,7 @@ __device__ __forceinline__ void walk8(const DevScene& S, const Walk8Tables& T, W
                 if (!ANY && ok && sm.best[e.y] == mine) sm.hit[e.y] = make_uint4(it.x, it.y, pack_uv(u, v), 0u);
                 if (!ANY && share && !more) {
                     const unsigned long long b = sm.best[e.y];
-                    tie = tie && (uint32_t)(b >> 32) == __float_as_uint(t) && b != mine && (uint32_t)b != 0xFFFFFFFFu;
+                    tie = tie && (uint32_t)(b >> 32) == __float_as_uint(t) && !(ok && b == mine) && (uint32_t)b != 0xFFFFFFFFu;
                     ties |= __reduce_or_sync(ALL_LANES, tie ? 1u << e.y : 0u);
                 }
                 __syncwarp();
