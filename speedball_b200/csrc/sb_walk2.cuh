@@ -27,7 +27,7 @@ struct Walk2Shared {
     float4 o[32];                 // local origin, determinant sign
     float4 d[32];                 // local direction, slot
     unsigned long long best[32];  // as in Walk8Shared
-    uint4 hit[32];
+    uint4 hit[32];                // triangle, slot, packed (u, v), the slack of reach
     uint32_t item[WALK2_QUEUE];   // lane of its ray << 24 | triangle
     uint32_t stk[WALK2_DEPTH][32];  // far children
     uint2 give[32];               // far children on their way to idle lanes; donor, lane of its ray
@@ -41,6 +41,16 @@ __device__ __forceinline__ bool walk2_usable(const DevScene& S) {
 }
 
 // gen and fin as for walk8; the best hit starts as none within tmax.
+//
+// Closest hits pass over a box only where it starts behind the hit in hand by more than
+// the rounding of both (`reach`). A BLAS's boxes are exact: a triangle in the plane of its
+// box starts, by the box, at or a few ulp behind its own t, so with the plain limit a
+// triangle as near as the hit in hand is tested or not as the one or the other is met
+// first, and the lanes that share a ray meet them in no fixed order (17 to 51 of 12,288
+// probe rays at planes of two sizes of triangles named another one than walks that share
+// nothing). Moeller-Trumbore's t is off by some 1e-7 of the triangle's size and distance over
+// the cosine to its normal: 1e-4 of the limit and of the BLAS's size cover all but rays
+// within a milliradian of the plane, and are less than a triangle of the meshes here.
 template <bool ANY, class Gen, class Fin>
 __device__ __forceinline__ void walk2(const DevScene& S, Walk2Shared& sm, Gen gen, Fin fin, Visits& vis,
                                       uint32_t* err) {
@@ -48,7 +58,9 @@ __device__ __forceinline__ void walk2(const DevScene& S, Walk2Shared& sm, Gen ge
     enum : uint32_t { FREE, WALK, ENDED };  // ENDED: this slot's nodes are done, items perhaps
     uint32_t state = FREE;
     float3 wo = mk(0.f, 0.f, 0.f), wd = wo, winv = wo, o = wo, inv = wo;
-    float tmax = 0.0f;
+    float tmax = 0.0f, lim = 0.0f;  // lim: reach(tmax)
+    auto reach = [](float t, float slack) { return ANY ? t : fmaf(t, 1.0001f, slack); };
+    auto shortest = [](float3 v) { return fminf(fminf(fabsf(v.x), fabsf(v.y)), fabsf(v.z)); };
     uint32_t tag = 0, k = 0, cur = PE_NONE, sp = 0, iter = 0, last = 0, head = 0, tail = 0;
     bool more = true;
     uint32_t home = lane, base = 0;  // as in walk8
@@ -60,9 +72,15 @@ __device__ __forceinline__ void walk2(const DevScene& S, Walk2Shared& sm, Gen ge
             const uint32_t slot = __ldg(S.dynList + k++);
             if (S.slotBounds) {
                 const float* b = S.slotBounds + 6u * slot;
-                if (!slab(mk(__ldg(b), __ldg(b + 1), __ldg(b + 2)), mk(__ldg(b + 3), __ldg(b + 4), __ldg(b + 5)), wo,
-                          winv, tmax))
-                    continue;
+                const float3 lo = mk(__ldg(b), __ldg(b + 1), __ldg(b + 2)),
+                             hi = mk(__ldg(b + 3), __ldg(b + 4), __ldg(b + 5));
+                float slack = 0.0f;
+                if (!ANY) {  // (rounded to FP32 at the scene's scale)
+                    const float far = fmaxf(fmaxf(fmaxf(fabsf(lo.x), fabsf(hi.x)), fmaxf(fabsf(lo.y), fabsf(hi.y))),
+                                            fmaxf(fabsf(lo.z), fabsf(hi.z)));
+                    slack = 1e-5f * far * shortest(winv);
+                }
+                if (!slab(lo, hi, wo, winv, reach(tmax, slack))) continue;
             }
             ++vis.inst;
             const float4 m = __ldg(S.inst + 4 * slot + 3);
@@ -76,9 +94,12 @@ __device__ __forceinline__ void walk2(const DevScene& S, Walk2Shared& sm, Gen ge
             if (root >= __float_as_uint(m.y) || root >= S.nodeCount) continue;
             const uint4 a = __ldg(S.nodes + 2 * root), b = __ldg(S.nodes + 2 * root + 1);
             ++vis.blas;
-            if (!slab(mk(__uint_as_float(a.x), __uint_as_float(a.y), __uint_as_float(a.z)),
-                      mk(__uint_as_float(a.w), __uint_as_float(b.x), __uint_as_float(b.y)), o, inv, tmax))
-                continue;
+            const float3 lo = mk(__uint_as_float(a.x), __uint_as_float(a.y), __uint_as_float(a.z)),
+                         hi = mk(__uint_as_float(a.w), __uint_as_float(b.x), __uint_as_float(b.y));
+            const float slack = 1e-4f * fmaxf(fmaxf(hi.x - lo.x, hi.y - lo.y), hi.z - lo.z) * shortest(inv);
+            lim = reach(tmax, slack);
+            if (!slab(lo, hi, o, inv, lim)) continue;
+            if (!ANY) sm.hit[lane].w = __float_as_uint(slack);
             cur = b.w == INTERIOR ? PE_BLAS | root : ((b.w >> 24) ? b.w : PE_NONE);
             if (cur == PE_NONE) continue;
             sm.o[lane] = make_float4(o.x, o.y, o.z, m.z);
@@ -171,7 +192,7 @@ __device__ __forceinline__ void walk2(const DevScene& S, Walk2Shared& sm, Gen ge
                 inv.x = __shfl_sync(ALL_LANES, inv.x, from);
                 inv.y = __shfl_sync(ALL_LANES, inv.y, from);
                 inv.z = __shfl_sync(ALL_LANES, inv.z, from);
-                tmax = __shfl_sync(ALL_LANES, tmax, from);
+                lim = __shfl_sync(ALL_LANES, lim, from);
                 if (take) {
                     cur = e.x;
                     home = e.y & 31u;
@@ -194,10 +215,10 @@ __device__ __forceinline__ void walk2(const DevScene& S, Walk2Shared& sm, Gen ge
                 float t0 = 0.f, t1 = 0.f;
                 const bool h0 = slab_near(__uint_as_float(q0.x), __uint_as_float(q0.z), __uint_as_float(q2.x),
                                           __uint_as_float(q0.y), __uint_as_float(q0.w), __uint_as_float(q2.y), o, inv,
-                                          tmax, t0) && q3.x != PE_NONE;
+                                          lim, t0) && q3.x != PE_NONE;
                 const bool h1 = slab_near(__uint_as_float(q1.x), __uint_as_float(q1.z), __uint_as_float(q2.z),
                                           __uint_as_float(q1.y), __uint_as_float(q1.w), __uint_as_float(q2.w), o, inv,
-                                          tmax, t1) && q3.y != PE_NONE;
+                                          lim, t1) && q3.y != PE_NONE;
                 const bool swap = h0 && h1 && t1 < t0;
                 uint32_t a = h0 ? q3.x : PE_NONE, b = h1 ? q3.y : PE_NONE;
                 if (swap) {
@@ -281,7 +302,7 @@ __device__ __forceinline__ void walk2(const DevScene& S, Walk2Shared& sm, Gen ge
                         else atomicMin(&sm.best[of], key);
                     }
                     __syncwarp();
-                    if (!ANY && ok && sm.best[of] == key) sm.hit[of] = make_uint4(tri, slot, pack_uv(u, v), 0u);
+                    if (!ANY && ok && sm.best[of] == key) sm.hit[of] = make_uint4(tri, slot, pack_uv(u, v), sm.hit[of].w);
                     if (!ANY && !more) {
                         const unsigned long long b = sm.best[of];
                         tie = tie && (uint32_t)(b >> 32) == __float_as_uint(t) && !(ok && b == key) && (uint32_t)b != 0xFFFFFFFFu;
@@ -290,7 +311,7 @@ __device__ __forceinline__ void walk2(const DevScene& S, Walk2Shared& sm, Gen ge
                     __syncwarp();
                     if (state != FREE) {
                         const unsigned long long b = sm.best[home];
-                        if (!ANY) tmax = __uint_as_float((uint32_t)(b >> 32));
+                        if (!ANY) lim = reach(tmax = __uint_as_float((uint32_t)(b >> 32)), __uint_as_float(sm.hit[home].w));
                         else if ((uint32_t)b == 0u) state = ENDED;
                     }
                 }
