@@ -184,6 +184,7 @@ __device__ __forceinline__ void walk8(const DevScene& S, const Walk8Tables& T, W
                                       uint32_t depth, Gen gen, Fin fin, Visits& vis, uint32_t* err) {
     const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
     stk += lane;
+    vis.inst -= vis.tri;  // every item test of this walk reads its instance's rows: with the end, one each
     enum : uint32_t { FREE, WALK, ENDED };  // ENDED: no node left, items perhaps
     uint32_t state = FREE;
     float3 o = mk(0.f, 0.f, 0.f), inv = o;
@@ -428,7 +429,7 @@ __device__ __forceinline__ void walk8(const DevScene& S, const Walk8Tables& T, W
             ANY && (uint32_t)b == 0u);
     }
     vis.blas += 8u * iter;
-    vis.inst += vis.tri;
+    vis.inst += vis.tri;  // (see the start)
 }
 
 }  // namespace sb
