@@ -557,6 +557,7 @@ __global__ void __launch_bounds__(SHADE_BWD_THREADS) k_shade_bwd(WaveCtx W, cons
     const float v[6] = {gBase.x, gBase.y, gBase.z, gEm.x, gEm.y, gEm.z};
 #pragma unroll
     for (uint32_t c = 0; c < 6u; ++c) rows[33u * c + lane] = v[c];
+    __syncwarp();  // (the match below orders no memory)
     uint32_t same = __match_any_sync(0xFFFFFFFFu, material);
     if (material != 0xFFFFFFFFu && __ffs(same) - 1 == (int)lane) {
         float sum[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
