@@ -16,6 +16,8 @@
 //   k_shade_bwd   dL/d(ray radiance) -> material albedo / emissive, light scale
 //                 and dL/dAtlas(s) through the NEE terms and the bounce read
 //                 (traceKernel shading, gi_probes.js:2020-2206).
+#include <type_traits>
+
 #include "sb_wave.cuh"
 #include "sb_kernels.cuh"
 
@@ -452,9 +454,10 @@ constexpr int SHADE_BWD_THREADS = 256;
 // Rows of a warp's table: a light each, and six for the materials' terms.
 __host__ __device__ inline uint32_t shade_bwd_rows(uint32_t lights) { return lights > 6u ? lights : 6u; }
 
-// One thread per ray. Parameter gradients gather per CTA in shared memory
-// (FP32) and flush with one FP64 atomic per touched entry; atlas gradients go
-// straight to global memory as float4 atomics.
+// One thread per ray. Parameter gradients gather per CTA in shared memory (SHARED: FP32,
+// for the 8,192 entries that fit 32 KB) and flush with one FP64 atomic per touched entry;
+// with more, each warp's sums go straight to global memory, formed in FP64 as the entries
+// are. Atlas gradients go straight to global memory as float4 atomics.
 //
 // A warp's rays share most of their lights and several of their materials, and a float
 // atomic in shared memory is a loop that the lanes with one address go through one by
@@ -462,23 +465,25 @@ __host__ __device__ inline uint32_t shade_bwd_rows(uint32_t lights) { return lig
 // (rows 33 apart: columns and rows are free of bank conflicts) and each light's row is
 // summed by one lane; a material's terms are summed by the first lane that has it.
 // 32,768 rays, 32 lights, 64 materials: 81 -> 31 us.
+template <bool SHARED>
 __global__ void __launch_bounds__(SHADE_BWD_THREADS) k_shade_bwd(WaveCtx W, const float4* gR, double* gParam,
-                                                                 float4* gA, uint32_t nParam, int useSmem) {
+                                                                 float4* gA, uint32_t nParam) {
+    using Sum = std::conditional_t<SHARED, float, double>;
     extern __shared__ float sParam[];
     if (!*W.S.valid) return;
     const DevCascade& C = W.C;
     const DevParams& P = W.P;
     const uint32_t N = C.rays, mc = W.S.materialCount, lc = W.S.lightCount, lane = threadIdx.x & 31u;
-    if (useSmem) {
+    if (SHARED) {
         for (uint32_t i = threadIdx.x; i < nParam; i += blockDim.x) sParam[i] = 0.0f;
         __syncthreads();
     }
-    float* rows = sParam + (useSmem ? nParam : 0u) + (threadIdx.x / 32u) * shade_bwd_rows(lc) * 33u;
+    float* rows = sParam + (SHARED ? nParam : 0u) + (threadIdx.x / 32u) * shade_bwd_rows(lc) * 33u;
     for (uint32_t i = 0; i < lc; ++i) rows[33u * i + lane] = 0.0f;
-    auto add = [&](uint32_t i, float v) {
-        if (v == 0.0f) return;
-        if (useSmem) atomicAdd(&sParam[i], v);
-        else atomicAdd(&gParam[i], (double)v);
+    auto add = [&](uint32_t i, Sum v) {
+        if (v == Sum(0)) return;
+        if constexpr (SHARED) atomicAdd(&sParam[i], v);
+        else atomicAdd(&gParam[i], v);
     };
     uint32_t material = 0xFFFFFFFFu;
     float3 gBase = mk(0.f, 0.f, 0.f), gEm = gBase;
@@ -548,7 +553,7 @@ __global__ void __launch_bounds__(SHADE_BWD_THREADS) k_shade_bwd(WaveCtx W, cons
     }
     __syncwarp();
     for (uint32_t li = lane; li < lc; li += 32u) {
-        float sum = 0.0f;
+        Sum sum = 0;
 #pragma unroll 8
         for (uint32_t j = 0; j < 32u; ++j) sum += rows[33u * li + j];
         add(6u * mc + li, sum);
@@ -560,7 +565,7 @@ __global__ void __launch_bounds__(SHADE_BWD_THREADS) k_shade_bwd(WaveCtx W, cons
     __syncwarp();  // (the match below orders no memory)
     uint32_t same = __match_any_sync(0xFFFFFFFFu, material);
     if (material != 0xFFFFFFFFu && __ffs(same) - 1 == (int)lane) {
-        float sum[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        Sum sum[6] = {};
         for (; same; same &= same - 1u) {
             const uint32_t j = __ffs(same) - 1u;
 #pragma unroll
@@ -572,7 +577,7 @@ __global__ void __launch_bounds__(SHADE_BWD_THREADS) k_shade_bwd(WaveCtx W, cons
             add(3u * (mc + material) + c, sum[3u + c]);
         }
     }
-    if (useSmem) {
+    if (SHARED) {
         __syncthreads();
         for (uint32_t i = threadIdx.x; i < nParam; i += blockDim.x)
             if (sParam[i] != 0.0f) atomicAdd(&gParam[i], (double)sParam[i]);
@@ -590,13 +595,14 @@ cudaError_t launch_shade_bwd(const DevScene& S, const DevCascade& C, const DevPa
     W.slotCount = C.probeTotal;
     W.dirs = const_cast<float4*>(dirs);
     const uint32_t nParam = 6u * S.materialCount + S.lightCount;
-    const int useSmem = (size_t)nParam * sizeof(float) <= 32u * 1024u ? 1 : 0;
-    const size_t smem = ((useSmem ? nParam : 0u) + SHADE_BWD_THREADS / 32u * shade_bwd_rows(S.lightCount) * 33u) *
+    const bool shared = (size_t)nParam * sizeof(float) <= 32u * 1024u;
+    const auto kernel = shared ? k_shade_bwd<true> : k_shade_bwd<false>;
+    const size_t smem = ((shared ? nParam : 0u) + SHADE_BWD_THREADS / 32u * shade_bwd_rows(S.lightCount) * 33u) *
                         sizeof(float);  // at most 98 KB (64 lights)
-    cudaError_t e = cudaFuncSetAttribute(k_shade_bwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    k_shade_bwd<<<(rays + SHADE_BWD_THREADS - 1) / SHADE_BWD_THREADS, SHADE_BWD_THREADS, smem, st>>>(W, gR, gParam, gA,
-                                                                                                  nParam, useSmem);
+    kernel<<<(rays + SHADE_BWD_THREADS - 1) / SHADE_BWD_THREADS, SHADE_BWD_THREADS, smem, st>>>(W, gR, gParam, gA,
+                                                                                             nParam);
     note_launch();
     return cudaGetLastError();
 }
