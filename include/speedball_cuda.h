@@ -295,7 +295,9 @@ sb_status sb_occluded(sb_ctx* ctx, const float* ro, const float* rd, const float
  * ray; one byte per ray), enqueued on the context's stream with no copy and
  * no synchronisation: the traversal reused by a GPU path tracer, as the
  * reference's spectral kernel reuses traverseClosest / traverseAny
- * (spectral_kernel.js:288, 451). Results equal sb_raycast / sb_occluded. */
+ * (spectral_kernel.js:288, 451). Results equal sb_raycast / sb_occluded.
+ * Queries only read the scene: those on different streams (sb_set_stream
+ * between them), and captured ones replayed side by side, may overlap. */
 sb_status sb_raycast_device(sb_ctx* ctx, const float* ro, const float* rd, uint32_t n, float* tOut,
                             int32_t* triOut, int32_t* instOut);
 sb_status sb_occluded_device(sb_ctx* ctx, const float* ro, const float* rd, const float* maxDist,

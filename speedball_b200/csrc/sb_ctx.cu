@@ -26,6 +26,8 @@ uint64_t launches() { return g_launches.load(std::memory_order_relaxed); }
 
 namespace {
 
+constexpr uint32_t QUERY_STREAMS = 64;  // streams whose queries have a cursor of their own
+
 struct Cascade {
     sb_grid grid{};
     bool configured = false;
@@ -101,6 +103,8 @@ struct sb_ctx {
     RefitRange refitRanges[REFIT_RANGES];
     uint32_t packEpoch = 1, refitNext = 0;
     uint32_t* dWork = nullptr;
+    unsigned long long queryStream[QUERY_STREAMS];  // ids of the streams that a query has run on
+    uint32_t queryStreams = 0;
     float4* dDirs = nullptr;  // ray directions: a batch's items (a solve: the first), then the adjoint's
     unsigned long long* dCounters = nullptr;
     bool countersOn = false;
@@ -217,7 +221,7 @@ template <class T> void release(T*& p) {
     p = nullptr;
 }
 
-constexpr uint32_t QUERY_CURSOR = SB_BATCH_MAX * WORK_WORDS;  // in dWork, behind the solves' words
+constexpr uint32_t ALL_WORK = SB_BATCH_MAX * WORK_WORDS;      // the solves' words in dWork; the queries' follow
 constexpr uint32_t ADJOINT_DIRS = SB_BATCH_MAX * MAX_RAYS;    // in dDirs
 constexpr uint64_t kJobCapMax = 64ull << 20;  // 64 Mi shadow jobs (2 GiB) per trace chunk
 
@@ -478,7 +482,7 @@ sb_status sb_create(const sb_device_opts* opts, sb_ctx** out) {
         if (cudaStreamCreateWithFlags(&ctx->ownStream, cudaStreamNonBlocking) != cudaSuccess) { st = SB_ERR_CUDA; break; }
         ctx->stream = ctx->ownStream;
         if (cudaMalloc(&ctx->dErr, 4) != cudaSuccess || cudaMalloc(&ctx->dGate, 4 * REFIT_RANGES * 4) != cudaSuccess ||
-            cudaMalloc(&ctx->dWork, (QUERY_CURSOR + 8) * 4) != cudaSuccess ||
+            cudaMalloc(&ctx->dWork, (ALL_WORK + QUERY_STREAMS) * 4) != cudaSuccess ||
             cudaMalloc(&ctx->dStamps, STAGE_STAMPS * 8) != cudaSuccess ||
             cudaMalloc(&ctx->dDirs, (ADJOINT_DIRS + MAX_RAYS) * sizeof(float4)) != cudaSuccess ||
             cudaMalloc(&ctx->dCounters, 16 * 8) != cudaSuccess ||
@@ -968,7 +972,7 @@ static cudaError_t clear_work(sb_ctx* ctx) {
         ctx->workClear = false;
         return cudaSuccess;
     }
-    return cudaMemsetAsync(ctx->dWork, 0, QUERY_CURSOR * sizeof(uint32_t), ctx->stream);
+    return cudaMemsetAsync(ctx->dWork, 0, ALL_WORK * sizeof(uint32_t), ctx->stream);
 }
 
 sb_status sb_solve(sb_ctx* ctx, uint32_t ci, uint32_t probeOffset, uint32_t updatedCount) {
@@ -1735,6 +1739,18 @@ sb_status sb_backward(sb_ctx* ctx, sb_grads* grads) {
     return SB_OK;
 }
 
+// A cursor for a query on the context's stream: queries of one stream follow one another,
+// so each stream has a word of its own. None for captured ones, and when the words are out.
+static uint32_t* query_cursor(sb_ctx* ctx) {
+    unsigned long long id = 0;
+    if (in_capture(ctx) || cudaStreamGetId(ctx->stream, &id) != cudaSuccess) return nullptr;
+    uint32_t k = 0;
+    while (k < ctx->queryStreams && ctx->queryStream[k] != id) ++k;
+    if (k == QUERY_STREAMS) return nullptr;
+    if (k == ctx->queryStreams) ctx->queryStream[ctx->queryStreams++] = id;
+    return ctx->dWork + ALL_WORK + k;
+}
+
 sb_status sb_raycast(sb_ctx* ctx, const float* ro, const float* rd, uint32_t n, float* tOut, int32_t* triOut,
                      int32_t* instOut) {
     if (!ctx || (n && (!ro || !rd || !tOut || !triOut || !instOut))) return fail(ctx, SB_ERR_INVALID_ARG, "null argument");
@@ -1754,8 +1770,7 @@ sb_status sb_raycast(sb_ctx* ctx, const float* ro, const float* rd, uint32_t n, 
     CK(cudaMallocAsync(&dinst, (size_t)n * 4, ctx->stream));
     CK(cudaMemcpyAsync(dro, ro, (size_t)n * 12, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(drd, rd, (size_t)n * 12, cudaMemcpyHostToDevice, ctx->stream));
-    CK(launch_raycast(dev_scene(ctx), dro, drd, n, dt, dtri, dinst, ctx->dWork + QUERY_CURSOR, ctx->numSms,
-                      ctx->dErr, ctx->stream));
+    CK(launch_raycast(dev_scene(ctx), dro, drd, n, dt, dtri, dinst, query_cursor(ctx), ctx->numSms, ctx->dErr, ctx->stream));
     CK(cudaMemcpyAsync(tOut, dt, (size_t)n * 4, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaMemcpyAsync(triOut, dtri, (size_t)n * 4, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaMemcpyAsync(instOut, dinst, (size_t)n * 4, cudaMemcpyDeviceToHost, ctx->stream));
@@ -1782,8 +1797,7 @@ sb_status sb_raycast_device(sb_ctx* ctx, const float* ro, const float* rd, uint3
     if (n == 0) return ctx->sceneLoaded ? SB_OK : fail(ctx, SB_ERR_NOT_READY, "no scene uploaded");
     sb_status s = device_query_ready(ctx);
     if (s != SB_OK) return s;
-    CK(launch_raycast(dev_scene(ctx), ro, rd, n, tOut, triOut, instOut, ctx->dWork + QUERY_CURSOR, ctx->numSms,
-                      ctx->dErr, ctx->stream));
+    CK(launch_raycast(dev_scene(ctx), ro, rd, n, tOut, triOut, instOut, query_cursor(ctx), ctx->numSms, ctx->dErr, ctx->stream));
     return SB_OK;
 }
 
@@ -1793,8 +1807,7 @@ sb_status sb_occluded_device(sb_ctx* ctx, const float* ro, const float* rd, cons
     if (n == 0) return ctx->sceneLoaded ? SB_OK : fail(ctx, SB_ERR_NOT_READY, "no scene uploaded");
     sb_status s = device_query_ready(ctx);
     if (s != SB_OK) return s;
-    CK(launch_occluded(dev_scene(ctx), ro, rd, maxDist, n, blockedOut, ctx->dWork + QUERY_CURSOR, ctx->numSms,
-                       ctx->dErr, ctx->stream));
+    CK(launch_occluded(dev_scene(ctx), ro, rd, maxDist, n, blockedOut, query_cursor(ctx), ctx->numSms, ctx->dErr, ctx->stream));
     return SB_OK;
 }
 
@@ -2013,7 +2026,7 @@ sb_status sb_occluded(sb_ctx* ctx, const float* ro, const float* rd, const float
     CK(cudaMemcpyAsync(dro, ro, (size_t)n * 12, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(drd, rd, (size_t)n * 12, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(dm, maxDist, (size_t)n * 4, cudaMemcpyHostToDevice, ctx->stream));
-    CK(launch_occluded(dev_scene(ctx), dro, drd, dm, n, dout, ctx->dWork + QUERY_CURSOR, ctx->numSms, ctx->dErr, ctx->stream));
+    CK(launch_occluded(dev_scene(ctx), dro, drd, dm, n, dout, query_cursor(ctx), ctx->numSms, ctx->dErr, ctx->stream));
     CK(cudaMemcpyAsync(out, dout, (size_t)n, cudaMemcpyDeviceToHost, ctx->stream));
     cudaFreeAsync(dro, ctx->stream); cudaFreeAsync(drd, ctx->stream); cudaFreeAsync(dm, ctx->stream);
     cudaFreeAsync(dout, ctx->stream);

@@ -210,7 +210,7 @@ cudaError_t launch_ray_dirs(uint32_t rays, float jitter, float4* dirs, cudaStrea
 cudaError_t launch_probe_rays(const DevCascade& C, float jitter, float* ro, float* rd, cudaStream_t st);
 
 // Arbitrary-ray queries through the same traversal (raycastFirst-like); `cursor`: one word of
-// scratch for the stream's next query.
+// scratch that only this stream's queries use, or null.
 cudaError_t launch_raycast(const DevScene& S, const float* ro, const float* rd, uint32_t n, float* tOut,
                            int32_t* triOut, int32_t* instOut, uint32_t* cursor, int numSms, uint32_t* err,
                            cudaStream_t st);

@@ -963,10 +963,14 @@ __global__ void k_occluded(DevScene S, const float* ro, const float* rd, const f
                  : 0;
 }
 
-// The same on the 8-wide tree. MOVED: the scene has moved slots, walked as a ray is
+// The same on the 8-wide tree. The warps share the rays by a cursor, a word of the stream's
+// own: queries on several streams run side by side. OWN: without one (a captured query, which
+// may be replayed beside any other) each CTA takes every gridDim.x-th 32 rays and its warps
+// share those: 603 -> 644 us (closest) and 438 -> 467 us (any) for 2.07M bounce rays, 2%
+// less to 5% more for 230,400 and 9,216. MOVED: the scene has moved slots, walked as a ray is
 // taken; without that walk's code the kernel spilled less at 64 registers: 554 -> 528 us
 // (closest) and 362 -> 341 us (any) for 2.07M bounce rays.
-template <bool ANY, bool MOVED>
+template <bool ANY, bool MOVED, bool OWN>
 __global__ void __launch_bounds__(256, SB_WALK8_MIN_BLOCKS) k_query_walk8(DevScene S, const float* ro, const float* rd,
                                                                           const float* maxDist, uint32_t n,
                                                                           float* tOut, int32_t* triOut,
@@ -975,12 +979,20 @@ __global__ void __launch_bounds__(256, SB_WALK8_MIN_BLOCKS) k_query_walk8(DevSce
     extern __shared__ float4 smem[];
     if (!*S.valid) return;
     const uint32_t lane = threadIdx.x & 31u;
+    uint32_t end = n;  // of the cursor's positions
+    if (OWN) {
+        __shared__ uint32_t own;
+        if (threadIdx.x == 0) own = 0u;  // (walk_shared synchronizes)
+        cursor = &own;
+        end = ((n + 31u) / 32u + gridDim.x - 1u - blockIdx.x) / gridDim.x * 32u;
+    }
     const WalkSmem m = walk_shared(smem, S.wideDepth + 1u, false);
     Visits vis = {0, 0, 0, 0};
     auto gen = [&](bool& more, uint32_t idle, float3& o, float3& d, float3& winv, float& tmax, uint32_t& tag,
                    uint4& hit) {
-        const uint32_t i = take(cursor, n, idle, more);
-        const bool ok = i < n && (idle >> lane & 1u);
+        const uint32_t p = take(cursor, end, idle, more);
+        const uint32_t i = OWN ? (p / 32u * gridDim.x + blockIdx.x) * 32u + p % 32u : p;
+        const bool ok = p < end && i < n && (idle >> lane & 1u);
         if (!ok) return false;
         const size_t i3 = 3 * (size_t)i;
         o = mk(ro[i3], ro[i3 + 1], ro[i3 + 2]);
@@ -1025,9 +1037,10 @@ cudaError_t launch_raycast(const DevScene& S, const float* ro, const float* rd, 
     if (n == 0) return cudaSuccess;
     if (S.wideNodes) {
         const size_t smem = walk_smem(S.wideDepth + 1u, false, 256u);
-        cudaError_t e = cudaMemsetAsync(cursor, 0, 4, st);
+        cudaError_t e = cursor ? cudaMemsetAsync(cursor, 0, 4, st) : cudaSuccess;
         if (e != cudaSuccess) return e;
-        const auto kernel = S.dynCount ? k_query_walk8<false, true> : k_query_walk8<false, false>;
+        const auto kernel = cursor ? S.dynCount ? k_query_walk8<false, true, false> : k_query_walk8<false, false, false>
+                                   : S.dynCount ? k_query_walk8<false, true, true> : k_query_walk8<false, false, true>;
         kernel<<<walk8_grid((const void*)kernel, 256, smem, query_tuning(numSms), n), 256, smem, st>>>(
             S, ro, rd, nullptr, n, tOut, triOut, instOut, nullptr, cursor, err);
     } else {
@@ -1044,9 +1057,10 @@ cudaError_t launch_occluded(const DevScene& S, const float* ro, const float* rd,
     if (n == 0) return cudaSuccess;
     if (S.wideNodes) {
         const size_t smem = walk_smem(S.wideDepth + 1u, false, 256u);
-        cudaError_t e = cudaMemsetAsync(cursor, 0, 4, st);
+        cudaError_t e = cursor ? cudaMemsetAsync(cursor, 0, 4, st) : cudaSuccess;
         if (e != cudaSuccess) return e;
-        const auto kernel = S.dynCount ? k_query_walk8<true, true> : k_query_walk8<true, false>;
+        const auto kernel = cursor ? S.dynCount ? k_query_walk8<true, true, false> : k_query_walk8<true, false, false>
+                                   : S.dynCount ? k_query_walk8<true, true, true> : k_query_walk8<true, false, true>;
         kernel<<<walk8_grid((const void*)kernel, 256, smem, query_tuning(numSms), n), 256, smem, st>>>(
             S, ro, rd, maxDist, n, nullptr, nullptr, nullptr, out, cursor, err);
     } else {
