@@ -40,7 +40,7 @@ struct Cascade {
     float4* rayData = nullptr;
     uint4* hits = nullptr;
     uint4* vis = nullptr;
-    size_t rayCap = 0;
+    size_t rayCap = 0, visCap = 0;
     float4* probePos = nullptr;     // every probe's position
     uint32_t* tileOrder = nullptr;  // probe index per issue position in 4 x 4 x 2 tiles (sortKey 2)
     // sortKey 3: cycles per 32-ray closest-hit batch of the last full solve, and the batch
@@ -907,13 +907,13 @@ sb_status sb_configure_cascade(sb_ctx* ctx, uint32_t ci, const sb_grid* g) {
         CK(cudaMemcpy(K.tileOrder, order.data(), (size_t)probeTotal * 4, cudaMemcpyHostToDevice));
     }
     if (rays > K.rayCap || !K.rayData) {
-        release(K.rayData); release(K.hits); release(K.vis);
+        release(K.rayData); release(K.hits);
         size_t c = 0;
         CK(grow(K.rayData, c, rays));
         c = 0; CK(grow(K.hits, c, rays));
-        c = 0; CK(grow(K.vis, c, rays));
         K.rayCap = rays;
     }
+    CK(grow(K.vis, K.visCap, rays + probeTotal));  // the rays', then the probes' emitter rays'
     {
         const size_t batches = (rays + 31) / 32;
         size_t c = K.batchCap;
@@ -996,9 +996,10 @@ sb_status sb_solve(sb_ctx* ctx, uint32_t ci, uint32_t probeOffset, uint32_t upda
     DevCascade D = dev_cascade(ctx, ci, probeOffset, updatedCount);
     DevParams P;
     std::memcpy(&P, &ctx->params, sizeof P);
-    // shadow-job queue: up to one job per (ray, light); solves larger than the
-    // queue cap run as several probe-slot chunks before the blend
-    const uint64_t perProbe = (uint64_t)K.grid.raysPerProbe * (ctx->lightCount ? ctx->lightCount : 1u);
+    // shadow-job queue: up to one job per (ray, light) and (probe, emitter); solves larger
+    // than the queue cap run as several probe-slot chunks before the blend
+    const uint64_t perProbe =
+        (uint64_t)K.grid.raysPerProbe * (ctx->lightCount ? ctx->lightCount : 1u) + ctx->emitterCount;
     uint64_t want = perProbe * updatedCount;
     if (want > kJobCapMax) want = kJobCapMax - kJobCapMax % perProbe;
     if (want < perProbe) want = perProbe;

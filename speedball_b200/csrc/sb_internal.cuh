@@ -110,7 +110,8 @@ struct DevCascade {
     unsigned long long* stamps;  // when each stage started (stage_begin), or null
     float4* rayData;           // updatedCount*rays
     uint4* hits;               // 16-byte hit records: tri, inst | facing << 31, t, packed uv
-    uint4* vis;                // NEE masks: tested lights (lo, hi), unblocked lights (lo, hi)
+    uint4* vis;                // per ray, NEE masks: tested lights (lo, hi), unblocked lights (lo, hi); behind all rays
+                               // one per slot: its emitters' rays
     float4* irr;               // history, probeTotal*64
     float2* depth;             // history
     const uint4* footPrev;     // the previous upload's colour footprints (sb_math.cuh)

@@ -371,7 +371,7 @@ __device__ __forceinline__ void shade_ray(const WaveCtx& W, uint32_t g) {
             if (!(diffuseEnergy > 0.02f || emissivePeak > 1e-6f)) hitT = -(t + ROUGH_UNSHADED_T_BIAS);
         }
         uint4 v = C.vis[rayIdx];
-        unsigned long long ok = (unsigned long long)(v.z & v.x) | (unsigned long long)(v.w & v.y) << 32;
+        unsigned long long ok = (unsigned long long)v.z | (unsigned long long)v.w << 32;
         while (ok) {
             uint32_t li = (uint32_t)(__ffsll((long long)ok) - 1);
             ok &= ok - 1ull;
@@ -615,9 +615,8 @@ __global__ void __launch_bounds__(128) k_shade(WaveCtx W) {
 // The rays join stage B's jobs. By themselves they are too few to fill the chip (2,197
 // probes and 3 emitters: 206 warps) and take as long as their longest walk, 72 us,
 // while stage B walks ninety times as many in 155: there they cost 9 us, the jobs' and
-// the fold's launches included. A ray's outcome is its emitter's record bit in the
-// unblocked mask of its probe's ray 0: the NEE tests no such record, so the bit is free
-// until the fold takes it out again.
+// the fold's launches included. The outcomes of a probe's rays are the emitters' bits of an
+// unblocked mask behind the rays' own.
 __global__ void __launch_bounds__(128) k_emitter_jobs(WaveCtx W) {
     stage_wait();
     if (!*W.S.valid) return;
@@ -625,9 +624,9 @@ __global__ void __launch_bounds__(128) k_emitter_jobs(WaveCtx W) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
     const bool active = i < W.slotCount;
     const uint32_t slot = W.slotBegin + (active ? i : 0u), probeIndex = probe_of(C, slot);
-    const uint32_t ray = slot * C.rays;
+    const uint32_t ray = C.probeTotal * C.rays + slot;
     const float3 ro = slot_origin(C, slot);
-    unsigned long long open = 0ull;
+    uint32_t open = 0u;
     for (uint32_t e = 0; e < C.emitterCount; ++e) {
         const uint32_t li = C.emitterBase + e;
         const float* L = C.lights + (size_t)li * 17u;
@@ -643,7 +642,7 @@ __global__ void __launch_bounds__(128) k_emitter_jobs(WaveCtx W) {
         j = __shfl_sync(ALL_LANES, j, 0) + (uint32_t)__popc(jobs & ((1u << lane) - 1u));
         if (!far) continue;
         if (j >= W.jobCap) {
-            latch(W.err, ERR_CAPACITY);  // (unreachable: no ray tests an emitter's record)
+            latch(W.err, ERR_CAPACITY);  // (unreachable: the queue has a job per probe and emitter too)
             continue;
         }
         const float3 d = axis * (1.0f / dist);
@@ -661,29 +660,22 @@ __global__ void __launch_bounds__(128) k_emitter_jobs(WaveCtx W) {
         const float3 sdir = normalize3(target - ro);
         const float traceBias = fmaxf(C.cellMin * 0.005f * W.P.debugTraceBiasScale, RAY_EPS * W.P.debugRayEpsScale);
         store32(W.jobs + 2 * j, make_float4(ro.x, ro.y, ro.z, fmaxf(dist - sourceRadius - traceBias, 1e-4f)),
-                make_float4(sdir.x, sdir.y, sdir.z, __uint_as_float(ray << 6 | li)));
-        open |= 1ull << li;
+                make_float4(sdir.x, sdir.y, sdir.z, __uint_as_float(ray << 6 | e)));
+        open |= 1u << e;
     }
-    if (open) {
-        C.vis[ray].z |= (uint32_t)open;
-        C.vis[ray].w |= (uint32_t)(open >> 32);
-    }
+    if (active) C.vis[ray] = make_uint4(open, 0u, open, 0u);
 }
 
 __global__ void __launch_bounds__(128) k_emitter_vis(DevScene S, DevCascade C) {
     stage_wait();
     const uint32_t slot = blockIdx.x * blockDim.x + threadIdx.x;
     if (slot >= C.updatedCount || !*S.valid) return;
-    uint4* ray = C.vis + (size_t)slot * C.rays;
-    const uint4 v = *ray;
-    const unsigned long long open = (unsigned long long)v.z | (unsigned long long)v.w << 32;
+    const uint32_t open = C.vis[C.probeTotal * C.rays + slot].z;
     float* vp = C.emitterVis + (size_t)probe_of(C, slot) * EMITTER_CAP;
     for (uint32_t e = 0; e < C.emitterCount; ++e) {
-        const float sample = open >> (C.emitterBase + e) & 1ull ? 1.0f : 0.0f;
+        const float sample = open >> e & 1u ? 1.0f : 0.0f;
         vp[e] = sample * (1.0f - EMITTER_VIS_RETENTION) + vp[e] * EMITTER_VIS_RETENTION;
     }
-    ray->z = v.z & v.x;
-    ray->w = v.w & v.y;
 }
 
 cudaError_t launch_emitter_vis(const DevScene& S, const DevCascade& C, cudaStream_t st) {
