@@ -2212,6 +2212,9 @@ sb_status sb_get_stats(sb_ctx* ctx, sb_stats* out) {
     out->sceneBvhBuilding = ctx->flat.building() ? 1u : 0u;
     out->lastSceneBvhBuildMs = ctx->flat.lastBuildMs;
     cudaSetDevice(ctx->device);
+    const bool stages = ctx->timed && !ctx->lastWasGraph;
+    unsigned long long t[STAGE_STAMPS];
+    if (stages) CK(cudaMemcpyAsync(t, ctx->dStamps, sizeof t, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     if (ctx->countersOn) {
         unsigned long long c[16];
@@ -2230,12 +2233,10 @@ sb_status sb_get_stats(sb_ctx* ctx, sb_stats* out) {
     if (ctx->timed && ctx->lastWasGraph) {
         float ms = 0.0f;
         if (cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1) == cudaSuccess) out->lastSolveMs = ms;  // whole frame
-    } else if (ctx->timed) {
+    } else if (stages) {
         float ms = 0.0f;
         if (cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1) == cudaSuccess) out->lastSolveMs = ms;
         // a stage from its start to the next one's; the blend what the trace leaves of the solve
-        unsigned long long t[STAGE_STAMPS];
-        CK(cudaMemcpy(t, ctx->dStamps, sizeof t, cudaMemcpyDeviceToHost));
         auto between = [&](int a, int b) { return t[b] > t[a] ? (float)((double)(t[b] - t[a]) * 1e-6) : 0.0f; };
         if (ctx->stamped) {
             out->lastTraceMs = std::min(between(0, 4), out->lastSolveMs);
