@@ -84,9 +84,9 @@ struct Build {
     uint32_t V, T, leafSize, chunk;  // chunk: positions per CTA and phase, a multiple of kThreads
     uint32_t levels;                 // prefix and box levels above the positions (32 per step)
     float4* centre;                  // T
-    uint32_t* part;                  // kMaxCtas x 8: centre bounds; then leaf and node sums
+    uint32_t* part;                  // per CTA 8: centre bounds; then leaf and node sums
     uint32_t *keyA, *keyB, *valA;    // T each; the sorted triangles lie in `order`
-    uint32_t* hist;                  // kMaxCtas x kDigits
+    uint32_t* hist;                  // per CTA of a sort pass kDigits
     uint8_t* prefix;                 // per position and level: common prefix with the next, minima above
     uint32_t *first, *last;          // T: range of the interior node of the output that splits after a position
     uint32_t *starts, *leafCount;    // T: interior nodes that start here; triangles of the output leaf that does
@@ -719,7 +719,14 @@ cudaError_t blas_build(BlasBuilder* b, const float* pos, uint32_t V, const uint3
         B.levels = k;
         if (k >= 2 && n <= 32u) break;
     }
-    // scratch, laid out 256-byte aligned; the first call sizes, the second places
+    const uint32_t tiles = (T + kThreads - 1u) / kThreads;
+    uint32_t clusterCtas = 1;
+    while (clusterCtas < 8 && clusterCtas * kThreads < T) clusterCtas *= 2;
+    const bool byCluster = T <= BUILD_CLUSTER_TRIS;
+    const uint32_t sortCtas = byCluster ? clusterCtas : std::min(kSortCtas, tiles);
+    const uint32_t maxCtas = byCluster ? clusterCtas : std::min(kMaxCtas, tiles);
+    // scratch, laid out 256-byte aligned; the first call sizes, the second places. The boxes
+    // come after the last use of centres and keys, and take their place.
     uint8_t* base = nullptr;
     size_t at = 0;
     auto place = [&](auto*& p, size_t count) {
@@ -728,28 +735,34 @@ cudaError_t blas_build(BlasBuilder* b, const float* pos, uint32_t V, const uint3
     };
     auto layout = [&] {
         at = 0;
+        place(B.boxLo, boxes);
+        place(B.boxHi, boxes);
+        const size_t end = at;
+        at = 0;
         place(B.centre, T);
-        place(B.part, kMaxCtas * 8);
         place(B.keyA, T);
         place(B.keyB, T);
         place(B.valA, T);
-        place(B.hist, kSortCtas * kDigits);
+        at = std::max(at, end);
+        place(B.part, maxCtas * 8);
+        place(B.hist, sortCtas * kDigits);
         place(B.prefix, boxes);
         place(B.first, T);
         place(B.last, T);
         place(B.starts, T);
         place(B.leafCount, T);
         place(B.before, (size_t)T + 1);
-        place(B.boxLo, boxes);
-        place(B.boxHi, boxes);
     };
     layout();
-    // grown in powers of two, so that a pass over meshes of rising size frees and
-    // allocates a few times, not for each; exactly where that much is not to be had
+    // Grown in powers of two, so that a pass over meshes of rising size frees and allocates
+    // a few times, not for each; exactly where that much is not to be had. A block of up to
+    // 1 MB is a part of the driver's 2 MB ones (3 us, or 350 when a new one has to be
+    // mapped: so no more than the mesh needs, 58 bytes a triangle); larger ones are always
+    // mapped, and unmapped again (350 + 280 us): powers of four.
     cudaError_t e = cudaSuccess;
     if (at > b->cap) {
-        size_t want = 1u << 20;
-        while (want < at) want *= 2;
+        size_t want = 64u << 10;
+        while (want < at) want *= want < 1u << 20 ? 2 : 4;
         if ((e = grow(b->scratch, b->cap, want)) != cudaSuccess) {
             cudaGetLastError();
             e = grow(b->scratch, b->cap, at);
@@ -764,10 +777,8 @@ cudaError_t blas_build(BlasBuilder* b, const float* pos, uint32_t V, const uint3
             if ((e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) != cudaSuccess) return e;
         b->ready = true;
     }
-    if (T <= BUILD_CLUSTER_TRIS) {
-        B.levels = 2;  // up to 64 boxes of 1024 positions
-        uint32_t ctas = 1;
-        while (ctas < 8 && ctas * kThreads < T) ctas *= 2;
+    if (byCluster) {
+        const uint32_t ctas = clusterCtas;
         B.chunk = ((T + ctas - 1) / ctas + kThreads - 1) / kThreads * kThreads;
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3(ctas);
@@ -793,8 +804,7 @@ cudaError_t blas_build(BlasBuilder* b, const float* pos, uint32_t V, const uint3
         const bool upper = phase == PHASE_UPPER || phase == PHASE_UPPER_BOXES;
         const bool sort = phase >= PHASE_SORT && phase < PHASE_PREFIXES;
         if (upper && B.levels < 3) continue;
-        const uint32_t most = phase < PHASE_PREFIXES ? kSortCtas : kMaxCtas;
-        const uint32_t ctas = std::min(most, (T + kThreads - 1u) / kThreads);
+        const uint32_t ctas = phase < PHASE_PREFIXES ? sortCtas : maxCtas;
         B.chunk = ((T + ctas - 1) / ctas + kThreads - 1) / kThreads * kThreads;
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3(upper ? 1u : ctas);
