@@ -630,26 +630,29 @@ __global__ void k_clear_cascade(DevCascade C) {
     }
 }
 
-// The footprints of the atlases as they are (a host upload, a clear).
-__global__ void k_footprints(DevCascade C) {
-    const uint32_t at = blockIdx.x * blockDim.x + threadIdx.x;
-    if (at >= C.probeTotal * FOOT) return;
-    const uint32_t probe = at / FOOT, f = at % FOOT;
+// The footprints of probes [first, first + count) from the atlases as they are (a host
+// upload, a clear).
+__global__ void k_footprints(DevCascade C, uint32_t first, uint32_t count, uint32_t which) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= count * FOOT) return;
+    const uint32_t at = first * FOOT + i, probe = at / FOOT, f = at % FOOT;
     const uint32_t col = probe % C.res[0], row = (probe / (C.res[0] * C.res[1])) * C.res[1] + (probe / C.res[0]) % C.res[1];
     const size_t t = (size_t)(row * TILE + f / 7u) * C.atlasW + col * TILE + f % 7u, W = C.atlasW;
-    store_foot(C.foot, at, C.atlas[t], C.atlas[t + 1], C.atlas[t + W], C.atlas[t + W + 1]);
-    C.footDepth[at] = make_uint4(C.depthAtlas[t].x, C.depthAtlas[t + 1].x, C.depthAtlas[t + W].x, C.depthAtlas[t + W + 1].x);
+    const uint2 *a = C.atlas + t, *d = C.depthAtlas + t;
+    if (which & FOOT_COLOUR) store_foot(C.foot, at, a[0], a[1], a[W], a[W + 1]);
+    if (which & FOOT_DEPTH) C.footDepth[at] = make_uint4(d[0].x, d[1].x, d[W].x, d[W + 1].x);
 }
 
-cudaError_t launch_footprints(const DevCascade& C, cudaStream_t st) {
-    const uint32_t n = C.probeTotal * FOOT;
-    k_footprints<<<(n + 255) / 256, 256, 0, st>>>(C); note_launch();
+cudaError_t launch_footprints(const DevCascade& C, uint32_t first, uint32_t count, uint32_t which, cudaStream_t st) {
+    const uint32_t n = count * FOOT;
+    if (n == 0) return cudaSuccess;
+    k_footprints<<<(n + 255) / 256, 256, 0, st>>>(C, first, count, which); note_launch();
     return cudaGetLastError();
 }
 
 cudaError_t launch_clear_cascade(const DevCascade& C, cudaStream_t st) {
     k_clear_cascade<<<148 * 4, 256, 0, st>>>(C); note_launch();
-    return launch_footprints(C, st);
+    return launch_footprints(C, 0, C.probeTotal, FOOT_COLOUR | FOOT_DEPTH, st);
 }
 
 }  // namespace sb

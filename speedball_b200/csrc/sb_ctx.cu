@@ -715,8 +715,14 @@ sb_status sb_upload_range(sb_ctx* ctx, uint32_t which, uint32_t start, uint32_t 
     if (!dst) return fail(ctx, SB_ERR_NOT_READY, "buffer %u not allocated", buf);
     if ((size_t)start + count > len) return fail(ctx, SB_ERR_INVALID_ARG, "range [%u,+%u) outside %zu", start, count, len);
     CK(cudaMemcpyAsync((char*)dst + (size_t)start * esz, src, (size_t)count * esz, cudaMemcpyHostToDevice, ctx->stream));
-    if (buf == SB_BUF_IRRADIANCE_ATLAS || buf == SB_BUF_DEPTH_ATLAS)
-        CK(launch_footprints(dev_cascade(ctx, ci, 0, 0), ctx->stream));
+    if (count && (buf == SB_BUF_IRRADIANCE_ATLAS || buf == SB_BUF_DEPTH_ATLAS)) {
+        // the rows of tiles that the range touches: a row of tiles is a row of probes along x
+        const Cascade& K = ctx->casc[ci];
+        const size_t row = (size_t)K.atlasW * 4 * TILE;
+        const uint32_t from = (uint32_t)(start / row), to = (uint32_t)(((size_t)start + count - 1) / row) + 1u;
+        CK(launch_footprints(dev_cascade(ctx, ci, 0, 0), from * K.grid.res[0], (to - from) * K.grid.res[0],
+                             buf == SB_BUF_IRRADIANCE_ATLAS ? FOOT_COLOUR : FOOT_DEPTH, ctx->stream));
+    }
     ++ctx->epoch;
     if (buf <= SB_BUF_MATERIALS && !(buf == SB_BUF_MATERIALS && shading_only(B, start, count))) {
         ++ctx->structGen;

@@ -104,8 +104,9 @@ cudaError_t launch_light_grid(float* lights, uint32_t lightCount, const DevCasca
 // (direction, type), (colour, emitter class).
 cudaError_t launch_light_gates(const float* lights, float4* gates, cudaStream_t st);
 cudaError_t launch_clear_cascade(const DevCascade& C, cudaStream_t st);
-// The footprints of the irradiance and depth atlases as they are.
-cudaError_t launch_footprints(const DevCascade& C, cudaStream_t st);
+// The footprints of probes [first, first + count) from the irradiance and / or depth atlas.
+constexpr uint32_t FOOT_COLOUR = 1, FOOT_DEPTH = 2;
+cudaError_t launch_footprints(const DevCascade& C, uint32_t first, uint32_t count, uint32_t which, cudaStream_t st);
 
 // Validation + derived-layout packing (sb_pack.cu).
 cudaError_t launch_pack_scene(const SceneBuffers& B, uint32_t* err, cudaStream_t st);
