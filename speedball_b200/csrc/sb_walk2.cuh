@@ -104,7 +104,7 @@ __device__ __forceinline__ void walk2(const DevScene& S, Walk2Shared& sm, Gen ge
             if (cur == PE_NONE) continue;
             sm.o[lane] = make_float4(o.x, o.y, o.z, m.z);
             sm.d[lane] = make_float4(d.x, d.y, d.z, __uint_as_float(slot));
-            sp = base = 0;
+            sp = base = iter = 0;  // (a step limit holds for each slot, as in dyn_walk)
             home = lane;
             last = head;
             state = WALK;
@@ -127,7 +127,7 @@ __device__ __forceinline__ void walk2(const DevScene& S, Walk2Shared& sm, Gen ge
                 if (want && gen(more, want, wo, wd, winv, tmax, tag)) {
                     sm.best[lane] = (unsigned long long)__float_as_uint(tmax) << 32 | 0xFFFFFFFFull;
                     if (!ANY) sm.hit[lane] = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u);
-                    k = iter = 0;
+                    k = 0;
                     own = true;
                 }
                 if (done) {
