@@ -26,7 +26,8 @@ constexpr uint32_t WALK2_DEPTH = 24;   // stacked far children; deeper BLASes: d
 struct Walk2Shared {
     float4 o[32];                 // local origin, determinant sign
     float4 d[32];                 // local direction, slot
-    unsigned long long best[32];  // as in Walk8Shared
+    unsigned long long best[32];  // bits of the ray's limit << 32 | its hit's place in the order
+    uint32_t place[32];           // of the slot the ray is in: number in dynList << 24
     uint4 hit[32];                // triangle, slot, packed (u, v), the slack of reach
     uint32_t item[WALK2_QUEUE];   // lane of its ray << 24 | triangle
     uint32_t stk[WALK2_DEPTH][32];  // far children
@@ -40,7 +41,10 @@ __device__ __forceinline__ bool walk2_usable(const DevScene& S) {
     return db != DEPTH_UNKNOWN && db <= WALK2_DEPTH;
 }
 
-// gen and fin as for walk8; the best hit starts as none within tmax.
+// gen and fin as for walk8; the best hit starts as none within tmax. Of several hits of the
+// nearest t it is the first slot's lowest triangle, the one that the reference's order meets
+// first: the lanes' items meet in no fixed order, so the place in that order is the low
+// half of what they take the minimum of.
 //
 // Closest hits pass over a box only where it starts behind the hit in hand by more than
 // the rounding of both (`reach`). A BLAS's boxes are exact: a triangle in the plane of its
@@ -64,8 +68,8 @@ __device__ __forceinline__ void walk2(const DevScene& S, Walk2Shared& sm, Gen ge
     uint32_t tag = 0, k = 0, cur = PE_NONE, sp = 0, iter = 0, last = 0, head = 0, tail = 0;
     bool more = true;
     uint32_t home = lane, base = 0;  // as in walk8
-    bool own = false, alone = S.iterCapRef < SB_WALK_STEPS_REF_DEFAULT, again = false;
-    uint32_t ties = 0;
+    bool own = false;
+    const bool share = S.iterCapRef >= SB_WALK_STEPS_REF_DEFAULT;  // as in walk8
     // the lane's ray into its next slot; false: none left
     auto next_slot = [&]() {
         for (; k < S.dynCount; ) {
@@ -104,6 +108,7 @@ __device__ __forceinline__ void walk2(const DevScene& S, Walk2Shared& sm, Gen ge
             if (cur == PE_NONE) continue;
             sm.o[lane] = make_float4(o.x, o.y, o.z, m.z);
             sm.d[lane] = make_float4(d.x, d.y, d.z, __uint_as_float(slot));
+            sm.place[lane] = (k - 1u) << 24;
             sp = base = iter = 0;  // (a step limit holds for each slot, as in dyn_walk)
             home = lane;
             last = head;
@@ -142,41 +147,28 @@ __device__ __forceinline__ void walk2(const DevScene& S, Walk2Shared& sm, Gen ge
         } else {
             // no rays are left to take: the lanes share those in hand, as in walk8. A ray goes
             // on to its next slot when no lane is in this one and the queue is empty (its
-            // local ray is the lanes' and the items'); a tie sends it through its slots again.
+            // local ray is the lanes' and the items').
             const uint32_t busy = __reduce_or_sync(ALL_LANES, state == WALK ? 1u << home : 0u);
             const bool ready = own && state != WALK && !(busy >> lane & 1u);
             flush = __any_sync(ALL_LANES, ready);
             if (!flush && !busy && tail == head) break;
             if (flush && tail == head) {
-                bool settled = false;
                 if (ready) {
                     const unsigned long long b = sm.best[lane];
                     const bool blocked = ANY && (uint32_t)b == 0u;
                     tmax = __uint_as_float((uint32_t)(b >> 32));
                     state = FREE;
-                    bool ended = blocked || !next_slot();
-                    settled = ended;
-                    if (ended && ties >> lane & 1u) {
-                        tmax = __uint_as_float((uint32_t)(b >> 32) + 1u);
-                        sm.best[lane] = (unsigned long long)__float_as_uint(tmax) << 32 | 0xFFFFFFFFull;
-                        k = 0;
-                        alone = again = true;
-                        ended = !next_slot();
-                    }
-                    if (ended) {
-                        const unsigned long long e = sm.best[lane];
-                        const uint32_t t = (uint32_t)(e >> 32) - (again && (uint32_t)e == 0xFFFFFFFFu ? 1u : 0u);
-                        fin(tag, __uint_as_float(t), ANY ? make_uint4(0u, 0u, 0u, 0u) : sm.hit[lane], blocked);
+                    if (blocked || !next_slot()) {
+                        fin(tag, tmax, ANY ? make_uint4(0u, 0u, 0u, 0u) : sm.hit[lane], blocked);
                         own = false;
                     }
                 }
-                ties &= ~__ballot_sync(ALL_LANES, settled);
                 __syncwarp();
             }
             // (a lane whose own ray waits for the queue takes nothing)
             const uint32_t walking =
                 __ballot_sync(ALL_LANES, state == WALK || (ready && tail != head));
-            const bool spare = state == WALK && sp > base && !(home == lane && alone);
+            const bool spare = share && state == WALK && sp > base;
             const uint32_t donors = __popc(~walking) >= WALK8_GIVE ? __ballot_sync(ALL_LANES, spare) : 0u;
             if (donors) {
                 const uint32_t n = min(__popc(donors), __popc(~walking)), r = __popc(donors & below);
@@ -276,38 +268,37 @@ __device__ __forceinline__ void walk2(const DevScene& S, Walk2Shared& sm, Gen ge
                 }
                 __syncwarp();
                 const uint32_t n = min(32u, tail - head);
-                bool ok = false, tie = false;
+                bool ok = false;
                 float t = 0.0f, u, v;
                 uint32_t tri = 0, of = 0, slot = 0;  // of: the lane whose ray it is
+                unsigned long long key = 0ull;       // (any hits: blocked)
                 if (lane < n) {
                     tri = sm.item[(head + lane) % WALK2_QUEUE];
                     of = tri >> 24;
                     tri &= 0x00FFFFFFu;
                     const float4 ro = sm.o[of], rd = sm.d[of];
-                    const float limit = __uint_as_float((uint32_t)(sm.best[of] >> 32));
+                    const unsigned long long best = sm.best[of];
+                    const uint32_t limit = (uint32_t)(best >> 32);
                     slot = __float_as_uint(rd.w);
                     float det;
                     uint32_t hb;
-                    const float upTo = ANY || more ? limit : __uint_as_float(__float_as_uint(limit) + 1u);
+                    const float upTo = __uint_as_float(ANY ? limit : limit + 1u);  // as near counts too
                     ok = tri_hit(S, tri, xyz(ro), xyz(rd), upTo, t, det, u, v, hb) &&
                          (hb & (ANY ? TB_SHADOW_OK : TB_CLOSEST_OK)) && side_ok(hb, det * ro.w);
-                    tie = ok;
-                    ok = ok && t < limit;
+                    if (!ANY) {
+                        key = (unsigned long long)__float_as_uint(t) << 32 | sm.place[of] | tri;
+                        ok = ok && key < best;
+                    }
                     ++vis.tri;
                 }
-                if (__any_sync(ALL_LANES, ok || tie)) {
-                    const unsigned long long key = ANY ? 0ull : (unsigned long long)__float_as_uint(t) << 32 | lane;
+                if (__any_sync(ALL_LANES, ok)) {
                     if (ok) {
-                        if (ANY) sm.best[of] = 0ull;  // blocked
+                        if (ANY) sm.best[of] = 0ull;
                         else atomicMin(&sm.best[of], key);
                     }
                     __syncwarp();
-                    if (!ANY && ok && sm.best[of] == key) sm.hit[of] = make_uint4(tri, slot, pack_uv(u, v), sm.hit[of].w);
-                    if (!ANY && !more) {
-                        const unsigned long long b = sm.best[of];
-                        tie = tie && (uint32_t)(b >> 32) == __float_as_uint(t) && !(ok && b == key) && (uint32_t)b != 0xFFFFFFFFu;
-                        ties |= __reduce_or_sync(ALL_LANES, tie ? 1u << of : 0u) & ~__ballot_sync(ALL_LANES, alone);
-                    }
+                    if (!ANY && ok && sm.best[of] == key)
+                        sm.hit[of] = make_uint4(tri, slot, pack_uv(u, v), sm.hit[of].w);
                     __syncwarp();
                     if (state != FREE) {
                         const unsigned long long b = sm.best[home];

@@ -141,3 +141,37 @@ def test_probe_rays_of_equal_t_do_not_depend_on_the_company(seed, moved):
         assert not any(bad.values()), bad
     finally:
         f.dispose()
+
+
+def test_moved_ties_name_the_first_slot_and_lowest_triangle():
+    """A ball whose triangles stand three times over, twice in one place, moved: of the six
+    equal hits a ray names the first listed slot's lowest triangle (the reference's order)."""
+    s, _ = _scene(0)
+    P, F, _ = synth.icosphere(2, 1.5)
+    F = np.random.default_rng(1).permutation(np.repeat(F, 3, 0)).astype(np.uint32)
+    s.meshes.append(Mesh(P, F, np.zeros(len(F), np.uint32)))
+    first = len(s.instances)
+    s.instances += [Instance(len(s.meshes) - 1, synth.trs((2.5, 7.5, 7.5))) for _ in range(2)]
+    s.meta["grid"] = dict(s.meta["grid"], res=(4, 6, 4), rays=128)
+    f = gu.make_field(s)
+    try:
+        f.tick()
+        f.markTransformsDirty([first, first + 1])
+        f.tick()
+        f.synchronize()
+        P, R = f._probeTotal, f.getRays()
+        _abi.check(f._lib.sb_solve(f.ctx, 0, 0, P), f.ctx)
+        f.synchronize()
+        hits = gu.read(f, "HIT_RECORDS", P * R * 4, np.uint32).reshape(-1, 4)
+        order = gu.read(f, "TLAS_ORDER", len(s.instances), np.uint32)
+        slots = [int(np.flatnonzero(order == first + k)[0]) for k in range(2)]
+        tri, slot = hits[:, 0], hits[:, 1] & 0x7FFFFFFF
+        on = np.isin(slot, slots) & (tri != 0xFFFFFFFF)
+        assert on.sum() > 100 and np.array_equal(np.unique(slot[on]), slots[:1])
+        corners = np.sort(f.pool.triIndex.reshape(-1, 3), 1)
+        _, group = np.unique(corners, axis=0, return_inverse=True)
+        lowest = np.full(group.max() + 1, len(group))
+        np.minimum.at(lowest, group, np.arange(len(group)))
+        assert np.array_equal(lowest[group[tri[on]]], tri[on])
+    finally:
+        f.dispose()
