@@ -18,6 +18,8 @@
 // other layouts warps pull 32 items per atomic. A issues rays direction-major: a
 // warp holds ray k of 32 neighbouring probes, i.e. 32 parallel rays, which keeps
 // the BVH walks of a warp together.
+#include <algorithm>
+
 #include "sb_walk2.cuh"
 #include "sb_wave.cuh"
 
@@ -955,53 +957,103 @@ __global__ void k_occluded(DevScene S, const float* ro, const float* rd, const f
                  : 0;
 }
 
-// The same on the 8-wide tree. The warps share the rays by a cursor, a word of the stream's
-// own: queries on several streams run side by side. OWN: without one (a captured query, which
-// may be replayed beside any other) each CTA takes every gridDim.x-th 32 rays and its warps
-// share those: 603 -> 644 us (closest) and 438 -> 467 us (any) for 2.07M bounce rays, 2%
-// less to 5% more for 230,400 and 9,216. MOVED: the scene has moved slots, walked as a ray is
-// taken; without that walk's code the kernel spilled less at 64 registers: 554 -> 528 us
-// (closest) and 362 -> 341 us (any) for 2.07M bounce rays.
-template <bool ANY, bool MOVED, bool OWN>
-__global__ void __launch_bounds__(256, SB_WALK8_MIN_BLOCKS) k_query_walk8(DevScene S, const float* ro, const float* rd,
-                                                                          const float* maxDist, uint32_t n,
-                                                                          float* tOut, int32_t* triOut,
-                                                                          int32_t* instOut, uint8_t* out,
-                                                                          uint32_t* cursor, uint32_t* err) {
-    extern __shared__ float4 smem[];
-    if (!*S.valid) return;
-    const uint32_t lane = threadIdx.x & 31u;
-    uint32_t end = n;  // of the cursor's positions
-    if (OWN) {
-        __shared__ uint32_t own;
-        if (threadIdx.x == 0) own = 0u;  // (walk_shared synchronizes)
-        cursor = &own;
-        end = ((n + 31u) / 32u + gridDim.x - 1u - blockIdx.x) / gridDim.x * 32u;
+// The rays of a query for the walks: the next ones of the lanes in `want` (all lanes call
+// it), by a cursor. Two cursors: 0 the tree's walk, 1 the moved slots'.
+template <bool ANY, bool OWN> struct QueryRays {
+    const float *ro, *rd, *maxDist;
+    uint32_t n, end;  // end: of the cursor's positions
+    uint32_t* cursor;
+    // (OWN: the CTA synchronizes before the first call)
+    __device__ QueryRays(const float* ro, const float* rd, const float* maxDist, uint32_t n, uint32_t* words)
+        : ro(ro), rd(rd), maxDist(maxDist), n(n), end(n), cursor(words) {
+        if (OWN) {
+            __shared__ uint32_t own[2];
+            if (threadIdx.x < 2u) own[threadIdx.x] = 0u;
+            cursor = own;
+            end = ((n + 31u) / 32u + gridDim.x - 1u - blockIdx.x) / gridDim.x * 32u;
+        }
     }
-    const WalkSmem m = walk_shared(smem, S.wideDepth + 1u, false);
-    Visits vis = {0, 0, 0, 0};
-    auto gen = [&](bool& more, uint32_t idle, float3& o, float3& d, float3& winv, float& tmax, uint32_t& tag,
-                   uint4& hit) {
-        const uint32_t p = take(cursor, end, idle, more);
+    __device__ QueryRays moved() const {  // the same rays by the other cursor
+        QueryRays r = *this;
+        ++r.cursor;
+        return r;
+    }
+    __device__ __forceinline__ bool operator()(bool& more, uint32_t want, float3& o, float3& d, float3& winv,
+                                               float& tmax, uint32_t& tag) const {
+        const uint32_t p = take(cursor, end, want, more);
         const uint32_t i = OWN ? (p / 32u * gridDim.x + blockIdx.x) * 32u + p % 32u : p;
-        const bool ok = p < end && i < n && (idle >> lane & 1u);
-        if (!ok) return false;
+        if (!(p < end && i < n && (want >> (threadIdx.x & 31u) & 1u))) return false;
         const size_t i3 = 3 * (size_t)i;
         o = mk(ro[i3], ro[i3 + 1], ro[i3 + 2]);
         d = mk(rd[i3], rd[i3 + 1], rd[i3 + 2]);
         winv = mk(1.0f / d.x, 1.0f / d.y, 1.0f / d.z);
         tmax = ANY ? maxDist[i] : T_MAX;
         tag = i;
+        return true;
+    }
+};
+
+// A warp's rays through the moved slots, by walk2 (a BLAS too deep for it: one ray per lane).
+template <bool ANY, class Rays, class Fin>
+__device__ __forceinline__ void walk2_rays(const DevScene& S, Walk2Shared& sm, Rays rays, Fin fin, Visits& vis,
+                                           uint32_t* err) {
+    if (walk2_usable(S)) {
+        walk2<ANY>(S, sm, rays, fin, vis, err);
+        return;
+    }
+    for (bool more = true; more;) {
+        float3 o, d, winv;
+        float t, u = 0.0f, v = 0.0f;
+        uint32_t i;
         int tri = -1, inst = -1;
-        float bu = 0.0f, bv = 0.0f;
-        const bool blocked = MOVED && dyn_walk<ANY>(S, o, d, winv, tmax, tri, inst, bu, bv, vis, err);
-        hit = make_uint4((uint32_t)tri, (uint32_t)inst, 0u, 0u);
-        if (ANY && blocked) out[i] = 1;
-        return !(ANY && blocked);
+        if (rays(more, ALL_LANES, o, d, winv, t, i)) {
+            const bool blocked = dyn_walk<ANY, !ANY>(S, o, d, winv, t, tri, inst, u, v, vis, err);
+            fin(i, t, make_uint4((uint32_t)tri, (uint32_t)inst, 0u, 0u), blocked);
+        }
+        __syncwarp();
+    }
+}
+
+// The same on the 8-wide tree. The warps share the rays by a cursor, a word of the stream's
+// own: queries on several streams run side by side. OWN: without one (a captured query, which
+// may be replayed beside any other) each CTA takes every gridDim.x-th 32 rays and its warps
+// share those: 603 -> 644 us (closest) and 438 -> 467 us (any) for 2.07M bounce rays, 2%
+// less to 5% more for 230,400 and 9,216. MOVED: the scene has moved slots, and what they gave
+// is in the outputs; `here`: these warps walk them first (any hits: a ray is blocked by either,
+// and `out` is 0 before).
+template <bool ANY, bool MOVED, bool OWN>
+__global__ void __launch_bounds__(256, SB_WALK8_MIN_BLOCKS) k_query_walk8(DevScene S, const float* ro, const float* rd,
+                                                                          const float* maxDist, uint32_t n,
+                                                                          float* tOut, int32_t* triOut,
+                                                                          int32_t* instOut, uint8_t* out,
+                                                                          uint32_t here, uint32_t* cursors,
+                                                                          uint32_t* err) {
+    extern __shared__ float4 smem[];
+    if (!*S.valid) return;
+    const QueryRays<ANY, OWN> rays(ro, rd, maxDist, n, cursors);
+    const WalkSmem m = walk_shared(smem, S.wideDepth + 1u, ANY && MOVED && here);  // (synchronizes)
+    Visits vis = {0, 0, 0, 0};
+    if (ANY && MOVED && here) {
+        walk2_rays<true>(S, *m.w2, rays.moved(), [&](uint32_t i, float, uint4, bool blocked) {
+            if (blocked) out[i] = 1;
+        }, vis, err);
+        __syncwarp();
+    }
+    auto gen = [&](bool& more, uint32_t idle, float3& o, float3& d, float3& winv, float& tmax, uint32_t& tag,
+                   uint4& hit) {
+        if (!rays(more, idle, o, d, winv, tmax, tag)) return false;
+        hit = make_uint4(0xFFFFFFFFu, 0xFFFFFFFFu, 0u, 0u);
+        if (MOVED && ANY) return out[tag] == 0;  // (not seen yet: walked in vain)
+        if (MOVED) {
+            tmax = tOut[tag];
+            hit.x = (uint32_t)triOut[tag];
+            hit.y = (uint32_t)instOut[tag];
+        }
+        return true;
     };
     auto fin = [&](uint32_t i, float t, uint4 hit, bool blocked) {
         if (ANY) {
-            out[i] = blocked ? 1 : 0;
+            if (!MOVED || blocked) out[i] = blocked ? 1 : 0;
         } else {
             tOut[i] = t;
             triOut[i] = (int32_t)hit.x;
@@ -1009,6 +1061,82 @@ __global__ void __launch_bounds__(256, SB_WALK8_MIN_BLOCKS) k_query_walk8(DevSce
         }
     };
     walk8<ANY>(S, *m.tables, *m.w8, m.stk, S.wideDepth + 1u, gen, fin, vis, err);
+}
+
+// The moved slots ahead of the tree, into the outputs, for queries of BY_THREAD rays or
+// more one thread per ray: rays that neighbour one another walk the slots together, and there
+// are enough of them. Fewer go by walk2, whose launch does not last as long as its longest
+// ray. (Walked by each lane of the tree's walk as it took a ray, 8 lanes or so together, as
+// they were, three slots cost 400,000 rays in the atrium 182 and 89 us (closest, any) and 29
+// of them 776 and 352; so 149 and 75, 567 and 274. 65,536 rays by thread / by walk2, closest:
+// 103 / 82 us with three slots, 254 / 160 with 29; 10^6 of a camera's 306 / 341, 426 / 677.)
+constexpr uint32_t BY_THREAD = 1u << 18;
+template <bool ANY>
+__global__ void __launch_bounds__(128) k_query_moved(DevScene S, const float* ro, const float* rd,
+                                                     const float* maxDist, uint32_t n, float* tOut, int32_t* triOut,
+                                                     int32_t* instOut, uint8_t* out, uint32_t* err) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n || !*S.valid) return;
+    const size_t i3 = 3 * (size_t)i;
+    const float3 o = mk(ro[i3], ro[i3 + 1], ro[i3 + 2]), d = mk(rd[i3], rd[i3 + 1], rd[i3 + 2]);
+    float t = ANY ? maxDist[i] : T_MAX, bu = 0.0f, bv = 0.0f;
+    int tri = -1, inst = -1;
+    Visits vis = {0, 0, 0, 0};
+    const bool blocked =
+        dyn_walk<ANY, !ANY>(S, o, d, mk(1.0f / d.x, 1.0f / d.y, 1.0f / d.z), t, tri, inst, bu, bv, vis, err);
+    if (ANY) {
+        out[i] = blocked ? 1 : 0;
+    } else {
+        tOut[i] = t;
+        triOut[i] = tri;
+        instOut[i] = inst;
+    }
+}
+template <bool OWN>  // closest hits by walk2 (any hits: k_query_walk8)
+__global__ void __launch_bounds__(256, SB_WALK8_MIN_BLOCKS) k_query_walk2(DevScene S, const float* ro, const float* rd,
+                                                                          uint32_t n, float* tOut, int32_t* triOut,
+                                                                          int32_t* instOut, uint32_t* cursors,
+                                                                          uint32_t* err) {
+    extern __shared__ float4 smem[];
+    if (!*S.valid) return;
+    const QueryRays<false, OWN> rays(ro, rd, nullptr, n, cursors);
+    __syncthreads();
+    Visits vis = {0, 0, 0, 0};
+    walk2_rays<false>(S, reinterpret_cast<Walk2Shared*>(smem)[threadIdx.x / 32u], rays.moved(),
+                      [&](uint32_t i, float t, uint4 hit, bool) {
+                          tOut[i] = t;
+                          triOut[i] = (int32_t)hit.x;
+                          instOut[i] = (int32_t)hit.y;
+                      }, vis, err);
+}
+
+// A query on the 8-wide tree.
+template <bool ANY>
+static cudaError_t launch_query(const DevScene& S, const float* ro, const float* rd, const float* maxDist, uint32_t n,
+                                float* tOut, int32_t* triOut, int32_t* instOut, uint8_t* out, uint32_t* cursors,
+                                int numSms, uint32_t* err, cudaStream_t st) {
+    const TraceTuning tune{256u, 0u, 0u, numSms, 0u};
+    const bool moved = S.dynCount != 0u, byThread = moved && n >= BY_THREAD, here = ANY && moved && !byThread;
+    cudaError_t e = cursors ? cudaMemsetAsync(cursors, 0, 4u * QUERY_WORDS, st) : cudaSuccess;
+    if (e == cudaSuccess && here) e = cudaMemsetAsync(out, 0, n, st);
+    if (e != cudaSuccess) return e;
+    if (byThread) {
+        k_query_moved<ANY><<<(n + 127) / 128, 128, 0, st>>>(S, ro, rd, maxDist, n, tOut, triOut, instOut, out, err);
+        note_launch();
+    } else if (!ANY && moved) {
+        const auto kernel = cursors ? k_query_walk2<false> : k_query_walk2<true>;
+        const size_t smem = 8u * sizeof(Walk2Shared);
+        kernel<<<walk8_grid((const void*)kernel, 256, smem, tune, n), 256, smem, st>>>(S, ro, rd, n, tOut, triOut,
+                                                                                      instOut, cursors, err);
+        note_launch();
+    }
+    const auto kernel = cursors ? moved ? k_query_walk8<ANY, true, false> : k_query_walk8<ANY, false, false>
+                                : moved ? k_query_walk8<ANY, true, true> : k_query_walk8<ANY, false, true>;
+    const size_t smem = walk_smem(S.wideDepth + 1u, here, 256u);
+    kernel<<<walk8_grid((const void*)kernel, 256, smem, tune, n), 256, smem, st>>>(
+        S, ro, rd, maxDist, n, tOut, triOut, instOut, out, here ? 1u : 0u, cursors, err);
+    note_launch();
+    return cudaGetLastError();
 }
 
 // The hits' parameters in FP64 (refine_t), one thread per ray.
@@ -1021,43 +1149,29 @@ __global__ void k_refine_hits(DevScene S, const float* ro, const float* rd, uint
                     mk(rd[i3], rd[i3 + 1], rd[i3 + 2]));
 }
 
-static const TraceTuning query_tuning(int numSms) { return TraceTuning{256u, 0u, 0u, numSms, 0u}; }
-
 cudaError_t launch_raycast(const DevScene& S, const float* ro, const float* rd, uint32_t n, float* tOut,
-                           int32_t* triOut, int32_t* instOut, uint32_t* cursor, int numSms, uint32_t* err,
+                           int32_t* triOut, int32_t* instOut, uint32_t* cursors, int numSms, uint32_t* err,
                            cudaStream_t st) {
     if (n == 0) return cudaSuccess;
     if (S.wideNodes) {
-        const size_t smem = walk_smem(S.wideDepth + 1u, false, 256u);
-        cudaError_t e = cursor ? cudaMemsetAsync(cursor, 0, 4, st) : cudaSuccess;
+        const cudaError_t e =
+            launch_query<false>(S, ro, rd, nullptr, n, tOut, triOut, instOut, nullptr, cursors, numSms, err, st);
         if (e != cudaSuccess) return e;
-        const auto kernel = cursor ? S.dynCount ? k_query_walk8<false, true, false> : k_query_walk8<false, false, false>
-                                   : S.dynCount ? k_query_walk8<false, true, true> : k_query_walk8<false, false, true>;
-        kernel<<<walk8_grid((const void*)kernel, 256, smem, query_tuning(numSms), n), 256, smem, st>>>(
-            S, ro, rd, nullptr, n, tOut, triOut, instOut, nullptr, cursor, err);
     } else {
         k_raycast<<<(n + 127) / 128, 128, 0, st>>>(S, ro, rd, n, tOut, triOut, instOut, err);
+        note_launch();
     }
-    note_launch();
     k_refine_hits<<<(n + 127) / 128, 128, 0, st>>>(S, ro, rd, n, tOut, triOut, instOut);
     note_launch();
     return cudaGetLastError();
 }
 
 cudaError_t launch_occluded(const DevScene& S, const float* ro, const float* rd, const float* maxDist, uint32_t n,
-                            uint8_t* out, uint32_t* cursor, int numSms, uint32_t* err, cudaStream_t st) {
+                            uint8_t* out, uint32_t* cursors, int numSms, uint32_t* err, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
-    if (S.wideNodes) {
-        const size_t smem = walk_smem(S.wideDepth + 1u, false, 256u);
-        cudaError_t e = cursor ? cudaMemsetAsync(cursor, 0, 4, st) : cudaSuccess;
-        if (e != cudaSuccess) return e;
-        const auto kernel = cursor ? S.dynCount ? k_query_walk8<true, true, false> : k_query_walk8<true, false, false>
-                                   : S.dynCount ? k_query_walk8<true, true, true> : k_query_walk8<true, false, true>;
-        kernel<<<walk8_grid((const void*)kernel, 256, smem, query_tuning(numSms), n), 256, smem, st>>>(
-            S, ro, rd, maxDist, n, nullptr, nullptr, nullptr, out, cursor, err);
-    } else {
-        k_occluded<<<(n + 127) / 128, 128, 0, st>>>(S, ro, rd, maxDist, n, out, err);
-    }
+    if (S.wideNodes)
+        return launch_query<true>(S, ro, rd, maxDist, n, nullptr, nullptr, nullptr, out, cursors, numSms, err, st);
+    k_occluded<<<(n + 127) / 128, 128, 0, st>>>(S, ro, rd, maxDist, n, out, err);
     note_launch();
     return cudaGetLastError();
 }

@@ -241,9 +241,24 @@ __device__ __forceinline__ bool walk(const DevScene& S, const uint4* tl, float3 
     return ANY ? false : bestTri >= 0;
 }
 
+// The limit up to which a closest hit's walk that others share or answer for too (walk2's)
+// looks into boxes: the hit in hand's t with room for the rounding of both (sb_walk2.cuh).
+__device__ __forceinline__ float reach(float t, float slack) { return fmaf(t, 1.0001f, slack); }
+__device__ __forceinline__ float shortest(float3 v) { return fminf(fminf(fabsf(v.x), fabsf(v.y)), fabsf(v.z)); }
+// Its slack, for a slot's world bounds (rounded to FP32 at the scene's scale) and in its
+// BLAS (root box lo, hi; local ray).
+__device__ __forceinline__ float slot_slack(float3 lo, float3 hi, float3 winv) {
+    const float far = fmaxf(fmaxf(fmaxf(fabsf(lo.x), fabsf(hi.x)), fmaxf(fabsf(lo.y), fabsf(hi.y))),
+                            fmaxf(fabsf(lo.z), fabsf(hi.z)));
+    return 1e-5f * far * shortest(winv);
+}
+__device__ __forceinline__ float blas_slack(float3 lo, float3 hi, float3 inv) {
+    return 1e-4f * fmaxf(fmaxf(hi.x - lo.x, hi.y - lo.y), hi.z - lo.z) * shortest(inv);
+}
+
 // One BLAS (spectral_traverse.js:354-435 / 477-536) for the nested schedule.
-// POSTPONE = while-while: walk interior nodes until a leaf, then test it.
-template <bool ANY, bool POSTPONE>
+// POSTPONE = while-while: walk interior nodes until a leaf, then test it. ROOM: `reach`.
+template <bool ANY, bool POSTPONE, bool ROOM = false>
 __device__ __forceinline__ bool blas_walk(const DevScene& S, uint32_t inst, float3 wro, float3 wrd, float& tmax,
                                           int& bestTri, int& bestInst, float& bu, float& bv, Visits& vis,
                                           uint32_t* err) {
@@ -255,6 +270,12 @@ __device__ __forceinline__ bool blas_walk(const DevScene& S, uint32_t inst, floa
     uint32_t cursor = __float_as_uint(m.x);
     const uint32_t end = __float_as_uint(m.y);
     const float dSign = m.z;
+    float slack = 0.0f;
+    if (ROOM && cursor < S.nodeCount) {
+        const uint4 a = __ldg(S.nodes + 2 * cursor), b = __ldg(S.nodes + 2 * cursor + 1);
+        slack = blas_slack(mk(__uint_as_float(a.x), __uint_as_float(a.y), __uint_as_float(a.z)),
+                           mk(__uint_as_float(a.w), __uint_as_float(b.x), __uint_as_float(b.y)), invD);
+    }
     uint32_t it = 0;
     while (cursor < end) {
         uint32_t leafOff = 0, leafCnt = 0, leafMiss = 0;
@@ -268,7 +289,7 @@ __device__ __forceinline__ bool blas_walk(const DevScene& S, uint32_t inst, floa
             ++vis.blas;
             float3 bmin = mk(__uint_as_float(a.x), __uint_as_float(a.y), __uint_as_float(a.z));
             float3 bmax = mk(__uint_as_float(a.w), __uint_as_float(b.x), __uint_as_float(b.y));
-            if (!slab(bmin, bmax, ro, invD, tmax)) {
+            if (!slab(bmin, bmax, ro, invD, ROOM ? reach(tmax, slack) : tmax)) {
                 cursor = b.z;
             } else if (b.w == INTERIOR) {
                 cursor = cursor + 1;
@@ -543,8 +564,8 @@ constexpr uint32_t FLAT_NONE = 0xFFFFFFFFu;
 #endif
 
 // A slot that left the tree: its world bounds (the reference's TLAS leaf
-// test), then its BLAS in the reference's order.
-template <bool ANY>
+// test), then its BLAS in the reference's order. ROOM: `reach`, so that the hit is walk2's.
+template <bool ANY, bool ROOM = false>
 __device__ __forceinline__ bool dyn_walk(const DevScene& S, float3 wro, float3 wrd, float3 winv, float& tmax,
                                          int& bestTri, int& bestInst, float& bu, float& bv, Visits& vis,
                                          uint32_t* err) {
@@ -552,23 +573,23 @@ __device__ __forceinline__ bool dyn_walk(const DevScene& S, float3 wro, float3 w
         const uint32_t inst = __ldg(S.dynList + k);
         if (S.slotBounds) {
             const float* b = S.slotBounds + 6u * inst;
-            if (!slab(mk(__ldg(b), __ldg(b + 1), __ldg(b + 2)), mk(__ldg(b + 3), __ldg(b + 4), __ldg(b + 5)), wro,
-                      winv, tmax))
-                continue;
+            const float3 lo = mk(__ldg(b), __ldg(b + 1), __ldg(b + 2)), hi = mk(__ldg(b + 3), __ldg(b + 4), __ldg(b + 5));
+            if (!slab(lo, hi, wro, winv, ROOM ? reach(tmax, slot_slack(lo, hi, winv)) : tmax)) continue;
         }
         ++vis.inst;
         if (__ldg(&S.inst[4 * inst + 3].w) > 0.5f &&
-            blas_walk<ANY, false>(S, inst, wro, wrd, tmax, bestTri, bestInst, bu, bv, vis, err) && ANY)
+            blas_walk<ANY, false, ROOM>(S, inst, wro, wrd, tmax, bestTri, bestInst, bu, bv, vis, err) && ANY)
             return true;
     }
     return false;
 }
 
-template <bool ANY>
+// DYN = false: without the moved slots (walked before).
+template <bool ANY, bool DYN = true>
 __device__ __forceinline__ bool flat_walk(const DevScene& S, float3 wro, float3 wrd, float& tmax, int& bestTri,
                                           int& bestInst, float& bu, float& bv, Visits& vis, uint32_t* err) {
     const float3 winv = mk(1.0f / wrd.x, 1.0f / wrd.y, 1.0f / wrd.z);
-    if (SB_DYN_FIRST && dyn_walk<ANY>(S, wro, wrd, winv, tmax, bestTri, bestInst, bu, bv, vis, err)) return true;
+    if (DYN && SB_DYN_FIRST && dyn_walk<ANY>(S, wro, wrd, winv, tmax, bestTri, bestInst, bu, bv, vis, err)) return true;
     uint2 stk[SB_STACK];
     int sp = 0;
     uint32_t cur = S.flatRoot;
@@ -656,7 +677,7 @@ __device__ __forceinline__ bool flat_walk(const DevScene& S, float3 wro, float3 
         }
     }
     // after the tree, the nearest hit so far culls the moved slots
-    if (!SB_DYN_FIRST && dyn_walk<ANY>(S, wro, wrd, winv, tmax, bestTri, bestInst, bu, bv, vis, err)) return true;
+    if (DYN && !SB_DYN_FIRST && dyn_walk<ANY>(S, wro, wrd, winv, tmax, bestTri, bestInst, bu, bv, vis, err)) return true;
     return ANY ? false : bestTri >= 0;
 }
 

@@ -63,8 +63,6 @@ __device__ __forceinline__ void walk2(const DevScene& S, Walk2Shared& sm, Gen ge
     uint32_t state = FREE;
     float3 wo = mk(0.f, 0.f, 0.f), wd = wo, winv = wo, o = wo, inv = wo;
     float tmax = 0.0f, lim = 0.0f;  // lim: reach(tmax)
-    auto reach = [](float t, float slack) { return ANY ? t : fmaf(t, 1.0001f, slack); };
-    auto shortest = [](float3 v) { return fminf(fminf(fabsf(v.x), fabsf(v.y)), fabsf(v.z)); };
     uint32_t tag = 0, k = 0, cur = PE_NONE, sp = 0, iter = 0, last = 0, head = 0, tail = 0;
     bool more = true;
     uint32_t home = lane, base = 0;  // as in walk8
@@ -78,13 +76,7 @@ __device__ __forceinline__ void walk2(const DevScene& S, Walk2Shared& sm, Gen ge
                 const float* b = S.slotBounds + 6u * slot;
                 const float3 lo = mk(__ldg(b), __ldg(b + 1), __ldg(b + 2)),
                              hi = mk(__ldg(b + 3), __ldg(b + 4), __ldg(b + 5));
-                float slack = 0.0f;
-                if (!ANY) {  // (rounded to FP32 at the scene's scale)
-                    const float far = fmaxf(fmaxf(fmaxf(fabsf(lo.x), fabsf(hi.x)), fmaxf(fabsf(lo.y), fabsf(hi.y))),
-                                            fmaxf(fabsf(lo.z), fabsf(hi.z)));
-                    slack = 1e-5f * far * shortest(winv);
-                }
-                if (!slab(lo, hi, wo, winv, reach(tmax, slack))) continue;
+                if (!slab(lo, hi, wo, winv, ANY ? tmax : reach(tmax, slot_slack(lo, hi, winv)))) continue;
             }
             ++vis.inst;
             const float4 m = __ldg(S.inst + 4 * slot + 3);
@@ -100,8 +92,8 @@ __device__ __forceinline__ void walk2(const DevScene& S, Walk2Shared& sm, Gen ge
             ++vis.blas;
             const float3 lo = mk(__uint_as_float(a.x), __uint_as_float(a.y), __uint_as_float(a.z)),
                          hi = mk(__uint_as_float(a.w), __uint_as_float(b.x), __uint_as_float(b.y));
-            const float slack = 1e-4f * fmaxf(fmaxf(hi.x - lo.x, hi.y - lo.y), hi.z - lo.z) * shortest(inv);
-            lim = reach(tmax, slack);
+            const float slack = blas_slack(lo, hi, inv);
+            lim = ANY ? tmax : reach(tmax, slack);
             if (!slab(lo, hi, o, inv, lim)) continue;
             if (!ANY) sm.hit[lane].w = __float_as_uint(slack);
             cur = b.w == INTERIOR ? PE_BLAS | root : ((b.w >> 24) ? b.w : PE_NONE);

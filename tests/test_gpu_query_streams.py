@@ -15,30 +15,34 @@ pytestmark = pytest.mark.gpu
 RAYS = 600_011
 
 
-@pytest.mark.parametrize("captured", [False, True])
-def test_queries_on_two_streams(captured):
+@pytest.mark.parametrize("captured,moved", [(False, False), (True, False), (False, True), (True, True)])
+def test_queries_on_two_streams(captured, moved):
     torch = pytest.importorskip("torch")
     f = gu.make_field(synth.room_spheres(4))
     try:
         f.tick()
+        if moved:
+            f.markTransformsDirty([3, 17, 40])
+            f.tick()
         f.synchronize()
+        n = 100_003 if moved else RAYS  # with moved slots: by walk2 too
         rng = np.random.default_rng(1)
         streams = [torch.cuda.Stream() for _ in range(2)]
         jobs = []
         for k in range(2):
-            ro = rng.uniform(0.2, 9.8, (RAYS, 3)).astype(np.float32)
-            rd = rng.normal(size=(RAYS, 3)).astype(np.float32)
+            ro = rng.uniform(0.2, 9.8, (n, 3)).astype(np.float32)
+            rd = rng.normal(size=(n, 3)).astype(np.float32)
             rd /= np.linalg.norm(rd, axis=1, keepdims=True)
-            ins = [torch.from_numpy(x).cuda() for x in (ro, rd, rng.uniform(0, 8, RAYS).astype(np.float32))]
-            outs = [torch.empty(RAYS, dtype=d, device="cuda") for d in (torch.float32, torch.int32, torch.int32, torch.uint8)]
+            ins = [torch.from_numpy(x).cuda() for x in (ro, rd, rng.uniform(0, 8, n).astype(np.float32))]
+            outs = [torch.empty(n, dtype=d, device="cuda") for d in (torch.float32, torch.int32, torch.int32, torch.uint8)]
             jobs.append((ins, outs))
         p = lambda t: C.c_void_p(t.data_ptr())  # noqa: E731
 
         def enqueue(k):
             (ro, rd, dist), (t, tri, inst, occ) = jobs[k]
             _abi.check(f._lib.sb_set_stream(f.ctx, C.c_void_p(streams[k].cuda_stream)), f.ctx)
-            _abi.check(f._lib.sb_raycast_device(f.ctx, p(ro), p(rd), RAYS, p(t), p(tri), p(inst)), f.ctx)
-            _abi.check(f._lib.sb_occluded_device(f.ctx, p(ro), p(rd), p(dist), RAYS, p(occ)), f.ctx)
+            _abi.check(f._lib.sb_raycast_device(f.ctx, p(ro), p(rd), n, p(t), p(tri), p(inst)), f.ctx)
+            _abi.check(f._lib.sb_occluded_device(f.ctx, p(ro), p(rd), p(dist), n, p(occ)), f.ctx)
 
         def results():
             torch.cuda.synchronize()

@@ -8,6 +8,8 @@ in walks that share nothing (a step limit below the default). Slots that have mo
 walked through their own BLAS ahead of the tree, the same for the rays of one probe, of
 all, and of walks that share nothing. Every launch does the same arithmetic on a ray: no
 tolerance."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -91,8 +93,8 @@ def test_hits_of_equal_t_do_not_depend_on_the_company(seed, moved):
         n = 3_000
         ro, rd = _rays(n, seed)
         rng = np.random.default_rng(9)
-        fro = rng.uniform(0.2, 9.8, (250_000, 3)).astype(np.float32)
-        frd = rng.normal(size=(250_000, 3)).astype(np.float32)
+        fro = rng.uniform(0.2, 9.8, (270_000, 3)).astype(np.float32)
+        frd = rng.normal(size=(270_000, 3)).astype(np.float32)
         frd /= np.linalg.norm(frd, axis=1, keepdims=True)
         _abi.check(f._lib.sb_set_walk_step_limit(f.ctx, NO_SHARING), f.ctx)
         want = _cast(f, ro, rd)
@@ -173,5 +175,48 @@ def test_moved_ties_name_the_first_slot_and_lowest_triangle():
         lowest = np.full(group.max() + 1, len(group))
         np.minimum.at(lowest, group, np.arange(len(group)))
         assert np.array_equal(lowest[group[tri[on]]], tri[on])
+    finally:
+        f.dispose()
+
+
+def _kind(f, kind):
+    t = _abi.sb_tuning()
+    _abi.check(f._lib.sb_get_tuning(f.ctx, C.byref(t)), f.ctx)
+    t.bvhKind = kind
+    _abi.check(f._lib.sb_set_tuning(f.ctx, C.byref(t)), f.ctx)
+
+
+@pytest.mark.parametrize("seed", [1, 2])
+def test_moved_queries_name_the_hits_of_one_thread_a_ray(seed):
+    """Every plane moved. By the warps' walk (few rays), one thread per ray (from 2^18) and
+    beside the binary tree, whose rays each walk the moved slots in the reference's order: the
+    same triangle, instance and t of two that are as near, and the same rays blocked."""
+    s, first = _scene(seed)
+    f = gu.make_field(s, record=False)
+    try:
+        f.tick()
+        f.markTransformsDirty(list(range(first, len(s.instances))))
+        f.tick()
+        f.synchronize()
+        n, large = 3_000, (1 << 18) + 5
+        ro, rd = _rays(n, seed)
+        at = np.arange(large) % n
+
+        def occluded(ro, rd):
+            out = np.zeros(len(ro), np.uint8)
+            dist = np.full(len(ro), 2.0, np.float32)
+            _abi.check(f._lib.sb_occluded(f.ctx, _abi.ptr(ro), _abi.ptr(rd), _abi.ptr(dist), len(ro), _abi.ptr(out)), f.ctx)
+            return out
+        got, occ = _cast(f, ro, rd), occluded(ro, rd)
+        assert np.array_equal(_cast(f, ro[at], rd[at]), got[at])
+        assert np.array_equal(occluded(ro[at], rd[at]), occ[at])
+        _kind(f, 2)
+        _abi.check(f._lib.sb_rebuild_scene_bvh(f.ctx), f.ctx)
+        f.tick()
+        f.markTransformsDirty(list(range(first, len(s.instances))))
+        f.tick()
+        f.synchronize()
+        assert np.array_equal(_cast(f, ro, rd), got) and np.array_equal(occluded(ro, rd), occ)
+        assert 0.1 < occ.mean() < 0.9
     finally:
         f.dispose()
