@@ -955,7 +955,8 @@ __global__ void __launch_bounds__(32 * TLAS_WARPS) k_update_refit_tlas(SceneBuff
             sCnt[i] = N[8] > 0.0f ? (uint16_t)N[8] : 0u;
             sDepth[i] = (uint16_t)I.nodeDepth[i];
         }
-        for (uint32_t i = threadIdx.x - firstStage; i < 6u * slots; i += step) sBounds[i % 6u][i / 6u] = I.liveBounds[i];
+        if (byWarp)  // (else they are all read anew below)
+            for (uint32_t i = threadIdx.x - firstStage; i < 6u * slots; i += step) sBounds[i % 6u][i / 6u] = I.liveBounds[i];
     }
     if (byWarp) {
         for (uint32_t i = warp; i < total; i += TLAS_WARPS) {
