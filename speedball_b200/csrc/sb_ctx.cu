@@ -10,6 +10,7 @@
 #include <cstring>
 #include <functional>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "sb_flat_scene.cuh"
@@ -32,28 +33,33 @@ struct Cascade {
     sb_grid grid{};
     bool configured = false;
     uint32_t probeTotal = 0, atlasW = 0, atlasH = 0;
+    // the probes' arrays lie in one block: each of these is more than the driver's 2 MB at
+    // 16^3 probes, and a block of that size takes 350 us to map (configuring a cascade of
+    // 16^3 probes in a new context 3.0 -> 1.4 ms, 2.4 before there were footprints)
+    uint8_t* block = nullptr;
     float4* irr = nullptr;
     float2* depth = nullptr;
     uint2* atlas = nullptr;
     uint2* depthAtlas = nullptr;
-    uint4 *foot = nullptr, *footDepth = nullptr, *footRough = nullptr;  // the atlases' footprints (sb_math.cuh)
+    uint4 *foot = nullptr, *footDepth = nullptr;  // the atlases' footprints (sb_math.cuh)
+    float4* probePos = nullptr;     // every probe's position
+    uint32_t* tileOrder = nullptr;  // probe index per issue position in 4 x 4 x 2 tiles (sortKey 2)
+    float* emitterVis = nullptr;    // probeTotal x 16 emitter visibility history
     float4* rayData = nullptr;
     uint4* hits = nullptr;
     uint4* vis = nullptr;
     size_t rayCap = 0, visCap = 0;
-    float4* probePos = nullptr;     // every probe's position
-    uint32_t* tileOrder = nullptr;  // probe index per issue position in 4 x 4 x 2 tiles (sortKey 2)
     // sortKey 3: cycles per 32-ray closest-hit batch of the last full solve, and the batch
     // order (costliest first) built from them; ready once a full solve has recorded costs
     uint32_t* batchCost = nullptr;
     uint32_t* batchOrder = nullptr;
     size_t batchCap = 0;
     bool batchOrderReady = false;
-    float* emitterVis = nullptr;  // probeTotal x 16 emitter visibility history
     // reflection lobes, allocated for reflTier (sb_set_reflection_quality)
     uint32_t reflTier = 0;
     float4* roughSpec = nullptr;
     uint2* roughAtlas = nullptr;
+    uint4* footRough = nullptr;  // its footprints
     float4* glossyNum = nullptr;
     float* glossyDen = nullptr;
     uint2* glossyAtlas = nullptr;
@@ -329,8 +335,8 @@ DevCascade dev_cascade(const sb_ctx* c, uint32_t ci, uint32_t probeOffset, uint3
 // and glossy atlases to vec4(0) (clearAtlasKernel / clearGlossyAtlasKernel,
 // 2703-2724). The glossy phase restarts at 0.
 sb_status alloc_reflection(sb_ctx* ctx, Cascade& K) {
-    release(K.roughSpec); release(K.roughAtlas); release(K.footRough); release(K.glossyNum); release(K.glossyDen);
-    release(K.glossyAtlas);
+    release(K.roughSpec); release(K.footRough); release(K.glossyNum); release(K.glossyDen); release(K.glossyAtlas);
+    K.roughAtlas = nullptr;
     const uint32_t tier = ctx->reflectTier, P = K.probeTotal;
     K.reflTier = tier;
     K.glossyPhase = 0;
@@ -343,12 +349,11 @@ sb_status alloc_reflection(sb_ctx* ctx, Cascade& K) {
     size_t c = 0;
     const size_t texels = (size_t)P * 64u;
     CK(grow(K.roughSpec, c, texels)); c = 0;
-    CK(grow(K.roughAtlas, c, texels)); c = 0;
-    const size_t foot = (size_t)P * FOOT * FOOT_U4;
-    CK(grow(K.footRough, c, foot)); c = 0;
-    CK(cudaMemsetAsync(K.footRough, 0, foot * sizeof(uint4), ctx->stream));
+    const size_t foot = (size_t)P * FOOT * FOOT_U4, both = foot + texels / 2u;  // the atlas behind its footprints
+    CK(grow(K.footRough, c, both)); c = 0;
+    K.roughAtlas = reinterpret_cast<uint2*>(K.footRough + foot);
+    CK(cudaMemsetAsync(K.footRough, 0, both * sizeof(uint4), ctx->stream));
     CK(cudaMemsetAsync(K.roughSpec, 0, texels * sizeof(float4), ctx->stream));
-    CK(cudaMemsetAsync(K.roughAtlas, 0, texels * sizeof(uint2), ctx->stream));
     if (tier >= SB_REFLECT_HIGH) {
         const size_t gt = (size_t)P * K.glossyTile * K.glossyTile;
         const size_t ga = (size_t)K.glossyTilesX * K.glossyTile * K.glossyTilesY * K.glossyTile;
@@ -526,13 +531,10 @@ void sb_destroy(sb_ctx* ctx) {
     release(I.detSign); release(I.order); release(I.slotOf); release(I.liveBounds); release(I.nodeDepth);
     release(I.scratch); release(ctx->instOwner); release(ctx->dStage); release(ctx->dStageM);
     for (auto& K : ctx->casc) {
-        release(K.irr); release(K.depth); release(K.atlas); release(K.depthAtlas); release(K.rayData); release(K.hits);
-        release(K.emitterVis);
-        release(K.probePos); release(K.tileOrder); release(K.batchCost); release(K.batchOrder);
-        release(K.vis);
-        release(K.roughSpec); release(K.roughAtlas); release(K.glossyNum); release(K.glossyDen);
-        release(K.foot); release(K.footDepth); release(K.footRough);
-        release(K.glossyAtlas);
+        release(K.block); release(K.rayData); release(K.hits); release(K.vis);
+        release(K.batchCost); release(K.batchOrder);
+        release(K.roughSpec); release(K.glossyNum); release(K.glossyDen);
+        release(K.footRough); release(K.glossyAtlas);
     }
     release(ctx->jobs);
     auto& G = ctx->graph;
@@ -885,19 +887,38 @@ sb_status sb_configure_cascade(sb_ctx* ctx, uint32_t ci, const sb_grid* g) {
                     K.grid.res[2] == g->res[2];
     size_t rays = (size_t)probeTotal * g->raysPerProbe;
     if (!sameDims) {
-        release(K.irr); release(K.depth); release(K.atlas); release(K.depthAtlas); release(K.tileOrder);
-        release(K.foot); release(K.footDepth);
-        release(K.emitterVis); release(K.probePos);
+        K.configured = false;  // until the arrays stand
+        release(K.block);
+        uint8_t* base = nullptr;
+        size_t at = 0;
+        auto place = [&](auto*& p, size_t perProbe) {
+            p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(base + at);
+            at += ((size_t)probeTotal * perProbe * sizeof(*p) + 255) & ~size_t(255);
+        };
+        auto layout = [&] {  // the first call sizes, the second places
+            at = 0;
+            place(K.irr, 64);
+            place(K.depth, 64);
+            place(K.atlas, 64);
+            place(K.depthAtlas, 64);
+            place(K.foot, FOOT * FOOT_U4);
+            place(K.footDepth, FOOT);
+            place(K.emitterVis, EMITTER_CAP);
+            place(K.probePos, 1);
+            place(K.tileOrder, 1);
+        };
+        layout();
         size_t c = 0;
-        CK(grow(K.probePos, c, (size_t)probeTotal)); c = 0;
-        CK(grow(K.emitterVis, c, (size_t)probeTotal * EMITTER_CAP)); c = 0;
+        const cudaError_t e = grow(K.block, c, at);
+        base = K.block;
+        if (e == cudaSuccess) {
+            layout();
+        } else {
+            K.irr = nullptr; K.depth = nullptr; K.atlas = K.depthAtlas = nullptr; K.foot = K.footDepth = nullptr;
+            K.emitterVis = nullptr; K.probePos = nullptr; K.tileOrder = nullptr;
+        }
+        CK(e);
         CK(cudaMemsetAsync(K.emitterVis, 0, (size_t)probeTotal * EMITTER_CAP * sizeof(float), ctx->stream));
-        CK(grow(K.irr, c, (size_t)probeTotal * 64)); c = 0;
-        CK(grow(K.depth, c, (size_t)probeTotal * 64)); c = 0;
-        CK(grow(K.atlas, c, (size_t)probeTotal * 64)); c = 0;
-        CK(grow(K.depthAtlas, c, (size_t)probeTotal * 64)); c = 0;
-        CK(grow(K.foot, c, (size_t)probeTotal * FOOT * FOOT_U4)); c = 0;
-        CK(grow(K.footDepth, c, (size_t)probeTotal * FOOT)); c = 0;
         // the probes in 4 x 4 x 2 tiles (row-major over tiles, x fastest inside;
         // edge tiles clipped): 32 consecutive entries form one compact block
         std::vector<uint32_t> order;
@@ -909,7 +930,6 @@ sb_status sb_configure_cascade(sb_ctx* ctx, uint32_t ci, const sb_grid* g) {
                     for (uint32_t z = tz; z < tz + 2 && z < rz; ++z)
                         for (uint32_t y = ty; y < ty + 4 && y < ry; ++y)
                             for (uint32_t x = tx; x < tx + 4 && x < rx; ++x) order.push_back((z * ry + y) * rx + x);
-        CK(grow(K.tileOrder, c, (size_t)probeTotal));
         CK(cudaMemcpy(K.tileOrder, order.data(), (size_t)probeTotal * 4, cudaMemcpyHostToDevice));
     }
     if (rays > K.rayCap || !K.rayData) {
