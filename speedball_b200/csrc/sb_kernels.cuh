@@ -113,11 +113,11 @@ cudaError_t launch_pack_scene(const SceneBuffers& B, uint32_t* err, cudaStream_t
 cudaError_t launch_pack_tris(const SceneBuffers& B, uint32_t triBegin, uint32_t triEnd, uint32_t* err, cudaStream_t st);
 cudaError_t launch_pack_dynamic(const SceneBuffers& B, uint32_t* err, cudaStream_t st);
 
-constexpr uint32_t REFIT_RANGES = 16;  // cached refit ranges; four words each (launch_refit_blas's gate)
-// Refit and TLAS lanes (sb_refit.cu). `validated`: the range's parent links
-// and layout checks from an earlier call on the same layout are still current
-// (their verdict is in *gate, the range's subtree count in gate[16]), so only
-// the bottom-up pass runs.
+constexpr uint32_t REFIT_RANGES = 16;  // cached refit ranges
+// Refit and TLAS lanes (sb_refit.cu). `gate`: the range's first of four words, REFIT_RANGES
+// apart (verdict, subtrees, planned nodes above them, subtrees done). `validated`: the range's
+// parent links and layout checks from an earlier call on the same layout are still
+// current, so only the bottom-up pass runs.
 cudaError_t launch_refit_blas(const SceneBuffers& B, uint32_t root, uint32_t end, uint32_t* err, uint32_t* gate,
                               cudaStream_t st, bool validated = false);
 
@@ -140,9 +140,9 @@ struct InstanceTable {
 constexpr uint32_t TLAS_BUILD_MAX = 4096;  // instances per single-CTA TLAS build
 
 cudaError_t launch_tlas_build(const SceneBuffers& B, const InstanceTable& I, uint32_t* err, cudaStream_t st);
+// The transform lane (instances, then the TLAS over them) as one single-CTA launch.
 // srcList/world16 are device arrays (count entries); srcList == null updates every
 // source instance from its stored matrix (rewriteRows = 0 after a BLAS refit).
-// The transform lane (instances, then the TLAS over them) as one single-CTA launch.
 cudaError_t launch_update_refit_tlas(const SceneBuffers& B, const InstanceTable& I, const uint32_t* srcList,
                                      const double* world16, uint32_t count, int rewriteRows, uint32_t* err,
                                      cudaStream_t st);
@@ -204,10 +204,10 @@ bool fine_box_from_hist(const uint32_t* hist, const double mn[3], const double s
                         double outSize[3]);
 // emitterVisKernel (sb_trace.cu): folds the emitter rays of the shadow stage into the history.
 cudaError_t launch_emitter_vis(const DevScene& S, const DevCascade& C, cudaStream_t st);
-// The FP32 probe rays of a solve as the trace forms them (sb_probe_rays).
 // The tables a solve's stages read: probe positions, ray directions.
 cudaError_t launch_probe_positions(const DevCascade& C, float4* pos, cudaStream_t st);
 cudaError_t launch_ray_dirs(uint32_t rays, float jitter, float4* dirs, cudaStream_t st);
+// The FP32 probe rays of a solve as the trace forms them (sb_probe_rays).
 cudaError_t launch_probe_rays(const DevCascade& C, float jitter, float* ro, float* rd, cudaStream_t st);
 
 // Arbitrary-ray queries through the same traversal (raycastFirst-like); `cursors`: QUERY_WORDS
