@@ -487,7 +487,7 @@ sb_status sb_create(const sb_device_opts* opts, sb_ctx** out) {
         if (cudaStreamCreateWithFlags(&ctx->ownStream, cudaStreamNonBlocking) != cudaSuccess) { st = SB_ERR_CUDA; break; }
         ctx->stream = ctx->ownStream;
         if (cudaMalloc(&ctx->dErr, 4) != cudaSuccess || cudaMalloc(&ctx->dGate, 4 * REFIT_RANGES * 4) != cudaSuccess ||
-            cudaMalloc(&ctx->dWork, (ALL_WORK + QUERY_STREAMS * QUERY_WORDS) * 4) != cudaSuccess ||
+            cudaMalloc(&ctx->dWork, (ALL_WORK + QUERY_STREAMS) * 4) != cudaSuccess ||
             cudaMalloc(&ctx->dStamps, STAGE_STAMPS * 8) != cudaSuccess ||
             cudaMalloc(&ctx->dDirs, (ADJOINT_DIRS + MAX_RAYS) * sizeof(float4)) != cudaSuccess ||
             cudaMalloc(&ctx->dCounters, 16 * 8) != cudaSuccess ||
@@ -1766,8 +1766,8 @@ sb_status sb_backward(sb_ctx* ctx, sb_grads* grads) {
     return SB_OK;
 }
 
-// Cursors for a query on the context's stream: queries of one stream follow one another,
-// so each stream has words of its own. None for captured ones, and when the words are out.
+// The cursor for a query on the context's stream: queries of one stream follow one another,
+// so each stream has a word of its own. None for captured ones, and when the words are out.
 static uint32_t* query_cursor(sb_ctx* ctx) {
     unsigned long long id = 0;
     if (in_capture(ctx) || cudaStreamGetId(ctx->stream, &id) != cudaSuccess) return nullptr;
@@ -1775,7 +1775,7 @@ static uint32_t* query_cursor(sb_ctx* ctx) {
     while (k < ctx->queryStreams && ctx->queryStream[k] != id) ++k;
     if (k == QUERY_STREAMS) return nullptr;
     if (k == ctx->queryStreams) ctx->queryStream[ctx->queryStreams++] = id;
-    return ctx->dWork + ALL_WORK + k * QUERY_WORDS;
+    return ctx->dWork + ALL_WORK + k;
 }
 
 sb_status sb_raycast(sb_ctx* ctx, const float* ro, const float* rd, uint32_t n, float* tOut, int32_t* triOut,

@@ -200,7 +200,6 @@ __device__ __forceinline__ uint32_t divide(uint32_t g, uint32_t d, uint32_t magi
 
 constexpr uint32_t MAX_RAYS = 256;  // per probe
 constexpr uint32_t WORK_WORDS = 8;  // WaveCtx::work of one solve
-constexpr uint32_t QUERY_WORDS = 2;  // of a query: cursors of the tree's and of the moved slots' walk
 
 // Several solves (scenes, cascades) through one launch of each stage: a
 // shared ray index space in which item i owns [rayBase, rayBase + rays), with

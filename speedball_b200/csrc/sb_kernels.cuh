@@ -210,12 +210,12 @@ cudaError_t launch_ray_dirs(uint32_t rays, float jitter, float4* dirs, cudaStrea
 // The FP32 probe rays of a solve as the trace forms them (sb_probe_rays).
 cudaError_t launch_probe_rays(const DevCascade& C, float jitter, float* ro, float* rd, cudaStream_t st);
 
-// Arbitrary-ray queries through the same traversal (raycastFirst-like); `cursors`: QUERY_WORDS
-// words of scratch that only this stream's queries use, or null.
+// Arbitrary-ray queries through the same traversal (raycastFirst-like); `cursor`: a word
+// of scratch that only this stream's queries use, or null.
 cudaError_t launch_raycast(const DevScene& S, const float* ro, const float* rd, uint32_t n, float* tOut,
-                           int32_t* triOut, int32_t* instOut, uint32_t* cursors, int numSms, uint32_t* err,
+                           int32_t* triOut, int32_t* instOut, uint32_t* cursor, int numSms, uint32_t* err,
                            cudaStream_t st);
 cudaError_t launch_occluded(const DevScene& S, const float* ro, const float* rd, const float* maxDist, uint32_t n,
-                            uint8_t* out, uint32_t* cursors, int numSms, uint32_t* err, cudaStream_t st);
+                            uint8_t* out, uint32_t* cursor, int numSms, uint32_t* err, cudaStream_t st);
 
 }  // namespace sb

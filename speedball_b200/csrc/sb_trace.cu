@@ -940,6 +940,7 @@ __global__ void k_raycast(DevScene S, const float* ro, const float* rd, uint32_t
     float3 o = mk(ro[3 * i], ro[3 * i + 1], ro[3 * i + 2]), d = mk(rd[3 * i], rd[3 * i + 1], rd[3 * i + 2]);
     const bool pairs = closest_pairs(S);
     trace_closest(S, pairs ? S.tlasPairs : S.tlas, o, d, t, tri, inst, bu, bv, vis, err, pairs);
+    if (tri >= 0) t = refine_t(S, (uint32_t)tri, (uint32_t)inst, o, d);
     tOut[i] = t;
     triOut[i] = tri;
     instOut[i] = inst;
@@ -958,22 +959,23 @@ __global__ void k_occluded(DevScene S, const float* ro, const float* rd, const f
 }
 
 // The rays of a query for the walks: the next ones of the lanes in `want` (all lanes call
-// it), by a cursor. Two cursors: 0 the tree's walk, 1 the moved slots'.
+// it), by a cursor: the query's, or (OWN) one of the CTA's two, 0 the tree's walk, 1 the moved
+// slots'.
 template <bool ANY, bool OWN> struct QueryRays {
     const float *ro, *rd, *maxDist;
     uint32_t n, end;  // end: of the cursor's positions
     uint32_t* cursor;
     // (OWN: the CTA synchronizes before the first call)
-    __device__ QueryRays(const float* ro, const float* rd, const float* maxDist, uint32_t n, uint32_t* words)
-        : ro(ro), rd(rd), maxDist(maxDist), n(n), end(n), cursor(words) {
+    __device__ QueryRays(const float* ro, const float* rd, const float* maxDist, uint32_t n, uint32_t* cursor)
+        : ro(ro), rd(rd), maxDist(maxDist), n(n), end(n), cursor(cursor) {
         if (OWN) {
             __shared__ uint32_t own[2];
             if (threadIdx.x < 2u) own[threadIdx.x] = 0u;
-            cursor = own;
+            this->cursor = own;
             end = ((n + 31u) / 32u + gridDim.x - 1u - blockIdx.x) / gridDim.x * 32u;
         }
     }
-    __device__ QueryRays moved() const {  // the same rays by the other cursor
+    __device__ QueryRays moved() const {  // (OWN) the same rays by the other cursor
         QueryRays r = *this;
         ++r.cursor;
         return r;
@@ -1014,11 +1016,17 @@ __device__ __forceinline__ void walk2_rays(const DevScene& S, Walk2Shared& sm, R
     }
 }
 
+// Queries of fewer rays are one launch that needs nothing ahead of it and nothing after.
+constexpr uint32_t FEW_RAYS = 1u << 18;
+
 // The same on the 8-wide tree. The warps share the rays by a cursor, a word of the stream's
-// own: queries on several streams run side by side. OWN: without one (a captured query, which
-// may be replayed beside any other) each CTA takes every gridDim.x-th 32 rays and its warps
-// share those: 603 -> 644 us (closest) and 438 -> 467 us (any) for 2.07M bounce rays, 2%
-// less to 5% more for 230,400 and 9,216. MOVED: the scene has moved slots, and what they gave
+// own: queries on several streams run side by side. OWN, without one, for few rays and for
+// captured queries (which may be replayed beside any other): each CTA takes every
+// gridDim.x-th 32 rays, its warps share those, and the hits' parameters are formed here
+// (refine_t). With a clear of the cursor ahead and a launch for the parameters behind, closest
+// hits of 1 / 100 / 10,000 / 131,072 rays take 16.6 / 27.3 / 35.1 / 53.5 us in the atrium
+// instead of 11.0 / 21.6 / 29.0 / 47.0; from 2^19 rays the cursor spreads them better (2.07M:
+// 417 against 437). MOVED: the scene has moved slots, and what they gave
 // is in the outputs; `here`: these warps walk them first (any hits: a ray is blocked by either,
 // and `out` is 0 before).
 template <bool ANY, bool MOVED, bool OWN>
@@ -1026,14 +1034,14 @@ __global__ void __launch_bounds__(256, SB_WALK8_MIN_BLOCKS) k_query_walk8(DevSce
                                                                           const float* maxDist, uint32_t n,
                                                                           float* tOut, int32_t* triOut,
                                                                           int32_t* instOut, uint8_t* out,
-                                                                          uint32_t here, uint32_t* cursors,
+                                                                          uint32_t here, uint32_t* cursor,
                                                                           uint32_t* err) {
     extern __shared__ float4 smem[];
     if (!*S.valid) return;
-    const QueryRays<ANY, OWN> rays(ro, rd, maxDist, n, cursors);
-    const WalkSmem m = walk_shared(smem, S.wideDepth + 1u, ANY && MOVED && here);  // (synchronizes)
+    const QueryRays<ANY, OWN> rays(ro, rd, maxDist, n, cursor);
+    const WalkSmem m = walk_shared(smem, S.wideDepth + 1u, ANY && MOVED && OWN && here);  // (synchronizes)
     Visits vis = {0, 0, 0, 0};
-    if (ANY && MOVED && here) {
+    if (ANY && MOVED && OWN && here) {
         walk2_rays<true>(S, *m.w2, rays.moved(), [&](uint32_t i, float, uint4, bool blocked) {
             if (blocked) out[i] = 1;
         }, vis, err);
@@ -1055,6 +1063,10 @@ __global__ void __launch_bounds__(256, SB_WALK8_MIN_BLOCKS) k_query_walk8(DevSce
         if (ANY) {
             if (!MOVED || blocked) out[i] = blocked ? 1 : 0;
         } else {
+            if (OWN && hit.x != 0xFFFFFFFFu) {
+                const size_t i3 = 3 * (size_t)i;
+                t = refine_t(S, hit.x, hit.y, mk(ro[i3], ro[i3 + 1], ro[i3 + 2]), mk(rd[i3], rd[i3 + 1], rd[i3 + 2]));
+            }
             tOut[i] = t;
             triOut[i] = (int32_t)hit.x;
             instOut[i] = (int32_t)hit.y;
@@ -1063,14 +1075,13 @@ __global__ void __launch_bounds__(256, SB_WALK8_MIN_BLOCKS) k_query_walk8(DevSce
     walk8<ANY>(S, *m.tables, *m.w8, m.stk, S.wideDepth + 1u, gen, fin, vis, err);
 }
 
-// The moved slots ahead of the tree, into the outputs, for queries of BY_THREAD rays or
+// The moved slots ahead of the tree, into the outputs, for queries of FEW_RAYS rays or
 // more one thread per ray: rays that neighbour one another walk the slots together, and there
 // are enough of them. Fewer go by walk2, whose launch does not last as long as its longest
 // ray. (Walked by each lane of the tree's walk as it took a ray, 8 lanes or so together, as
 // they were, three slots cost 400,000 rays in the atrium 182 and 89 us (closest, any) and 29
 // of them 776 and 352; so 149 and 75, 567 and 274. 65,536 rays by thread / by walk2, closest:
 // 103 / 82 us with three slots, 254 / 160 with 29; 10^6 of a camera's 306 / 341, 426 / 677.)
-constexpr uint32_t BY_THREAD = 1u << 18;
 template <bool ANY>
 __global__ void __launch_bounds__(128) k_query_moved(DevScene S, const float* ro, const float* rd,
                                                      const float* maxDist, uint32_t n, float* tOut, int32_t* triOut,
@@ -1092,14 +1103,13 @@ __global__ void __launch_bounds__(128) k_query_moved(DevScene S, const float* ro
         instOut[i] = inst;
     }
 }
-template <bool OWN>  // closest hits by walk2 (any hits: k_query_walk8)
+// Closest hits by walk2 (any hits: k_query_walk8).
 __global__ void __launch_bounds__(256, SB_WALK8_MIN_BLOCKS) k_query_walk2(DevScene S, const float* ro, const float* rd,
                                                                           uint32_t n, float* tOut, int32_t* triOut,
-                                                                          int32_t* instOut, uint32_t* cursors,
-                                                                          uint32_t* err) {
+                                                                          int32_t* instOut, uint32_t* err) {
     extern __shared__ float4 smem[];
     if (!*S.valid) return;
-    const QueryRays<false, OWN> rays(ro, rd, nullptr, n, cursors);
+    const QueryRays<false, true> rays(ro, rd, nullptr, n, nullptr);
     __syncthreads();
     Visits vis = {0, 0, 0, 0};
     walk2_rays<false>(S, reinterpret_cast<Walk2Shared*>(smem)[threadIdx.x / 32u], rays.moved(),
@@ -1108,35 +1118,6 @@ __global__ void __launch_bounds__(256, SB_WALK8_MIN_BLOCKS) k_query_walk2(DevSce
                           triOut[i] = (int32_t)hit.x;
                           instOut[i] = (int32_t)hit.y;
                       }, vis, err);
-}
-
-// A query on the 8-wide tree.
-template <bool ANY>
-static cudaError_t launch_query(const DevScene& S, const float* ro, const float* rd, const float* maxDist, uint32_t n,
-                                float* tOut, int32_t* triOut, int32_t* instOut, uint8_t* out, uint32_t* cursors,
-                                int numSms, uint32_t* err, cudaStream_t st) {
-    const TraceTuning tune{256u, 0u, 0u, numSms, 0u};
-    const bool moved = S.dynCount != 0u, byThread = moved && n >= BY_THREAD, here = ANY && moved && !byThread;
-    cudaError_t e = cursors ? cudaMemsetAsync(cursors, 0, 4u * QUERY_WORDS, st) : cudaSuccess;
-    if (e == cudaSuccess && here) e = cudaMemsetAsync(out, 0, n, st);
-    if (e != cudaSuccess) return e;
-    if (byThread) {
-        k_query_moved<ANY><<<(n + 127) / 128, 128, 0, st>>>(S, ro, rd, maxDist, n, tOut, triOut, instOut, out, err);
-        note_launch();
-    } else if (!ANY && moved) {
-        const auto kernel = cursors ? k_query_walk2<false> : k_query_walk2<true>;
-        const size_t smem = 8u * sizeof(Walk2Shared);
-        kernel<<<walk8_grid((const void*)kernel, 256, smem, tune, n), 256, smem, st>>>(S, ro, rd, n, tOut, triOut,
-                                                                                      instOut, cursors, err);
-        note_launch();
-    }
-    const auto kernel = cursors ? moved ? k_query_walk8<ANY, true, false> : k_query_walk8<ANY, false, false>
-                                : moved ? k_query_walk8<ANY, true, true> : k_query_walk8<ANY, false, true>;
-    const size_t smem = walk_smem(S.wideDepth + 1u, here, 256u);
-    kernel<<<walk8_grid((const void*)kernel, 256, smem, tune, n), 256, smem, st>>>(
-        S, ro, rd, maxDist, n, tOut, triOut, instOut, out, here ? 1u : 0u, cursors, err);
-    note_launch();
-    return cudaGetLastError();
 }
 
 // The hits' parameters in FP64 (refine_t), one thread per ray.
@@ -1149,28 +1130,55 @@ __global__ void k_refine_hits(DevScene S, const float* ro, const float* rd, uint
                     mk(rd[i3], rd[i3 + 1], rd[i3 + 2]));
 }
 
-cudaError_t launch_raycast(const DevScene& S, const float* ro, const float* rd, uint32_t n, float* tOut,
-                           int32_t* triOut, int32_t* instOut, uint32_t* cursors, int numSms, uint32_t* err,
-                           cudaStream_t st) {
-    if (n == 0) return cudaSuccess;
-    if (S.wideNodes) {
-        const cudaError_t e =
-            launch_query<false>(S, ro, rd, nullptr, n, tOut, triOut, instOut, nullptr, cursors, numSms, err, st);
-        if (e != cudaSuccess) return e;
-    } else {
-        k_raycast<<<(n + 127) / 128, 128, 0, st>>>(S, ro, rd, n, tOut, triOut, instOut, err);
+// A query on the 8-wide tree.
+template <bool ANY>
+static cudaError_t launch_query(const DevScene& S, const float* ro, const float* rd, const float* maxDist, uint32_t n,
+                                float* tOut, int32_t* triOut, int32_t* instOut, uint8_t* out, uint32_t* cursor,
+                                int numSms, uint32_t* err, cudaStream_t st) {
+    const TraceTuning tune{256u, 0u, 0u, numSms, 0u};
+    const bool moved = S.dynCount != 0u, few = n < FEW_RAYS, here = ANY && moved && few;
+    if (few) cursor = nullptr;
+    cudaError_t e = cursor ? cudaMemsetAsync(cursor, 0, 4u, st) : cudaSuccess;
+    if (e == cudaSuccess && here) e = cudaMemsetAsync(out, 0, n, st);
+    if (e != cudaSuccess) return e;
+    if (moved && !few) {
+        k_query_moved<ANY><<<(n + 127) / 128, 128, 0, st>>>(S, ro, rd, maxDist, n, tOut, triOut, instOut, out, err);
+        note_launch();
+    } else if (!ANY && moved) {
+        const size_t smem = 8u * sizeof(Walk2Shared);
+        k_query_walk2<<<walk8_grid((const void*)k_query_walk2, 256, smem, tune, n), 256, smem, st>>>(
+            S, ro, rd, n, tOut, triOut, instOut, err);
         note_launch();
     }
-    k_refine_hits<<<(n + 127) / 128, 128, 0, st>>>(S, ro, rd, n, tOut, triOut, instOut);
+    const auto kernel = cursor ? moved ? k_query_walk8<ANY, true, false> : k_query_walk8<ANY, false, false>
+                               : moved ? k_query_walk8<ANY, true, true> : k_query_walk8<ANY, false, true>;
+    const size_t smem = walk_smem(S.wideDepth + 1u, here, 256u);
+    kernel<<<walk8_grid((const void*)kernel, 256, smem, tune, n), 256, smem, st>>>(
+        S, ro, rd, maxDist, n, tOut, triOut, instOut, out, here ? 1u : 0u, cursor, err);
+    note_launch();
+    if (!ANY && cursor) {
+        k_refine_hits<<<(n + 127) / 128, 128, 0, st>>>(S, ro, rd, n, tOut, triOut, instOut);
+        note_launch();
+    }
+    return cudaGetLastError();
+}
+
+cudaError_t launch_raycast(const DevScene& S, const float* ro, const float* rd, uint32_t n, float* tOut,
+                           int32_t* triOut, int32_t* instOut, uint32_t* cursor, int numSms, uint32_t* err,
+                           cudaStream_t st) {
+    if (n == 0) return cudaSuccess;
+    if (S.wideNodes)
+        return launch_query<false>(S, ro, rd, nullptr, n, tOut, triOut, instOut, nullptr, cursor, numSms, err, st);
+    k_raycast<<<(n + 127) / 128, 128, 0, st>>>(S, ro, rd, n, tOut, triOut, instOut, err);
     note_launch();
     return cudaGetLastError();
 }
 
 cudaError_t launch_occluded(const DevScene& S, const float* ro, const float* rd, const float* maxDist, uint32_t n,
-                            uint8_t* out, uint32_t* cursors, int numSms, uint32_t* err, cudaStream_t st) {
+                            uint8_t* out, uint32_t* cursor, int numSms, uint32_t* err, cudaStream_t st) {
     if (n == 0) return cudaSuccess;
     if (S.wideNodes)
-        return launch_query<true>(S, ro, rd, maxDist, n, nullptr, nullptr, nullptr, out, cursors, numSms, err, st);
+        return launch_query<true>(S, ro, rd, maxDist, n, nullptr, nullptr, nullptr, out, cursor, numSms, err, st);
     k_occluded<<<(n + 127) / 128, 128, 0, st>>>(S, ro, rd, maxDist, n, out, err);
     note_launch();
     return cudaGetLastError();
