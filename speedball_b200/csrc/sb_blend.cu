@@ -14,21 +14,6 @@ namespace sb {
 // are half of the blend's instructions, and issue bounds it: 32 -> 29.5 us for the
 // atrium's 4,096 probes x 64 rays, 51 -> 47 for 128 rays. Packed, they take 68 registers;
 // held to 56 (four CTAs per SM) 29.5 us, at three CTAs 32.7.
-__device__ __forceinline__ unsigned long long f32x2(float lo, float hi) {
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-__device__ __forceinline__ float2 unpack2(unsigned long long v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-    unsigned long long r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
 __device__ __forceinline__ void kahan_fma2(unsigned long long& s, unsigned long long& nc, unsigned long long w,
                                            unsigned long long x) {
     const unsigned long long neg = 0xBF800000BF800000ull;  // (-1, -1)
@@ -167,17 +152,17 @@ __device__ __forceinline__ void blend_upload_block(const DevCascade& C, const De
             for (uint32_t k = 0; k < n; ++k) {
                 const float2 wv = S.w[k][lane];
                 const float4 a = S.u.f.fa[p][k], b = S.u.f.fb[p][k];
-                const unsigned long long ww = f32x2(wv.x, wv.x);
-                kahan_fma2(srg, crg, ww, f32x2(a.x, a.y));
-                kahan_fma2(sbl, cbl, ww, f32x2(a.z, a.w));
-                kahan_fma2(sld, cld, f32x2(wv.x, wv.y), f32x2(b.x, b.y));  // luma^2, distance
+                const unsigned long long ww = pack2(wv.x, wv.x);
+                kahan_fma2(srg, crg, ww, pack2(a.x, a.y));
+                kahan_fma2(sbl, cbl, ww, pack2(a.z, a.w));
+                kahan_fma2(sld, cld, pack2(wv.x, wv.y), pack2(b.x, b.y));  // luma^2, distance
                 kahan_fma(sd2, cd2, wv.y, b.z);
                 if (ROUGH) {
                     const float r = S.wr[k][lane];
                     const float rv = r * b.w;  // coverage is 0 or 1: exact
-                    const unsigned long long rr = f32x2(rv, rv);
-                    kahan_fma2(xrg, kxrg, rr, f32x2(a.x, a.y));
-                    kahan_fma2(xbh, kxbh, rr, f32x2(a.z, 1.0f));
+                    const unsigned long long rr = pack2(rv, rv);
+                    kahan_fma2(xrg, kxrg, rr, pack2(a.x, a.y));
+                    kahan_fma2(xbh, kxbh, rr, pack2(a.z, 1.0f));
                 }
             }
             if (p == 0)  // the weight sums depend on (texel, ray) only: the first probe's lanes form them
@@ -485,13 +470,13 @@ __global__ void __launch_bounds__(352) k_glossy(DevCascade C, DevParams P, uint3
     for (uint32_t k = 0; k < N; ++k) {
         const float4 d = dir[k];
         const float gw = pow64(fmaxf(td.x * d.x + td.y * d.y + td.z * d.z, 0.0f));
-        const unsigned long long ww = f32x2(gw, gw);
+        const unsigned long long ww = pack2(gw, gw);
         aw += gw;
 #pragma unroll
         for (uint32_t q = 0; q < GLOSSY_PROBES; ++q) {
             const float4 r = rad[q * N + k];
-            arg[q] = fma2(ww, f32x2(r.x, r.y), arg[q]);
-            abh[q] = fma2(ww, f32x2(r.z, r.w), abh[q]);
+            arg[q] = fma2(ww, pack2(r.x, r.y), arg[q]);
+            abh[q] = fma2(ww, pack2(r.z, r.w), abh[q]);
         }
     }
     if (!active) return;

@@ -109,26 +109,6 @@ __device__ __forceinline__ FootTap tap_of(float2 o) {
 struct Sum2 {
     unsigned long long rg, b;
 };
-__device__ __forceinline__ unsigned long long pair2(float2 v) {
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(v.x), "f"(v.y));
-    return r;
-}
-__device__ __forceinline__ float2 unpair2(unsigned long long v) {
-    float2 r;
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-    return r;
-}
-__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
-    unsigned long long r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
-    unsigned long long r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
 // Bilinear weights, each twice and by column.
 struct Weights2 {
     unsigned long long w[4], row0, row1;
@@ -136,32 +116,32 @@ struct Weights2 {
 __device__ __forceinline__ Weights2 weights2(const FootTap& t) {
     const float4 w = foot_weights(t);
     Weights2 r;
-    r.w[0] = pair2(make_float2(w.x, w.x));
-    r.w[1] = pair2(make_float2(w.y, w.y));
-    r.w[2] = pair2(make_float2(w.z, w.z));
-    r.w[3] = pair2(make_float2(w.w, w.w));
-    r.row0 = pair2(make_float2(w.x, w.y));
-    r.row1 = pair2(make_float2(w.z, w.w));
+    r.w[0] = pack2(w.x, w.x);
+    r.w[1] = pack2(w.y, w.y);
+    r.w[2] = pack2(w.z, w.z);
+    r.w[3] = pack2(w.w, w.w);
+    r.row0 = pack2(w.x, w.y);
+    r.row1 = pack2(w.z, w.w);
     return r;
 }
 __device__ __forceinline__ Sum2 foot_rgb2(const uint4* foot, uint32_t at, const Weights2& w) {
     uint32_t u[8];
     load_foot(foot + FOOT_U4 * at, u);
     Sum2 s;
-    s.rg = mul2(pair2(half2_at(u[0])), w.w[0]);
-    s.rg = fma2(pair2(half2_at(u[1])), w.w[1], s.rg);
-    s.rg = fma2(pair2(half2_at(u[2])), w.w[2], s.rg);
-    s.rg = fma2(pair2(half2_at(u[3])), w.w[3], s.rg);
-    s.b = fma2(pair2(half2_at(u[5])), w.row1, mul2(pair2(half2_at(u[4])), w.row0));
+    s.rg = mul2(pack2(half2_at(u[0])), w.w[0]);
+    s.rg = fma2(pack2(half2_at(u[1])), w.w[1], s.rg);
+    s.rg = fma2(pack2(half2_at(u[2])), w.w[2], s.rg);
+    s.rg = fma2(pack2(half2_at(u[3])), w.w[3], s.rg);
+    s.b = fma2(pack2(half2_at(u[5])), w.row1, mul2(pack2(half2_at(u[4])), w.row0));
     return s;
 }
 __device__ __forceinline__ void add_scaled(Sum2& acc, const Sum2& s, float w) {
-    const unsigned long long w2 = pair2(make_float2(w, w));
+    const unsigned long long w2 = pack2(w, w);
     acc.rg = fma2(s.rg, w2, acc.rg);
     acc.b = fma2(s.b, w2, acc.b);
 }
 __device__ __forceinline__ float3 sum_of(const Sum2& s, float scale) {
-    const float2 rg = unpair2(s.rg), b = unpair2(s.b);
+    const float2 rg = unpack2(s.rg), b = unpack2(s.b);
     return mk(rg.x * scale, rg.y * scale, (b.x + b.y) * scale);
 }
 // An rgba footprint read: (r, g) and, over the columns, b and a.
@@ -172,12 +152,12 @@ __device__ __forceinline__ Sum4 foot_rgba2(const uint4* foot, uint32_t at, const
     uint32_t u[8];
     load_foot(foot + FOOT_U4 * at, u);
     Sum4 s;
-    s.rg = mul2(pair2(half2_at(u[0])), w.w[0]);
-    s.rg = fma2(pair2(half2_at(u[1])), w.w[1], s.rg);
-    s.rg = fma2(pair2(half2_at(u[2])), w.w[2], s.rg);
-    s.rg = fma2(pair2(half2_at(u[3])), w.w[3], s.rg);
-    s.b = fma2(pair2(half2_at(u[5])), w.row1, mul2(pair2(half2_at(u[4])), w.row0));
-    s.a = fma2(pair2(half2_at(u[7])), w.row1, mul2(pair2(half2_at(u[6])), w.row0));
+    s.rg = mul2(pack2(half2_at(u[0])), w.w[0]);
+    s.rg = fma2(pack2(half2_at(u[1])), w.w[1], s.rg);
+    s.rg = fma2(pack2(half2_at(u[2])), w.w[2], s.rg);
+    s.rg = fma2(pack2(half2_at(u[3])), w.w[3], s.rg);
+    s.b = fma2(pack2(half2_at(u[5])), w.row1, mul2(pack2(half2_at(u[4])), w.row0));
+    s.a = fma2(pack2(half2_at(u[7])), w.row1, mul2(pack2(half2_at(u[6])), w.row0));
     return s;
 }
 
@@ -359,16 +339,16 @@ __device__ __forceinline__ void combined_cascade(const GatherCascade& C, const G
             const float bw[4] = {(1.0f - fx) * (1.0f - fy) * gw, fx * (1.0f - fy) * gw, (1.0f - fx) * fy * gw, fx * fy * gw};
 #pragma unroll
             for (int c = 0; c < 4; ++c) {
-                const unsigned long long w2 = pair2(make_float2(bw[c], bw[c]));
-                glossyRg = fma2(pair2(half2_at(t[c].x)), w2, glossyRg);
-                glossyBa = fma2(pair2(half2_at(t[c].y)), w2, glossyBa);
+                const unsigned long long w2 = pack2(bw[c], bw[c]);
+                glossyRg = fma2(pack2(half2_at(t[c].x)), w2, glossyRg);
+                glossyBa = fma2(pack2(half2_at(t[c].y)), w2, glossyBa);
             }
             glossyW += gw;
         }
         if (wantsRough) {
             const FootTap tB = tap_of(oSR);
             const Sum4 br = foot_rgba2(C.footRough, foot + tB.at, weights2(tB));
-            const unsigned long long w2 = pair2(make_float2(probeW, probeW));
+            const unsigned long long w2 = pack2(probeW, probeW);
             rough.rg = fma2(br.rg, w2, rough.rg);
             rough.b = fma2(br.b, w2, rough.b);
             rough.a = fma2(br.a, w2, rough.a);
@@ -376,13 +356,13 @@ __device__ __forceinline__ void combined_cascade(const GatherCascade& C, const G
         }
     }
     irr = sum_of(acc, 1.0f / fmaxf(wsum, 1e-4f));
-    const float2 rrg = unpair2(rough.rg), rb = unpair2(rough.b), ra = unpair2(rough.a);
+    const float2 rrg = unpack2(rough.rg), rb = unpack2(rough.b), ra = unpack2(rough.a);
     const float4 roughAcc = make_float4(rrg.x, rrg.y, rb.x + rb.y, ra.x + ra.y);
     const float ri = 1.0f / fmaxf(roughW, 1e-4f);
     refl = make_float4(roughAcc.x * ri, roughAcc.y * ri, roughAcc.z * ri, roughAcc.w * ri);
     if (glossyOn) {
         const float gi = 1.0f / fmaxf(glossyW, 1e-4f);
-        const float2 grg = unpair2(glossyRg), gba = unpair2(glossyBa);
+        const float2 grg = unpack2(glossyRg), gba = unpack2(glossyBa);
         const float4 glossyAcc = make_float4(grg.x, grg.y, gba.x, gba.y);
         refl = make_float4(glossyAcc.x * gi * (1.0f - lobeMix) + refl.x * lobeMix,
                            glossyAcc.y * gi * (1.0f - lobeMix) + refl.y * lobeMix,

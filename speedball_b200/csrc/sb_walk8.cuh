@@ -72,12 +72,6 @@ __device__ __forceinline__ float min3f(float a, float b, float c) {
     return d;
 }
 
-__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
-    unsigned long long r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
-    return r;
-}
-
 // Plane distances of bytes b and b + 1 of w: q * s + o for both, where
 // s2 = (s, s) and o2 = (o, o). A byte becomes the float 2^23 + q with one permute,
 // and q with one subtraction.
