@@ -1027,8 +1027,10 @@ constexpr uint32_t FEW_RAYS = 1u << 18;
 // hits of 1 / 100 / 10,000 / 131,072 rays take 16.6 / 27.3 / 35.1 / 53.5 us in the atrium
 // instead of 11.0 / 21.6 / 29.0 / 47.0; from 2^19 rays the cursor spreads them better (2.07M:
 // 417 against 437). MOVED: the scene has moved slots, and what they gave
-// is in the outputs; `here`: these warps walk them first (any hits: a ray is blocked by either,
-// and `out` is 0 before).
+// is in the outputs; `here` (OWN): these warps walk them first (any hits: a ray is blocked by
+// either, and `out` is 0 before; in a launch of their own closest hits of 1 / 100 /
+// 200,000 rays took 15.5 / 41.3 / 109.8 us in the atrium with three slots moved, so 12.5 /
+// 39.2 / 103.5).
 template <bool ANY, bool MOVED, bool OWN>
 __global__ void __launch_bounds__(256, SB_WALK8_MIN_BLOCKS) k_query_walk8(DevScene S, const float* ro, const float* rd,
                                                                           const float* maxDist, uint32_t n,
@@ -1039,13 +1041,20 @@ __global__ void __launch_bounds__(256, SB_WALK8_MIN_BLOCKS) k_query_walk8(DevSce
     extern __shared__ float4 smem[];
     if (!*S.valid) return;
     const QueryRays<ANY, OWN> rays(ro, rd, maxDist, n, cursor);
-    const WalkSmem m = walk_shared(smem, S.wideDepth + 1u, ANY && MOVED && OWN && here);  // (synchronizes)
+    const WalkSmem m = walk_shared(smem, S.wideDepth + 1u, MOVED && OWN && here);  // (synchronizes)
     Visits vis = {0, 0, 0, 0};
-    if (ANY && MOVED && OWN && here) {
-        walk2_rays<true>(S, *m.w2, rays.moved(), [&](uint32_t i, float, uint4, bool blocked) {
-            if (blocked) out[i] = 1;
+    if (MOVED && OWN && here) {
+        walk2_rays<ANY>(S, *m.w2, rays.moved(), [&](uint32_t i, float t, uint4 hit, bool blocked) {
+            if (ANY) {
+                if (blocked) out[i] = 1;
+            } else {
+                tOut[i] = t;
+                triOut[i] = (int32_t)hit.x;
+                instOut[i] = (int32_t)hit.y;
+            }
         }, vis, err);
-        __syncwarp();
+        if (ANY) __syncwarp();
+        else __syncthreads();  // the tree's walk takes the CTA's rays anew, each with its hit
     }
     auto gen = [&](bool& more, uint32_t idle, float3& o, float3& d, float3& winv, float& tmax, uint32_t& tag,
                    uint4& hit) {
@@ -1103,23 +1112,6 @@ __global__ void __launch_bounds__(128) k_query_moved(DevScene S, const float* ro
         instOut[i] = inst;
     }
 }
-// Closest hits by walk2 (any hits: k_query_walk8).
-__global__ void __launch_bounds__(256, SB_WALK8_MIN_BLOCKS) k_query_walk2(DevScene S, const float* ro, const float* rd,
-                                                                          uint32_t n, float* tOut, int32_t* triOut,
-                                                                          int32_t* instOut, uint32_t* err) {
-    extern __shared__ float4 smem[];
-    if (!*S.valid) return;
-    const QueryRays<false, true> rays(ro, rd, nullptr, n, nullptr);
-    __syncthreads();
-    Visits vis = {0, 0, 0, 0};
-    walk2_rays<false>(S, reinterpret_cast<Walk2Shared*>(smem)[threadIdx.x / 32u], rays.moved(),
-                      [&](uint32_t i, float t, uint4 hit, bool) {
-                          tOut[i] = t;
-                          triOut[i] = (int32_t)hit.x;
-                          instOut[i] = (int32_t)hit.y;
-                      }, vis, err);
-}
-
 // The hits' parameters in FP64 (refine_t), one thread per ray.
 __global__ void k_refine_hits(DevScene S, const float* ro, const float* rd, uint32_t n, float* t, const int32_t* tri,
                               const int32_t* inst) {
@@ -1136,18 +1128,13 @@ static cudaError_t launch_query(const DevScene& S, const float* ro, const float*
                                 float* tOut, int32_t* triOut, int32_t* instOut, uint8_t* out, uint32_t* cursor,
                                 int numSms, uint32_t* err, cudaStream_t st) {
     const TraceTuning tune{256u, 0u, 0u, numSms, 0u};
-    const bool moved = S.dynCount != 0u, few = n < FEW_RAYS, here = ANY && moved && few;
+    const bool moved = S.dynCount != 0u, few = n < FEW_RAYS, here = moved && few;
     if (few) cursor = nullptr;
     cudaError_t e = cursor ? cudaMemsetAsync(cursor, 0, 4u, st) : cudaSuccess;
-    if (e == cudaSuccess && here) e = cudaMemsetAsync(out, 0, n, st);
+    if (e == cudaSuccess && ANY && here) e = cudaMemsetAsync(out, 0, n, st);
     if (e != cudaSuccess) return e;
-    if (moved && !few) {
+    if (moved && !here) {
         k_query_moved<ANY><<<(n + 127) / 128, 128, 0, st>>>(S, ro, rd, maxDist, n, tOut, triOut, instOut, out, err);
-        note_launch();
-    } else if (!ANY && moved) {
-        const size_t smem = 8u * sizeof(Walk2Shared);
-        k_query_walk2<<<walk8_grid((const void*)k_query_walk2, 256, smem, tune, n), 256, smem, st>>>(
-            S, ro, rd, n, tOut, triOut, instOut, err);
         note_launch();
     }
     const auto kernel = cursor ? moved ? k_query_walk8<ANY, true, false> : k_query_walk8<ANY, false, false>

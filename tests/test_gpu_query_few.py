@@ -1,6 +1,6 @@
 """Queries of few rays: one launch on every layout of the scene (a second one, for the hits'
-parameters or to clear a cursor, doubled the time of a handful of rays), two after motion for
-closest hits; and the same hits, bit for bit, whichever way a query of its size goes."""
+parameters, for the moved slots or to clear a cursor, doubled the time of a handful of rays);
+and the same hits, bit for bit, whichever way a query of its size goes."""
 import ctypes as C
 
 import numpy as np
@@ -64,6 +64,6 @@ def test_few_rays(kind, moved):
             for g, w in zip(got, want):
                 assert np.array_equal(g, w[a:b]), (a, b)
             if b - a < FEW:
-                assert launches == (2 if moved and kind == 1 else 1, 1), (a, b, launches)
+                assert launches == (1, 1), (a, b, launches)
     finally:
         f.dispose()
